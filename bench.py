@@ -326,7 +326,7 @@ def run_bit(args):
         "counted": "near (target, source) pairs plus far (target, cluster) pairs, screened and "
                    "Coulomb, all ranks"}
     # rooflines: the dominant kernel of the FP64 step first, then the others
-    fpp = far_flops_per_pair(NTERMS)
+    fpp = far_harmonic_flops(NTERMS)
     roofs = []
     for prec, st, pk in (("fp64", st64_s, peaks["fp64"]), ("fp64", st64_c, peaks["fp64"]),
                          ("mixed", st_s, peaks["fp32"]), ("mixed", st_c, peaks["fp32"])):
@@ -366,7 +366,7 @@ def run_bit(args):
 
 
 def roofline_far(prec, kname, st, flops_pair, peak_tflops):
-    """Far field (k_far): the reference recurrence's flops per (target, cluster) pair, as the
+    """Far field (k_far): the generated evaluation's flops per (target, cluster) pair, as the
     generator counts them, times the pairs of the launch, over its device time."""
     ach = flops_pair * st["far_pairs"] / st["t_far"] / 1e12
     t = "double" if prec == "fp64" else "float"
@@ -378,8 +378,8 @@ def roofline_far(prec, kname, st, flops_pair, peak_tflops):
             "traffic": TRAFFIC.get(key), "traffic_unit": "bytes per launch (dram read+write)",
             "traffic_source": TRAFFIC_SOURCE if TRAFFIC.get(key) else None,
             "seconds": st["t_far"],
-            "algorithmic": f"{flops_pair} flops (the reference's {kname} recurrence to degree "
-                           f"{NTERMS - 1} and the moment dot product) x {st['far_pairs']} "
+            "algorithmic": f"{flops_pair} flops (the {kname} Taylor polynomial to degree "
+                           f"{NTERMS - 1} in solid harmonics) x {st['far_pairs']} "
                            "(target, cluster) pairs per launch"}
 
 
@@ -757,15 +757,24 @@ def run_serving(ctx, args, matched=False):
             "at_most_1e-6": bool(max(derr + serr) <= 1e-6)}
 
 
-def far_flops_per_pair(nterms):
-    """Flops per (target, cluster) pair of the generated far-field recurrences, counted from
-    the generator (bit_b200/csrc/gen_farfield.py)."""
+def _generator(name):
     import importlib.util
     spec = importlib.util.spec_from_file_location(
-        "gen_farfield", os.path.join(ROOT, "bit_b200", "csrc", "gen_farfield.py"))
+        name, os.path.join(ROOT, "bit_b200", "csrc", name + ".py"))
     g = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(g)
-    return g.flops_per_pair(nterms)
+    return g
+
+
+def far_flops_per_pair(nterms):
+    """Flops per (target, cluster) pair of the reference's far-field recurrences, counted from
+    the generator (bit_b200/csrc/gen_farfield.py)."""
+    return _generator("gen_farfield").flops_per_pair(nterms)
+
+
+def far_harmonic_flops(nterms):
+    """Flops per (target, cluster) pair of the far-field kernels (bit_b200/csrc/gen_harmonics.py)."""
+    return _generator("gen_harmonics").flops_per_pair(nterms)
 
 
 def accuracy(ctx, x, y, z, q, s32, c32, s64, c64, args):

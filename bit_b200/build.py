@@ -2,7 +2,7 @@
 
     python -m bit_b200.build [--force] [--verbose]
 
-Generates the unrolled far-field recurrences (csrc/gen_farfield.py), compiles every
+Generates the unrolled far-field evaluations (csrc/gen_farfield.py, gen_harmonics.py), compiles every
 csrc/*.cu for sm_100a with nvcc, and links one shared library exporting the C ABI of
 include/bit_b200.h.  Objects are rebuilt only when a source or header is newer.
 """
@@ -47,10 +47,11 @@ def headers():
 def build(force=False, verbose=False, extra=()):
     os.makedirs(GEN, exist_ok=True)
     os.makedirs(OBJ, exist_ok=True)
-    gen_out = os.path.join(GEN, "farfield_gen.cuh")
-    gen_src = os.path.join(CSRC, "gen_farfield.py")
-    if force or _newer(gen_out, [gen_src]):
-        subprocess.run([sys.executable, gen_src, gen_out], check=True)
+    for stem in ("farfield", "harmonics"):
+        gen_out = os.path.join(GEN, f"{stem}_gen.cuh")
+        gen_src = os.path.join(CSRC, f"gen_{stem}.py")
+        if force or _newer(gen_out, [gen_src]):
+            subprocess.run([sys.executable, gen_src, gen_out], check=True)
     deps = headers()
     jobs = []
     for s in sources():

@@ -103,12 +103,13 @@ struct SysEval {
   int kernel, nterms;
   int near_sign, eps_check, self_term, particles;
   int kernel_order;  // regularised Coulomb field: the reference's KERNEL_ORDER (src/problem.h:13)
-  int pad_;
+  int far_kind;      // potentials: bit 0 screened, bit 1 regularised (far_add > 0)
 };
 
 // One launch of a far / near kernel: the groups of one (nterms, kernel) class.
 struct LaunchClass {
   int nterms, kernel, eps;  // eps: near field skips r^2 <= 1e-14
+  int kind;                 // far field: SysEval::far_kind
   int begin, count;         // range in the class-ordered group array
 };
 
@@ -157,6 +158,7 @@ struct Lists {
   bool valid = false;
   int ngroups = 0;
   int ntargets = 0;                         // targets the groups cover
+  int max_targets = 0;                      // of the largest group, rounded up to 32
   long long nfar = 0, nnear = 0;            // entries
   long long far_pairs = 0, near_pairs = 0;  // interactions
   DBuf<int> g_tstart, g_tcount;             // group: first target, count
@@ -255,18 +257,14 @@ struct Tree {
   bool has_moments = false;
   bool lists_built = false;  // the last evaluation built its particle-target lists
   DBuf<double> mom64;
-  DBuf<float> mom32;
   std::vector<long long> h_mom_off;  // first moment of each node (systems may differ in nterms)
   DBuf<long long> mom_off;
-  // the same moments in the far field's shell order, each node's block padded with zeros to
-  // a multiple of 4 (16-byte aligned blocks, copied whole into shared memory by TMA)
-  DBuf<double> msh64;
-  DBuf<float> msh32;
-  DBuf<long long> msh_off;
+  // every node's far-field coefficients for the evaluation under way (far.cu)
+  DBuf<double> far_coef;
   // moment work plan: (node, first, last) member chunks and per-chunk partial sums
   long long mplan_gen = -1;
   int mplan_nch = 0;
-  long long mom_total = 0, msh_total = 0;
+  long long mom_total = 0;
   std::vector<int> mplan_cls;  // chunk range of each nterms class
   DBuf<int4> mplan_chunks;
   DBuf<int> mplan_c0, mplan_c1, mplan_T;
@@ -283,16 +281,6 @@ struct Tree {
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
-
-// FP32 moments are stored normalised: M_v / h^|v| with h = 2^e the smallest power of two
-// above the cluster radius (sqrt(sqradius)), so the scaling is exact (exponent shifts) and
-// the FP32 far field works with (h/r)^n, which stays bounded at any scale.  Both the
-// moment pass and the far kernels call this on the same FP64 sqradius.
-__device__ __forceinline__ int mom32_scale_exp(double sqradius) {
-  if (!(sqradius > 0.0) || !(sqradius < 1e300)) return 0;
-  const int e = ilogb(sqrt(sqradius)) + 1;
-  return e < -100 ? -100 : (e > 100 ? 100 : e);
-}
 
 // ---- entry points implemented in the .cu files -----------------------------------------
 void tree_build(Tree* t, const double* dx, const double* dy, const double* dz);

@@ -2,14 +2,19 @@
 // shielded_treetaylorpot, treetaylorforce; src/tree3d.cpp:4468-4640, 3004-3227, 456-810),
 // one CTA per target group.
 //
-// The CTA's warps take the group's far entries round-robin.  A warp packs the targets of
-// its entry (the set bits of the entry's mask) into a dense list while a TMA bulk copy
-// brings the cluster's moments (a padded shell-order block, no multicast) into the warp's
-// shared-memory slot, and its lanes run the unrolled recurrence (generated per nterms by
-// gen_farfield.py) for one target each, against those moments (warp-uniform loads).  Each warp accumulates into its own
-// shared-memory row; rows are summed in warp order at the end, so the result does not
-// depend on timing.  The target-centre offset is formed in FP64; the mixed path rounds it
-// once to FP32 and runs recurrence and dot product in FP32, accumulating with two-sum.
+// Potentials: the reference's Taylor polynomial regrouped in solid harmonics
+// (gen_harmonics.py), the same value to rounding.  k_far_coefs turns every node's Cartesian
+// moments into the coefficients of the evaluation's kernel and parameters.  The CTA's warps
+// then take the group's far entries, each a contiguous run.  A warp packs the targets of its
+// entry (the set bits of the entry's mask) into a dense list while a TMA bulk copy brings
+// the cluster's coefficients (a padded block, no multicast) into the warp's shared-memory
+// slot, and its lanes run the unrolled evaluation for one target each, against those
+// coefficients (warp-uniform loads).  Each warp accumulates into its own shared-memory row;
+// rows are summed in warp order at the end, so the result does not depend on timing.  The
+// target-centre offset is formed in FP64; the mixed path rounds it once to FP32 and runs
+// the evaluation in FP32, accumulating with two-sum.
+//
+// Forces: the reference's recurrences (gen_farfield.py) on the moments themselves.
 #include <algorithm>
 
 #include "common.cuh"
@@ -44,6 +49,7 @@ __device__ __forceinline__ V4<double> ld4(const double* M, int q) {
 }  // namespace bit
 
 #include "generated/farfield_gen.cuh"
+#include "generated/harmonics_gen.cuh"
 
 namespace bit {
 
@@ -57,10 +63,11 @@ struct FarArgs {
   const int* node;
   const unsigned* mask;
   const double4* nodec;
-  const void* mom;  // float or double, T(nterms of the node's system) per node
+  const double* mom;         // T(nterms of the node's system) moments per node
   const long long* mom_off;  // first moment of each node
-  const void* msh;           // the same in shell order, padded blocks (potential kernels)
-  const long long* msh_off;  // first element of each node's block
+  const void* coef;          // float or double: every node's coefficients (potential kernels)
+  int stride;                // elements from one node's coefficients to the next's
+  int rows;                  // targets of the largest group, rounded up to 32 (potentials)
   int* err;                  // device error flags (a bounded wait that gave up: 8)
   int* cost;                 // scratch, one int per far entry: its number of targets
   const SysEval* sys;        // per system: far_add, kappa, far_sign
@@ -68,23 +75,18 @@ struct FarArgs {
   double *out, *out_y, *out_z;
 };
 
-// Pack the set bits of a group mask (W words, lane l holds word l) into tl; returns count.
-__device__ __forceinline__ int warp_pack(unsigned wd, unsigned short* tl) {
+// Pack the set bits of a group mask (W words, lane l holds word l) into tl in ascending
+// order: word by word, each lane placing its own bit.
+__device__ __forceinline__ void warp_pack(unsigned wd, int W, unsigned short* tl) {
   const int lane = threadIdx.x & 31;
-  const int c = __popc(wd);
-  int pre = c;
-  for (int o = 1; o < 32; o <<= 1) {
-    int t = __shfl_up_sync(0xffffffffu, pre, o);
-    if (lane >= o) pre += t;
-  }
-  int base = pre - c;
-  while (wd) {
-    const int b = __ffs(wd) - 1;
-    wd &= wd - 1;
-    tl[base++] = (unsigned short)(32 * lane + b);
+  const unsigned lt = (1u << lane) - 1u;
+  int base = 0;
+  for (int j = 0; j < W; j++) {
+    const unsigned b = __shfl_sync(0xffffffffu, wd, j);
+    if ((b >> lane) & 1u) tl[base + __popc(b & lt)] = (unsigned short)(32 * j + lane);
+    base += __popc(b);
   }
   __syncwarp();
-  return __shfl_sync(0xffffffffu, pre, 31);
 }
 
 template <class T>
@@ -92,72 +94,173 @@ struct WarpAcc;  // per-warp accumulator rows in shared memory
 template <>
 struct WarpAcc<float> {
   static constexpr int words = 2;  // hi, lo
-  __device__ static void add(float* row, int i, float v) {
+  __device__ static void add(float* row, int rows, int i, float v) {
     float& s = row[i];
-    float& e = row[kGroupMax + i];
+    float& e = row[rows + i];
     float t = s + v, bp = t - s;
     e += (s - (t - bp)) + (v - bp);
     s = t;
   }
-  __device__ static double get(const float* row, int i) {
-    return (double)row[i] + (double)row[kGroupMax + i];
+  __device__ static double get(const float* row, int rows, int i) {
+    return (double)row[i] + (double)row[rows + i];
   }
 };
 template <>
 struct WarpAcc<double> {
   static constexpr int words = 1;
-  __device__ static void add(double* row, int i, double v) { row[i] += v; }
-  __device__ static double get(const double* row, int i) { return row[i]; }
+  __device__ static void add(double* row, int, int i, double v) { row[i] += v; }
+  __device__ static double get(const double* row, int, int i) { return row[i]; }
 };
 
-template <int NW>
-constexpr size_t far_smem(size_t acc_bytes_per_row_target, size_t moment_bytes) {
-  return 3 * kGroupMax * sizeof(double) + NW * kGroupMax * sizeof(unsigned short) +
-         NW * kGroupMax * acc_bytes_per_row_target + NW * moment_bytes;
+constexpr int NWF = 4;  // warps per CTA, force (three accumulators)
+// Warps per CTA, potentials.  Resident CTAs per SM: two at 128 registers, where every order's
+// evaluation fits without spills; three (80 registers) up to nterms 6, whose leaves and
+// entries are small in use, so that more warps cover the per-entry work.  Device time in us,
+// two / three / four CTAs: FP64 screened, 2M clustered, nterms 9: 4116 / 4471 / 4748; mixed:
+// 2585 / 2587 / 2889; 300k in leaves of 100, nterms 5, FP64: 791 / 635 / 619, mixed 663 / 514
+// / 449 (at four, nterms 6 starts to spill).  A second slot per warp (the next entry's
+// coefficients in flight during this one's evaluation) and two targets per lane were both
+// within 1% or slower.
+constexpr int NWP = 8;
+constexpr int far_blocks(int nt) { return nt <= 6 ? 3 : 2; }
+
+constexpr size_t force_smem(size_t moment_bytes) {
+  return 3 * kGroupMax * sizeof(double) + NWF * kGroupMax * sizeof(unsigned short) +
+         NWF * kGroupMax * 3 * sizeof(double) + NWF * moment_bytes;
 }
 
-// Warps per CTA of the potential kernels (NW).  FP32: 8 warps, two CTAs per SM at 128
-// registers.  FP64 (254 registers): with many groups, 4 warps, so that two CTAs share an SM
-// and one keeps the FP64 pipe busy while the other waits at its group's closing barrier;
-// with few, 8 warps, so that each group is spread over more warps (eval_far).  Measured on
-// clustered systems, p = 8 (screened, ms, 4 / 8 warps): 378 groups 1.41 / 1.07, 835 groups
-// 3.17 / 3.23, 3,091 groups (2M) 17.25 / 18.12.
-template <class T>
-constexpr int min_blocks(int nw) { return sizeof(T) == 8 && nw == 8 ? 1 : 2; }
-constexpr int NWF = 4;  // warps per CTA, force (three accumulators)
+// ---- coefficients of the potential kernels ------------------------------------------------
 
-// The far field of one target group g (the CTA's whole work for that group).  Shared
-// memory: the group's target coordinates, per warp a packed target list, an accumulator row
-// and one cluster's moments (NW * TP of them; a kernel running several orders sizes this for
-// the largest).  bar: one mbarrier per warp, phase: this warp's count of its completed
-// copies.  Returns false (in every thread) if a warp's bounded wait for its moments gave up:
-// the error flag is set, the warp has waited (bounded again) for that copy, and the group's
-// result is not valid.
-template <int NT, int KER, class T, int NW>
+// Kind of a system's far field: bit 0 screened, bit 1 regularised (delta > 0).
+constexpr int FAR_SCREENED = 1, FAR_REG = 2;
+
+__host__ __device__ constexpr int far_count(int nt, int kind) {
+  return kind & FAR_REG ? harm_count_reg(nt) : harm_count(nt);
+}
+// A node's block: its coefficients, then the scaling length H, padded to 16-byte TMA copies.
+__host__ __device__ constexpr int far_block(int nt, int kind) {
+  return (far_count(nt, kind) + 1 + 3) / 4 * 4;
+}
+
+// Exponent of H = 2^e, the smallest power of two above the cluster's radius and (regularised)
+// sqrt(delta): the scaled evaluation then works with ratios H / distance of at most about
+// one, and scaling by H is exact.  A cluster of coincident particles has moments of degree 0
+// only, and takes the lowest exponent.
+__device__ __forceinline__ int far_scale_exp(double sqradius, double delta) {
+  const double s = fmax(sqradius, delta);
+  if (!(s > 0.0)) return -100;
+  if (!(s < 1e300)) return 100;
+  const int e = ilogb(sqrt(s)) + 1;
+  return e < -100 ? -100 : (e > 100 ? 100 : e);
+}
+
+// Canonical moment index t (i outer, j, k inner, i + j + k < nt) to shell order: by degree
+// d, then i, then j descending.
+__device__ int canon_shell_pos(int t, int nt, int& d) {
+  int i = 0, j = 0;
+  for (; t >= (nt - i) * (nt - i + 1) / 2; i++) t -= (nt - i) * (nt - i + 1) / 2;
+  for (; t >= nt - i - j; j++) t -= nt - i - j;
+  d = i + j + t;
+  return d * (d + 1) * (d + 2) / 6 + (d - i) * (d - i + 1) / 2 + (d - i - j);
+}
+
+// One CTA per node: moments -> harmonic moments -> the coefficients of the node's system
+// (gen_harmonics.py), all in FP64, stored once as T.  Every value is a short fixed sum, so
+// the kernel is bound by latency; 2M clustered (4,319 nodes, nterms 9): 26 us a launch.
+constexpr int kCoefThreads = 128;
+template <class T>
+__global__ void __launch_bounds__(kCoefThreads)
+    k_far_coefs(const int* node_sys, const SysEval* sys, const double4* nodec, const double* mom,
+                const long long* mom_off, T* coef, int stride) {
+  constexpr int TMAX = num_terms(kNtermsMax);
+  constexpr int KMAX = (kNtermsMax - 1) / 2 + 1;
+  __shared__ double s_m[TMAX], s_a[TMAX];
+  __shared__ double s_e[KMAX][2 * KMAX];  // lap^k f = sum_s s_e[k][s] E_s, scaled by H^2(k-s)
+  const int node = blockIdx.x;
+  const SysEval* se = sys + node_sys[node];
+  const int nt = se->nterms, kind = se->far_kind;
+  const int nm = num_terms(nt), cnt = far_count(nt, kind);
+  // (an FP32 distance overflows past 3.4e38, where the potential is 0: keep H and the
+  // coefficients finite)
+  const double delta = kind & FAR_REG ? (sizeof(T) == 4 ? fmin(se->far_add, 3e38) : se->far_add) : 0.0;
+  const int he = far_scale_exp(nodec[node].w, delta);
+  const double* M = mom + mom_off[node];
+  for (int t = threadIdx.x; t < nm; t += kCoefThreads) {
+    int d;
+    const int p = canon_shell_pos(t, nt, d);
+    s_m[p] = ldexp(M[t], -he * d);
+  }
+  if (threadIdx.x == 0) {
+    const double kh = kind & FAR_SCREENED ? ldexp(se->kappa, he) : 0.0;
+    const double k2 = kh * kh, dd = ldexp(delta, -2 * he);
+    for (int k = 0; k < KMAX; k++)
+      for (int s = 0; s < 2 * KMAX; s++) s_e[k][s] = 0.0;
+    s_e[0][0] = 1.0;
+    for (int k = 0; k + 1 < KMAX; k++)
+      for (int s = 0; s <= 2 * k; s++) {
+        const double v = s_e[k][s];
+        s_e[k + 1][s] += k2 * v;
+        s_e[k + 1][s + 1] += 2 * s * v;
+        s_e[k + 1][s + 2] -= dd * v;
+      }
+  }
+  __syncthreads();
+  for (int h = threadIdx.x; h < nm; h += kCoefThreads) {
+    double a = 0.0;
+    for (int e = kHarmBegin[h]; e < kHarmBegin[h + 1]; e++)
+      a = fma(kHarmFactor[e], s_m[kHarmShell[e]], a);
+    s_a[h] = a;
+  }
+  __syncthreads();
+  const HarmCoef* hc = kHarmCoef + (kind & FAR_REG ? kHarmCoefBeginReg[nt] : kHarmCoefBegin[nt]);
+  T* C = coef + (long long)node * stride;
+  for (int p = threadIdx.x; p < far_block(nt, kind); p += kCoefThreads) {
+    double v = 0.0;
+    if (p < cnt) {
+      const HarmCoef q = hc[p];
+      for (int k = (q.s + 1) / 2; q.l + 2 * k < nt; k++)
+        v = fma(s_e[k][q.s], s_a[harm_index(q.l, q.m, q.part, k)], v);
+      for (int j = 3; j < 2 * (q.l + q.s); j += 2) v *= j;  // (2(l + s) - 1)!!
+    } else if (p == cnt) {
+      v = ldexp(1.0, he);
+    }
+    C[p] = (T)v;
+  }
+}
+
+// The far field of one target group g (the CTA's whole work for that group).  Bound by the
+// FP64 / FP32 pipe and issue: 244 instructions a pair (nterms 9, screened) where the
+// reference's recurrence took 1,333 (FP64) and 1,118 (FP32); 324 against 738 and 683 with
+// delta > 0.  2M clustered, theta = 0.7, 181 M pairs, before / now: FP64 screened 17.2 / 4.1
+// ms, Coulomb (delta = 0.005) 11.0 / 5.4, screened regularised 17.2 / 7.0; mixed 9.1 / 2.6,
+// 6.1 / 3.4, 9.1 / 4.2; mixed against FP64 (relative L2, screened) 1.91e-7 / 1.78e-7.
+// Shared memory: per warp an accumulator row, one cluster's coefficients and a packed target list
+// (a kernel running several orders sizes the coefficients for the largest).  bar: one
+// mbarrier per warp, phase: this warp's count of its completed copies.  Returns false (in
+// every thread) if a warp's bounded wait for its coefficients gave up: the error flag is
+// set, the warp has waited (bounded again) for that copy, and the group's result is not
+// valid.
+template <int NT, int KIND, class T, int NW>
 __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar, unsigned& phase) {
-  constexpr int TT = num_terms(NT);
-  constexpr int TP = FarField<NT>::kPadded;
+  constexpr int CNT = far_count(NT, KIND);
+  constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
-  double* cx = reinterpret_cast<double*>(sm);
-  double* cy = cx + kGroupMax;
-  double* cz = cy + kGroupMax;
-  unsigned short* tlb = reinterpret_cast<unsigned short*>(cz + kGroupMax);
-  T* accb = reinterpret_cast<T*>(tlb + NW * kGroupMax);
-  constexpr int ROW = WarpAcc<T>::words * kGroupMax;
-  T* msb = accb + NW * ROW;  // one cluster's moments per warp
+  const int rows = a.rows;
+  const int ROW = WarpAcc<T>::words * rows;
+  T* msb = reinterpret_cast<T*>(sm);  // per warp a slot of a.stride elements
+  T* accb = msb + NW * a.stride;
+  unsigned short* tlb = reinterpret_cast<unsigned short*>(accb + NW * ROW);
 
   const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
   const int W = (tc + 31) >> 5;
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int i = tid; i < tc; i += 32 * NW) {
-    cx[i] = a.tx[t0 + i]; cy[i] = a.ty[t0 + i]; cz[i] = a.tz[t0 + i];
-  }
+  const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
   for (int i = tid; i < NW * ROW; i += 32 * NW) accb[i] = T(0);
-  __syncthreads();
-  unsigned short* tl = tlb + w * kGroupMax;
+  unsigned short* tl = tlb + w * rows;
   T* row = accb + w * ROW;
-  const T* msh = reinterpret_cast<const T*>(a.msh);
+  T* M = msb + w * a.stride;
+  const T* coef = reinterpret_cast<const T*>(a.coef);
   const SysEval* se = a.sys + a.g_sys[g];
   const T tadd = (T)se->far_add, tk = (T)se->kappa;
   const double sign = se->far_sign;
@@ -193,19 +296,20 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
   }
   for (long long e = e0 + eb; e < e0 + ee; e++) {
     const int node = a.node[e];
-    T* M = msb + w * TP;
-    // The cluster's moments, its whole padded shell-order block (TP values, 16-byte aligned
-    // in global and shared memory), by one TMA bulk copy into the warp's slot while the
-    // warp packs the entry's targets.  The previous entry's reads of the slot ended at the
-    // __syncwarp closing its loop.
+    // The cluster's coefficients, its whole block (TP values, 16-byte aligned in global and
+    // shared memory), by one TMA bulk copy into the warp's slot while the warp packs the
+    // entry's targets.  The previous entry's reads of the slot ended at the __syncwarp
+    // closing its loop.
     if (lane == 0) {
       fence_proxy_async();
       mbar_expect_tx(&bar[w], TP * (unsigned)sizeof(T));
-      tma_load_1d(M, msh + a.msh_off[node], TP * (unsigned)sizeof(T), &bar[w]);
+      tma_load_1d(M, coef + (long long)node * a.stride, TP * (unsigned)sizeof(T), &bar[w]);
     }
     const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-    const int cnt = warp_pack(wd, tl);
+    const int cnt = __ldcg(a.cost + e);
     const double4 c = a.nodec[node];
+    const bool all = cnt == tc;  // a cluster accepted by the whole group needs no list
+    if (!all) warp_pack(wd, W, tl);
     const bool landed = __all_sync(0xffffffffu, mbar_wait(&bar[w], phase & 1));
     phase++;
     if (!landed) {
@@ -217,41 +321,30 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
       failed = true;
       break;
     }
-    // Both precisions run the scaled form of the reference's recurrence (fewer operations
-    // than the literal one, the same function).  FP32 moments are normalised by h^|v|,
-    // h = 2^e; FP64 moments are the plain ones, i.e. h = 1.  The FP32 kernels take the
-    // forms with per-pair products hoisted (at nterms 9, screened: 886 fma + 189 mul per
-    // pair against 886 + 447, Coulomb: 572 + 68 against 572 + 123; at 2M clustered, p = 8,
-    // theta = 0.7: screened 9.77 -> 9.09 ms, Coulomb 6.41 -> 6.07 ms); the FP64
-    // ones keep the plain forms, since the hoisted screened one spilled there and ran 1%
-    // slower.
-    const T h = sizeof(T) == 4 ? (T)ldexpf(1.f, mom32_scale_exp(c.w)) : T(1);
-    __syncwarp();
+    const T H = M[CNT];
     for (int r = lane; r < cnt; r += 32) {
-      const int i = tl[r];
+      const int i = all ? r : tl[r];
       const T dx = (T)(cx[i] - c.x), dy = (T)(cy[i] - c.y), dz = (T)(cz[i] - c.z);
-      const T r2 = dx * dx + dy * dy + dz * dz + tadd;
+      const T r2 = dx * dx + dy * dy + dz * dz;
       T v;
-      if (sizeof(T) == 4)
-        v = KER == BIT_KERNEL_COULOMB ? FarField<NT>::template coulomb_s<T>(dx, dy, dz, r2, h, M)
-                                      : FarField<NT>::template screened_s<T>(dx, dy, dz, r2, tk, h, M);
-      else
-        v = KER == BIT_KERNEL_COULOMB ? FarField<NT>::template coulomb_sp<T>(dx, dy, dz, r2, h, M)
-                                      : FarField<NT>::template screened_sp<T>(dx, dy, dz, r2, tk, h, M);
-      WarpAcc<T>::add(row, i, v);
+      if constexpr (KIND == 0) v = Harmonics<NT>::template hc<T>(dx, dy, dz, r2, tadd, tk, H, M);
+      else if constexpr (KIND == FAR_SCREENED) v = Harmonics<NT>::template hs<T>(dx, dy, dz, r2, tadd, tk, H, M);
+      else if constexpr (KIND == FAR_REG) v = Harmonics<NT>::template rc<T>(dx, dy, dz, r2, tadd, tk, H, M);
+      else v = Harmonics<NT>::template rs<T>(dx, dy, dz, r2, tadd, tk, H, M);
+      WarpAcc<T>::add(row, rows, i, v);
     }
     __syncwarp();
   }
   if (__syncthreads_or(failed)) return false;
   for (int i = tid; i < tc; i += 32 * NW) {
     double s = 0.0;
-    for (int q = 0; q < NW; q++) s += WarpAcc<T>::get(accb + q * ROW, i);
+    for (int q = 0; q < NW; q++) s += WarpAcc<T>::get(accb + q * ROW, rows, i);
     a.out[t0 + i] = sign * s;
   }
   return true;
 }
 
-// One mbarrier per warp for the moment copies, initialised before the kernel's first
+// One mbarrier per warp for the coefficient copies, initialised before the kernel's first
 // __syncthreads.
 template <int NW>
 __device__ __forceinline__ void far_bars_init(uint64_t* bar) {
@@ -262,12 +355,12 @@ __device__ __forceinline__ void far_bars_init(uint64_t* bar) {
 }
 
 // One launch class: CTA b takes group order[b].
-template <int NT, int KER, class T, int NW>
-__global__ void __launch_bounds__(32 * NW, min_blocks<T>(NW)) k_far(FarArgs a) {
+template <int NT, int KIND, class T, int NW>
+__global__ void __launch_bounds__(32 * NW, far_blocks(NT)) k_far(FarArgs a) {
   __shared__ uint64_t bar[NW];
   far_bars_init<NW>(bar);
   unsigned phase = 0;
-  far_group<NT, KER, T, NW>(a, a.order[blockIdx.x], bar, phase);
+  far_group<NT, KIND, T, NW>(a, a.order[blockIdx.x], bar, phase);
 }
 
 // Persistent work queue over the groups of every class: each CTA takes the next item
@@ -276,8 +369,7 @@ __global__ void __launch_bounds__(32 * NW, min_blocks<T>(NW)) k_far(FarArgs a) {
 // same order within the group, as k_far, so the results are identical.  No CTA waits for
 // another; the counter is the only shared state.
 template <class T, int NW>
-__global__ void __launch_bounds__(32 * NW, min_blocks<T>(NW))
-    k_far_queue(FarArgs a, int count, int* head) {
+__global__ void __launch_bounds__(32 * NW, 2) k_far_queue(FarArgs a, int count, int* head) {
   __shared__ int s_item;
   __shared__ uint64_t bar[NW];
   far_bars_init<NW>(bar);
@@ -290,16 +382,14 @@ __global__ void __launch_bounds__(32 * NW, min_blocks<T>(NW))
     if (item >= count) return;
     const int g = a.order[item];
     const SysEval* se = a.sys + a.g_sys[g];
-    const bool coul = se->kernel == BIT_KERNEL_COULOMB;
     bool ok = true;
-    switch (se->nterms) {
-#define FQ(N)                                                                   \
-  case N:                                                                       \
-    ok = coul ? far_group<N, BIT_KERNEL_COULOMB, T, NW>(a, g, bar, phase)       \
-              : far_group<N, BIT_KERNEL_SCREENED, T, NW>(a, g, bar, phase);     \
-    break;
+    switch (se->nterms * 4 + se->far_kind) {
+#define FK(N, K) \
+  case 4 * N + K: ok = far_group<N, K, T, NW>(a, g, bar, phase); break;
+#define FQ(N) FK(N, 0) FK(N, 1) FK(N, 2) FK(N, 3)
       FQ(1) FQ(2) FQ(3) FQ(4) FQ(5) FQ(6) FQ(7) FQ(8) FQ(9) FQ(10)
 #undef FQ
+#undef FK
       default:
         break;
     }
@@ -338,29 +428,18 @@ __global__ void __launch_bounds__(32 * NWF) k_far_force(FarArgs a) {
   __syncthreads();
   unsigned short* tl = tlb + w * kGroupMax;
   double* row = accb + w * 3 * kGroupMax;
-  const T* mom = reinterpret_cast<const T*>(a.mom);
   const SysEval* se = a.sys + a.g_sys[g];
   const T tadd = (T)se->far_add, tk = (T)se->kappa, tdel = (T)se->near_del;
   const int korder = se->kernel_order;
   for (long long e = e0 + w; e < e1; e += NW) {
     const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-    const int cnt = warp_pack(wd, tl);
+    const int cnt = __reduce_add_sync(0xffffffffu, __popc(wd));
+    warp_pack(wd, W, tl);
     const int node = a.node[e];
     const double4 c = a.nodec[node];
     T* M = msb + w * TP;
-    const T* mn = mom + a.mom_off[node];
-    // FP32 moments are stored normalised by h^|v| (h = 2^e): undo it exactly here, since
-    // the force recurrence takes the moments themselves
-    const int se = sizeof(T) == 4 ? mom32_scale_exp(c.w) : 0;
-    for (int k = lane; k < TP; k += 32) {
-      T m = k < TT ? mn[FarField<NT>::canon(k)] : T(0);
-      if constexpr (sizeof(T) == 4) {
-        int d = 0;  // degree of shell-order index k
-        while (num_terms(d + 1) <= k) d++;
-        m = ldexpf(m, se * d);
-      }
-      M[k] = m;
-    }
+    const double* mn = a.mom + a.mom_off[node];
+    for (int k = lane; k < TP; k += 32) M[k] = k < TT ? (T)mn[FarField<NT>::canon(k)] : T(0);
     __syncwarp();
     for (int r = lane; r < cnt; r += 32) {
       const int i = tl[r];
@@ -396,17 +475,22 @@ void set_smem(K kernel, size_t bytes) {
   ensure_smem_attr(reinterpret_cast<const void*>(kernel), (int)bytes);
 }
 
-template <int NT, int KER, class T, int NW>
+template <class T, int NW>
+size_t far_smem(const FarArgs& a) {
+  return NW * ((size_t)a.stride * sizeof(T) + (size_t)a.rows * (WarpAcc<T>::words * sizeof(T) + sizeof(unsigned short)));
+}
+constexpr size_t kFarSmemMax =
+    NWP * ((far_block(kNtermsMax, FAR_REG) + kGroupMax) * sizeof(double) + kGroupMax * sizeof(unsigned short));
+
+template <int NT, int KIND, class T, int NW>
 void launch_far(const FarArgs& a, int ng, cudaStream_t s) {
-  const size_t bytes =
-      far_smem<NW>(WarpAcc<T>::words * sizeof(T), FarField<NT>::kPadded * sizeof(T));
-  set_smem(k_far<NT, KER, T, NW>, bytes);
-  count_launch(), k_far<NT, KER, T, NW><<<ng, 32 * NW, bytes, s>>>(a);
+  set_smem(k_far<NT, KIND, T, NW>, kFarSmemMax);
+  count_launch(), k_far<NT, KIND, T, NW><<<ng, 32 * NW, far_smem<T, NW>(a), s>>>(a);
 }
 
 template <int NT, int FK, class T>
 void launch_force(const FarArgs& a, int ng, cudaStream_t s) {
-  const size_t bytes = far_smem<NWF>(3 * sizeof(double), FarField<NT>::kPadded * sizeof(T));
+  const size_t bytes = force_smem(FarField<NT>::kPadded * sizeof(T));
   set_smem(k_far_force<NT, FK, T>, bytes);
   count_launch(), k_far_force<NT, FK, T><<<ng, 32 * NWF, bytes, s>>>(a);
 }
@@ -423,10 +507,8 @@ FarArgs far_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const d
   a.node = L->far_node.p;
   a.mask = L->far_mask.p;
   a.nodec = t->nodec.p;
-  a.mom = P.f32 ? (const void*)t->mom32.p : (const void*)t->mom64.p;
+  a.mom = t->mom64.p;
   a.mom_off = t->mom_off.p;
-  a.msh = P.f32 ? (const void*)t->msh32.p : (const void*)t->msh64.p;
-  a.msh_off = t->msh_off.p;
   a.err = t->ctx->dev_err();
   L->far_cost.ensure(t->ctx, std::max(L->nfar, 1LL));
   a.cost = L->far_cost.p;
@@ -437,23 +519,30 @@ FarArgs far_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const d
 
 }  // namespace
 
-// One launch per (nterms, kernel) class, each over its groups (P.far_ord + begin).
 template <class T, int NW>
-void launch_far_queue(Ctx* c, const FarArgs& a, int count, int max_nterms, int* head,
-                      cudaStream_t s) {
-  int tp = 0;
-  switch (max_nterms) {
-#define TPN(N) case N: tp = FarField<N>::kPadded; break;
-    TPN(1) TPN(2) TPN(3) TPN(4) TPN(5) TPN(6) TPN(7) TPN(8) TPN(9) TPN(10)
-#undef TPN
-    default: fail(BIT_ERR_STATE, "moments not computed");
-  }
-  const size_t bytes = far_smem<NW>(WarpAcc<T>::words * sizeof(T), tp * sizeof(T));
-  set_smem(k_far_queue<T, NW>, bytes);
+void launch_far_queue(Ctx* c, const FarArgs& a, int count, int* head, cudaStream_t s) {
+  const size_t bytes = far_smem<T, NW>(a);
+  set_smem(k_far_queue<T, NW>, kFarSmemMax);
   int per_sm = 0;
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_far_queue<T, NW>, 32 * NW, bytes));
   const int grid = std::max(1, std::min(count, c->num_sms * std::max(per_sm, 1)));
   count_launch(), k_far_queue<T, NW><<<grid, 32 * NW, bytes, s>>>(a, count, head);
+}
+
+// Every node's coefficients for this plan's systems, at one stride (the largest system's
+// block).  The buffer is sized in doubles whatever the precision, so that a tree evaluated
+// in both (iterative refinement, whose matvecs are replayed as CUDA graphs on fixed
+// buffers) keeps one buffer.
+template <class T>
+void far_coefs(Tree* t, const EvalPlan& P, FarArgs& a, cudaStream_t s) {
+  a.stride = 0;
+  for (const SysEval& se : P.h_sys) a.stride = std::max(a.stride, far_block(se.nterms, se.far_kind));
+  t->far_coef.ensure(t->ctx, (size_t)a.stride * t->numtree);
+  a.coef = t->far_coef.p;
+  count_launch(), k_far_coefs<T><<<t->numtree, kCoefThreads, 0, s>>>(
+      t->node_sys.p, P.sys.p, t->nodec.p, t->mom64.p, t->mom_off.p, reinterpret_cast<T*>(t->far_coef.p),
+      a.stride);
+  BIT_CHECK_LAUNCH();
 }
 
 // The work-queue form is used for plans of several classes when the context allows it;
@@ -468,48 +557,40 @@ int* queue_head(Ctx* c, int which, cudaStream_t s) {
   return c->queue_heads.p + which;
 }
 
+// One launch per (nterms, kind) class, each over its groups (P.far_ord + begin), or one
+// work queue over them all.
 void eval_far(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
               const double* tz, double* out) {
   FarArgs a = far_args(t, L, P, tx, ty, tz);
   a.out = out;
+  a.rows = L->max_targets;
   cudaStream_t s = t->ctx->stream;
   const bool f32 = P.f32;
-  // FP64: 4-warp CTAs when the evaluation has at least 4 groups per SM.  The choice
-  // follows the whole list (not a launch class), so the queue and the class launches of
-  // one evaluation sum in the same order.
-  const bool narrow = !f32 && L->ngroups >= 4 * t->ctx->num_sms;
+  if (f32) far_coefs<float>(t, P, a, s);
+  else far_coefs<double>(t, P, a, s);
   if (use_queue(t->ctx, P.far_classes)) {
-    int nt_max = 0, count = 0;
-    for (const LaunchClass& k : P.far_classes) nt_max = std::max(nt_max, k.nterms);
+    int count = 0;
     for (const LaunchClass& k : P.far_classes) count += k.count;
     a.order = L->order.p;
     int* head = queue_head(t->ctx, 0, s);
-    if (f32) launch_far_queue<float, 8>(t->ctx, a, count, nt_max, head, s);
-    else if (narrow) launch_far_queue<double, 4>(t->ctx, a, count, nt_max, head, s);
-    else launch_far_queue<double, 8>(t->ctx, a, count, nt_max, head, s);
+    if (f32) launch_far_queue<float, NWP>(t->ctx, a, count, head, s);
+    else launch_far_queue<double, NWP>(t->ctx, a, count, head, s);
     BIT_CHECK_LAUNCH();
     return;
   }
   for (const LaunchClass& k : P.far_classes) {
     a.order = P.far_ord + k.begin;
     const int ng = k.count;
-    const bool coul = k.kernel == BIT_KERNEL_COULOMB;
-    switch (k.nterms) {
-#define CASE(N)                                                                   \
-  case N:                                                                         \
-    if (f32) {                                                                    \
-      if (coul) launch_far<N, BIT_KERNEL_COULOMB, float, 8>(a, ng, s);            \
-      else launch_far<N, BIT_KERNEL_SCREENED, float, 8>(a, ng, s);                \
-    } else if (narrow) {                                                          \
-      if (coul) launch_far<N, BIT_KERNEL_COULOMB, double, 4>(a, ng, s);           \
-      else launch_far<N, BIT_KERNEL_SCREENED, double, 4>(a, ng, s);               \
-    } else {                                                                      \
-      if (coul) launch_far<N, BIT_KERNEL_COULOMB, double, 8>(a, ng, s);           \
-      else launch_far<N, BIT_KERNEL_SCREENED, double, 8>(a, ng, s);               \
-    }                                                                             \
+    switch (k.nterms * 4 + k.kind) {
+#define FK(N, K)                                             \
+  case 4 * N + K:                                            \
+    if (f32) launch_far<N, K, float, NWP>(a, ng, s);         \
+    else launch_far<N, K, double, NWP>(a, ng, s);            \
     break;
+#define CASE(N) FK(N, 0) FK(N, 1) FK(N, 2) FK(N, 3)
       CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)
 #undef CASE
+#undef FK
       default:
         fail(BIT_ERR_STATE, "moments not computed");
     }

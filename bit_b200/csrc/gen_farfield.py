@@ -726,31 +726,6 @@ def main(out):
         parts.append(f"  static constexpr int kPadded = {len(table)};")
         parts.append("  // canonical (i outer, j, k inner) index of the k-th moment in shell order")
         parts.append(f"  static __device__ __forceinline__ int canon(int k) {{ return kShellCanon{nt}[k]; }}")
-        parts.append("  template <class T> static __device__ __forceinline__ T coulomb("
-                     "T dx, T dy, T dz, T rs, const T* __restrict__ M) {")
-        parts += gen_coulomb(nt)
-        parts.append("  }")
-        parts.append("  template <class T> static __device__ __forceinline__ T screened("
-                     "T dx, T dy, T dz, T dist2, T kappa, const T* __restrict__ M) {")
-        parts += gen_screened(nt)
-        parts.append("  }")
-        parts.append("  // scaled forms for normalised moments (M_v / h^|v|), used by the FP32 path")
-        parts.append("  template <class T> static __device__ __forceinline__ T coulomb_s("
-                     "T dx, T dy, T dz, T rs, T h, const T* __restrict__ M) {")
-        parts += gen_coulomb_scaled(nt)
-        parts.append("  }")
-        parts.append("  template <class T> static __device__ __forceinline__ T coulomb_sp("
-                     "T dx, T dy, T dz, T rs, T h, const T* __restrict__ M) {")
-        parts += gen_coulomb_scaled(nt, hoisted=False)
-        parts.append("  }")
-        parts.append("  template <class T> static __device__ __forceinline__ T screened_s("
-                     "T dx, T dy, T dz, T dist2, T kappa, T h, const T* __restrict__ M) {")
-        parts += gen_screened_scaled(nt)
-        parts.append("  }")
-        parts.append("  template <class T> static __device__ __forceinline__ T screened_sp("
-                     "T dx, T dy, T dz, T dist2, T kappa, T h, const T* __restrict__ M) {")
-        parts += gen_screened_scaled_plain(nt)
-        parts.append("  }")
         parts.append("  template <class T> static __device__ __forceinline__ void force("
                      "T dx, T dy, T dz, T rs, const T* __restrict__ M, T& fx, T& fy, T& fz) {")
         parts += gen_force(nt)

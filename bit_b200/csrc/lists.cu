@@ -461,6 +461,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   // nodes (far) and leaves (near), each with at most 32 mask words.
   int maxw = 1;
   for (int g = 0; g < ng; g++) maxw = std::max(maxw, (tc[g] + 31) / 32);
+  L->max_targets = 32 * maxw;
   int per_sm = 0;
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists_queue, LT, STACK_BYTES));
   const int slots = std::max(1, std::min(ng, c->num_sms * std::max(per_sm, 1)));

@@ -80,6 +80,7 @@ SysEval make_sys_eval(const bit_eval_params& p, int nterms, int points, int forc
       s.near_sign = 1;
       break;
   }
+  s.far_kind = (p.kernel != BIT_KERNEL_COULOMB ? 1 : 0) + (s.far_add > 0.0 ? 2 : 0);
   return s;
 }
 
@@ -130,7 +131,7 @@ ListKey plan_key(const Tree* t, const EvalPlan& P, int points) {
 }
 
 namespace {
-long long far_class_of(const SysEval& s) { return s.nterms * 2 + (s.kernel == BIT_KERNEL_COULOMB ? 0 : 1); }
+long long far_class_of(const SysEval& s) { return s.nterms * 4 + s.far_kind; }
 long long near_class_of(const SysEval& s) { return (s.kernel == BIT_KERNEL_COULOMB ? 0 : 2) + s.eps_check; }
 
 // Groups ordered by class, then by decreasing work; one LaunchClass per class present.
@@ -147,7 +148,7 @@ void order_by_class(const Lists* L, const std::vector<long long>& gcls, const Ev
   for (int i = 0; i < ng; i++) {
     if (i == 0 || gcls[ord[i]] != gcls[ord[i - 1]]) {
       const SysEval& s = P.h_sys[L->h_g_sys[ord[i]]];
-      cls.push_back(LaunchClass{far ? s.nterms : 0, s.kernel, s.eps_check, i, 0});
+      cls.push_back(LaunchClass{far ? s.nterms : 0, s.kernel, s.eps_check, s.far_kind, i, 0});
     }
     cls.back().count++;
   }
@@ -178,7 +179,7 @@ void plan_classes(Tree* t, Lists* L, EvalPlan* P) {
   std::vector<int> ord;
   const SysEval& s0 = P->h_sys[0];
   if (one_far) {
-    P->far_classes.assign(1, LaunchClass{s0.nterms, s0.kernel, s0.eps_check, 0, ng});
+    P->far_classes.assign(1, LaunchClass{s0.nterms, s0.kernel, s0.eps_check, s0.far_kind, 0, ng});
     P->far_ord = L->order.p;
   } else {
     order_by_class(L, gf, *P, ord, P->far_classes, true);
@@ -187,7 +188,7 @@ void plan_classes(Tree* t, Lists* L, EvalPlan* P) {
     P->far_ord = P->far_order.p;
   }
   if (one_near) {
-    P->near_classes.assign(1, LaunchClass{0, s0.kernel, s0.eps_check, 0, ng});
+    P->near_classes.assign(1, LaunchClass{0, s0.kernel, s0.eps_check, s0.far_kind, 0, ng});
     P->near_ord = L->order.p;
   } else {
     order_by_class(L, gn, *P, ord, P->near_classes, false);
