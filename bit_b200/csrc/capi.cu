@@ -663,7 +663,12 @@ bit_status bit_eval_points(bit_tree* th, const bit_eval_params* prm, int m, cons
     copy_h2d(c, dord.p, ord.data(), m * sizeof(int));
     Lists L;
     EvalPlan P;
-    plan_sys(t, &P, {*prm}, 1, 0);
+    double reach = 0.0;  // of the points' box, from the tree's box centre
+    for (int a = 0; a < 3; a++) {
+      const double c0 = t->h_fields[6 + a], d = std::max(std::fabs(hi[a] - c0), std::fabs(lo[a] - c0));
+      reach += d * d;
+    }
+    plan_sys(t, &P, {*prm}, 1, 0, 0, std::sqrt(reach));
     build_lists(t, &L, plan_key(t, P, 1), m, dx.p, dy.p, dz.p, P.sys.p);
     plan_classes(t, &L, &P);
     eval_far(t, &L, P, dx.p, dy.p, dz.p, out.p);

@@ -17,6 +17,8 @@ constexpr int kWarp = 32;
 constexpr int kNtermsMax = BIT_NTERMS_MAX;
 constexpr int kGroupMax = 1024;   // targets per group (one CTA; 32 mask words)
 constexpr int kPointGroup = 256;  // external points per group
+constexpr int kNearParts = 8;         // near-field items of a group, at most
+constexpr long long kNearChunk = 512 << 10;  // and the pairs of one, at least
 constexpr double kEpsNear = 1e-14;  // src/constants.h:35
 
 __host__ __device__ constexpr int num_terms(int n) { return n * (n + 1) * (n + 2) / 6; }
@@ -104,6 +106,8 @@ struct SysEval {
   int near_sign, eps_check, self_term, particles;
   int kernel_order;  // regularised Coulomb field: the reference's KERNEL_ORDER (src/problem.h:13)
   int far_kind;      // potentials: bit 0 screened, bit 1 regularised (far_add > 0)
+  int underflow;     // some pair's exp(-kappa R) may fall below the smallest normal number
+  int pad_;
 };
 
 // One launch of a far / near kernel: the groups of one (nterms, kernel) class.
@@ -111,6 +115,7 @@ struct LaunchClass {
   int nterms, kernel, eps;  // eps: near field skips r^2 <= 1e-14
   int kind;                 // far field: SysEval::far_kind
   int begin, count;         // range in the class-ordered group array
+  int ibegin, icount;       // near field: range in the class-ordered item array
 };
 
 struct EvalPlan {
@@ -122,6 +127,8 @@ struct EvalPlan {
   DBuf<int> far_order, near_order;   // used when there is more than one class
   const int* far_ord = nullptr;      // group order of the far / near launches
   const int* near_ord = nullptr;
+  DBuf<int2> near_items;             // used when there is more than one near class
+  const int2* near_it = nullptr;
   long long lists_version = -1;      // lists the classes were planned for
   std::vector<long long> class_key;  // per system: far and near class of the last plan
 };
@@ -170,8 +177,18 @@ struct Lists {
   DBuf<int> far_node, near_node;            // entry -> node
   DBuf<unsigned> far_mask, near_mask;       // (tcount+31)/32 words per entry
   DBuf<int> order;                          // groups by decreasing work
-  DBuf<int> far_cost;                       // far field scratch: targets of each far entry
+  DBuf<int> far_tgt, near_tgt;              // targets of each entry
+  DBuf<long long> far_pre, near_pre;        // work of the group's entries before it
+  DBuf<long long> far_tot, near_tot;        // per group: work of all its entries
   std::vector<long long> h_work;            // estimated work of each group
+  // the potentials' near-field items (group, part | parts << 16), heaviest first; groups of
+  // several parts add them up in near_part (from part_off[g]) when part_done[g] is complete
+  std::vector<int2> h_items;
+  DBuf<int2> items;
+  DBuf<unsigned long long> g_near;          // near pairs of each group
+  DBuf<long long> part_off;
+  DBuf<int> part_done;
+  DBuf<double> near_part;
   long long version = 0;                    // bumped by every build
   ListSizing last;                          // the last build's sizes
   bool fallback = false;                    // the last build used count, scan and fill
@@ -240,6 +257,11 @@ struct Tree {
   DBuf<double> sx, sy, sz, sq, sw;
   DBuf<double4> src64;   // (x, y, z, q)
   DBuf<float4> src32;    // leaf-centred (x-c, y-c, z-c, q)
+  // the same for the mixed potentials, two sources to a record (x0 x1 y0 y1, z0 z1 q0 q1),
+  // each leaf from record pstart[leaf]; an odd leaf's last record ends with its last source
+  // once more, without charge
+  DBuf<float4> src2;
+  DBuf<int> pstart;
   DBuf<int> leaf_of;     // leaf node of each sorted position
   // nodes
   DBuf<int> nummemb, start, children, level, parent;
@@ -319,9 +341,9 @@ void direct_field(Ctx* c, int n, const double* x, const double* y, const double*
 SysEval make_sys_eval(const bit_eval_params& p, int nterms, int points, int force,
                       int kernel_order = 0);
 // Fill P->h_sys (one entry per system; prm holds one entry for all or one per system) and
-// its device copy.
+// its device copy.  reach (points): no target is farther than this from the tree's box centre.
 void plan_sys(Tree* t, EvalPlan* P, const std::vector<bit_eval_params>& prm, int points,
-              int force, int kernel_order = 0);
+              int force, int kernel_order = 0, double reach = 0.0);
 // Key of the lists the plan's MAC needs.
 ListKey plan_key(const Tree* t, const EvalPlan& P, int points);
 // Launch classes and class-ordered groups of P over the lists L.

@@ -69,7 +69,9 @@ struct FarArgs {
   int stride;                // elements from one node's coefficients to the next's
   int rows;                  // targets of the largest group, rounded up to 32 (potentials)
   int* err;                  // device error flags (a bounded wait that gave up: 8)
-  int* cost;                 // scratch, one int per far entry: its number of targets
+  const int* tgt;            // targets of each far entry (potentials)
+  const long long* pre;      // targets of the group's entries before it
+  const long long* tot;      // per group: targets of all its entries
   const SysEval* sys;        // per system: far_add, kappa, far_sign
   const int* g_sys;          // per group: system
   double *out, *out_y, *out_z;
@@ -270,30 +272,15 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
   // w C <= NW P < (w + 1) C, C the group's total.  The entries' costs vary widely, so the
   // round-robin deal this replaces left warps idle at the group's closing barrier.  The
   // split depends on the lists only, so results stay deterministic.
-  for (long long e = e0 + w; e < e1; e += NW) {
-    const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-    const int c = __reduce_add_sync(0xffffffffu, __popc(wd));
-    if (lane == 0) a.cost[e] = c;
-  }
-  __syncthreads();
-  long long tot = 0;
-  for (long long b = e0; b < e1; b += 32)
-    tot += __reduce_add_sync(0xffffffffu, b + lane < e1 ? __ldcg(a.cost + b + lane) : 0);
-  long long run = 0;
-  int eb = 0, ee = 0;
+  const long long tot = a.tot[g];
+  long long eb = 0, ee = 0;
   for (long long b = e0; b < e1; b += 32) {
     const bool in = b + lane < e1;
-    const int c = in ? __ldcg(a.cost + b + lane) : 0;
-    int inc = c;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    const long long P = (run + inc - c) * NW;
+    const long long P = in ? a.pre[b + lane] * NW : 0;
     eb += __popc(__ballot_sync(0xffffffffu, in && P < w * tot));
     ee += __popc(__ballot_sync(0xffffffffu, in && P < (w + 1) * tot));
-    run += __shfl_sync(0xffffffffu, inc, 31);
   }
+  __syncthreads();  // the rows are zero
   for (long long e = e0 + eb; e < e0 + ee; e++) {
     const int node = a.node[e];
     // The cluster's coefficients, its whole block (TP values, 16-byte aligned in global and
@@ -306,7 +293,7 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
       tma_load_1d(M, coef + (long long)node * a.stride, TP * (unsigned)sizeof(T), &bar[w]);
     }
     const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-    const int cnt = __ldcg(a.cost + e);
+    const int cnt = a.tgt[e];
     const double4 c = a.nodec[node];
     const bool all = cnt == tc;  // a cluster accepted by the whole group needs no list
     if (!all) warp_pack(wd, W, tl);
@@ -510,8 +497,9 @@ FarArgs far_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const d
   a.mom = t->mom64.p;
   a.mom_off = t->mom_off.p;
   a.err = t->ctx->dev_err();
-  L->far_cost.ensure(t->ctx, std::max(L->nfar, 1LL));
-  a.cost = L->far_cost.p;
+  a.tgt = L->far_tgt.p;
+  a.pre = L->far_pre.p;
+  a.tot = L->far_tot.p;
   a.sys = P.sys.p;
   a.g_sys = L->g_sys.p;
   return a;

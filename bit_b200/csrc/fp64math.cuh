@@ -91,6 +91,50 @@ __device__ __forceinline__ double exp_tang(double t) {
   return n < -65280 ? 0.0 : e;  // m < -1020: exp(t) < 1e-307
 }
 
+// The same exponential for exp(-kappa r), kappa fixed: the argument in units of L = ln 2 / 64
+// is r * (64 kappa / ln 2), with that factor as a leading double and a correction, so that
+// neither kappa r nor the reduction rounds it: n = rint(r nh), f = r nh - n (one fma, exact)
+// + r nl, |f| <= 1/2, and e^(f L) - 1 from the same Taylor polynomial with L^k folded into
+// its coefficients.  One operation less than -kappa r and exp_tang, and no rounded product.
+// tab: this lane's copy of the table in shared memory (exp_tab_fill): 4 copies of 16-byte
+// entries side by side, so that at most two of the 8 lanes served together meet in a bank
+// (the gather through L1 took up to eight wavefronts a load; 8 copies were no faster).  exp(-kappa r) below 1e-307 is 0.
+struct ExpScale {
+  double nh, nl;  // -64 kappa / ln 2
+};
+constexpr double kExpNoUnderflow = 700.0;
+constexpr double kExpInvLlo = 0x1.777d0ffda0d24p-50;  // 64 / ln 2 - kExpInvL
+__device__ __forceinline__ ExpScale exp_scale(double kappa) {
+  ExpScale k;
+  k.nh = -kappa * kExpInvL;
+  k.nl = fma(-kappa, kExpInvL, -k.nh) - kappa * kExpInvLlo;
+  return k;
+}
+constexpr int kExpTabCopies = 4;
+constexpr int kExpTabBytes = 64 * kExpTabCopies * 16;
+__device__ __forceinline__ void exp_tab_fill(double2* tab, int tid, int threads) {
+  for (int i = tid; i < 64 * kExpTabCopies; i += threads) tab[i] = kExp2Tab64[i / kExpTabCopies];
+}
+// COPIES: of the table at tab (1: kExp2Tab64 itself).  UF: the result is checked for underflow; without, kappa r < kExpNoUnderflow is required.
+template <bool UF, int COPIES>
+__device__ __forceinline__ double exp_scaled(double r, ExpScale k, const double2* tab) {
+  const double kd = fma(r, k.nh, kRoundShift);
+  const int n = __double2loint(kd);
+  const double kf = kd - kRoundShift;
+  const double f = fma(r, k.nl, fma(r, k.nh, -kf));
+  // (ln 2 / 64)^k / k!, k = 5 .. 1
+  double p = fma(f, 0x1.5d87fe78a6731p-40, 0x1.3b2ab6fba4e77p-31);
+  p = fma(p, f, 0x1.c6b08d704a0c0p-23);
+  p = fma(p, f, 0x1.ebfbdff82c58fp-15);
+  p = fma(p, f, 0x1.62e42fefa39efp-7);
+  p *= f;
+  const double2 s = tab[(n & 63) * COPIES];
+  const double v = s.x + fma(s.x, p, s.y);
+  const double e = __hiloint2double(__double2hiint(v) + ((n >> 6) << 20), __double2loint(v));
+  if (!UF) return e;
+  return kd < kRoundShift - 65280.0 ? 0.0 : e;  // below 2^-1020, however far
+}
+
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

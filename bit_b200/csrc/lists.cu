@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "near.cuh"
 
 namespace bit {
 
@@ -55,6 +56,11 @@ struct ListArgs {
   // per group
   long long *far_off, *near_off, *far_moff, *near_moff;
   int *far_cnt, *near_cnt;
+  unsigned long long* g_near;  // near pairs of each group
+  // per entry: its targets, and the work of the group's entries before it (far: targets,
+  // near: near_weight x sources); per group: that of all
+  int *far_tgt, *near_tgt;
+  long long *far_pre, *near_pre, *far_tot, *near_tot;
   // lists
   int *far_node, *near_node;
   unsigned *far_mask, *near_mask;
@@ -85,6 +91,46 @@ __device__ __forceinline__ void bar_sync_n(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// The per-entry targets and work prefixes of group g, whose lists begin at far / near entry
+// fo / no and mask word fmo / nmo (written by this CTA): the potentials' kernels share a
+// group's work out by them, without a pass over the masks of their own.
+__device__ void finish_group(const ListArgs& a, int g, long long nf, long long fo, long long fmo,
+                             long long nn, long long no, long long nmo) {
+  const int W = (a.g_tcount[g] + 31) >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  __syncthreads();
+  for (long long k = threadIdx.x; k < nf + nn; k += LT) {
+    const unsigned* m = k < nf ? a.far_mask + fmo + k * W : a.near_mask + nmo + (k - nf) * W;
+    int c = 0;
+    for (int q = 0; q < W; q++) c += __popc(m[q]);
+    if (k < nf) a.far_tgt[fo + k] = c;
+    else a.near_tgt[no + k - nf] = c;
+  }
+  __syncthreads();
+  if (w > 1) return;  // warp 0 the far list, warp 1 the near list
+  const long long n = w ? nn : nf;
+  long long run = 0;
+  for (long long b = 0; b < n; b += 32) {
+    const long long k = b + lane;
+    long long v = 0;
+    if (k < n) v = w ? (long long)near_weight(a.near_tgt[no + k]) * a.kids[a.near_node[no + k]].y : a.far_tgt[fo + k];
+    long long inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (k < n) {
+      if (w) a.near_pre[no + k] = run + inc - v;
+      else a.far_pre[fo + k] = run + inc - v;
+    }
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) {
+    if (w) a.near_tot[g] = run;
+    else a.far_tot[g] = run;
+  }
+}
+
 // The walk of group g by the whole CTA.  MODE_COUNT counts the group's entries, MODE_FILL
 // writes them at the offsets a scan gave, MODE_STAGE writes them into the CTA's staging
 // region and then copies them into room reserved with one atomic per list.
@@ -95,6 +141,7 @@ __device__ __forceinline__ void walk_group(const ListArgs& a, int g) {
   __shared__ unsigned long long s_base[4];
   __shared__ int s_flags;  // the walk's overflow (1) / full staging (2), for every warp
   __shared__ long long s_n[2];  // the walk's far and near entry counts, for every warp
+  __shared__ unsigned long long s_np;  // the group's near pairs
   extern __shared__ unsigned dyn[];
   // dynamic shared memory: each warp's own copy of the node stack
   int (*s_node)[LSTK] = reinterpret_cast<int (*)[LSTK]>(dyn);
@@ -126,7 +173,7 @@ __device__ __forceinline__ void walk_group(const ListArgs& a, int g) {
     s_am[threadIdx.x >> 5][lane] = 0u;
     s_rm[threadIdx.x >> 5][lane] = 0u;
   }
-  if (threadIdx.x == 0) s_flags = 0;
+  if (threadIdx.x == 0) { s_flags = 0; s_np = 0; }
   int sp = 1;
   long long nf = 0, nn = 0, fpairs = 0, npairs = 0;
   const long long fo = MODE == MODE_FILL ? a.far_off[g] : 0, no = MODE == MODE_FILL ? a.near_off[g] : 0;
@@ -216,13 +263,21 @@ __device__ __forceinline__ void walk_group(const ListArgs& a, int g) {
   if (MODE != MODE_FILL && lane == 0 && (fpairs || npairs)) {
     atomicAdd(&a.pairs[0], (unsigned long long)fpairs);
     atomicAdd(&a.pairs[1], (unsigned long long)npairs);
+    if (npairs) atomicAdd(&s_np, (unsigned long long)npairs);
   }
-  if (MODE == MODE_COUNT && threadIdx.x == 0) {
-    a.far_cnt[g] = (int)nf;
-    a.near_cnt[g] = (int)nn;
+  if (MODE == MODE_FILL) {
+    finish_group(a, g, nf, fo, fmo, nn, no, nmo);
+    return;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.g_near[g] = s_np;
+    if (MODE == MODE_COUNT) {
+      a.far_cnt[g] = (int)nf;
+      a.near_cnt[g] = (int)nn;
+    }
   }
   if (MODE != MODE_STAGE || overflow || full) return;
-  __syncthreads();
   if (threadIdx.x == 0) {
     s_base[0] = atomicAdd(&a.totals[0], (unsigned long long)nf);
     s_base[1] = atomicAdd(&a.totals[1], (unsigned long long)(nf * W));
@@ -247,6 +302,8 @@ __device__ __forceinline__ void walk_group(const ListArgs& a, int g) {
   for (int k = threadIdx.x; k < nf * W; k += LT) a.far_mask[s_base[1] + k] = sf_mask[k];
   for (int k = threadIdx.x; k < nn; k += LT) a.near_node[s_base[2] + k] = sn_node[k];
   for (int k = threadIdx.x; k < nn * W; k += LT) a.near_mask[s_base[3] + k] = sn_mask[k];
+  finish_group(a, g, nf, (long long)s_base[0], (long long)s_base[1], nn, (long long)s_base[2],
+               (long long)s_base[3]);
 }
 
 // Count / fill passes: CTA b walks group b.
@@ -372,6 +429,43 @@ static void particle_groups(Tree* t, int G, std::vector<int>& ts, std::vector<in
   flush();
 }
 
+// The potentials' near-field items, heaviest first: a group's near work in one item, or in up
+// to kNearParts equal parts of at least kNearChunk pairs each, whose sums meet in scratch
+// (near_part).  The count follows from the group's own lists alone, so that its result does
+// not depend on what else is evaluated; without room in the memory budget for the scratch,
+// every group is one item.
+static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& pairs,
+                       const std::vector<int>& tc) {
+  const int ng = (int)pairs.size();
+  std::vector<int> K(ng);
+  std::vector<long long> off(ng, 0);
+  long long tot = 0;
+  for (int g = 0; g < ng; g++) {
+    K[g] = (int)std::max(1ull, std::min<unsigned long long>(kNearParts, pairs[g] / kNearChunk));
+    off[g] = tot;
+    if (K[g] > 1) tot += (long long)K[g] * tc[g];
+  }
+  if (L->near_part.n < (size_t)tot && c->budget && c->in_use + tot * sizeof(double) > c->budget) {
+    std::fill(K.begin(), K.end(), 1);
+    tot = 0;
+  }
+  std::vector<std::pair<unsigned long long, int2>> it;
+  for (int g = 0; g < ng; g++)
+    for (int k = 0; k < K[g]; k++) it.push_back({pairs[g] / K[g], make_int2(g, k | K[g] << 16)});
+  std::stable_sort(it.begin(), it.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  L->h_items.resize(it.size());
+  for (size_t i = 0; i < it.size(); i++) L->h_items[i] = it[i].second;
+  cudaStream_t s = c->stream;
+  L->items.ensure(c, it.size());
+  L->part_off.ensure(c, ng);
+  L->part_done.ensure(c, ng);
+  L->near_part.ensure(c, tot);
+  BIT_CUDA(cudaMemcpyAsync(L->items.p, L->h_items.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+  BIT_CUDA(cudaMemcpyAsync(L->part_off.p, off.data(), ng * sizeof(long long), cudaMemcpyHostToDevice, s));
+  BIT_CUDA(cudaMemsetAsync(L->part_done.p, 0, ng * sizeof(int), s));
+  BIT_CUDA(cudaStreamSynchronize(s));
+}
+
 void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const double* tx,
                  const double* ty, const double* tz, const SysEval* d_sys, const ListKey* alt) {
   if (alt && (!alt->sysmac.empty() || !key.sysmac.empty() || t->nsys != 1)) alt = nullptr;
@@ -406,6 +500,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->near_moff.ensure(c, ng);
   L->far_cnt.ensure(c, ng);
   L->near_cnt.ensure(c, ng);
+  L->g_near.ensure(c, ng);
   DBuf<unsigned long long> cnt;  // totals[4], pairs[2], err (as the 7th word)
   cnt.ensure(c, 8);
   BIT_CUDA(cudaMemsetAsync(cnt.p, 0, 8 * sizeof(unsigned long long), s));
@@ -420,6 +515,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   a.far_off = L->far_off.p; a.near_off = L->near_off.p;
   a.far_moff = L->far_moff.p; a.near_moff = L->near_moff.p;
   a.far_cnt = L->far_cnt.p; a.near_cnt = L->near_cnt.p;
+  a.g_near = L->g_near.p;
   a.totals = cnt.p;
   a.pairs = cnt.p + 4;
   a.err = reinterpret_cast<int*>(cnt.p + 6);
@@ -454,8 +550,20 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->near_node.ensure(c, cap[2]);
   L->near_mask.ensure(c, cap[3]);
   for (int k = 0; k < 4; k++) a.cap[k] = cap[k];
-  a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
-  a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
+  auto point_at_lists = [&] {
+    L->far_tgt.ensure(c, L->far_node.n);
+    L->near_tgt.ensure(c, L->near_node.n);
+    L->far_pre.ensure(c, L->far_node.n);
+    L->near_pre.ensure(c, L->near_node.n);
+    a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
+    a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
+    a.far_tgt = L->far_tgt.p; a.near_tgt = L->near_tgt.p;
+    a.far_pre = L->far_pre.p; a.near_pre = L->near_pre.p;
+  };
+  point_at_lists();
+  L->far_tot.ensure(c, ng);
+  L->near_tot.ensure(c, ng);
+  a.far_tot = L->far_tot.p; a.near_tot = L->near_tot.p;
   set_stage_attr();
   // staging: one region per resident CTA.  A group's entries number at most the tree's
   // nodes (far) and leaves (near), each with at most 32 mask words.
@@ -479,6 +587,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
                       !c->budget || c->in_use + stage_words * sizeof(unsigned) <= c->budget;
   unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   std::vector<int> hf(ng), hn(ng);
+  std::vector<unsigned long long> hp(ng);
   int err = 2;  // no single pass: straight to count, scan and fill
   if (staged) {
     L->gstage.ensure(c, stage_words);
@@ -492,6 +601,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     BIT_CUDA(cudaMemcpyAsync(h, cnt.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaMemcpyAsync(hf.data(), L->far_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaMemcpyAsync(hn.data(), L->near_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
+    BIT_CUDA(cudaMemcpyAsync(hp.data(), L->g_near.p, ng * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaStreamSynchronize(s));
     err = (int)(h[6] & 0xffffffffu);
     if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded (tree deeper than supported)");
@@ -508,6 +618,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     BIT_CUDA(cudaMemcpyAsync(h, cnt.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaMemcpyAsync(hf.data(), L->far_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaMemcpyAsync(hn.data(), L->near_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
+    BIT_CUDA(cudaMemcpyAsync(hp.data(), L->g_near.p, ng * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaStreamSynchronize(s));
     err = (int)(h[6] & 0xffffffffu);  // this pass walked every group to the end
     if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded");
@@ -515,8 +626,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     L->far_mask.ensure(c, h[1]);
     L->near_node.ensure(c, h[2]);
     L->near_mask.ensure(c, h[3]);
-    a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
-    a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
+    point_at_lists();
     count_launch(), k_lists<MODE_FILL><<<ng, LT, STACK_BYTES, s>>>(a);
     BIT_CHECK_LAUNCH();
   }
@@ -545,6 +655,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->h_work = wk;
   L->order.ensure(c, ng);
   BIT_CUDA(cudaMemcpyAsync(L->order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s));
+  near_items(L, c, hp, tc);
   BIT_CUDA(cudaStreamSynchronize(s));
   L->key = key;
   L->valid = true;

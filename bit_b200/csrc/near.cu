@@ -1,718 +1,630 @@
-// Near field: the leaf direct sums of treepotential / shielded_treepot / treeforce
-// (src/tree3d.cpp:4737-4774, 3539-3623, 923-967), one CTA per target group.
+// Near field of the potentials: the leaf direct sums of treepotential / shielded_treepot
+// (src/tree3d.cpp:4737-4774, 3539-3623), one CTA per item: a target group, or one of the
+// equal parts a heavy group's work is cut into.
 //
-// For each near entry (source leaf, bitmask over the group's targets) the CTA packs the
-// targets that need the leaf into a dense list and splits the leaf's sources across 1..32
-// threads per target, whichever keeps the most threads busy (partial sums combined by
-// warp shuffles).  Source tiles are staged in shared memory by TMA bulk
-// copies (cp.async.bulk with an mbarrier), double buffered so the next tile streams in
-// while the current one is consumed; every thread then reads each source from shared
-// memory, broadcast across the targets.  Accumulation per target is in shared memory in a
-// fixed order, so results are deterministic.
+// A group's near work is the sum over its near entries (source leaf, bitmask over the
+// group's targets) of targets x sources.  The CTA's warps share it out by source: entry
+// after entry, source after source, each warp takes the contiguous run that holds 1/8 of the
+// group's pair steps, so that all finish together without meeting at a barrier per tile, and
+// every lane of a warp reads the same source (one shared-memory wavefront a load).  For each
+// entry of its run a warp packs the targets that need the leaf into a list, streams its
+// sources through two of its own shared-memory tiles by TMA bulk copies (the next tile lands
+// while this one is consumed), and takes the targets 64 at a time, two per lane, so that one
+// source load serves two pairs and four pairs are in flight; the last few targets of a list
+// share a source among several lanes.  Sums go to the warp's own accumulator row; rows are
+// added in warp order at the end.  Everything follows from the lists alone, so results do
+// not depend on timing.
 //
-// FP64 path: the reference's arithmetic.  Mixed path: sources in FP32 relative to their
-// leaf centre, the target's offset from that centre formed in FP64 and rounded once, MUFU
-// rsqrt / ex2, and per-target compensated (two-sum) accumulation; pairs too close for FP32
-// coordinates are summed in FP64 (below).  The self pair is skipped by splitting each
-// lane's index range around it.
+// FP64: bound by the FP64 pipe (12 operations a Coulomb pair, 25 a screened one; the kernel
+// this replaces, one target a thread and a barrier per tile, was held up by shared-memory
+// wavefronts).  Mixed: by the MUFU (one or two a pair) and issue.  Before / now, ms, default
+// settings: 2M clustered (leaves of 1000, theta = 0.7, 9.25 G pairs) FP64 screened 20.7 / 17.1,
+// Coulomb 13.4 / 7.5, mixed 6.0 / 5.9 and 3.6 / 3.8; 100k, theta = 0.15 (1.61 G pairs): 10.8 /
+// 3.1, 6.5 / 1.34, mixed 2.26 / 1.16, 1.72 / 0.60; 300k uniform in leaves of 100: 1.17 / 0.50,
+// 0.75 / 0.32, mixed 0.68 / 0.29, 0.50 / 0.24.  Eight warps a CTA: four are 5% faster in the
+// mixed 2M case and up to 50% slower on 20k; parts of at least 512k pairs: 64k cost 10% at
+// 200k for 10% at 20k.
 #include <algorithm>
 #include <climits>
 
 #include "common.cuh"
 #include "fp64math.cuh"
+#include "near.cuh"
 #include "tma.cuh"
 
 namespace bit {
 
 namespace {
 
-constexpr int NT = 256;  // threads per CTA
+constexpr int NW = 8;  // warps per CTA
 
-struct NearArgs {
-  const int *order, *g_tstart, *g_tcount;
-  const double *tx, *ty, *tz;
-  const long long *off, *moff;
-  const int* cnt;
-  const int* node;
-  const unsigned* mask;
-  const int *start, *nummemb;
-  const double4* nodec;
-  const void* src;  // float4 (mixed) or double4 (FP64) in tree order
-  const double4* src64;
-  const float4* nodeh;  // per node: half extents of the box, rounded up
-  const double* sw;
-  const SysEval* sys;  // per system: near_del, kappa, intg, near_sign, self_term, particles
-  const int* g_sys;    // per group: system
-  double *out, *out_y, *out_z;  // potential, or the three field components
-  int* err;
-  // mixed potentials: close pairs left out of the FP32 sums, per target (k_close)
-  int* ccnt;    // tiles recorded for the target
-  int2* crec;   // up to kCloseRec (near entry, first source of the tile) per target
-  int2* clist;  // (target, group) of every target with a record
-  int* cn;      // entries of clist
-  int tile;     // sources per tile (Prec<>::TILE_MIN..TILE_MAX)
-  int split;    // threads per target: 0 the precision's rule, else at most this many
-};
-
-constexpr int kCloseRec = 2;  // record slots per target; beyond them k_close scans them all
-
-__device__ __forceinline__ float rsqrt_approx(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// Knuth two-sum: s + e accumulates b with the rounding error of each step kept in e.
-__device__ __forceinline__ void two_sum(float& s, float& e, float b) {
-  float t = s + b;
-  float bp = t - s;
-  e += (s - (t - bp)) + (b - bp);
-  s = t;
+// Pack the set bits of a group mask (W words, lane l holds word l) into tl in ascending order.
+__device__ __forceinline__ void pack_list(unsigned wd, int W, unsigned short* tl) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  int base = 0;
+  for (int j = 0; j < W; j++) {
+    const unsigned b = __shfl_sync(0xffffffffu, wd, j);
+    if ((b >> lane) & 1u) tl[base + __popc(b & lt)] = (unsigned short)(32 * j + lane);
+    base += __popc(b);
+  }
+  __syncwarp();
 }
 
-template <bool F32>
-struct Prec;
-// Source tile (records per TMA copy): the default, and the range a context may choose
-// (bit_ctx_set_near_config); shared memory holds two tiles.
-template <>
-struct Prec<true> {
-  using S = float4;
-  using T = float;
-  static constexpr int TILE = 1024, TILE_MIN = 256, TILE_MAX = 2048;
-};
-template <>
-struct Prec<false> {
-  using S = double4;
-  using T = double;
-  static constexpr int TILE = 512, TILE_MIN = 128, TILE_MAX = 1024;
-};
-
-// One pair's contribution in FP64, added to acc: the reference's q / sqrt(r^2) and
-// q e^{-kappa r} / r (src/tree3d.cpp:4765-4769, 3609-3618).  1/r comes from a refined
-// reciprocal square root (rsqrt_nr, within an ulp of 1/sqrt) in place of a square root
-// and a division, the exponential from a branch-free exp (exp_tang, within an ulp), so
-// that the unrolled pairs of a sweep interleave; r^2 + del is one FMA chain, and the
-// Coulomb pair folds q and the accumulation into the Newton step's last FMA.  At 2M
-// clustered, p = 8, theta = 0.7, the screened FP64 near field takes 21.2 ms against 26.2
-// ms with CUDA's exp and rsqrt and the plain forms, the Coulomb one 10.8 against 12.1 ms
-// (the same tuned tiles); the results move by about 2e-16 (relative L2).  EPS: a pair with
-// r^2 <= 1e-14 adds nothing.  SMALL: kappa r < kSmallExpArg, the exponential's
-// small-argument form (no underflow check; the same value).
-template <int KER, bool EPS, bool SMALL = false>
-__device__ __forceinline__ void pair_acc(double x, double y, double z, double4 s, double del,
-                                         double kappa, double& acc) {
+// -------------------------------------------------------------------------------- FP64 pair
+// One pair's q / sqrt(r^2 + del) or q e^(-kappa R) / R (src/tree3d.cpp:4765-4769, 3609-3618)
+// added to acc.  1/R: the hardware seed and one third-order Newton step (rsqrt_nr); the
+// exponential: exp_scaled.  12 (Coulomb) / 25 (screened) FP64 operations.  EPS: a pair with
+// r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`).  UF: the
+// exponential may underflow.
+template <int KER, bool EPS, bool SELF, bool UF, int COPIES = kExpTabCopies>
+__device__ __forceinline__ void pair64(double x, double y, double z, double4 s, double del,
+                                       ExpScale k, const double2* tab, bool own, double& acc) {
   const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
-  const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, del)));
-  double q = s.w, rr = r2;
-  if (EPS) {
-    const bool skip = !(r2 > kEpsNear);
+  double rr = fma(dx, dx, fma(dy, dy, fma(dz, dz, del)));
+  double q = s.w;
+  if (EPS || SELF) {
+    const bool skip = (SELF && own) || (EPS && !(rr > kEpsNear));
     q = skip ? 0.0 : q;
     rr = skip ? 1.0 : rr;
   }
   double y0;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(rr));
-  // one third-order Newton step, as rsqrt_nr: y0 (1 + e c), e = 1 - rr y0^2, c = 1/2 + 3e/8
-  const double e = fma(-rr * y0, y0, 1.0);
-  const double ec = e * fma(e, 0.375, 0.5);
+  const double t = rr * y0;
+  const double e = fma(-t, y0, 1.0);
+  const double f = fma(e, 0.375, 0.5);
   if (KER == BIT_KERNEL_COULOMB) {
-    const double qy = q * y0;
-    acc = fma(qy, ec, acc + qy);
+    acc = fma(q * y0, fma(e, f, 1.0), acc);
   } else {
+    const double ec = e * f;
     const double ri = fma(y0, ec, y0);
-    acc = fma(q * exp_tang<SMALL>(-kappa * (rr * ri)), ri, acc);
+    acc = fma(q * exp_scaled<UF, COPIES>(fma(t, ec, t), k, tab), ri, acc);
   }
-}
-// Field of eval_grad_kernel_reg (src/tree3d.cpp:73-97), KERNEL_ORDER = 0:
-// q * (-(x_j - x) / (r * r^2)).
-__device__ __forceinline__ void fpair(double x, double y, double z, double4 s, double del,
-                                      double& ax, double& ay, double& az) {
-  const double dx = s.x - x, dy = s.y - y, dz = s.z - z;
-  const double rs = dx * dx + dy * dy + dz * dz + del;
-  const double r = sqrt(rs);
-  const double t = s.w / (r * rs);
-  ax -= dx * t; ay -= dy * t; az -= dz * t;
-}
-// The same with the reference's KERNEL_ORDER family (eval_grad_kernel_reg,
-// src/tree3d.cpp:80-91): 1/(r rs) plus korder terms, each the previous one times
-// (l + 1/2)/l * del/rs.
-__device__ __forceinline__ void fpair_order(double x, double y, double z, double4 s, double del,
-                                            int korder, double& ax, double& ay, double& az) {
-  const double dx = s.x - x, dy = s.y - y, dz = s.z - z;
-  const double rs = dx * dx + dy * dy + dz * dz + del;
-  const double r = sqrt(rs);
-  double temp = 1.0 / (r * rs), f = temp;
-  for (int l = 1; l <= korder; l++) {
-    f = f * (l + 0.5) / l * del / rs;
-    temp += f;
-  }
-  const double t = s.w * temp;
-  ax -= dx * t; ay -= dy * t; az -= dz * t;
-}
-// Screened 2-D field of one pair (shielded_treeforce's leaf loop, src/tree3d.cpp:3384-3398):
-// t = q e^{-kappa r} / r^2 (kappa + 1/r), fx -= dy t, fy += dx t, no del.
-__device__ __forceinline__ void cpair(double x, double y, double z, double4 s, double kappa,
-                                      double& ax, double& ay) {
-  const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
-  const double rs = dx * dx + dy * dy + dz * dz;
-  const double r = sqrt(rs);
-  const double t = s.w * exp(-kappa * r) / rs * (kappa + 1 / r);
-  ax -= dy * t; ay += dx * t;
 }
 
-template <class T>
-__device__ __forceinline__ T shfl_sum(T v, int tpt) {
-  for (int o = tpt >> 1; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+struct Range64 {
+  const double4* src;  // the tile
+  int n;               // its sources
+  double del;
+  ExpScale k;
+  const double2* tab;
+};
+
+// Two targets against every source of the tile, two sources (four pairs) at a time; o0, o1:
+// the targets' own tile index (SELF).  (Four sources: 3% faster at 2M, 20% slower on leaves
+// of 55.)
+template <int KER, bool EPS, bool SELF, bool UF>
+__device__ __forceinline__ void two64(const Range64& r, double x0, double y0, double z0, double x1,
+                                      double y1, double z1, int o0, int o1, double& p0, double& p1) {
+  constexpr int UN = 2;
+  double a0[UN], a1[UN];
+#pragma unroll
+  for (int u = 0; u < UN; u++) a0[u] = a1[u] = 0.0;
+  auto add = [&](int j, int u) {
+    const double4 s = r.src[j];
+    pair64<KER, EPS, SELF, UF>(x0, y0, z0, s, r.del, r.k, r.tab, j == o0, a0[u]);
+    pair64<KER, EPS, SELF, UF>(x1, y1, z1, s, r.del, r.k, r.tab, j == o1, a1[u]);
+  };
+  int j = 0;
+#pragma unroll 1
+  for (; j + UN - 1 < r.n; j += UN) {
+#pragma unroll
+    for (int u = 0; u < UN; u++) add(j + u, u);
+  }
+#pragma unroll 1
+  for (; j < r.n; j++) add(j, 0);
+  p0 = a0[0] + a0[1];
+  p1 = a1[0] + a1[1];
+}
+
+// One target against sources j, j + step, ... of the tile.
+template <int KER, bool EPS, bool SELF, bool UF>
+__device__ __forceinline__ double one64(const Range64& r, double x, double y, double z, int o, int j,
+                                        int step) {
+  constexpr int UN = 4;
+  double a[UN] = {0.0, 0.0, 0.0, 0.0};
+  auto add = [&](int k, int u) {
+    pair64<KER, EPS, SELF, UF>(x, y, z, r.src[k], r.del, r.k, r.tab, k == o, a[u]);
+  };
+#pragma unroll 1
+  for (; j + (UN - 1) * step < r.n; j += UN * step) {
+#pragma unroll
+    for (int u = 0; u < UN; u++) add(j + u * step, u);
+  }
+#pragma unroll 1
+  for (; j < r.n; j += step) add(j, 0);
+  return (a[0] + a[2]) + (a[1] + a[3]);
+}
+
+// Every listed target against one tile; sums into the warp's row.
+template <int KER, bool EPS, bool SELF, bool UF>
+__device__ __forceinline__ void tile64(const Range64& r, const double* cx, const double* cy,
+                                       const double* cz, const unsigned short* tl, bool all, int cnt,
+                                       int own0, double* row) {
+  const int lane = threadIdx.x & 31;
+  const NearSteps st = near_steps(cnt);
+  for (int b = 0; b < st.full; b++) {
+    const int r0 = 64 * b + lane, r1 = r0 + 32;
+    const bool v1 = r1 < cnt;  // (a partial last block holds more than 48: r0 is a target)
+    const int i0 = all ? r0 : tl[r0], i1 = v1 ? (all ? r1 : tl[r1]) : i0;
+    double p0, p1;
+    two64<KER, EPS, SELF, UF>(r, cx[i0], cy[i0], cz[i0], cx[i1], cy[i1], cz[i1], i0 + own0, i1 + own0, p0, p1);
+    row[i0] += p0;
+    if (v1) row[i1] += p1;
+  }
+  int base = 64 * st.full;
+  if (st.one) {
+    const int i = all ? base + lane : tl[base + lane];
+    row[i] += one64<KER, EPS, SELF, UF>(r, cx[i], cy[i], cz[i], i + own0, 0, 1);
+    base += 32;
+  }
+  if (st.tail) {
+    const int sh = near_tail_shift(st.tail), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+    const bool v = slot < st.tail;
+    const int r0 = base + (v ? slot : 0);
+    const int i = all ? r0 : tl[r0];
+    double p = one64<KER, EPS, SELF, UF>(r, cx[i], cy[i], cz[i], i + own0, slice, 1 << sh);
+    for (int o = 1 << sh >> 1; o; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+    if (v && slice == 0) row[i] += p;
+  }
+  __syncwarp();
+}
+
+// -------------------------------------------------------------------------------- FP32 pairs
+// Mixed precision: sources in FP32 relative to their leaf's centre, two to a 32-byte record
+// (x0 x1 y0 y1 z0 z1 q0 q1), the target's offset from that centre formed in FP64 and rounded
+// once.  Differences, squares and sums run on packed pairs of sources (f32x2: one issue slot
+// for two), 1/r and 2^x on the MUFU.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
   return v;
 }
 
-// Close pairs in the mixed path.  FP32 leaf-centred coordinates carry an absolute error of
-// about 6e-8 of their magnitude, so a pair much closer than the leaf's size loses relative
-// accuracy in its FP32 difference (two particles 1e-4 apart in a leaf of size 0.1 give
-// ~1e-5).  Pairs closer than r_t = 1/32 of the source leaf's radius (r^2 below thr) are
-// left out of the FP32 sum and summed in FP64 from the FP64 sources instead, with the
-// reference's rules (including its r^2 <= 1e-14 skip, which only such pairs can meet:
-// thr >= 2e-14).  Every other pair keeps at most ~4e-6 relative error, far below 1e-6 of a
-// target's total.  Close pairs can only occur where a target lies within r_t of the source
-// leaf's box (its own leaf, or a neighbour's boundary), and only where the kernel's del is
-// below thr (FP32 r^2 >= del), so a warp runs the checked loop on those tiles and the plain
-// loop, with no test at all, everywhere else.
-constexpr float kCloseFrac = 1.0f / 1024.0f;  // (1/32)^2
-constexpr float kThrMin = 2e-14f;             // above the 1e-14 skip of src/constants.h:35
-
-// Squared distance from a point (relative to a leaf's centre) to the leaf's box (half
-// extents h, rounded up); 0 inside.
-__device__ __forceinline__ float box_d2(float x, float y, float z, float4 h) {
-  const float dx = fmaxf(fabsf(x) - h.x, 0.f), dy = fmaxf(fabsf(y) - h.y, 0.f),
-              dz = fmaxf(fabsf(z) - h.z, 0.f);
-  return dx * dx + dy * dy + dz * dz;
-}
-
-// FP32 r^2 of a pair (identical wherever it is formed, so the FP32 and FP64 sums split the
-// pairs exactly).
-__device__ __forceinline__ float r2_32(float xt, float yt, float zt, float4 s, float del) {
-  const float dx = s.x - xt, dy = s.y - yt, dz = s.z - zt;
-  return fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, del)));
-}
-
-// p += q * G(r); CHK: pairs with r^2 < thr are left out and flagged.
-template <int KER, bool CHK>
-__device__ __forceinline__ void acc_pot(float xt, float yt, float zt, float4 s, float del,
-                                        float kl2, float thr, float& p, bool& close) {
-  float r2 = r2_32(xt, yt, zt, s, del);
-  float q = s.w;
-  if (CHK) {
-    const bool cl = r2 < thr;
-    close |= cl;
-    q = cl ? 0.f : q;
-    r2 = cl ? 1.f : r2;
-  }
-  const float ri = rsqrt_approx(r2);
-  if (KER == BIT_KERNEL_COULOMB) p = fmaf(q, ri, p);
-  else p = fmaf(q * ri, ex2_approx(r2 * ri * kl2), p);
-}
-
-// FP64: this lane's pairs j, j + tpt, ... < je (the target's own source excluded by the
-// caller's split of the range), eight pairs per iteration into four independent
-// accumulators so that consecutive pairs do not wait on one another's additions.  SMALL:
-// kappa r < kSmallExpArg for every pair (exp_tang's small-argument form).
-template <int KER, bool EPS, bool SMALL = false>
-__device__ __forceinline__ void sweep_pot64(const double4* ds, int j, int je, int tpt, double x,
-                                            double y, double z, double del, double kappa,
-                                            double& p0, double& p1) {
-  double p2 = 0.0, p3 = 0.0;
-  for (; j + 7 * tpt < je; j += 8 * tpt) {
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j], del, kappa, p0);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + tpt], del, kappa, p1);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 2 * tpt], del, kappa, p2);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 3 * tpt], del, kappa, p3);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 4 * tpt], del, kappa, p0);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 5 * tpt], del, kappa, p1);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 6 * tpt], del, kappa, p2);
-    pair_acc<KER, EPS, SMALL>(x, y, z, ds[j + 7 * tpt], del, kappa, p3);
-  }
-  for (; j < je; j += tpt) pair_acc<KER, EPS, SMALL>(x, y, z, ds[j], del, kappa, p0);
-  p0 += p2;
-  p1 += p3;
-}
-
-// This lane's pairs j = jb, jb + tpt, ... < je, eight per iteration into four independent
-// accumulators (against four per iteration: Coulomb 4.13 -> 3.89 ms at 2M).  Both
-// exponentials and reciprocal square roots stay on the MUFU: moving 1, 2 or 3 of every 8
-// screened exponentials to the FMA pipe (a Cody-Waite / minimax exp2) measured 3-12%
-// slower at 2M, since this loop is bound by latency and issue, not by MUFU throughput.
-template <int KER, bool CHK>
-__device__ __forceinline__ void sweep_pot(const float4* fs, int j, int je, int tpt, float xt,
-                                          float yt, float zt, float del, float kl2, float thr,
-                                          float& p0, float& p1, bool& close) {
-  float p2 = 0.f, p3 = 0.f;
-  for (; j + 7 * tpt < je; j += 8 * tpt) {
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j], del, kl2, thr, p0, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + tpt], del, kl2, thr, p1, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 2 * tpt], del, kl2, thr, p2, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 3 * tpt], del, kl2, thr, p3, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 4 * tpt], del, kl2, thr, p0, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 5 * tpt], del, kl2, thr, p1, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 6 * tpt], del, kl2, thr, p2, close);
-    acc_pot<KER, CHK>(xt, yt, zt, fs[j + 7 * tpt], del, kl2, thr, p3, close);
-  }
-  for (; j < je; j += tpt) acc_pot<KER, CHK>(xt, yt, zt, fs[j], del, kl2, thr, p0, close);
-  p1 += p2 + p3;
-}
-
-// Target t left close pairs out of this job's FP32 sum (near entry e, tile at toff).  One
-// thread handles a target per job, and the CTA's jobs are separated by barriers, so the
-// target's records need no atomics and come in job order.
-__device__ __forceinline__ void record_close(const NearArgs& a, int t, int g, long long e,
-                                             int toff) {
-  const int c = a.ccnt[t];
-  if (c < kCloseRec) a.crec[(long long)t * kCloseRec + c] = make_int2((int)e, toff);
-  a.ccnt[t] = c + 1;
-  if (c == 0) a.clist[atomicAdd(a.cn, 1)] = make_int2(t, g);
-}
-
-// Field of one pair, q (x - x_j) / r^3 (eval_grad_kernel_reg, src/tree3d.cpp:73-97,
-// KERNEL_ORDER = 0); CHK as acc_pot.
-template <bool CHK>
-__device__ __forceinline__ void acc_force(float xt, float yt, float zt, float4 s, float del,
-                                          float thr, float& ax, float& ay, float& az,
-                                          bool& close) {
-  const float dx = xt - s.x, dy = yt - s.y, dz = zt - s.z;
-  float rs = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, del)));
-  float q = s.w;
-  if (CHK) {
-    const bool cl = rs < thr;
-    close |= cl;
-    q = cl ? 0.f : q;
-    rs = cl ? 1.f : rs;
-  }
-  const float ri = rsqrt_approx(rs);
-  const float tq = q * ri * ri * ri;
-  ax = fmaf(dx, tq, ax); ay = fmaf(dy, tq, ay); az = fmaf(dz, tq, az);
-}
-
-__device__ __forceinline__ void close_force(float xt, float yt, float zt, double x, double y,
-                                         double z, const float4* fs, const double4* s64,
-                                         int slice, int tpt, int ns, int selfj, float del,
-                                         float thr, double del64, double& cx, double& cy,
-                                         double& cz) {
-  for (int j = slice; j < ns; j += tpt)
-    if (j != selfj && r2_32(xt, yt, zt, fs[j], del) < thr) fpair(x, y, z, s64[j], del64, cx, cy, cz);
-}
-
-// Threads per target for an entry with cnt targets.  FP64 pairs (slow arithmetic): the
-// power of two (1..32) that keeps the most of the CTA's threads busy over the rounds of NT
-// units (a larger split must win by 4% to be taken, since it adds a shuffle reduction and
-// shortens each thread's run).  FP32 pairs are cheap enough that the per-unit overhead
-// weighs more: split only until half the threads are busy (measured: the utilisation rule
-// gains 1.5% on 2M clustered screened targets but loses 14% on 82k-node BIE matvecs).
-// cap > 0 (a tuned setting): the utilisation rule over 1..cap threads.
-template <bool CHEAP>
-__device__ __forceinline__ int split_for(int cnt, int cap) {
-  if (CHEAP && cap == 0) {
-    int tpt = 1;
-    while (tpt < 32 && cnt * tpt * 2 <= NT) tpt <<= 1;
-    return tpt;
-  }
-  const int maxtp = cap > 0 ? cap : 32;
-  int best = 1;
-  float bu = 0.f;
-  for (int tp = 1; tp <= maxtp; tp <<= 1) {
-    const int units = cnt * tp;
-    const int rounds = (units + NT - 1) / NT;
-    const float util = (float)units / (float)(rounds * NT);
-    if (util > bu + 0.04f) {
-      bu = util;
-      best = tp;
-    }
-  }
-  return best;
-}
-
-// Shared-memory layout of one CTA: two source tiles of `tile` records, then the
-// accumulators, the self terms, the packed target list and the mbarriers (target
-// coordinates are read through L1).
-template <bool F32, bool FORCE>
-struct Smem {
-  using S = typename Prec<F32>::S;
-  static constexpr int NACC = FORCE ? 3 : 1;
-  // mixed: float hi + lo per target; FP64: one double; force: three doubles
-  static constexpr size_t acc = (FORCE ? 3 : 1) * kGroupMax * sizeof(double);
-  static constexpr size_t self = kGroupMax * sizeof(double);
-  static constexpr size_t list = kGroupMax * sizeof(int);
-  static constexpr size_t bars = 64;
-  __host__ __device__ static size_t tiles(int tile) { return 2 * (size_t)tile * sizeof(S); }
-  __host__ __device__ static size_t total(int tile) { return tiles(tile) + acc + self + list + bars; }
+struct Range32 {
+  const ulonglong2* rec;  // the tile: two vectors per record of two sources
+  int n;                  // its sources (the last record may be half empty: charge 0)
+  float del, kl2, thr;    // kl2 = -kappa log2(e); pairs below thr are close (near.cuh)
 };
 
-// The whole near field of group g, by the whole CTA.  FORCE: the three field components
-// instead of the potential.  Returns false (in every thread) if a bounded wait gave up:
-// the error flag is set, and the CTA has waited, bounded again, for its copies in flight.
-template <int KER, bool EPS, bool F32, bool FORCE>
-__device__ __forceinline__ bool near_group(const NearArgs& a, int g) {
-  using P = Prec<F32>;
-  using S = typename P::S;
-  using T = typename P::T;
-  using L = Smem<F32, FORCE>;
-  const int TILE = a.tile;
+// A target against one record; careful: the target's own source (index o), the empty half and
+// close pairs add nothing, and `close` tells that there was a close one.  Only the differences
+// and r^2 are packed: what follows the MUFU stays scalar, since gathering its results into
+// pairs costs a move each.
+template <int KER, bool CAREFUL>
+__device__ __forceinline__ void pair32(const Range32& r, int k, f32x2 nx, f32x2 ny, f32x2 nz, int o,
+                                       float2& acc, bool& close) {
+  const ulonglong2 u = r.rec[2 * k], v = r.rec[2 * k + 1];
+  const f32x2 dx = add2(u.x, nx), dy = add2(u.y, ny), dz = add2(v.x, nz);
+  float2 f = unpack2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, pack2(r.del, r.del)))));
+  float2 q = unpack2(v.y);
+  if (CAREFUL) {
+    const bool in0 = 2 * k != o, in1 = 2 * k + 1 != o && 2 * k + 1 < r.n;
+    const bool c0 = f.x < r.thr, c1 = f.y < r.thr;
+    close |= (in0 && c0) || (in1 && c1);
+    if (!in0 || c0) { q.x = 0.f; f.x = 1.f; }
+    if (!in1 || c1) { q.y = 0.f; f.y = 1.f; }
+  }
+  const float i0 = rsqrt_approx(f.x), i1 = rsqrt_approx(f.y);
+  if (KER == BIT_KERNEL_COULOMB) {
+    acc.x = fmaf(q.x, i0, acc.x);
+    acc.y = fmaf(q.y, i1, acc.y);
+  } else {
+    acc.x = fmaf(q.x * i0, ex2_approx(f.x * i0 * r.kl2), acc.x);
+    acc.y = fmaf(q.y * i1, ex2_approx(f.y * i1 * r.kl2), acc.y);
+  }
+}
+
+struct Target32 {
+  f32x2 nx, ny, nz;  // minus the offset from the leaf's centre, twice
+  int own;           // tile index of its own source
+  __device__ Target32(float x, float y, float z, int o)
+      : nx(pack2(-x, -x)), ny(pack2(-y, -y)), nz(pack2(-z, -z)), own(o) {}
+};
+
+template <int KER, bool CAREFUL>
+__device__ __forceinline__ void two32(const Range32& r, const Target32& a, const Target32& b, float& p0,
+                                      float& p1, bool& c0, bool& c1) {
+  float2 s0{0.f, 0.f}, s1{0.f, 0.f}, t0{0.f, 0.f}, t1{0.f, 0.f};
+  const int nr = (r.n + 1) >> 1;
+  int k = 0;
+#pragma unroll 1
+  for (; k + 1 < nr; k += 2) {
+    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c0);
+    pair32<KER, CAREFUL>(r, k, b.nx, b.ny, b.nz, b.own, t0, c1);
+    pair32<KER, CAREFUL>(r, k + 1, a.nx, a.ny, a.nz, a.own, s1, c0);
+    pair32<KER, CAREFUL>(r, k + 1, b.nx, b.ny, b.nz, b.own, t1, c1);
+  }
+  if (k < nr) {
+    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c0);
+    pair32<KER, CAREFUL>(r, k, b.nx, b.ny, b.nz, b.own, t0, c1);
+  }
+  p0 = (s0.x + s0.y) + (s1.x + s1.y);
+  p1 = (t0.x + t0.y) + (t1.x + t1.y);
+}
+
+// One target against records k, k + step, ...
+template <int KER, bool CAREFUL>
+__device__ __forceinline__ float one32(const Range32& r, const Target32& a, int k, int step, bool& c) {
+  float2 s0{0.f, 0.f}, s1{0.f, 0.f};
+  const int nr = (r.n + 1) >> 1;
+#pragma unroll 1
+  for (; k + step < nr; k += 2 * step) {
+    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c);
+    pair32<KER, CAREFUL>(r, k + step, a.nx, a.ny, a.nz, a.own, s1, c);
+  }
+  if (k < nr) pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c);
+  return (s0.x + s0.y) + (s1.x + s1.y);
+}
+
+// Every listed target against one tile of leaf `entry` (centre c, half extents hb); compensated
+// sums into the warp's row (rows values, then rows errors).  own0: the tile index of target
+// 0's own source if the leaf holds targets of the group (SELF).  A warp takes the careful
+// loops where one of its targets comes within the close distance of the leaf's box.
+template <int KER, bool SELF>
+__device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, const double* cx,
+                                       const double* cy, const double* cz, double4 c, float4 hb,
+                                       const unsigned short* tl, bool all, int cnt, int own0, float* row,
+                                       int rows, int t0, int g, long long e, int toff) {
+  const int lane = threadIdx.x & 31;
+  const NearSteps st = near_steps(cnt);
+  auto target = [&](int i) {
+    return Target32((float)(cx[i] - c.x), (float)(cy[i] - c.y), (float)(cz[i] - c.z), SELF ? i + own0 : -1);
+  };
+  auto near_box = [&](const Target32& t) {
+    return box_d2(unpack2(t.nx).x, unpack2(t.ny).x, unpack2(t.nz).x, hb) < r.thr;
+  };
+  auto add = [&](int i, float p, bool close) {
+    two_sum(row[i], row[rows + i], p);
+    if (close) record_close(a, t0 + i, g, e, toff);
+  };
+  for (int b = 0; b < st.full; b++) {
+    const int r0 = 64 * b + lane, r1 = r0 + 32;
+    const bool v1 = r1 < cnt;  // (a partial last block holds more than 48: r0 is a target)
+    const int i0 = all ? r0 : tl[r0], i1 = v1 ? (all ? r1 : tl[r1]) : i0;
+    const Target32 x = target(i0), y = target(i1);
+    float p0, p1;
+    bool c0 = false, c1 = false;
+    if (SELF || __any_sync(0xffffffffu, near_box(x) || near_box(y)))
+      two32<KER, true>(r, x, y, p0, p1, c0, c1);
+    else
+      two32<KER, false>(r, x, y, p0, p1, c0, c1);
+    add(i0, p0, c0);
+    if (v1) add(i1, p1, c1);
+  }
+  int base = 64 * st.full;
+  if (st.one) {
+    const int i = all ? base + lane : tl[base + lane];
+    const Target32 x = target(i);
+    bool cl = false;
+    const float p = SELF || __any_sync(0xffffffffu, near_box(x)) ? one32<KER, true>(r, x, 0, 1, cl)
+                                                                : one32<KER, false>(r, x, 0, 1, cl);
+    add(i, p, cl);
+    base += 32;
+  }
+  if (st.tail) {
+    const int sh = near_tail_shift(st.tail), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+    const bool v = slot < st.tail;
+    const int r0 = base + (v ? slot : 0);
+    const int i = all ? r0 : tl[r0];
+    const Target32 x = target(i);
+    bool cl = false;
+    float p = SELF || __any_sync(0xffffffffu, near_box(x)) ? one32<KER, true>(r, x, slice, 1 << sh, cl)
+                                                          : one32<KER, false>(r, x, slice, 1 << sh, cl);
+    int c = cl;
+    for (int o = 1 << sh >> 1; o; o >>= 1) {
+      p += __shfl_xor_sync(0xffffffffu, p, o);
+      c |= __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (v && slice == 0) add(i, p, c != 0);
+  }
+  __syncwarp();
+}
+
+// -------------------------------------------------------------------------------- the item
+// Shared memory of a CTA: the exponential's table (FP64 screened), per warp two source tiles,
+// an accumulator row (a double, or a float and its error, per target) and a target list.
+// Tiles are counted in 32-byte records: one FP64 source, two FP32 ones.
+constexpr int kRec = 32;
+struct Layout {
+  int recs, rows, tab;  // tab: bytes of the table
+  __host__ __device__ size_t warp_bytes() const {
+    return 2 * (size_t)recs * kRec + (size_t)rows * (sizeof(double) + sizeof(unsigned short));
+  }
+  __host__ __device__ size_t total() const { return tab + NW * warp_bytes(); }
+};
+
+// First source (a multiple of 8, or all ns) of an entry of weight wt whose work begins at P
+// that lies at or past T.
+__device__ __forceinline__ int cut(long long T, long long P, int wt, int ns) {
+  if (T <= P) return 0;
+  if (T >= P + (long long)wt * ns) return ns;
+  const long long j = (T - P + 8LL * wt - 1) / (8LL * wt) * 8;
+  return j < ns ? (int)j : ns;
+}
+
+// Returns false (in every thread) if a warp's bounded wait for a tile gave up: the error flag
+// is set, the warp has waited, bounded again, for its copies in flight, and the group's
+// result is not valid.  phase: this warp's count of completed copies, over the items of a
+// queue.
+template <int KER, bool EPS, bool F32>
+__device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, int2 item, uint64_t* bar,
+                                          unsigned& phase) {
+  constexpr int PER = F32 ? 2 : 1;  // sources of a record
+  const int TILE = L.recs * PER;
+  const int g = item.x, part = item.y & 0xffff, parts = item.y >> 16;
+  __shared__ int s_last;
   extern __shared__ __align__(128) unsigned char sm[];
-  S* tiles = reinterpret_cast<S*>(sm);
-  const double* cx = a.tx + 0;  // group targets, indexed t0 + i below
-  const double* cy = a.ty + 0;
-  const double* cz = a.tz + 0;
-  unsigned char* rest = sm + L::tiles(TILE);
-  double* accd = reinterpret_cast<double*>(rest);
-  float* acch = reinterpret_cast<float*>(accd);  // mixed: hi [0,1024), lo [1024,2048)
-  double* selfv = reinterpret_cast<double*>(rest + L::acc);
-  int* tl = reinterpret_cast<int*>(rest + L::acc + L::self);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(rest + L::acc + L::self + L::list);
-  __shared__ int s_cnt;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const double2* tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
+  unsigned char* tiles0 = sm + L.tab;
+  unsigned char* tiles = tiles0 + (size_t)w * 2 * L.recs * kRec;
+  double* rows = reinterpret_cast<double*>(tiles0 + NW * 2 * (size_t)L.recs * kRec);
+  double* row = rows + (size_t)w * L.rows;
+  unsigned short* tl = reinterpret_cast<unsigned short*>(rows + (size_t)NW * L.rows) + (size_t)w * L.rows;
 
   const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
   const SysEval* se = a.sys + a.g_sys[g];
-  const double sdel = se->near_del, skappa = se->kappa;
   const int W = (tc + 31) >> 5;
-  const long long e0 = a.off[g], e1 = e0 + a.cnt[g];
-  const long long m0 = a.moff[g];
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < tc; i += NT) selfv[i] = 0.0;
-  // the whole accumulator block (the mixed path views it as float hi / lo rows)
-  for (int k = tid; k < L::NACC * kGroupMax; k += NT) accd[k] = 0.0;
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+  const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
+  const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
+  for (int i = tid; i < NW * L.rows; i += 32 * NW) rows[i] = 0.0;
+  // this warp's run [T0, T1) of the group's work (all parts' warps share it), and the entry
+  // it begins in: the last whose prefix is at most T0
+  const long long tot = a.tot[g];
+  const int nv = NW * parts, v = part * NW + w;
+  const long long T0 = tot / nv * v + tot % nv * v / nv;
+  const long long T1 = tot / nv * (v + 1) + tot % nv * (v + 1) / nv;
+  long long e = e0 < e1 ? e0 - 1 : e1;  // (a group may have no near entries)
+  for (long long b = e0; b < e1; b += 32) {
+    const int c = __popc(__ballot_sync(0xffffffffu, b + lane < e1 && a.pre[b + lane] <= T0));
+    e += c;
+    if (c < 32) break;
+  }
+  __syncthreads();  // the rows are zero
+  const double del = se->near_del;
+  const ExpScale ks = exp_scale(se->kappa);
+  const float kl2 = (float)(-se->kappa * 1.4426950408889634);  // -kappa log2(e)
+  bool failed = false;
+  for (; e < e1; e++) {
+    const long long P = a.pre[e];
+    if (P >= T1) break;
+    const int node = a.node[e], ns = a.nummemb[node], cnt = a.tgt[e];
+    const int wt = near_weight(cnt);
+    const int ja = cut(T0, P, wt, ns), jb = cut(T1, P, wt, ns);
+    if (ja >= jb) continue;
+    const int s0 = a.start[node];
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(a.src) +
+                               (size_t)(F32 ? a.pstart[node] : s0) * kRec;
+    auto fetch = [&](int j, unsigned n) {  // the tile that begins at source j (even for FP32)
+      if (lane == 0) {
+        const int cnt_j = min(jb, (j / TILE + 1) * TILE) - j;
+        const unsigned bytes = (unsigned)((cnt_j + PER - 1) / PER) * kRec;
+        fence_proxy_async();
+        mbar_expect_tx(&bar[2 * w + (n & 1)], bytes);
+        tma_load_1d(tiles + (n & 1) * L.recs * kRec, src + (size_t)(j / PER) * kRec, bytes,
+                    &bar[2 * w + (n & 1)]);
+      }
+    };
+    // the first tile streams in while the targets are packed
+    fetch(ja, phase);
+    const bool all = cnt == tc;
+    if (!all) {
+      const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
+      pack_list(wd, W, tl);
+    }
+    // a particle target's own source is the leaf's source at its own sorted position
+    const bool self = se->particles && s0 < t0 + tc && t0 < s0 + ns;
+    Range32 r32;
+    double4 c{};
+    float4 hb{};
+    if (F32) {
+      c = a.nodec[node];
+      hb = a.nodeh[node];
+      r32.del = (float)del;
+      r32.kl2 = kl2;
+      // where del alone reaches the threshold no pair of this leaf can be close
+      r32.thr = near_close_thr(c.w);
+      if (!(r32.del < r32.thr)) r32.thr = 0.f;
+    }
+    for (int j = ja; j < jb;) {
+      const int jn = min(jb, (j / TILE + 1) * TILE);
+      if (jn < jb) fetch(jn, phase + 1);  // (its buffer's reads ended at the last __syncwarp)
+      if (!__all_sync(0xffffffffu, mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1))) {
+        if (lane == 0) {
+          atomicOr(a.err, 2);
+          mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1);
+          if (jn < jb) mbar_wait(&bar[2 * w + ((phase + 1) & 1)], ((phase + 1) >> 1) & 1);
+        }
+        __syncwarp();
+        failed = true;
+        break;
+      }
+      const unsigned char* tile = tiles + (phase & 1) * L.recs * kRec;
+      phase++;
+      const int own = t0 - s0 - j;
+      if constexpr (F32) {
+        r32.rec = reinterpret_cast<const ulonglong2*>(tile);
+        r32.n = jn - j;
+        float* row32 = reinterpret_cast<float*>(row);
+        const int toff = j / TILE * TILE;
+        if (self) tile32<KER, true>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, own, row32, L.rows, t0, g, e, toff);
+        else tile32<KER, false>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, 0, row32, L.rows, t0, g, e, toff);
+      } else {
+        const Range64 r{reinterpret_cast<const double4*>(tile), jn - j, del, ks, tab};
+        if (KER != BIT_KERNEL_COULOMB && se->underflow) {
+          if (self) tile64<KER, EPS, true, true>(r, cx, cy, cz, tl, all, cnt, own, row);
+          else tile64<KER, EPS, false, true>(r, cx, cy, cz, tl, all, cnt, 0, row);
+        } else {
+          if (self) tile64<KER, EPS, true, false>(r, cx, cy, cz, tl, all, cnt, own, row);
+          else tile64<KER, EPS, false, false>(r, cx, cy, cz, tl, all, cnt, 0, row);
+        }
+      }
+      j = jn;
+    }
+    if (failed) break;
+  }
+  const bool ok = !__syncthreads_or(failed);
+  auto warps_sum = [&](int i) {
+    double s = 0.0;
+    for (int q = 0; q < NW; q++) {
+      const double* x = rows + (size_t)q * L.rows;
+      if (F32) {
+        const float* f = reinterpret_cast<const float*>(x);
+        s += (double)f[i] + (double)f[L.rows + i];
+      } else {
+        s += x[i];
+      }
+    }
+    return s;
+  };
+  // this item's sums: straight into the result, or the group's scratch, which the CTA that
+  // completes the group adds up in part order (a failed item counts too: the error flag
+  // stands, and the count is left at 0 for the next evaluation)
+  double* sum = a.part + a.part_off[g];
+  if (parts > 1) {
+    for (int i = tid; i < tc; i += 32 * NW) sum[(long long)part * tc + i] = warps_sum(i);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      s_last = atomicAdd(&a.part_done[g], 1) == parts - 1;
+      if (s_last) {
+        a.part_done[g] = 0;
+        __threadfence();
+      }
+    }
+    __syncthreads();
+    if (!s_last) return ok;
+  }
+  for (int i = tid; i < tc; i += 32 * NW) {
+    double s = 0.0;
+    if (parts > 1) {
+      for (int q = 0; q < parts; q++) s += __ldcg(sum + (long long)q * tc + i);
+    } else {
+      s = warps_sum(i);
+    }
+    double self = 0.0;
+    if (se->self_term) {
+      // the reference's self term, where the target's own leaf is one of its near entries;
+      // added, not subtracted (src/tree3d.cpp:3596)
+      const int leaf = a.leaf_of[t0 + i];
+      for (long long k = e0; k < e1; k++)
+        if (a.node[k] == leaf) {
+          if ((a.mask[m0 + (k - e0) * W + (i >> 5)] >> (i & 31)) & 1u)
+            self = a.src64[t0 + i].w * se->intg / (a.sw ? a.sw[t0 + i] : 1.0);
+          break;
+        }
+    }
+    a.out[t0 + i] += se->near_sign * s + self;
+  }
+  return ok;
+}
+
+// Two mbarriers a warp for its tiles, and the exponential's table, before the kernel's first
+// __syncthreads.
+__device__ __forceinline__ void near_init(const Layout& L, uint64_t* bar) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  if (L.tab) exp_tab_fill(reinterpret_cast<double2*>(sm), threadIdx.x, 32 * NW);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 2 * NW; k++) mbar_init(&bar[k], 1);
     fence_mbar_init();
   }
-  __syncthreads();
-  if (e0 < e1) {
-    const S* src = reinterpret_cast<const S*>(a.src);
-    const float del = (float)sdel;
-    const float kl2 = (float)(-skappa * 1.4426950408889634);  // -kappa*log2(e)
-    // job iterator: (entry e, first source of the tile in the entry's leaf)
-    long long e = e0;
-    int node = a.node[e];
-    int j0 = a.start[node], jn = a.nummemb[node];
-    int toff = 0;
-    if (tid == 0) {
-      const int cnt0 = min(TILE, jn);
-      fence_proxy_async();
-      mbar_expect_tx(&bar[0], cnt0 * (unsigned)sizeof(S));
-      tma_load_1d(tiles, src + j0, cnt0 * (unsigned)sizeof(S), &bar[0]);
-    }
-    int k = 0, tpt = 1, cnt = 0;
-    while (true) {
-      const int buf = k & 1;
-      const int ns = min(TILE, jn - toff);
-      if (toff == 0 && tid < 32) {
-        // pack the targets of this entry (warp 0)
-        unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-        const int c = __popc(wd);
-        int pre = c;
-        for (int o = 1; o < 32; o <<= 1) {
-          int t = __shfl_up_sync(0xffffffffu, pre, o);
-          if (lane >= o) pre += t;
-        }
-        int base = pre - c;
-        while (wd) {
-          const int b = __ffs(wd) - 1;
-          wd &= wd - 1;
-          tl[base++] = 32 * lane + b;
-        }
-        if (lane == 31) s_cnt = pre;
-      }
-      // the next job streams into the other buffer while this one is consumed
-      long long ne = e;
-      int noff = toff + TILE;
-      if (noff >= jn) { ne = e + 1; noff = 0; }
-      if (tid == 0 && ne < e1) {
-        const int nd = a.node[ne];
-        const int cntn = min(TILE, a.nummemb[nd] - noff);
-        fence_proxy_async();
-        mbar_expect_tx(&bar[buf ^ 1], cntn * (unsigned)sizeof(S));
-        tma_load_1d(tiles + (buf ^ 1) * TILE, src + a.start[nd] + noff,
-                    cntn * (unsigned)sizeof(S), &bar[buf ^ 1]);
-      }
-      // Every thread waits (bounded) for this job's tile; the barrier then combines the
-      // outcomes, so the whole CTA takes the same branch.  On a timeout the CTA waits,
-      // bounded again, for both copies it may still have in flight into its shared memory
-      // before it returns, and the host reports the error flag.
-      const bool landed = mbar_wait(&bar[buf], (k >> 1) & 1);
-      if (__syncthreads_or(!landed)) {
-        if (tid == 0) {
-          atomicOr(a.err, 2);
-          mbar_wait(&bar[buf], (k >> 1) & 1);
-          if (ne < e1) mbar_wait(&bar[buf ^ 1], ((k + 1) >> 1) & 1);
-        }
-        __syncthreads();
-        return false;
-      }
-      if (toff == 0) {
-        cnt = s_cnt;
-        tpt = split_for<F32 && !FORCE>(cnt, a.split);
-      }
-      const S* ts = tiles + buf * TILE;
-      const double4 c = a.nodec[node];
-      // Particle targets: target i's own source sits at its sorted position t0 + i, i.e.
-      // at tile index i + selfbase, which is inside this tile only if the target is one
-      // of the tile's sources.
-      const int selfbase = se->particles ? (t0 - (j0 + toff)) : INT_MIN;
-      const int units = cnt * tpt;
-      const int lt = __ffs(tpt) - 1;
-      // close-pair checks are needed only where a target comes within r_t of this leaf's box
-      float thr = fmaxf((float)c.w * kCloseFrac, kThrMin);  // r_t^2 = sqradius / 1024
-      // the FP32 r^2 is at least del (fmaf of non-negative squares onto del), so where del
-      // reaches thr no pair of this tile can be close: thr = 0 keeps every warp on the
-      // plain loop (no box distance is below 0), which is then exact
-      if (!(del < thr)) thr = 0.f;
-      const float4 hb = a.nodeh[node];
-      const double4* s64 = a.src64 + j0 + toff;
-      for (int u0 = 0; u0 < units; u0 += NT) {
-        const int u = u0 + tid;
-        const bool valid = u < units;
-        const int slot = u >> lt, slice = u & (tpt - 1);
-        const int i = valid ? tl[slot] : 0;
-        const int selfj = selfbase == INT_MIN ? -1 : i + selfbase;
-        // the target's own source in this lane's slice: sum around it
-        const bool self_in = selfj >= 0 && selfj < ns && ((selfj - slice) & (tpt - 1)) == 0;
-        const int je = self_in ? selfj : ns;
-        if (!FORCE) {
-          T part = 0;
-          bool close = false;  // mixed: a pair of this lane was left for the FP64 pass
-          if constexpr (F32) {
-            const float4* fs = reinterpret_cast<const float4*>(ts);
-            const float xt = (float)(cx[t0 + i] - c.x), yt = (float)(cy[t0 + i] - c.y),
-                        zt = (float)(cz[t0 + i] - c.z);
-            const bool chk = __any_sync(0xffffffffu, valid && box_d2(xt, yt, zt, hb) < thr);
-            if (valid) {
-              float p0 = 0.f, p1 = 0.f;
-              if (!chk) {
-                sweep_pot<KER, false>(fs, slice, je, tpt, xt, yt, zt, del, kl2, thr, p0, p1, close);
-                if (self_in)
-                  sweep_pot<KER, false>(fs, selfj + tpt, ns, tpt, xt, yt, zt, del, kl2, thr, p0, p1, close);
-              } else {
-                sweep_pot<KER, true>(fs, slice, je, tpt, xt, yt, zt, del, kl2, thr, p0, p1, close);
-                if (self_in)
-                  sweep_pot<KER, true>(fs, selfj + tpt, ns, tpt, xt, yt, zt, del, kl2, thr, p0, p1, close);
-              }
-              part = p0 + p1;
-            }
-          } else {
-            // screened: kappa r stays below kSmallExpArg for every pair of this warp's
-            // targets and tile if it does at r^2 = dmax^2 + del, dmax the target's distance
-            // to the leaf centre plus the leaf's half diagonal (a warp-uniform choice of
-            // the exp form)
-            bool small = false;
-            if (KER == BIT_KERNEL_SCREENED) {
-              const double ox = cx[t0 + i] - c.x, oy = cy[t0 + i] - c.y, oz = cz[t0 + i] - c.z;
-              const double dmax = sqrt(fma(ox, ox, fma(oy, oy, oz * oz))) + sqrt(c.w);
-              small = __all_sync(0xffffffffu, !valid || skappa * sqrt(fma(dmax, dmax, sdel)) < kSmallExpArg);
-            }
-            if (valid) {
-              const double4* ds = reinterpret_cast<const double4*>(ts);
-              double p0 = 0.0, p1 = 0.0;
-              const double x = cx[t0 + i], y = cy[t0 + i], z = cz[t0 + i];
-              if (small) {
-                sweep_pot64<KER, EPS, true>(ds, slice, je, tpt, x, y, z, sdel, skappa, p0, p1);
-                if (self_in) sweep_pot64<KER, EPS, true>(ds, selfj + tpt, ns, tpt, x, y, z, sdel, skappa, p0, p1);
-              } else {
-                sweep_pot64<KER, EPS>(ds, slice, je, tpt, x, y, z, sdel, skappa, p0, p1);
-                if (self_in) sweep_pot64<KER, EPS>(ds, selfj + tpt, ns, tpt, x, y, z, sdel, skappa, p0, p1);
-              }
-              part = p0 + p1;
-            }
-          }
-          if (valid && se->self_term && self_in) {
-            const int jg = j0 + toff + selfj;  // added, not subtracted (src/tree3d.cpp:3596)
-            selfv[i] = a.src64[jg].w * se->intg / (a.sw ? a.sw[jg] : 1.0);
-          }
-          part = shfl_sum(part, tpt);
-          if (valid && slice == 0) {
-            if constexpr (F32) two_sum(acch[i], acch[kGroupMax + i], (float)part);
-            else accd[i] += (double)part;
-          }
-          if constexpr (F32) {
-            if (a.ccnt) {  // (null where no pair can be close)
-              // a target's tpt slices share a warp: one record per target and tile
-              for (int o = tpt >> 1; o; o >>= 1) close |= __shfl_xor_sync(0xffffffffu, (int)close, o) != 0;
-              if (valid && slice == 0 && close) record_close(a, t0 + i, g, e, toff);
-            }
-          }
-        } else {
-          T fx = 0, fy = 0, fz = 0;
-          if constexpr (F32) {
-            const float4* fs = reinterpret_cast<const float4*>(ts);
-            const float xt = (float)(cx[t0 + i] - c.x), yt = (float)(cy[t0 + i] - c.y),
-                        zt = (float)(cz[t0 + i] - c.z);
-            const bool chk = __any_sync(0xffffffffu, valid && box_d2(xt, yt, zt, hb) < thr);
-            if (valid) {
-              bool close = false;
-              if (!chk) {
-                for (int j = slice; j < je; j += tpt)
-                  acc_force<false>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-                if (self_in)
-                  for (int j = selfj + tpt; j < ns; j += tpt)
-                    acc_force<false>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-              } else {
-                for (int j = slice; j < je; j += tpt)
-                  acc_force<true>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-                if (self_in)
-                  for (int j = selfj + tpt; j < ns; j += tpt)
-                    acc_force<true>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-              }
-              if (close) {
-                double qx = 0.0, qy = 0.0, qz = 0.0;
-                close_force(xt, yt, zt, cx[t0 + i], cy[t0 + i], cz[t0 + i], fs, s64, slice, tpt,
-                            ns, selfj, del, thr, sdel, qx, qy, qz);
-                fx += (float)qx; fy += (float)qy; fz += (float)qz;
-              }
-            }
-          } else {
-            if (valid) {
-              const double4* ds = reinterpret_cast<const double4*>(ts);
-              const double x = cx[t0 + i], y = cy[t0 + i], z = cz[t0 + i];
-              const int korder = se->kernel_order;
-              if (KER == BIT_KERNEL_SCREENED) {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) cpair(x, y, z, ds[j], skappa, fx, fy);
-              } else if (korder > 0) {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) fpair_order(x, y, z, ds[j], sdel, korder, fx, fy, fz);
-              } else {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) fpair(x, y, z, ds[j], sdel, fx, fy, fz);
-              }
-            }
-          }
-          fx = shfl_sum(fx, tpt);
-          fy = shfl_sum(fy, tpt);
-          fz = shfl_sum(fz, tpt);
-          if (valid && slice == 0) {
-            accd[i] += (double)fx;
-            accd[kGroupMax + i] += (double)fy;
-            accd[2 * kGroupMax + i] += (double)fz;
-          }
-        }
-      }
-      __syncthreads();
-      k++;
-      if (ne >= e1) break;
-      if (ne != e) {
-        e = ne;
-        node = a.node[e];
-        j0 = a.start[node];
-        jn = a.nummemb[node];
-      }
-      toff = noff;
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < tc; i += NT) {
-    if (FORCE) {
-      a.out[t0 + i] += accd[i];
-      a.out_y[t0 + i] += accd[kGroupMax + i];
-      a.out_z[t0 + i] += accd[2 * kGroupMax + i];
-    } else if (F32) {
-      a.out[t0 + i] += se->near_sign * ((double)acch[i] + (double)acch[kGroupMax + i]) + selfv[i];
-    } else {
-      a.out[t0 + i] += se->near_sign * accd[i] + selfv[i];
-    }
-  }
-  return true;
 }
 
-// One launch class: CTA b takes group order[b].  Potential kernels keep four CTAs per SM
-// (64 registers; the FP64 one chose 72 and three CTAs unconstrained, 4% slower at 2M),
-// except the mixed screened one, which runs three (85 registers): at 2M clustered, p = 8,
-// theta = 0.7, 6.43 -> 6.13 ms, while the mixed Coulomb one went 3.92 -> 4.26 ms with three.
-template <int KER, bool EPS, bool F32, bool FORCE>
-__global__ void __launch_bounds__(NT, FORCE ? 0 : ((F32 && KER == BIT_KERNEL_SCREENED) ? 3 : 4))
-    k_near(NearArgs a) {
-  near_group<KER, EPS, F32, FORCE>(a, a.order[blockIdx.x]);
+// One launch class: CTA b takes item b.
+template <int KER, bool EPS, bool F32>
+__global__ void __launch_bounds__(32 * NW, 2) k_near(NearArgs a, Layout L) {
+  __shared__ uint64_t bar[2 * NW];
+  near_init(L, bar);
+  unsigned phase = 0;
+  near_item<KER, EPS, F32>(a, L, a.items[blockIdx.x], bar, phase);
 }
 
-// Persistent work queue over the groups of every class of a potential evaluation: each CTA
-// takes the next item (a group, in the given order) from a device counter until none is
-// left and runs near_group for that group's kernel and eps rule -- the same device code as
-// k_near, so the results are identical.  A CTA whose bounded wait gave up stops taking
-// items (the host reports the error flag).
+// Persistent work queue over the items of every class (as k_far_queue): the same device code
+// per item, so the results are identical.
 template <bool F32>
-__global__ void __launch_bounds__(NT, 4) k_near_queue(NearArgs a, int count, int* head) {
+__global__ void __launch_bounds__(32 * NW, 2) k_near_queue(NearArgs a, Layout L, int count, int* head) {
   __shared__ int s_item;
+  __shared__ uint64_t bar[2 * NW];
+  near_init(L, bar);
+  unsigned phase = 0;
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(head, 1);
     __syncthreads();
-    const int item = s_item;
+    const int k = s_item;
     __syncthreads();  // every thread has read s_item before it is overwritten
-    if (item >= count) return;
-    const int g = a.order[item];
-    const SysEval* se = a.sys + a.g_sys[g];
+    if (k >= count) return;
+    const int2 item = a.items[k];
+    const SysEval* se = a.sys + a.g_sys[item.x];
     bool ok;
-    if (se->kernel == BIT_KERNEL_COULOMB) {
-      ok = se->eps_check ? near_group<BIT_KERNEL_COULOMB, true, F32, false>(a, g)
-                         : near_group<BIT_KERNEL_COULOMB, false, F32, false>(a, g);
-    } else {
-      ok = se->eps_check ? near_group<BIT_KERNEL_SCREENED, true, F32, false>(a, g)
-                         : near_group<BIT_KERNEL_SCREENED, false, F32, false>(a, g);
-    }
+    // (the mixed path applies the limit on r^2 in its FP64 pass over close pairs)
+    const bool eps = !F32 && se->eps_check;
+    if (se->kernel == BIT_KERNEL_COULOMB)
+      ok = eps ? near_item<BIT_KERNEL_COULOMB, !F32, F32>(a, L, item, bar, phase)
+               : near_item<BIT_KERNEL_COULOMB, false, F32>(a, L, item, bar, phase);
+    else
+      ok = eps ? near_item<BIT_KERNEL_SCREENED, !F32, F32>(a, L, item, bar, phase)
+               : near_item<BIT_KERNEL_SCREENED, false, F32>(a, L, item, bar, phase);
     if (!ok) return;
-    __syncthreads();  // the group's last reads of shared memory precede the next group's writes
+    __syncthreads();  // the item's last reads of shared memory precede the next item's writes
   }
 }
 
-template <int KER, bool EPS, bool F32, bool FORCE>
-void launch(const NearArgs& a, int ngroups, cudaStream_t s) {
-  const size_t bytes = Smem<F32, FORCE>::total(a.tile);
-  ensure_smem_attr(reinterpret_cast<const void*>(k_near<KER, EPS, F32, FORCE>),
-                   (int)Smem<F32, FORCE>::total(Prec<F32>::TILE_MAX));
-  count_launch(), k_near<KER, EPS, F32, FORCE><<<ngroups, NT, bytes, s>>>(a);
-}
-
-template <bool F32>
-void launch_queue(Ctx* c, const NearArgs& a, int count, cudaStream_t s) {
-  const size_t bytes = Smem<F32, false>::total(a.tile);
-  ensure_smem_attr(reinterpret_cast<const void*>(k_near_queue<F32>),
-                   (int)Smem<F32, false>::total(Prec<F32>::TILE_MAX));
-  int per_sm = 0;
-  BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32>, NT, bytes));
-  const int grid = std::max(1, std::min(count, c->num_sms * std::max(per_sm, 1)));
-  c->queue_heads.ensure(c, 2);
-  BIT_CUDA(cudaMemsetAsync(c->queue_heads.p + 1, 0, sizeof(int), s));
-  count_launch(), k_near_queue<F32><<<grid, NT, bytes, s>>>(a, count, c->queue_heads.p + 1);
-}
-
-// FP64 sum of the close pairs that the mixed near kernel left out (FP32 r^2 < thr, the
-// target's own source excluded), one warp per recorded target: the recorded tiles in job
-// order, or, for a target with more tiles than record slots, every near entry of its group
-// that covers it (tiles without close pairs add nothing, so the sum is the same).  Lanes
-// take the sources in the kernel's order and the warp reduces in a fixed order, so the
-// result does not depend on scheduling.
+// FP64 sum of the close pairs that the mixed kernel left out (FP32 r^2 < thr, the target's
+// own source excluded), one warp per recorded target: the recorded tiles in list order (two
+// warps whose runs meet in a tile may both have recorded it), or, for a target with more
+// records than slots, every near entry of its group that covers it (tiles without close pairs
+// add nothing, so the sum is the same).  Lanes take the sources in a fixed order and the warp
+// reduces in a fixed order, so the result does not depend on scheduling.
 template <int KER, bool EPS>
-__device__ double close_sum(const NearArgs& a, const SysEval* se, int t, int g, double x,
-                            double y, double z) {
+__device__ double close_sum(const NearArgs& a, const SysEval* se, int t, int g, double x, double y,
+                            double z) {
   const int lane = threadIdx.x & 31;
-  const double sdel = se->near_del, skappa = se->kappa;
+  const double sdel = se->near_del;
   const float del = (float)sdel;
   const int self = se->particles ? t : -1;  // sorted position of the target's own source
-  const float4* fs = reinterpret_cast<const float4*>(a.src);
   double acc = 0.0;
   auto tile = [&](int node, int j0, int j1) {
     const double4 c = a.nodec[node];
     const float xt = (float)(x - c.x), yt = (float)(y - c.y), zt = (float)(z - c.z);
-    const float thr = fmaxf((float)c.w * kCloseFrac, kThrMin);
+    const float thr = near_close_thr(c.w);
     const int s0 = a.start[node];
-    for (int j = s0 + j0 + lane; j < s0 + j1; j += 32)
-      if (j != self && r2_32(xt, yt, zt, fs[j], del) < thr)
-        pair_acc<KER, EPS>(x, y, z, a.src64[j], sdel, skappa, acc);
+    const float* f = reinterpret_cast<const float*>(a.src) + 8 * (size_t)a.pstart[node];
+    for (int j = j0 + lane; j < j1; j += 32) {
+      const float* p = f + 8 * (j >> 1) + (j & 1);
+      if (s0 + j != self && r2_32(xt, yt, zt, make_float4(p[0], p[2], p[4], 0.f), del) < thr)
+        pair64<KER, EPS, false, true, 1>(x, y, z, a.src64[s0 + j], sdel, exp_scale(se->kappa), kExp2Tab64, false, acc);
+    }
   };
   const int nrec = a.ccnt[t];
   if (nrec <= kCloseRec) {
+    int2 r[kCloseRec];
+    for (int k = 0; k < nrec; k++) r[k] = a.crec[(long long)t * kCloseRec + k];
+    if (nrec == 2 && (r[1].x < r[0].x || (r[1].x == r[0].x && r[1].y < r[0].y))) {
+      const int2 s = r[0];
+      r[0] = r[1];
+      r[1] = s;
+    }
     for (int k = 0; k < nrec; k++) {
-      const int2 r = a.crec[(long long)t * kCloseRec + k];
-      const int node = a.node[r.x];
-      tile(node, r.y, min(r.y + a.tile, a.nummemb[node]));
+      if (k && r[k].x == r[k - 1].x && r[k].y == r[k - 1].y) continue;
+      const int node = a.node[r[k].x];
+      tile(node, r[k].y, min(r[k].y + a.tile, a.nummemb[node]));
     }
   } else {
     const int i = t - a.g_tstart[g], W = (a.g_tcount[g] + 31) >> 5;
@@ -746,56 +658,74 @@ __global__ void __launch_bounds__(256) k_close(NearArgs a) {
   }
 }
 
-NearArgs base_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
-                   const double* tz) {
-  NearArgs a{};
-  a.g_tstart = L->g_tstart.p;
-  a.g_tcount = L->g_tcount.p;
-  a.tx = tx; a.ty = ty; a.tz = tz;
-  a.off = L->near_off.p;
-  a.cnt = L->near_cnt.p;
-  a.moff = L->near_moff.p;
-  a.node = L->near_node.p;
-  a.mask = L->near_mask.p;
-  a.start = t->start.p;
-  a.nummemb = t->nummemb.p;
-  a.nodec = t->nodec.p;
-  a.src = P.f32 ? (const void*)t->src32.p : (const void*)t->src64.p;
-  a.src64 = t->src64.p;
-  a.nodeh = t->nodeh.p;
-  a.sw = t->has_weights ? t->sw.p : nullptr;
-  a.sys = P.sys.p;
-  a.g_sys = L->g_sys.p;
-  a.err = t->ctx->dev_err();
-  // the context's tile, clamped to the precision's range (0: the default)
-  const int want = t->ctx->near_tile;
-  const int lo = P.f32 ? Prec<true>::TILE_MIN : Prec<false>::TILE_MIN;
-  const int hi = P.f32 ? Prec<true>::TILE_MAX : Prec<false>::TILE_MAX;
-  a.tile = want == 0 ? (P.f32 ? Prec<true>::TILE : Prec<false>::TILE) : std::min(hi, std::max(lo, want));
-  a.split = t->ctx->near_split;
-  return a;
+constexpr int kSmemMax = 227 * 1024;
+
+template <bool F32>
+void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
+  Ctx* c = t->ctx;
+  cudaStream_t s = c->stream;
+  Layout lay;
+  lay.rows = L->max_targets;
+  lay.tab = 0;
+  for (const LaunchClass& k : P.near_classes)
+    if (!F32 && k.kernel != BIT_KERNEL_COULOMB) lay.tab = kExpTabBytes;
+  // a context's tile setting counts the records of a CTA's eight warps
+  lay.recs = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 64;
+  // two CTAs an SM: rows of 1,024 targets and the table leave room for tiles of 48
+  while (lay.recs > 16 && lay.total() > kSmemMax / 2 - 1024) lay.recs -= 16;
+  a.tile = lay.recs * (F32 ? 2 : 1);
+  if (c->work_queue && P.near_classes.size() > 1) {
+    const int count = (int)L->h_items.size();
+    a.items = L->items.p;
+    ensure_smem_attr(reinterpret_cast<const void*>(k_near_queue<F32>), kSmemMax - 1024);
+    int per_sm = 0;
+    BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32>, 32 * NW, lay.total()));
+    const int grid = std::max(1, std::min(count, c->num_sms * std::max(per_sm, 1)));
+    c->queue_heads.ensure(c, 2);
+    BIT_CUDA(cudaMemsetAsync(c->queue_heads.p + 1, 0, sizeof(int), s));
+    count_launch(), k_near_queue<F32><<<grid, 32 * NW, lay.total(), s>>>(a, lay, count, c->queue_heads.p + 1);
+    BIT_CHECK_LAUNCH();
+    return;
+  }
+  for (const LaunchClass& k : P.near_classes) {
+    a.items = P.near_it + k.ibegin;
+    auto go = [&](auto kernel) {
+      ensure_smem_attr(reinterpret_cast<const void*>(kernel), kSmemMax - 1024);
+      count_launch(), kernel<<<k.icount, 32 * NW, lay.total(), s>>>(a, lay);
+      BIT_CHECK_LAUNCH();
+    };
+    const bool eps = !F32 && k.eps;
+    if (k.kernel == BIT_KERNEL_COULOMB) {
+      if (eps) go(k_near<BIT_KERNEL_COULOMB, !F32, F32>);
+      else go(k_near<BIT_KERNEL_COULOMB, false, F32>);
+    } else {
+      if (eps) go(k_near<BIT_KERNEL_SCREENED, !F32, F32>);
+      else go(k_near<BIT_KERNEL_SCREENED, false, F32>);
+    }
+  }
 }
 
 }  // namespace
 
-// One launch per (kernel, eps check) class, each over its groups (P.near_ord + begin).
+// One launch per (kernel, eps check) class over its items, or one work queue over all.
 void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
                const double* tz, double* out) {
   Ctx* c = t->ctx;
   cudaStream_t s = c->stream;
-  NearArgs a = base_args(t, L, P, tx, ty, tz);
+  NearArgs a = near_args(t, L, P, tx, ty, tz);
   a.out = out;
+  if (!P.f32) {
+    launch_near<false>(t, L, P, a);
+    return;
+  }
+  a.src = t->src2.p;
   // Mixed: close pairs need r^2 < thr = max(sqradius / 1024, 2e-14) of some leaf, and the
   // FP32 r^2 is at least the system's del (a rounded sum of non-negative terms and del);
   // where del reaches the largest leaf threshold no pair can be close, and the records
   // and the FP64 pass are skipped.
   bool close_possible = false;
-  if (P.f32)
-    for (size_t sy = 0; sy < P.h_sys.size(); sy++) {
-      const float thr_max = fmaxf((float)t->h_sys_leaf_sqr[sy] * kCloseFrac, kThrMin);
-      close_possible |= (float)P.h_sys[sy].near_del < thr_max;
-    }
-  const bool f32 = P.f32;
+  for (size_t sy = 0; sy < P.h_sys.size(); sy++)
+    close_possible |= (float)P.h_sys[sy].near_del < near_close_thr(t->h_sys_leaf_sqr[sy]);
   if (close_possible) {
     // close-pair records, cleared for this evaluation (k_close consumes them)
     const int nt = L->ntargets;
@@ -811,54 +741,9 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
     a.clist = c->close_list.p;
     a.cn = c->close_n.p;
   }
-  // several classes (a forest): one persistent launch over a work queue of all groups
-  if (c->work_queue && P.near_classes.size() > 1) {
-    int count = 0;
-    for (const LaunchClass& k : P.near_classes) count += k.count;
-    a.order = L->order.p;
-    if (f32) launch_queue<true>(c, a, count, s);
-    else launch_queue<false>(c, a, count, s);
-    BIT_CHECK_LAUNCH();
-  }
-  for (const LaunchClass& k : P.near_classes) {
-    if (c->work_queue && P.near_classes.size() > 1) break;
-    a.order = P.near_ord + k.begin;
-    const int ng = k.count;
-    const bool scr = k.kernel != BIT_KERNEL_COULOMB;
-    const bool eps = k.eps != 0;
-#define GO(K, E, F) launch<K, E, F, false>(a, ng, s)
-    if (f32) {
-      if (!scr) { if (eps) GO(BIT_KERNEL_COULOMB, true, true); else GO(BIT_KERNEL_COULOMB, false, true); }
-      else { if (eps) GO(BIT_KERNEL_SCREENED, true, true); else GO(BIT_KERNEL_SCREENED, false, true); }
-    } else {
-      if (!scr) { if (eps) GO(BIT_KERNEL_COULOMB, true, false); else GO(BIT_KERNEL_COULOMB, false, false); }
-      else { if (eps) GO(BIT_KERNEL_SCREENED, true, false); else GO(BIT_KERNEL_SCREENED, false, false); }
-    }
-#undef GO
-    BIT_CHECK_LAUNCH();
-  }
+  launch_near<true>(t, L, P, a);
   if (close_possible) {
     count_launch(), k_close<<<c->num_sms * 4, 256, 0, s>>>(a);
-    BIT_CHECK_LAUNCH();
-  }
-}
-
-void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* fy, double* fz) {
-  cudaStream_t s = t->ctx->stream;
-  NearArgs a = base_args(t, L, P, t->sx.p, t->sy.p, t->sz.p);
-  a.out = fx; a.out_y = fy; a.out_z = fz;
-  // P.force: 1 the regularised Coulomb field (kernel order per system; FP64 beyond order
-  // 0), 2 the screened 2-D field of shielded_treeforce (FP64)
-  for (const LaunchClass& k : P.near_classes) {
-    a.order = P.near_ord + k.begin;
-    if (P.force == 2) {
-      if (P.f32) fail(BIT_ERR_INVALID_ARGUMENT, "the screened field is FP64 only");
-      launch<BIT_KERNEL_SCREENED, false, false, true>(a, k.count, s);
-    } else if (P.f32) {
-      launch<BIT_KERNEL_COULOMB, false, true, true>(a, k.count, s);
-    } else {
-      launch<BIT_KERNEL_COULOMB, false, false, true>(a, k.count, s);
-    }
     BIT_CHECK_LAUNCH();
   }
 }

@@ -7,11 +7,13 @@
 // same for every group of one launch class, so a forest is evaluated by one far launch
 // per distinct (nterms, kernel) and one near launch per distinct (kernel, eps check).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <numeric>
 #include <vector>
 
 #include "common.cuh"
+#include "fp64math.cuh"
 
 namespace bit {
 
@@ -80,12 +82,14 @@ SysEval make_sys_eval(const bit_eval_params& p, int nterms, int points, int forc
       s.near_sign = 1;
       break;
   }
+  // (where del alone keeps r^2 + del above the limit, the near field need not check it)
+  if (s.near_del > kEpsNear) s.eps_check = 0;
   s.far_kind = (p.kernel != BIT_KERNEL_COULOMB ? 1 : 0) + (s.far_add > 0.0 ? 2 : 0);
   return s;
 }
 
 void plan_sys(Tree* t, EvalPlan* P, const std::vector<bit_eval_params>& prm, int points,
-              int force, int kernel_order) {
+              int force, int kernel_order, double reach) {
   const int ns = t->nsys;
   if (prm.empty() || ((int)prm.size() != 1 && (int)prm.size() != ns))
     fail(BIT_ERR_INVALID_ARGUMENT, "one parameter set, or one per system, expected");
@@ -95,9 +99,15 @@ void plan_sys(Tree* t, EvalPlan* P, const std::vector<bit_eval_params>& prm, int
     if (p.precision != prm[0].precision)
       fail(BIT_ERR_INVALID_ARGUMENT, "all systems of one call share a precision");
   std::vector<SysEval> h(ns);
-  for (int s = 0; s < ns; s++)
+  for (int s = 0; s < ns; s++) {
     h[s] = make_sys_eval(prm[prm.size() == 1 ? 0 : s], t->h_sys_nterms[s], points, force,
                          kernel_order);
+    // the largest kappa R of a pair: the sources lie within the root box's half diagonal of
+    // its centre, particle targets too
+    const double half = std::sqrt(t->h_fields[13LL * s + 12]);
+    const double far = half + (points ? reach : half);
+    h[s].underflow = !(h[s].kappa * std::sqrt(far * far + h[s].near_del) < kExpNoUnderflow);
+  }
   P->f32 = prm[0].precision == BIT_PREC_MIXED;
   P->force = force;
   const bool same = P->sys.p && P->h_sys.size() == h.size() &&
@@ -148,7 +158,7 @@ void order_by_class(const Lists* L, const std::vector<long long>& gcls, const Ev
   for (int i = 0; i < ng; i++) {
     if (i == 0 || gcls[ord[i]] != gcls[ord[i - 1]]) {
       const SysEval& s = P.h_sys[L->h_g_sys[ord[i]]];
-      cls.push_back(LaunchClass{far ? s.nterms : 0, s.kernel, s.eps_check, s.far_kind, i, 0});
+      cls.push_back(LaunchClass{far ? s.nterms : 0, s.kernel, s.eps_check, s.far_kind, i, 0, 0, 0});
     }
     cls.back().count++;
   }
@@ -179,7 +189,7 @@ void plan_classes(Tree* t, Lists* L, EvalPlan* P) {
   std::vector<int> ord;
   const SysEval& s0 = P->h_sys[0];
   if (one_far) {
-    P->far_classes.assign(1, LaunchClass{s0.nterms, s0.kernel, s0.eps_check, s0.far_kind, 0, ng});
+    P->far_classes.assign(1, LaunchClass{s0.nterms, s0.kernel, s0.eps_check, s0.far_kind, 0, ng, 0, (int)L->h_items.size()});
     P->far_ord = L->order.p;
   } else {
     order_by_class(L, gf, *P, ord, P->far_classes, true);
@@ -188,13 +198,25 @@ void plan_classes(Tree* t, Lists* L, EvalPlan* P) {
     P->far_ord = P->far_order.p;
   }
   if (one_near) {
-    P->near_classes.assign(1, LaunchClass{0, s0.kernel, s0.eps_check, s0.far_kind, 0, ng});
+    P->near_classes.assign(1, LaunchClass{0, s0.kernel, s0.eps_check, s0.far_kind, 0, ng, 0, (int)L->h_items.size()});
     P->near_ord = L->order.p;
+    P->near_it = L->items.p;
   } else {
     order_by_class(L, gn, *P, ord, P->near_classes, false);
     P->near_order.ensure(c, ng);
     BIT_CUDA(cudaMemcpyAsync(P->near_order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, st));
     P->near_ord = P->near_order.p;
+    std::vector<int2> it;
+    for (LaunchClass& k : P->near_classes) {
+      k.ibegin = (int)it.size();
+      for (const int2& i : L->h_items)
+        if (gn[i.x] == gn[ord[k.begin]]) it.push_back(i);
+      k.icount = (int)it.size() - k.ibegin;
+    }
+    P->near_items.ensure(c, it.size());
+    BIT_CUDA(cudaMemcpyAsync(P->near_items.p, it.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+    BIT_CUDA(cudaStreamSynchronize(st));
+    P->near_it = P->near_items.p;
   }
   if (!one_far || !one_near) BIT_CUDA(cudaStreamSynchronize(st));
   P->lists_version = L->version;

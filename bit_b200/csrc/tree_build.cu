@@ -666,11 +666,14 @@ __global__ void k_node_centres(int numtree, const double* fields, const int* chi
   }
 }
 
+// leaves in member order: leaf l's FP32 sources begin at record (start + l) / 2, which leaves
+// every leaf whole records of two
 __global__ void k_leaf_of(int nleaves, const int* leaves, const int* start, const int* nummemb,
-                          int* leaf_of) {
+                          int* leaf_of, int* pstart) {
   int l = blockIdx.x;
   if (l >= nleaves) return;
   int node = leaves[l];
+  if (threadIdx.x == 0) pstart[node] = (int)(((unsigned)start[node] + (unsigned)l) >> 1);
   for (int e = start[node] + threadIdx.x; e < start[node] + nummemb[node]; e += blockDim.x)
     leaf_of[e] = node;
 }
@@ -841,17 +844,19 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   count_launch(), k_node_centres<<<grid_for(b, 128), 128, 0, s>>>(b, t->fields.p, t->children.p, t->nummemb.p,
                                                                  t->nodec.p, t->nodeh.p, t->kids.p);
   tree_sync_host(t);
-  // leaves in node order
+  // leaves in member order
   std::vector<int> leaves;
   for (int i = 0; i < b; i++)
     if (t->h_children[8LL * i] == -1) leaves.push_back(i);
+  std::sort(leaves.begin(), leaves.end(), [&](int p, int q) { return t->h_start[p] < t->h_start[q]; });
   t->nleaves = (int)leaves.size();
+  t->pstart.ensure(c, b);
   t->leaves.ensure(c, leaves.size());
   BIT_CUDA(cudaMemcpyAsync(t->leaves.p, leaves.data(), leaves.size() * sizeof(int),
                            cudaMemcpyHostToDevice, s));
   t->leaf_of.ensure(c, n);
   count_launch(), k_leaf_of<<<t->nleaves, 256, 0, s>>>(t->nleaves, t->leaves.p, t->start.p, t->nummemb.p,
-                                                       t->leaf_of.p);
+                                                       t->leaf_of.p, t->pstart.p);
   t->iperm.ensure(c, n);
   count_launch(), k_iperm<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, t->iperm.p);
   BIT_CHECK_LAUNCH();
