@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <map>
 #include <string>
 #include <vector>
@@ -62,6 +63,12 @@ void dev_free(Ctx* c, void* p);
 // place.
 void copy_h2d(Ctx* c, void* dst, const void* src, size_t bytes);
 void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes);
+struct D2H {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+void copy_d2h_batch(Ctx* c, std::initializer_list<D2H> list);
 // Free cached (unused) blocks until live + cached bytes are at most `keep`.
 void ctx_trim(Ctx* c, size_t keep);
 
@@ -264,14 +271,13 @@ struct Tree {
   DBuf<int> pstart;
   DBuf<int> leaf_of;     // leaf node of each sorted position
   // nodes
-  DBuf<int> nummemb, start, children, level, parent;
+  DBuf<int> nummemb, start, children;
   DBuf<double> fields;   // 13 per node
   DBuf<double4> nodec;   // (xmid, ymid, zmid, sqradius)
   DBuf<float4> nodeh;    // half extents of the box about the midpoint (rounded up)
   DBuf<int2> kids;       // children: (first index or -1, count | slot order 3 bits each)
-  DBuf<int> leaves;
   // host mirror of the node structure
-  std::vector<int> h_nummemb, h_start, h_children, h_level, h_perm;
+  std::vector<int> h_nummemb, h_start, h_children, h_perm;
   std::vector<double> h_fields;
   // charges and moments
   bool has_charges = false, has_weights = false;

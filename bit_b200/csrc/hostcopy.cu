@@ -169,4 +169,30 @@ void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
   }
 }
 
+// Several device arrays into pageable host arrays with one synchronisation: all of them into
+// one pinned chunk, then out of it.  (A pageable cudaMemcpyAsync waits for its own copy.)
+void copy_d2h_batch(Ctx* c, std::initializer_list<D2H> list) {
+  cudaStream_t s = c->stream;
+  size_t total = 0;
+  for (const D2H& d : list) total += (d.bytes + 15) / 16 * 16;
+  if (total > kStageChunk) {
+    for (const D2H& d : list) copy_d2h(c, d.dst, d.src, d.bytes);
+    return;
+  }
+  ensure_stage(c);
+  BIT_CUDA(cudaEventSynchronize(c->stage_ev[0]));  // it may still feed a host-to-device copy
+  char* p = static_cast<char*>(c->stage[0]);
+  size_t off = 0;
+  for (const D2H& d : list) {
+    if (d.bytes) BIT_CUDA(cudaMemcpyAsync(p + off, d.src, d.bytes, cudaMemcpyDeviceToHost, s));
+    off += (d.bytes + 15) / 16 * 16;
+  }
+  BIT_CUDA(cudaStreamSynchronize(s));
+  off = 0;
+  for (const D2H& d : list) {
+    std::memcpy(d.dst, p + off, d.bytes);
+    off += (d.bytes + 15) / 16 * 16;
+  }
+}
+
 }  // namespace bit

@@ -463,7 +463,7 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
   BIT_CUDA(cudaMemcpyAsync(L->items.p, L->h_items.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
   BIT_CUDA(cudaMemcpyAsync(L->part_off.p, off.data(), ng * sizeof(long long), cudaMemcpyHostToDevice, s));
   BIT_CUDA(cudaMemsetAsync(L->part_done.p, 0, ng * sizeof(int), s));
-  BIT_CUDA(cudaStreamSynchronize(s));
+  BIT_CUDA(cudaStreamSynchronize(s));  // the host arrays are done with
 }
 
 void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const double* tx,
@@ -588,6 +588,12 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   std::vector<int> hf(ng), hn(ng);
   std::vector<unsigned long long> hp(ng);
+  auto read_back = [&] {
+    copy_d2h_batch(c, {{h, cnt.p, 8 * sizeof(unsigned long long)},
+                       {hf.data(), L->far_cnt.p, ng * sizeof(int)},
+                       {hn.data(), L->near_cnt.p, ng * sizeof(int)},
+                       {hp.data(), L->g_near.p, ng * sizeof(unsigned long long)}});
+  };
   int err = 2;  // no single pass: straight to count, scan and fill
   if (staged) {
     L->gstage.ensure(c, stage_words);
@@ -598,11 +604,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     a.ngroups = ng;
     count_launch(), k_lists_queue<<<slots, LT, STACK_BYTES, s>>>(a);
     BIT_CHECK_LAUNCH();
-    BIT_CUDA(cudaMemcpyAsync(h, cnt.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hf.data(), L->far_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hn.data(), L->near_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hp.data(), L->g_near.p, ng * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaStreamSynchronize(s));
+    read_back();
     err = (int)(h[6] & 0xffffffffu);
     if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded (tree deeper than supported)");
   }
@@ -615,11 +617,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->far_cnt.p, L->g_tcount.p, L->far_moff.p, ng, cnt.p + 1);
     count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->near_cnt.p, nullptr, L->near_off.p, ng, cnt.p + 2);
     count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->near_cnt.p, L->g_tcount.p, L->near_moff.p, ng, cnt.p + 3);
-    BIT_CUDA(cudaMemcpyAsync(h, cnt.p, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hf.data(), L->far_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hn.data(), L->near_cnt.p, ng * sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hp.data(), L->g_near.p, ng * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaStreamSynchronize(s));
+    read_back();
     err = (int)(h[6] & 0xffffffffu);  // this pass walked every group to the end
     if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded");
     L->far_node.ensure(c, h[0]);
@@ -655,8 +653,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->h_work = wk;
   L->order.ensure(c, ng);
   BIT_CUDA(cudaMemcpyAsync(L->order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s));
-  near_items(L, c, hp, tc);
-  BIT_CUDA(cudaStreamSynchronize(s));
+  near_items(L, c, hp, tc);  // (synchronises)
   L->key = key;
   L->valid = true;
   L->version++;

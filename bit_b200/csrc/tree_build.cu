@@ -5,19 +5,32 @@
 // parent order, which is the reference's breadth-first numbering.  Inside a node the
 // reference runs a short sequential program of up to seven bisections (treedivide,
 // src/tree3d.cpp:1163-1304), each needing the member count and bounding box of both
-// halves of the slot it splits.  Here every node keeps the results of its completed
-// bisections; a one-thread "decide" step replays the program from the start on those
-// cached results until it reaches the first bisection it has no result for, and a
-// "pass" kernel over all members of the level's nodes computes that bisection's counts
-// and bounding boxes (block reduction + atomics; min/max are order independent, so the
-// result is exact).  The first decision of a level is a kernel of its own; each later one
-// is made inside the pass, by the CTA that finishes the node's last chunk.  Members carry a slot label; a final stable counting scatter
-// lays each node's children out contiguously in slot order, members in ascending
-// original index (the reference's member order).  Field arithmetic (midpoints, aspect
-// ratios, sqradius) is the reference's, with no FMA contraction.
+// halves of the slot it splits (min/max are order independent, so the result is exact).
+//
+// A node of at most kSmallNode members is one cluster's work (k_node_split: one, four or eight
+// CTAs by its size): the members stay in shared memory through the whole program, and go to
+// the children's ranges in one stable scatter, members in ascending original index (the
+// reference's member order).  The level's last CTA scans the child counts, k_make_children
+// appends the children and sorts out which of them are to be split, all from device-side
+// level records, so the host launches four levels at a time and then looks.
+//
+// Larger nodes (the first levels of a large tree) are split by all SMs: a pass over all their
+// members relabels by each node's last bisection and reduces counts and bounding boxes of the
+// next (block reduction + atomics), and the CTA that finishes a node's last chunk takes the
+// program's next step.  Members carry a slot label; a stable counting scatter follows.
+//
+// Field arithmetic (midpoints, aspect ratios, sqradius) is the reference's, with no FMA
+// contraction.
+//
+// Bound by launches and latency.  With the passes for every node (18 launches and a round trip
+// a level), before / now: 10k uniform in leaves of 200 700 / 220 us, 100k clustered in leaves
+// of 500 1,757 / 780, 2M in leaves of 1000 4,200 / 2,900; with one CTA up to 16,384 members
+// that read them from L2 at every bisection: 320, 1,190, 4,030.
 #include <algorithm>
 #include <climits>
 #include <cstring>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 
@@ -25,8 +38,21 @@ namespace bit {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int CH = 2048;  // members per chunk (one block)
 constexpr int TB = 256;   // threads per block
+// Nodes that a cluster of CTAs splits with its members in shared memory, by size: one CTA of
+// up to 3,584 members (two such CTAs an SM), four of those, eight of 7,168.  Larger nodes take
+// all SMs.
+constexpr int kClasses = 3;
+constexpr int kClassCtas[kClasses] = {1, 4, 8};
+constexpr int kClassRows[kClasses] = {7, 7, 14};  // members of a thread
+constexpr int ST = 512;                           // threads of a CTA
+__host__ __device__ constexpr int class_members(int c) {
+  return (c == 0 ? 1 : c == 1 ? 4 : 8) * (c == 2 ? 14 : 7) * ST;
+}
+constexpr int kSmallNode = class_members(kClasses - 1);
 static_assert(CH % TB == 0, "a chunk is a whole number of block strides");
 
 __device__ __forceinline__ unsigned long long okey(double v) {
@@ -53,19 +79,121 @@ __device__ void box_fields(double* f, double x0, double x1, double y0, double y1
   f[12] = dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
 }
 
-struct Divide {
-  int dir, src, c1, c2;  // src -1: the node itself
-  double mid;
+// What a split leaves for k_make_children: the child slots and the order of children[].
+struct NodeOut {
+  int nchild;
+  int order[8], slot_n[8];
+  double slot_f[8][13];
 };
 
+// One level of the tree, on the device (a ring of kLevels records).
+constexpr int kLevels = 8;
+struct Level {
+  int a, b;            // its nodes
+  int nact;            // nodes to split, numbered in no particular order
+  int nsmall[kClasses], nbig;  // of those, by class
+  int arrive;          // CTAs of the level's last k_node_split that are done
+};
+struct Ctl {
+  Level lv[kLevels];
+  int cur;             // the first level whose children have not been made
+  int stop;            // the node arrays are full: nothing runs until they have grown
+  int err;             // 1 NaN, 2 a node that cannot be split, 4 / 8 consistency checks
+};
+
+// treemake's per-node program (src/tree3d.cpp:1412-1545), resumable at its bisections: slots
+// are relative to the first free node index, order[] receives the children in recorded order.
+struct Program {
+  int pc, j, k, xc, yc, ind2, nchild, nchild2;
+  int dir, src, c1, c2;  // the bisection to do: slot src (-1: the node) into c1 and c2
+  int n[8], order[8];    // the slots' members
+};
+
+__device__ __forceinline__ void program_init(Program& g) {
+  g.pc = g.nchild = g.nchild2 = 0;
+  for (int s = 0; s < 8; s++) g.n[s] = 0;
+}
+
+// Go on after the bisection in hand, which made `made` non-empty halves (the first call: none
+// in hand); P: the node's box, f: the slots' boxes.  True: the next bisection is in hand;
+// false: the program is done.
+__device__ bool program_next(Program& g, const double* P, const double (*f)[13], int made, double lim,
+                             int maxmemb) {
+  auto zsplit = [&](int s) { return f[s][10] < lim && f[s][11] < lim && g.n[s] > maxmemb; };
+  auto bisect = [&](int pc, int dir, int src, int c1, int c2) {
+    g.pc = pc; g.dir = dir; g.src = src; g.c1 = c1; g.c2 = c2;
+    return true;
+  };
+  auto second = [&] {  // a second half is a child of its own
+    if (made == 2) g.order[g.nchild++] = g.ind2++;
+    return made == 2;
+  };
+  bool in_k = false;
+  switch (g.pc) {
+    case 0:
+      if (P[9] > lim && P[10] > lim) return bisect(1, 0, -1, 0, 1);
+      if (P[9] < lim && P[11] > lim) return bisect(5, 1, -1, 0, 1);
+      return bisect(7, 2, -1, 0, 1);
+    case 1:  // x done
+    case 5:  // y done, no x
+      g.xc = g.ind2 = made;
+      g.j = 0;
+      break;
+    case 2:  // y of slot j done
+      g.yc = made;
+      second();
+      g.k = 0;
+      in_k = true;
+      break;
+    case 3:  // z of slot t done
+      if (second()) g.nchild2++;
+      g.k++;
+      in_k = true;
+      break;
+    case 4:  // z of slot j done, no y
+    case 6:
+      second();
+      g.j++;
+      break;
+    default:  // z only
+      for (int j = 0; j < made; j++) g.order[g.nchild++] = j;
+      return false;
+  }
+  if (g.pc >= 5) {
+    for (; g.j < g.xc; g.j++) {
+      g.order[g.nchild++] = g.j;
+      if (zsplit(g.j)) return bisect(6, 2, g.j, g.j, g.ind2);
+    }
+    return false;
+  }
+  for (;;) {
+    if (in_k) {
+      for (; g.k < g.yc; g.k++) {
+        // the reference's numtree+j+k*(nchild2+1) (src/tree3d.cpp:1460), as written
+        const int t = g.j + g.k * (g.nchild2 + 1);
+        if (t >= 8 || t >= g.ind2) continue;  // never-created slot: nummemb == 0
+        if (zsplit(t)) return bisect(3, 2, t, t, g.ind2);
+      }
+      in_k = false;
+      g.j++;
+    }
+    if (g.j >= g.xc) return false;
+    g.order[g.nchild++] = g.j;
+    if (f[g.j][9] < lim && f[g.j][11] > lim && g.n[g.j] > maxmemb) return bisect(2, 1, g.j, g.j, g.ind2);
+    if (zsplit(g.j)) return bisect(4, 2, g.j, g.j, g.ind2);
+    g.j++;
+  }
+}
+
+// A large node's split: its program, and the bisections its next pass relabels by and reduces.
+struct Divide {
+  int dir, src, c1, c2;
+  double mid;
+};
 struct SplitState {
-  int active, finished, ndone, has_cur, has_prev, nchild, prev_c2eff, pad;
-  Divide cur, prev;
-  int res_cnt[7][2];
-  double res_bb[7][2][6];
-  int order[8];
-  int slot_n[8];
-  double slot_f[8][13];
+  Program g;
+  int has_cur, has_prev;
+  Divide cur, prev;  // prev.c2: where the second half went
 };
 
 struct SplitAcc {
@@ -78,96 +206,6 @@ __device__ void acc_reset(SplitAcc* a) {
     a->cnt[h] = 0;
     for (int d = 0; d < 3; d++) { a->mn[h][d] = ~0ULL; a->mx[h][d] = 0ULL; }
   }
-}
-
-// Replay of the split program on cached bisection results.
-struct Replay {
-  SplitState* S;
-  const double* pf;
-  int maxmemb;
-  double lim;
-  int d;
-  bool need;
-  int n[8];
-  double f[8][13];
-};
-
-__device__ int rp_bisect(Replay& r, int dir, int src, int c1, int c2) {
-  if (r.need) return 0;
-  const double* f = src < 0 ? r.pf : r.f[src];
-  if (r.d >= r.S->ndone) {
-    r.S->cur.dir = dir; r.S->cur.src = src; r.S->cur.c1 = c1; r.S->cur.c2 = c2;
-    r.S->cur.mid = f[6 + dir];
-    r.need = true;
-    return 0;
-  }
-  const int* cnt = r.S->res_cnt[r.d];
-  int dst[2] = {c1, cnt[0] > 0 ? c2 : c1};
-  int made = 0;
-  for (int h = 0; h < 2; h++) {
-    if (!cnt[h]) continue;
-    const double* bb = r.S->res_bb[r.d][h];
-    r.n[dst[h]] = cnt[h];
-    box_fields(r.f[dst[h]], bb[0], bb[1], bb[2], bb[3], bb[4], bb[5]);
-    made++;
-  }
-  r.d++;
-  return made;
-}
-
-__device__ __forceinline__ bool zsplit_ok(const Replay& r, int s) {
-  return r.f[s][10] < r.lim && r.f[s][11] < r.lim && r.n[s] > r.maxmemb;
-}
-
-// treemake's per-node program (src/tree3d.cpp:1412-1545) on slots relative to the first
-// free node index.  Returns nchild; order[] receives the children in recorded order.
-__device__ int split_program(Replay& r, int* order) {
-  const double lim = r.lim;
-  const double* P = r.pf;
-  int nchild = 0, nchild2 = 0, ind2;
-  for (int s = 0; s < 8; s++) r.n[s] = 0;
-  if (P[9] > lim && P[10] > lim) {
-    int xc = rp_bisect(r, 0, -1, 0, 1);
-    ind2 = xc;
-    for (int j = 0; j < xc; j++) {
-      order[nchild++] = j;
-      if (r.f[j][9] < lim && r.f[j][11] > lim && r.n[j] > r.maxmemb) {
-        int yc = rp_bisect(r, 1, j, j, ind2);
-        if (yc == 2) { order[nchild++] = ind2; ind2++; }
-        for (int k = 0; k < yc; k++) {
-          // the reference's numtree+j+k*(nchild2+1) (src/tree3d.cpp:1460), as written
-          int t = j + k * (nchild2 + 1);
-          if (t >= 8 || t >= ind2) continue;  // never-created slot: nummemb == 0
-          if (zsplit_ok(r, t)) {
-            int zc = rp_bisect(r, 2, t, t, ind2);
-            if (zc == 2) { order[nchild++] = ind2; nchild2++; ind2++; }
-          }
-        }
-      } else if (zsplit_ok(r, j)) {
-        int zc = rp_bisect(r, 2, j, j, ind2);
-        if (zc == 2) { order[nchild++] = ind2; ind2++; }
-      }
-    }
-  } else if (P[9] < lim && P[11] > lim) {
-    int yc = rp_bisect(r, 1, -1, 0, 1);
-    ind2 = yc;
-    for (int j = 0; j < yc; j++) {
-      order[nchild++] = j;
-      if (zsplit_ok(r, j)) {
-        int zc = rp_bisect(r, 2, j, j, ind2);
-        if (zc == 2) { order[nchild++] = ind2; ind2++; }
-      }
-    }
-  } else {
-    int zc = rp_bisect(r, 2, -1, 0, 1);
-    for (int j = 0; j < zc; j++) order[nchild++] = j;
-  }
-  return nchild;
-}
-
-__global__ void k_iota(int* p, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = i;
 }
 
 template <class T>
@@ -185,16 +223,20 @@ __device__ __forceinline__ int warp_sum(int v) {
   return v;
 }
 
-// Bounding box of each system's particles (its root, src/tree3d.cpp:1385-1403); flags
-// NaNs.  grid.y = system, grid.x = blocks striding over that system.
+// The particles into tree order (the identity, to begin with) and the bounding box of each
+// system's (its root, src/tree3d.cpp:1385-1403); flags NaNs.  grid.y = system, grid.x =
+// blocks striding over that system.
 __global__ void k_root_bbox(const int* sys_start, const int* sys_n, const double* x,
-                            const double* y, const double* z, SplitAcc* acc, int* err) {
+                            const double* y, const double* z, int* perm, double* sx, double* sy_,
+                            double* sz, SplitAcc* acc, Ctl* ctl) {
   const int sy = blockIdx.y;
   const int i0 = sys_start[sy], i1 = i0 + sys_n[sy];
   unsigned long long mn[3] = {~0ULL, ~0ULL, ~0ULL}, mx[3] = {0, 0, 0};
   int bad = 0;
   for (int i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < i1; i += gridDim.x * blockDim.x) {
     double v[3] = {x[i], y[i], z[i]};
+    perm[i] = i;
+    sx[i] = v[0]; sy_[i] = v[1]; sz[i] = v[2];
     for (int d = 0; d < 3; d++) {
       if (isnan(v[d])) bad = 1;
       unsigned long long k = okey(v[d]);
@@ -212,7 +254,7 @@ __global__ void k_root_bbox(const int* sys_start, const int* sys_n, const double
       atomicMin(&acc[sy].mn[0][d], mn[d]);
       atomicMax(&acc[sy].mx[0][d], mx[d]);
     }
-    if (bad) atomicOr(err, 1);
+    if (bad) atomicOr(&ctl->err, 1);
   }
 }
 
@@ -221,9 +263,33 @@ __global__ void k_acc_reset(SplitAcc* acc, int n) {
   if (i < n) acc_reset(&acc[i]);
 }
 
-__global__ void k_root_init(int nsys, const int* sys_start, const int* sys_n, const SplitAcc* acc,
-                            int* nummemb, int* start, int* children, int* level, int* parent,
-                            double* fields, int* node_sys) {
+// The lists of the nodes to split, by level parity.
+struct Lists2 {
+  int* small[kClasses][2];
+  int* big[2];
+};
+
+// Node `node` of level lev (its record L) joins the list it belongs to; act: its number among
+// the nodes to split, or -1.
+__device__ __forceinline__ void enlist(int node, int cnt, int maxmemb, Level* L, int lev,
+                                       const Lists2& ls, int* act, int* nch) {
+  nch[node] = 0;
+  if (cnt <= maxmemb) {
+    act[node] = -1;
+    return;
+  }
+  act[node] = atomicAdd(&L->nact, 1);
+  if (cnt > kSmallNode) {
+    ls.big[lev & 1][atomicAdd(&L->nbig, 1)] = node;
+    return;
+  }
+  const int c = cnt <= class_members(0) ? 0 : cnt <= class_members(1) ? 1 : 2;
+  ls.small[c][lev & 1][atomicAdd(&L->nsmall[c], 1)] = node;
+}
+
+__global__ void k_root_init(int nsys, const int* sys_start, const int* sys_n, const int* sys_maxmemb,
+                            const SplitAcc* acc, int* nummemb, int* start, int* children,
+                            double* fields, int* node_sys, Ctl* ctl, Lists2 ls, int* act, int* nch) {
   const int sy = blockIdx.x * blockDim.x + threadIdx.x;
   if (sy >= nsys) return;
   double f[13];
@@ -231,24 +297,379 @@ __global__ void k_root_init(int nsys, const int* sys_start, const int* sys_n, co
   box_fields(f, okey_inv(A->mn[0][0]), okey_inv(A->mx[0][0]), okey_inv(A->mn[0][1]),
              okey_inv(A->mx[0][1]), okey_inv(A->mn[0][2]), okey_inv(A->mx[0][2]));
   for (int k = 0; k < 13; k++) fields[13LL * sy + k] = f[k];
-  nummemb[sy] = sys_n[sy]; start[sy] = sys_start[sy]; level[sy] = 0; parent[sy] = -1;
+  nummemb[sy] = sys_n[sy]; start[sy] = sys_start[sy];
   node_sys[sy] = sy;
   for (int c = 0; c < 8; c++) children[8LL * sy + c] = -1;
+  if (sy == 0) ctl->lv[0].b = nsys;
+  enlist(sy, sys_n[sy], sys_maxmemb[sy], &ctl->lv[0], 0, ls, act, nch);
 }
 
-// Per level node: active flag and the number of member chunks it needs.
-__global__ void k_level_init(int a, int nlev, const int* nummemb, const int* node_sys,
-                             const int* sys_maxmemb, SplitState* st, SplitAcc* acc, int* nchunk,
-                             int* done) {
+struct Arrays {
+  int *nummemb, *start, *children, *node_sys, *act, *nch, *cscan;
+  double* fields;
+  int* perm;
+  double *sx, *sy, *sz;
+  int* perm2;
+  double *sx2, *sy2, *sz2;
+  const int* sys_maxmemb;
+  NodeOut* out;
+  Ctl* ctl;
+  Lists2 ls;
+  double lim;
+  int cap;
+};
+
+// ---- nodes of up to kSmallNode members ------------------------------------------------------
+constexpr int SW = ST / 32;  // warps of a CTA
+
+struct NodeShared {
+  Program g;
+  double pf[13], f[8][13];      // the node's box, the slots'
+  double red[SW][14];           // per warp: min / max of x, y, z and the count, of both halves
+  double part[2][14], all[14];  // the CTA's (by parity of the bisection), the node's
+  int wcnt[SW][8], tot[8];      // members of each slot, per warp and in the CTA
+  int made;
+};
+
+// Value v = 7 h + q of a bisection: q = 2 d the smallest, 2 d + 1 the largest coordinate of
+// axis d in half h, 6 the count.
+__device__ __forceinline__ double combine(int v, double a, double b) {
+  const int q = v % 7;
+  return q == 6 ? a + b : ((q & 1) ? (b > a ? b : a) : (b < a ? b : a));
+}
+
+// Split every node of class C at level lev: a cluster of CTAs holds a node's members in shared
+// memory, each thread its own (a warp a contiguous run), with the slot labels in nibbles of a
+// register.  A bisection is a pass over the thread's members, a reduction over the warp, the
+// CTA and (through distributed shared memory) the cluster, and one thread's step of the
+// program, which every CTA takes for itself.  The members then go to the children's ranges in
+// order, in place: all of them were read before any is written.  The level's last CTA (of the
+// launch with `last`) scans the child counts.
+template <int C>
+__global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) {
+  constexpr int CS = kClassCtas[C], ROWS = kClassRows[C];
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ NodeShared N;
+  __shared__ int s_last;
+  double* xs = reinterpret_cast<double*>(sm);
+  double* ys = xs + ROWS * ST;
+  double* zs = ys + ROWS * ST;
+  int* ps = reinterpret_cast<int*>(zs + ROWS * ST);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = CS > 1 ? (int)cluster.block_rank() : 0;
+  Ctl* ctl = A.ctl;
+  if (ctl->stop) return;
+  Level* lv = &ctl->lv[lev % kLevels];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const double inf = __longlong_as_double(0x7ff0000000000000LL);
+  const int count = lv->nsmall[C];  // (not ctl->err: a cluster's CTAs have to agree)
+  int par = 0;
+  for (int k = blockIdx.x / CS; k < count; k += gridDim.x / CS) {
+    const int node = A.ls.small[C][lev & 1][k];
+    const int s0 = A.start[node], cnt = A.nummemb[node], maxmemb = A.sys_maxmemb[A.node_sys[node]];
+    if (tid < 13) N.pf[tid] = A.fields[13LL * node + tid];
+    if (tid == 0) program_init(N.g);
+    // this CTA's members, this warp's run of them
+    const int per = (cnt + CS - 1) / CS;
+    const int c0 = min(rank * per, cnt), c1 = min(c0 + per, cnt);
+    const int run = (c1 - c0 + ST - 1) / ST * 32;
+    const int r0 = min(c0 + w * run, c1), r1 = min(r0 + run, c1), rows = run / 32;
+    for (int i = 0; i < rows; i++) {
+      const int e = r0 + 32 * i + lane;
+      if (e < r1) {
+        ps[i * ST + tid] = A.perm[s0 + e];
+        // + 0.0: a -0.0 enters the boxes as +0.0, as the large nodes' ordered keys have it
+        xs[i * ST + tid] = A.sx[s0 + e];
+        ys[i * ST + tid] = A.sy[s0 + e];
+        zs[i * ST + tid] = A.sz[s0 + e];
+      }
+    }
+    unsigned long long lab = ~0ULL;  // 15: the node itself
+    __syncthreads();
+    if (tid == 0) N.made = program_next(N.g, N.pf, N.f, 0, A.lim, maxmemb) ? 0 : -1;
+    __syncthreads();
+    while (N.made >= 0) {
+      const int dir = N.g.dir, src = N.g.src;
+      const double mid = (src < 0 ? N.pf : N.f[src])[6 + dir];
+      const unsigned want = src < 0 ? 15u : (unsigned)src;
+      double v[14];
+#pragma unroll
+      for (int q = 0; q < 14; q++) v[q] = q % 7 == 6 ? 0.0 : ((q % 7) & 1 ? -inf : inf);
+      int n0 = 0, n1 = 0;
+      unsigned up = 0;
+      const double* cs = dir == 0 ? xs : (dir == 1 ? ys : zs);
+      for (int i = 0; i < rows; i++) {
+        if (r0 + 32 * i + lane >= r1 || ((unsigned)(lab >> (4 * i)) & 15u) != want) continue;
+        const int o = i * ST + tid;
+        const double x = xs[o] + 0.0, y = ys[o] + 0.0, z = zs[o] + 0.0;
+        if (cs[o] <= mid) {
+          n0++;
+          v[0] = x < v[0] ? x : v[0]; v[1] = x > v[1] ? x : v[1];
+          v[2] = y < v[2] ? y : v[2]; v[3] = y > v[3] ? y : v[3];
+          v[4] = z < v[4] ? z : v[4]; v[5] = z > v[5] ? z : v[5];
+        } else {
+          up |= 1u << i;
+          n1++;
+          v[7] = x < v[7] ? x : v[7]; v[8] = x > v[8] ? x : v[8];
+          v[9] = y < v[9] ? y : v[9]; v[10] = y > v[10] ? y : v[10];
+          v[11] = z < v[11] ? z : v[11]; v[12] = z > v[12] ? z : v[12];
+        }
+      }
+      n0 = __reduce_add_sync(0xffffffffu, n0);
+      n1 = __reduce_add_sync(0xffffffffu, n1);
+      if (n0)  // (the whole warp)
+#pragma unroll
+        for (int q = 0; q < 6; q++)
+#pragma unroll
+          for (int o = 16; o; o >>= 1) v[q] = combine(q, v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+      if (n1)
+#pragma unroll
+        for (int q = 7; q < 13; q++)
+#pragma unroll
+          for (int o = 16; o; o >>= 1) v[q] = combine(q, v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+      v[6] = n0;
+      v[13] = n1;
+      if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < 14; q++) N.red[w][q] = v[q];
+      __syncthreads();
+      if (w < 14) {  // warp q: value q over the CTA's warps
+        double x = N.red[lane & (SW - 1)][w];
+#pragma unroll
+        for (int o = SW / 2; o; o >>= 1) x = combine(w, x, __shfl_xor_sync(0xffffffffu, x, o));
+        if (lane == 0) (CS > 1 ? N.part[par] : N.all)[w] = x;
+      }
+      if constexpr (CS > 1) {
+        cluster.sync();
+        if (w < 14) {
+          double x = cluster.map_shared_rank(&N.part[par][0], lane & (CS - 1))[w];
+#pragma unroll
+          for (int o = CS / 2; o; o >>= 1) x = combine(w, x, __shfl_xor_sync(0xffffffffu, x, o));
+          if (lane == 0) N.all[w] = x;
+        }
+        par ^= 1;  // (a CTA past the next barrier has read these values)
+      }
+      __syncthreads();
+      const bool any0 = N.all[6] > 0.0, any1 = N.all[13] > 0.0;
+      const int d0 = N.g.c1, d1 = any0 ? N.g.c2 : N.g.c1;
+      __syncthreads();  // every thread has read the bisection in hand
+      if (lane == 0 && w < 2 && (w ? any1 : any0)) {  // a half's fields, one warp each
+        const double* bb = &N.all[7 * w];
+        box_fields(N.f[w ? d1 : d0], bb[0], bb[1], bb[2], bb[3], bb[4], bb[5]);
+        N.g.n[w ? d1 : d0] = (int)bb[6];
+      }
+      for (int i = 0; i < rows; i++)
+        if (((unsigned)(lab >> (4 * i)) & 15u) == want)
+          lab = (lab & ~(15ULL << (4 * i))) | ((unsigned long long)((up >> i) & 1u ? d1 : d0) << (4 * i));
+      __syncthreads();
+      if (tid == 0) {
+        const int made = (int)any0 + (int)any1;
+        N.made = program_next(N.g, N.pf, N.f, made, A.lim, maxmemb) ? made : -1;
+      }
+      __syncthreads();
+    }
+    const int nchild = N.g.nchild;
+    if (nchild < 2) {  // one child == the node itself: never terminates
+      if (tid == 0) atomicOr(&ctl->err, 2);
+      if (CS > 1) cluster.sync();
+      else __syncthreads();
+      continue;
+    }
+    // stable scatter: members of each slot per warp and CTA, then every member's place
+    unsigned mine = 0;  // lane s: this warp's members of slot s
+    for (int i = 0; i < rows; i++) {
+      const unsigned l = r0 + 32 * i + lane < r1 ? (unsigned)(lab >> (4 * i)) & 15u : 15u;
+      for (int s = 0; s < nchild; s++) {
+        const unsigned m = __ballot_sync(0xffffffffu, l == (unsigned)s);
+        if (lane == s) mine += __popc(m);
+      }
+    }
+    if (lane < 8) N.wcnt[w][lane] = lane < nchild ? mine : 0;
+    __syncthreads();
+    if (tid < 8) {
+      int t = 0;
+      for (int q = 0; q < SW; q++) t += N.wcnt[q][tid];
+      N.tot[tid] = t;
+    }
+    if (CS > 1) cluster.sync();  // (and every CTA of the cluster holds its members)
+    else __syncthreads();
+    int next = s0;  // lane s: where this warp's next member of slot s goes
+    if (lane < nchild) {
+      for (int s = 0; s < lane; s++) next += N.g.n[s];
+      if constexpr (CS > 1)
+        for (int r = 0; r < rank; r++) next += cluster.map_shared_rank(&N.tot[0], r)[lane];
+      for (int q = 0; q < w; q++) next += N.wcnt[q][lane];
+    }
+    for (int i = 0; i < rows; i++) {
+      const bool in = r0 + 32 * i + lane < r1;
+      const unsigned l = in ? (unsigned)(lab >> (4 * i)) & 15u : 15u;
+      int dst = __shfl_sync(0xffffffffu, next, l & 7);
+      for (int s = 0; s < nchild; s++) {
+        const unsigned m = __ballot_sync(0xffffffffu, l == (unsigned)s);
+        if (l == (unsigned)s) dst += __popc(m & lt);
+        if (lane == s) next += __popc(m);
+      }
+      if (in) {
+        const int o = i * ST + tid;
+        A.perm[dst] = ps[o]; A.sx[dst] = xs[o]; A.sy[dst] = ys[o]; A.sz[dst] = zs[o];
+      }
+    }
+    if (rank == 0) {
+      NodeOut* O = &A.out[A.act[node]];
+      if (tid < 13 * nchild) (&O->slot_f[0][0])[tid] = (&N.f[0][0])[tid];
+      if (tid < 8) {
+        O->slot_n[tid] = tid < nchild ? N.g.n[tid] : 0;
+        O->order[tid] = tid < nchild ? N.g.order[tid] : -1;
+      }
+      if (tid == 0) {
+        O->nchild = nchild;
+        A.nch[node] = nchild;
+      }
+    }
+    if (CS > 1) cluster.sync();  // the cluster's reads of each other's counts are done
+    else __syncthreads();
+  }
+  if (!last) return;
+  // the level's last CTA: where each node's children begin
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&lv->arrive, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int a = lv->a, b = lv->b;
+  int* ws = &N.wcnt[0][0];
+  int carry = b;
+  for (int base = a; base < b; base += ST) {
+    const int i = base + tid;
+    const int v = i < b ? __ldcg(A.nch + i) : 0;
+    int s = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    if (lane == 31) ws[w] = s;
+    __syncthreads();
+    int before = carry, all = 0;
+    for (int q = 0; q < SW; q++) {
+      if (q < w) before += ws[q];
+      all += ws[q];
+    }
+    if (i < b) A.cscan[i] = before + s - v;
+    carry += all;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    Level* nx = &ctl->lv[(lev + 1) % kLevels];
+    nx->a = b;
+    nx->b = __ldcg(&ctl->err) ? b : carry;  // (another CTA may have set it)
+    Level z{};
+    ctl->lv[(lev + 2) % kLevels] = z;
+  }
+}
+
+// The class's members in shared memory.
+template <int C>
+constexpr size_t split_smem() { return (size_t)kClassRows[C] * ST * (3 * sizeof(double) + sizeof(int)); }
+
+// `nodes`: at most that many nodes of the class.
+template <int C>
+void launch_split(const Ctx* c, const Arrays& A, int lev, int last, long long nodes, cudaStream_t s) {
+  ensure_smem_attr(reinterpret_cast<const void*>(k_node_split<C>), (int)split_smem<C>());
+  const int per_sm = C == 2 ? 1 : 2;
+  const long long fit = std::max(1, c->num_sms * per_sm / kClassCtas[C]);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(std::max(1LL, std::min(nodes, fit)) * kClassCtas[C]));
+  cfg.blockDim = dim3(ST);
+  cfg.dynamicSmemBytes = split_smem<C>();
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kClassCtas[C];
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  count_launch();
+  BIT_CUDA(cudaLaunchKernelEx(&cfg, k_node_split<C>, A, lev, last));
+}
+
+// The children of level lev's nodes, one warp per node: their records, and the lists of the
+// next level's nodes to split.
+__global__ void __launch_bounds__(256) k_make_children(Arrays A, int lev) {
+  Ctl* ctl = A.ctl;
+  if (ctl->stop || ctl->err) return;
+  const Level* lv = &ctl->lv[lev % kLevels];
+  Level* nx = &ctl->lv[(lev + 1) % kLevels];
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  const int lane = threadIdx.x & 31;
+  const int a = lv->a, b = lv->b;
+  if (a == b) return;  // past the last level
+  if (nx->b > A.cap) {
+    if (first) ctl->stop = 1;  // (read by the kernels that follow this one)
+    return;
+  }
+  for (int p = a + (blockIdx.x * blockDim.x + threadIdx.x) / 32; p < b; p += gridDim.x * blockDim.x / 32) {
+    if (A.act[p] < 0) continue;
+    const NodeOut* O = &A.out[A.act[p]];
+    const int nchild = O->nchild, base = A.cscan[p], sys = A.node_sys[p];
+    const int n = lane < 8 ? O->slot_n[lane] : 0;
+    int off = n;
+    for (int o = 1; o < 8; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, off, o);
+      if (lane >= o) off += t;
+    }
+    off -= n;
+    for (int i = lane; i < 13 * nchild; i += 32) A.fields[13LL * base + i] = (&O->slot_f[0][0])[i];
+    for (int i = lane; i < 8 * nchild; i += 32) A.children[8LL * base + i] = -1;
+    if (lane < 8) A.children[8LL * p + lane] = lane < nchild ? base + O->order[lane] : -1;
+    if (lane < nchild) {
+      const int node = base + lane;
+      A.nummemb[node] = n;
+      A.start[node] = A.start[p] + off;
+      A.node_sys[node] = sys;
+      enlist(node, n, A.sys_maxmemb[sys], nx, lev + 1, A.ls, A.act, A.nch);
+    }
+  }
+  if (first) ctl->cur = lev + 1;
+}
+
+// ---- nodes of more members: all SMs ---------------------------------------------------------
+// The large node's next bisection, or, its program done, what k_make_children needs.
+__device__ void plan_divide(const Arrays& A, int node, SplitState* S, int made) {
+  NodeOut* O = &A.out[A.act[node]];
+  const double* P = A.fields + 13LL * node;
+  S->has_cur = program_next(S->g, P, O->slot_f, made, A.lim, A.sys_maxmemb[A.node_sys[node]]);
+  if (S->has_cur) {
+    const Program& g = S->g;
+    S->cur.dir = g.dir; S->cur.src = g.src; S->cur.c1 = g.c1; S->cur.c2 = g.c2;
+    S->cur.mid = (g.src < 0 ? P : O->slot_f[g.src])[6 + g.dir];
+    return;
+  }
+  if (S->g.nchild < 2) {  // one child == the node itself: never terminates
+    atomicOr(&A.ctl->err, 2);
+    S->g.nchild = 0;
+  }
+  O->nchild = S->g.nchild;
+  A.nch[node] = S->g.nchild;
+  for (int c = 0; c < 8; c++) {
+    O->order[c] = c < S->g.nchild ? S->g.order[c] : -1;
+    O->slot_n[c] = c < S->g.nchild ? S->g.n[c] : 0;
+  }
+}
+
+// The large nodes of the level (list), numbered li = 0 .. nbig - 1.
+__global__ void k_big_init(Arrays A, int nbig, const int* list, SplitState* st, SplitAcc* acc, int* nchunk,
+                           int* done) {
   int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nlev) return;
-  SplitState* S = &st[li];
-  int cnt = nummemb[a + li];
-  S->active = cnt > sys_maxmemb[node_sys[a + li]];
-  S->finished = 0; S->ndone = 0; S->has_cur = 0; S->has_prev = 0; S->nchild = 0;
+  if (li >= nbig) return;
   acc_reset(&acc[li]);
-  nchunk[li] = S->active ? (cnt + CH - 1) / CH : 0;
+  nchunk[li] = (A.nummemb[list[li]] + CH - 1) / CH;
   done[li] = 0;
+  SplitState* S = &st[li];
+  program_init(S->g);
+  S->has_prev = 0;
+  plan_divide(A, list[li], S, 0);
 }
 
 // Exclusive scan of a small int array in one block; total in out[n].
@@ -286,70 +707,10 @@ __global__ void k_scan_small(const int* in, int* out, int n) {
   if (threadIdx.x == 0) out[n] = carry;
 }
 
-__global__ void k_fill_chunks(int a, int nlev, const int* start, const int* nummemb,
-                              const int* cbeg, int2* chunks) {
-  int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nlev) return;
-  int s = start[a + li];
-  for (int c = cbeg[li]; c < cbeg[li + 1]; c++) chunks[c] = make_int2(li, s + (c - cbeg[li]) * CH);
-}
-
-// Record the bisection step just reduced for node a + li and plan its next one.
-__device__ __noinline__ void decide_node(int a, int li, const double* fields, const int* node_sys,
-                                         const int* sys_maxmemb, SplitState* st, SplitAcc* acc,
-                                         double lim, int* err) {
-  SplitState* S = &st[li];
-  if (!S->active) return;
-  SplitAcc* A = &acc[li];
-  if (S->has_cur) {
-    // The sums arrived as atomics in L2 from other CTAs of this launch (when the decision
-    // is made inside k_split_pass); __ldcg reads them there, never from a line this SM's
-    // L1 may hold from a neighbouring node's decision.
-    int d = S->ndone;
-    for (int h = 0; h < 2; h++) {
-      S->res_cnt[d][h] = __ldcg(&A->cnt[h]);
-      for (int q = 0; q < 3; q++) {
-        S->res_bb[d][h][2 * q] = okey_inv(__ldcg(&A->mn[h][q]));
-        S->res_bb[d][h][2 * q + 1] = okey_inv(__ldcg(&A->mx[h][q]));
-      }
-    }
-    S->ndone = d + 1;
-    S->prev = S->cur;
-    S->prev_c2eff = S->res_cnt[d][0] > 0 ? S->cur.c2 : S->cur.c1;
-    S->has_prev = 1;
-    S->has_cur = 0;
-    acc_reset(A);
-  } else {
-    S->has_prev = 0;
-  }
-  if (S->finished) return;
-  Replay r;
-  r.S = S; r.pf = fields + 13 * (long long)(a + li); r.lim = lim;
-  r.maxmemb = sys_maxmemb[node_sys[a + li]];
-  r.d = 0; r.need = false;
-  int order[8];
-  int nchild = split_program(r, order);
-  if (r.need) {
-    S->has_cur = 1;
-    if (S->ndone >= 7) atomicOr(err, 4);  // cannot happen: at most 7 bisections per node
-    return;
-  }
-  S->finished = 1;
-  S->nchild = nchild;
-  for (int c = 0; c < 8; c++) S->order[c] = c < nchild ? order[c] : -1;
-  for (int s = 0; s < 8; s++) {
-    S->slot_n[s] = s < nchild ? r.n[s] : 0;
-    if (s < nchild)
-      for (int k = 0; k < 13; k++) S->slot_f[s][k] = r.f[s][k];
-  }
-  if (nchild < 2) atomicOr(err, 2);  // one child == the node itself: never terminates
-}
-
-__global__ void k_split_decide(int a, int nlev, const double* fields, const int* node_sys,
-                               const int* sys_maxmemb, SplitState* st, SplitAcc* acc, double lim,
-                               int* err) {
-  int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li < nlev) decide_node(a, li, fields, node_sys, sys_maxmemb, st, acc, lim, err);
+__global__ void k_fill_chunks(int nbig, const int* list, const int* start, const int* cbeg, int2* chunks) {
+  const int li = blockIdx.x, s = start[list[li]];
+  for (int c = cbeg[li] + threadIdx.x; c < cbeg[li + 1]; c += blockDim.x)
+    chunks[c] = make_int2(li, s + (c - cbeg[li]) * CH);
 }
 
 __device__ __forceinline__ double coord(int dir, const double* sx, const double* sy,
@@ -357,39 +718,28 @@ __device__ __forceinline__ double coord(int dir, const double* sx, const double*
   return dir == 0 ? sx[e] : (dir == 1 ? sy[e] : sz[e]);
 }
 
-// Per-level inputs of the decision a split pass makes for each node when its last chunk
-// is done (decide = 0: the level's final pass, which only relabels).
-struct DecideArgs {
-  const int* nchunk;
-  int* done;
-  const double* fields;
-  const int* node_sys;
-  const int* sys_maxmemb;
-  double lim;
-  int* err;
-  int decide;
-};
-
-// One bisection step for every active node of the level: apply the previous step's
+// One bisection step for every large node of the level (decide = 0: the level's final pass,
+// which only relabels): apply the previous step's
 // relabel, then reduce counts / bounding boxes of both halves of the current step.  The
 // CTA that finishes a node's last chunk then makes the node's decision for the next step.
 // 6 CTAs per SM as without the decision (40 registers); whatever the call to decide_node
 // needs beyond that is spilled on the deciding thread's path only
-__global__ void __launch_bounds__(TB, 6) k_split_pass(const int2* chunks, const int* nch, int a, const int* start,
-                                                   const int* nummemb, const double* __restrict__ sx,
-                                                   const double* __restrict__ sy,
-                                                   const double* __restrict__ sz,
-                                                   signed char* __restrict__ lab, SplitState* st,
-                                                   SplitAcc* acc, DecideArgs da) {
+__global__ void __launch_bounds__(TB, 6)
+    k_split_pass(const __grid_constant__ Arrays A, const int2* chunks, const int* nch, const int* list,
+                 const int* nchunk, int* done, signed char* __restrict__ lab, SplitState* st, SplitAcc* acc,
+                 int decide) {
+  const double* __restrict__ sx = A.sx;
+  const double* __restrict__ sy = A.sy;
+  const double* __restrict__ sz = A.sz;
   if ((int)blockIdx.x >= *nch) return;  // the grid is sized from a bound
   const int2 ck = chunks[blockIdx.x];
   const SplitState* S = &st[ck.x];
   const int hp = S->has_prev, hc = S->has_cur;
   if (!hp && !hc) return;  // (its decision would change nothing)
   const Divide pv = S->prev, cu = S->cur;
-  const int pc2 = S->prev_c2eff;
-  const int node = a + ck.x;
-  const int e1 = min(ck.y + CH, start[node] + nummemb[node]);
+  const int pc2 = pv.c2;
+  const int node = list[ck.x];
+  const int e1 = min(ck.y + CH, A.start[node] + A.nummemb[node]);
   int cnt[2] = {0, 0};
   unsigned long long mn[2][3], mx[2][3];
   for (int h = 0; h < 2; h++)
@@ -460,27 +810,53 @@ __global__ void __launch_bounds__(TB, 6) k_split_pass(const int2* chunks, const 
       }
     }
   }
-  if (!da.decide) return;
-  // the CTA that completes the node's chunk count decides (its atomics, and every other
-  // chunk's, are visible after the fences)
+  if (!decide) return;
+  // The CTA that completes the node's chunk count (its atomics, and every other chunk's, are
+  // visible after the fences) records the bisection and plans the next.  The sums arrived as
+  // atomics in L2 from other CTAs; __ldcg reads them there.
   __shared__ int s_last;
   __threadfence();  // this thread's atomics, before the count that may complete the node
   __syncthreads();
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(&da.done[ck.x], 1) == da.nchunk[ck.x] - 1;
-    if (s_last) {
-      __threadfence();
-      decide_node(a, ck.x, da.fields, da.node_sys, da.sys_maxmemb, st, acc, da.lim, da.err);
-      da.done[ck.x] = 0;
+  if (threadIdx.x == 0) s_last = atomicAdd(&done[ck.x], 1) == nchunk[ck.x] - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  SplitState* D = &st[ck.x];
+  SplitAcc* R = &acc[ck.x];
+  if (hc) {
+    const int n0 = __ldcg(&R->cnt[0]), n1 = __ldcg(&R->cnt[1]);
+    const int c2 = n0 > 0 ? cu.c2 : cu.c1;
+    if (threadIdx.x % 32 == 0 && threadIdx.x < 64) {  // a half's fields, one warp each
+      const int h = threadIdx.x / 32, c = h ? c2 : cu.c1;
+      if (h ? n1 : n0) {
+        double bb[6];
+        for (int q = 0; q < 3; q++) {
+          bb[2 * q] = okey_inv(__ldcg(&R->mn[h][q]));
+          bb[2 * q + 1] = okey_inv(__ldcg(&R->mx[h][q]));
+        }
+        box_fields(A.out[A.act[node]].slot_f[c], bb[0], bb[1], bb[2], bb[3], bb[4], bb[5]);
+        D->g.n[c] = h ? n1 : n0;
+      }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      D->prev = cu;
+      D->prev.c2 = c2;
+      D->has_prev = 1;
+      acc_reset(R);
+      plan_divide(A, node, D, (n0 > 0) + (n1 > 0));
+    }
+  } else if (threadIdx.x == 0) {
+    D->has_prev = 0;  // (relabelled above; nothing is left to do)
   }
+  if (threadIdx.x == 0) done[ck.x] = 0;
 }
 
-__global__ void k_scatter_count(const int2* chunks, const int* nch, int a, const int* start, const int* nummemb,
+__global__ void k_scatter_count(const int2* chunks, const int* nch, const int* list, const int* start, const int* nummemb,
                                 const signed char* lab, int* cc) {
   if ((int)blockIdx.x >= *nch) return;  // the grid is sized from a bound
   const int2 ck = chunks[blockIdx.x];
-  const int node = a + ck.x;
+  const int node = list[ck.x];
   const int e1 = min(ck.y + CH, start[node] + nummemb[node]);
   __shared__ int s[8];
   if (threadIdx.x < 8) s[threadIdx.x] = 0;
@@ -502,18 +878,17 @@ __global__ void k_scatter_count(const int2* chunks, const int* nch, int a, const
 
 // Per node (one block): destination offset of each chunk's members of each child slot,
 // an exclusive scan over the node's chunks of the per-slot counts, 8 slots at once.
-__global__ void __launch_bounds__(TB) k_scatter_offsets(int a, const int* start, const int* cbeg,
+__global__ void __launch_bounds__(TB) k_scatter_offsets(const int* list, const int* start, const int* cbeg,
                                                         const int* cc, int* coff,
                                                         const SplitState* st, int* err) {
   const int li = blockIdx.x;
-  const SplitState* S = &st[li];
-  if (!S->active) return;
+  const Program* S = &st[li].g;
   constexpr int NW = TB / 32;
   __shared__ int s_base[8], s_carry[8], s_warp[NW][8];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   if (tid == 0) {
     int acc = 0;
-    for (int v = 0; v < 8; v++) { s_base[v] = start[a + li] + acc; acc += S->slot_n[v]; s_carry[v] = 0; }
+    for (int v = 0; v < 8; v++) { s_base[v] = start[list[li]] + acc; acc += v < S->nchild ? S->n[v] : 0; s_carry[v] = 0; }
   }
   __syncthreads();
   const int c0 = cbeg[li], c1 = cbeg[li + 1];
@@ -542,11 +917,11 @@ __global__ void __launch_bounds__(TB) k_scatter_offsets(int a, const int* start,
       for (int q = 0; q < NW; q++) s_carry[tid] += s_warp[q][tid];
     __syncthreads();
   }
-  if (tid < 8 && s_carry[tid] != S->slot_n[tid]) atomicOr(err, 8);
+  if (tid < S->nchild && s_carry[tid] != S->n[tid]) atomicOr(err, 8);
 }
 
 // Stable scatter of each chunk's members to their child's range (order kept).
-__global__ void __launch_bounds__(TB) k_scatter(const int2* chunks, const int* nch, int a, const int* start,
+__global__ void __launch_bounds__(TB) k_scatter(const int2* chunks, const int* nch, const int* list, const int* start,
                                                 const int* nummemb, const signed char* __restrict__ lab,
                                                 const int* coff, const int* __restrict__ perm,
                                                 const double* __restrict__ sx,
@@ -556,7 +931,7 @@ __global__ void __launch_bounds__(TB) k_scatter(const int2* chunks, const int* n
                                                 double* __restrict__ sz2) {
   if ((int)blockIdx.x >= *nch) return;  // the grid is sized from a bound
   const int2 ck = chunks[blockIdx.x];
-  const int node = a + ck.x;
+  const int node = list[ck.x];
   const int e1 = min(ck.y + CH, start[node] + nummemb[node]);
   __shared__ int wcnt[TB / 32][8];
   __shared__ int run[8];
@@ -598,14 +973,14 @@ __global__ void __launch_bounds__(TB) k_scatter(const int2* chunks, const int* n
 
 // (restrict: the two copies never overlap, so a thread's members' loads need not wait
 // for its earlier stores)
-__global__ void k_copy_back(const int2* chunks, const int* nch, int a, const int* start, const int* nummemb,
+__global__ void k_copy_back(const int2* chunks, const int* nch, const int* list, const int* start, const int* nummemb,
                             const int* __restrict__ perm2, const double* __restrict__ sx2,
                             const double* __restrict__ sy2, const double* __restrict__ sz2,
                             int* __restrict__ perm, double* __restrict__ sx,
                             double* __restrict__ sy, double* __restrict__ sz) {
   if ((int)blockIdx.x >= *nch) return;  // the grid is sized from a bound
   const int2 ck = chunks[blockIdx.x];
-  const int node = a + ck.x;
+  const int node = list[ck.x];
   const int e1 = min(ck.y + CH, start[node] + nummemb[node]);
 #pragma unroll
   for (int e = ck.y + threadIdx.x; e < e1; e += TB) {
@@ -613,69 +988,34 @@ __global__ void k_copy_back(const int2* chunks, const int* nch, int a, const int
   }
 }
 
-__global__ void k_child_counts(int nlev, const SplitState* st, int* nch) {
-  int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li < nlev) nch[li] = st[li].active ? st[li].nchild : 0;
-}
-
-__global__ void k_make_children(int a, int b, int nlev, const SplitState* st, const int* cscan,
-                                int* nummemb, int* start, int* children, int* level,
-                                int* parent, double* fields, int* node_sys) {
-  int li = blockIdx.x * blockDim.x + threadIdx.x;
-  if (li >= nlev) return;
-  const SplitState* S = &st[li];
-  if (!S->active) return;
-  const int p = a + li, base = b + cscan[li];
-  int off = start[p];
-  for (int s = 0; s < S->nchild; s++) {
-    int node = base + s;
-    nummemb[node] = S->slot_n[s];
-    start[node] = off;
-    off += S->slot_n[s];
-    level[node] = level[p] + 1;
-    parent[node] = p;
-    node_sys[node] = node_sys[p];
-    for (int k = 0; k < 13; k++) fields[13LL * node + k] = S->slot_f[s][k];
-    for (int c = 0; c < 8; c++) children[8LL * node + c] = -1;
+// Per node (one warp): the packed forms the traversal and the near field read, and a leaf's
+// number at each of its members.
+__global__ void __launch_bounds__(256) k_finish_nodes(int numtree, const double* fields, const int* children,
+                                                      const int* nummemb, const int* start, double4* nodec,
+                                                      float4* nodeh, int2* kids, int* leaf_of) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
+  if (i >= numtree) return;
+  // children[] holds base + order[c] in its first nchild slots (consecutive node
+  // indices, in another order), so one int2 gives the traversal all of them:
+  // (base, nchild | order[c] << (4 + 3c)); a leaf is (-1, nummemb)
+  const int* ch = children + 8LL * i;
+  if (ch[0] == -1)
+    for (int e = start[i] + lane; e < start[i] + nummemb[i]; e += 32) leaf_of[e] = i;
+  if (lane) return;
+  int base = ch[0], cnt = 0;
+  for (int c = 0; c < 8 && ch[c] != -1; c++) {
+    base = min(base, ch[c]);
+    cnt++;
   }
-  for (int c = 0; c < 8; c++) children[8LL * p + c] = c < S->nchild ? base + S->order[c] : -1;
-}
-
-__global__ void k_node_centres(int numtree, const double* fields, const int* children,
-                               const int* nummemb, double4* nodec, float4* nodeh, int2* kids) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < numtree) {
-    // children[] holds base + order[c] in its first nchild slots (consecutive node
-    // indices, in another order), so one int2 gives the traversal all of them:
-    // (base, nchild | order[c] << (4 + 3c)); a leaf is (-1, nummemb)
-    const int* ch = children + 8LL * i;
-    int base = ch[0], cnt = 0;
-    for (int c = 0; c < 8 && ch[c] != -1; c++) {
-      base = min(base, ch[c]);
-      cnt++;
-    }
-    int code = cnt;
-    for (int c = 0; c < cnt; c++) code |= (ch[c] - base) << (4 + 3 * c);
-    kids[i] = cnt ? make_int2(base, code) : make_int2(-1, nummemb[i]);
-    const double* f = fields + 13LL * i;
-    nodec[i] = make_double4(f[6], f[7], f[8], f[12]);
-    // half extents about the midpoint, rounded up to FP32 (a box the members are inside of)
-    const double hx = fmax(f[1] - f[6], f[6] - f[0]), hy = fmax(f[3] - f[7], f[7] - f[2]),
-                 hz = fmax(f[5] - f[8], f[8] - f[4]);
-    nodeh[i] = make_float4(__double2float_ru(hx), __double2float_ru(hy), __double2float_ru(hz), 0.f);
-  }
-}
-
-// leaves in member order: leaf l's FP32 sources begin at record (start + l) / 2, which leaves
-// every leaf whole records of two
-__global__ void k_leaf_of(int nleaves, const int* leaves, const int* start, const int* nummemb,
-                          int* leaf_of, int* pstart) {
-  int l = blockIdx.x;
-  if (l >= nleaves) return;
-  int node = leaves[l];
-  if (threadIdx.x == 0) pstart[node] = (int)(((unsigned)start[node] + (unsigned)l) >> 1);
-  for (int e = start[node] + threadIdx.x; e < start[node] + nummemb[node]; e += blockDim.x)
-    leaf_of[e] = node;
+  int code = cnt;
+  for (int c = 0; c < cnt; c++) code |= (ch[c] - base) << (4 + 3 * c);
+  kids[i] = cnt ? make_int2(base, code) : make_int2(-1, nummemb[i]);
+  const double* f = fields + 13LL * i;
+  nodec[i] = make_double4(f[6], f[7], f[8], f[12]);
+  // half extents about the midpoint, rounded up to FP32 (a box the members are inside of)
+  const double hx = fmax(f[1] - f[6], f[6] - f[0]), hy = fmax(f[3] - f[7], f[7] - f[2]),
+               hz = fmax(f[5] - f[8], f[8] - f[4]);
+  nodeh[i] = make_float4(__double2float_ru(hx), __double2float_ru(hy), __double2float_ru(hz), 0.f);
 }
 
 __global__ void k_iperm(int n, const int* perm, int* iperm) {
@@ -720,146 +1060,183 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   t->sx.ensure(c, n); t->sy.ensure(c, n); t->sz.ensure(c, n);
   DBuf<int> perm2; DBuf<double> sx2, sy2, sz2;
   perm2.ensure(c, n); sx2.ensure(c, n); sy2.ensure(c, n); sz2.ensure(c, n);
-  DBuf<signed char> lab;
-  lab.ensure(c, n);
-  long long capl = 64;
-  for (int k = 0; k < nsys; k++)
-    capl += 16LL * (t->h_sys_n[k] / std::max(t->h_sys_maxmemb[k], 1) + 1) + 8;
+  // nodes: an estimate, grown when it is short; nodes to split at one level: more than maxmemb
+  // members each
+  long long capl = 64, actl = 1;
+  bool big = false;
+  for (int k = 0; k < nsys; k++) {
+    const int m = t->h_sys_maxmemb[k];
+    capl += 16LL * (t->h_sys_n[k] / std::max(m, 1) + 1) + 8;
+    actl += t->h_sys_n[k] / (m + 1LL);
+    big |= t->h_sys_n[k] > std::max(m, kSmallNode);
+  }
   int cap = (int)std::min<long long>(capl, 1LL << 30);
-  t->nummemb.ensure(c, cap); t->start.ensure(c, cap); t->level.ensure(c, cap);
-  t->parent.ensure(c, cap); t->children.ensure(c, 8LL * cap); t->fields.ensure(c, 13LL * cap);
-  t->node_sys.ensure(c, cap);
-  DBuf<int> err;
-  err.ensure(c, 4);
-  BIT_CUDA(cudaMemsetAsync(err.p, 0, 4 * sizeof(int), s));
-  long long* hp = c->h_pinned;
+  DBuf<int> act, nch, cscan, small, big0, big1;
+  DBuf<NodeOut> out;
+  DBuf<Ctl> ctl;
+  t->nummemb.ensure(c, cap); t->start.ensure(c, cap); t->children.ensure(c, 8LL * cap);
+  t->fields.ensure(c, 13LL * cap); t->node_sys.ensure(c, cap);
+  act.ensure(c, cap); nch.ensure(c, cap); cscan.ensure(c, cap);
+  small.ensure(c, 2 * kClasses * actl);
+  big0.ensure(c, n / kSmallNode + 1); big1.ensure(c, n / kSmallNode + 1);
+  out.ensure(c, actl);
+  ctl.ensure(c, 1);
+  BIT_CUDA(cudaMemsetAsync(ctl.p, 0, sizeof(Ctl), s));
+  static_assert(sizeof(Ctl) <= 64 * sizeof(long long), "the control block fits the pinned read-back area");
+  Ctl* h = reinterpret_cast<Ctl*>(c->h_pinned);
 
-  count_launch(), k_iota<<<grid_for(n, 256), 256, 0, s>>>(t->perm.p, n);
-  BIT_CUDA(cudaMemcpyAsync(t->sx.p, x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  BIT_CUDA(cudaMemcpyAsync(t->sy.p, y, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  BIT_CUDA(cudaMemcpyAsync(t->sz.p, z, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  BIT_CUDA(cudaMemsetAsync(lab.p, -1, n, s));
+  Arrays A{};
+  A.perm = t->perm.p; A.sx = t->sx.p; A.sy = t->sy.p; A.sz = t->sz.p;
+  A.perm2 = perm2.p; A.sx2 = sx2.p; A.sy2 = sy2.p; A.sz2 = sz2.p;
+  A.sys_maxmemb = t->sys_maxmemb.p;
+  A.out = out.p;
+  A.ctl = ctl.p;
+  for (int k = 0; k < kClasses; k++)
+    for (int p = 0; p < 2; p++) A.ls.small[k][p] = small.p + (2 * k + p) * actl;
+  A.ls.big[0] = big0.p;
+  A.ls.big[1] = big1.p;
+  A.lim = 1.0 / std::sqrt(2.0);  // src/tree3d.cpp:1371
+  auto point_at_nodes = [&] {
+    A.nummemb = t->nummemb.p; A.start = t->start.p; A.children = t->children.p;
+    A.node_sys = t->node_sys.p; A.fields = t->fields.p;
+    A.act = act.p; A.nch = nch.p; A.cscan = cscan.p;
+    A.cap = cap;
+  };
+  point_at_nodes();
 
   DBuf<SplitAcc> acc;
   acc.ensure(c, nsys);
   count_launch(), k_acc_reset<<<grid_for(nsys, 128), 128, 0, s>>>(acc.p, nsys);
   {
     const unsigned per = std::max(1u, std::min<unsigned>(grid_for(n / nsys + 1, 256), 4 * c->num_sms / nsys + 1));
-    count_launch(), k_root_bbox<<<dim3(per, nsys), 256, 0, s>>>(t->sys_start.p, t->sys_n.p, t->sx.p,
-                                                                t->sy.p, t->sz.p, acc.p, err.p);
+    count_launch(), k_root_bbox<<<dim3(per, nsys), 256, 0, s>>>(t->sys_start.p, t->sys_n.p, x, y, z, t->perm.p,
+                                                                t->sx.p, t->sy.p, t->sz.p, acc.p, ctl.p);
   }
   count_launch(), k_root_init<<<grid_for(nsys, 128), 128, 0, s>>>(
-      nsys, t->sys_start.p, t->sys_n.p, acc.p, t->nummemb.p, t->start.p, t->children.p,
-      t->level.p, t->parent.p, t->fields.p, t->node_sys.p);
+      nsys, t->sys_start.p, t->sys_n.p, t->sys_maxmemb.p, acc.p, t->nummemb.p, t->start.p, t->children.p,
+      t->fields.p, t->node_sys.p, ctl.p, A.ls, act.p, nch.p);
   BIT_CHECK_LAUNCH();
 
-  const double lim = 1.0 / std::sqrt(2.0);  // src/tree3d.cpp:1371
-  DBuf<SplitState> st;
-  DBuf<int> nchunk, cbeg, cc, coff, nch, cscan, done;
-  DBuf<int2> chunks;
-  int a = 0, b = nsys, depth = 1;
-  while (true) {
-    const int nlev = b - a;
-    st.ensure(c, nlev);
-    acc.ensure(c, nlev);
-    nchunk.ensure(c, nlev);
-    cbeg.ensure(c, nlev + 1);
-    nch.ensure(c, nlev);
-    cscan.ensure(c, nlev + 1);
-    const unsigned gl = grid_for(nlev, 128);
-    done.ensure(c, nlev);
-    count_launch(), k_level_init<<<gl, 128, 0, s>>>(a, nlev, t->nummemb.p, t->node_sys.p,
-                                                    t->sys_maxmemb.p, st.p, acc.p, nchunk.p, done.p);
-    count_launch(), k_scan_small<<<1, 1024, 0, s>>>(nchunk.p, cbeg.p, nlev);
-    // The level's chunk count stays on the device (cbeg[nlev]): the chunk kernels run on a
-    // grid sized from its bound, n / CH + one partial chunk per node, and CTAs past the
-    // count return.  A level of leaves only runs empty kernels, and ends the loop below
-    // with no children.
-    const int* nchk = cbeg.p + nlev;
-    const int nch_total = (int)std::min<long long>((long long)n / CH + nlev + 1, INT_MAX);
-    chunks.ensure(c, nch_total);
-    cc.ensure(c, 8LL * nch_total);
-    coff.ensure(c, 8LL * nch_total);
-    count_launch(), k_fill_chunks<<<gl, 128, 0, s>>>(a, nlev, t->start.p, t->nummemb.p, cbeg.p, chunks.p);
-    count_launch(), k_split_decide<<<gl, 128, 0, s>>>(a, nlev, t->fields.p, t->node_sys.p,
-                                                      t->sys_maxmemb.p, st.p, acc.p, lim, err.p);
-    DecideArgs da{nchunk.p, done.p, t->fields.p, t->node_sys.p, t->sys_maxmemb.p, lim, err.p, 1};
-    for (int step = 0; step < 8; step++) {  // 7 bisection steps at most, then the last relabel
-      da.decide = step < 7;
-      count_launch(), k_split_pass<<<nch_total, TB, 0, s>>>(chunks.p, nchk, a, t->start.p, t->nummemb.p, t->sx.p,
-                                                            t->sy.p, t->sz.p, lab.p, st.p, acc.p, da);
-    }
-    count_launch(), k_scatter_count<<<nch_total, TB, 0, s>>>(chunks.p, nchk, a, t->start.p, t->nummemb.p, lab.p, cc.p);
-    count_launch(), k_scatter_offsets<<<nlev, TB, 0, s>>>(a, t->start.p, cbeg.p, cc.p, coff.p, st.p, err.p);
-    count_launch(), k_scatter<<<nch_total, TB, 0, s>>>(chunks.p, nchk, a, t->start.p, t->nummemb.p, lab.p, coff.p,
-                                                       t->perm.p, t->sx.p, t->sy.p, t->sz.p, perm2.p, sx2.p,
-                                                       sy2.p, sz2.p);
-    count_launch(), k_copy_back<<<nch_total, TB, 0, s>>>(chunks.p, nchk, a, t->start.p, t->nummemb.p, perm2.p, sx2.p,
-                                                         sy2.p, sz2.p, t->perm.p, t->sx.p, t->sy.p, t->sz.p);
-    // the next level's members start unlabelled
-    BIT_CUDA(cudaMemsetAsync(lab.p, -1, n, s));
-    count_launch(), k_child_counts<<<gl, 128, 0, s>>>(nlev, st.p, nch.p);
-    count_launch(), k_scan_small<<<1, 1024, 0, s>>>(nch.p, cscan.p, nlev);
-    BIT_CUDA(cudaMemcpyAsync(hp, cscan.p + nlev, sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaMemcpyAsync(hp + 1, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  const unsigned gsplit = (unsigned)std::max(1LL, std::min(actl, 2LL * c->num_sms));
+  // the largest class a system's root may be in: the first levels launch no more
+  int top = 0;
+  for (int k = 0; k < nsys; k++)
+    if (t->h_sys_n[k] > t->h_sys_maxmemb[k])
+      for (int q = top + 1; q < kClasses; q++)
+        if (t->h_sys_n[k] > class_members(q - 1)) top = q;
+  auto sync_ctl = [&] {
+    BIT_CUDA(cudaMemcpyAsync(h, ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaStreamSynchronize(s));
-    const int total = *reinterpret_cast<int*>(hp);
-    const int e = *reinterpret_cast<int*>(hp + 1);
-    if (e & 1) fail(BIT_ERR_INVALID_ARGUMENT, "particle coordinates contain NaN");
-    if (e & 2)
+    if (h->err & 1) fail(BIT_ERR_INVALID_ARGUMENT, "particle coordinates contain NaN");
+    if (h->err & 2)
       fail(BIT_ERR_DEGENERATE,
            "a node with more than maxmemb members cannot be split (coincident particles); "
            "the reference's treemake would not terminate");
-    if (e & 12) fail(BIT_ERR_CUDA, "internal tree-build consistency check failed");
-    if (total == 0) break;
-    if (b + total > cap) {
-      int ncap = std::max(2 * cap, b + total + 64);
-      t->nummemb.grow(c, ncap, b, s); t->start.grow(c, ncap, b, s);
-      t->level.grow(c, ncap, b, s); t->parent.grow(c, ncap, b, s);
-      t->children.grow(c, 8LL * ncap, 8LL * b, s); t->fields.grow(c, 13LL * ncap, 13LL * b, s);
-      t->node_sys.grow(c, ncap, b, s);
-      cap = ncap;
+    if (h->err & 12) fail(BIT_ERR_CUDA, "internal tree-build consistency check failed");
+  };
+  auto make_children = [&](int lev) {
+    const int lo = lev == h->cur ? h->lv[lev % kLevels].b - h->lv[lev % kLevels].a : 0;
+    const unsigned grid = std::max(gsplit, std::min(grid_for(lo, 8), 4u * c->num_sms));
+    count_launch(), k_make_children<<<grid, 256, 0, s>>>(A, lev);
+  };
+  DBuf<signed char> lab;
+  DBuf<SplitState> st;
+  DBuf<int> nchunk, cbeg, cc, coff, done;
+  DBuf<int2> chunks;
+  int cur = 0;
+  h->cur = -1;
+  if (big) sync_ctl();
+  int nbig = big ? h->lv[0].nbig : 0;
+  while (true) {
+    if (nbig > 0) {
+      const int* list = A.ls.big[cur & 1];
+      lab.ensure(c, n);
+      st.ensure(c, nbig);
+      acc.ensure(c, nbig);
+      nchunk.ensure(c, nbig);
+      cbeg.ensure(c, nbig + 1);
+      done.ensure(c, nbig);
+      BIT_CUDA(cudaMemsetAsync(lab.p, -1, n, s));  // members start unlabelled
+      const unsigned gl = grid_for(nbig, 128);
+      count_launch(), k_big_init<<<gl, 128, 0, s>>>(A, nbig, list, st.p, acc.p, nchunk.p, done.p);
+      count_launch(), k_scan_small<<<1, 1024, 0, s>>>(nchunk.p, cbeg.p, nbig);
+      // The chunk count stays on the device (cbeg[nbig]): the chunk kernels run on a grid
+      // sized from its bound, n / CH + one partial chunk per node, and CTAs past it return.
+      const int* nchk = cbeg.p + nbig;
+      const int nch_total = (int)std::min<long long>((long long)n / CH + nbig + 1, INT_MAX);
+      chunks.ensure(c, nch_total);
+      cc.ensure(c, 8LL * nch_total);
+      coff.ensure(c, 8LL * nch_total);
+      count_launch(), k_fill_chunks<<<nbig, 128, 0, s>>>(nbig, list, t->start.p, cbeg.p, chunks.p);
+      for (int step = 0; step < 8; step++)  // 7 bisection steps at most, then the last relabel
+        count_launch(), k_split_pass<<<nch_total, TB, 0, s>>>(A, chunks.p, nchk, list, nchunk.p, done.p, lab.p,
+                                                              st.p, acc.p, step < 7);
+      count_launch(), k_scatter_count<<<nch_total, TB, 0, s>>>(chunks.p, nchk, list, t->start.p, t->nummemb.p, lab.p, cc.p);
+      count_launch(), k_scatter_offsets<<<nbig, TB, 0, s>>>(list, t->start.p, cbeg.p, cc.p, coff.p, st.p, &ctl.p->err);
+      count_launch(), k_scatter<<<nch_total, TB, 0, s>>>(chunks.p, nchk, list, t->start.p, t->nummemb.p, lab.p, coff.p,
+                                                         t->perm.p, t->sx.p, t->sy.p, t->sz.p, perm2.p, sx2.p,
+                                                         sy2.p, sz2.p);
+      count_launch(), k_copy_back<<<nch_total, TB, 0, s>>>(chunks.p, nchk, list, t->start.p, t->nummemb.p, perm2.p,
+                                                           sx2.p, sy2.p, sz2.p, t->perm.p, t->sx.p, t->sy.p, t->sz.p);
     }
-    count_launch(), k_make_children<<<gl, 128, 0, s>>>(a, b, nlev, st.p, cscan.p, t->nummemb.p, t->start.p,
-                                                       t->children.p, t->level.p, t->parent.p, t->fields.p,
-                                                       t->node_sys.p);
+    // Without large nodes, four levels before the next look (a level past the last costs two
+    // empty launches).
+    const int batch = nbig > 0 ? 1 : 4;
+    for (int k = 0; k < batch; k++) {
+      // (a class's nodes are disjoint and larger than the class below)
+      if (top >= 2) launch_split<2>(c, A, cur + k, 0, n / class_members(1) + 1, s);
+      if (top >= 1) launch_split<1>(c, A, cur + k, 0, n / class_members(0) + 1, s);
+      launch_split<0>(c, A, cur + k, 1, actl, s);
+      make_children(cur + k);
+    }
     BIT_CHECK_LAUNCH();
-    a = b;
-    b += total;
-    depth++;
+    sync_ctl();
+    while (h->stop) {  // the node arrays are full: grow them, and go on where it stopped
+      const int have = h->lv[h->cur % kLevels].b, need = h->lv[(h->cur + 1) % kLevels].b;
+      const int ncap = std::max(2 * cap, need + 64);
+      t->nummemb.grow(c, ncap, have, s); t->start.grow(c, ncap, have, s);
+      t->children.grow(c, 8LL * ncap, 8LL * have, s); t->fields.grow(c, 13LL * ncap, 13LL * have, s);
+      t->node_sys.grow(c, ncap, have, s);
+      act.grow(c, ncap, have, s); nch.grow(c, ncap, have, s); cscan.grow(c, ncap, have, s);
+      cap = ncap;
+      point_at_nodes();
+      BIT_CUDA(cudaMemsetAsync(&ctl.p->stop, 0, sizeof(int), s));
+      make_children(h->cur);
+      BIT_CHECK_LAUNCH();
+      sync_ctl();
+    }
+    cur = h->cur;
+    const Level& L = h->lv[cur % kLevels];
+    if (L.a == L.b) break;
+    nbig = L.nbig;
+    // children are no larger than their parents
+    while (nbig == 0 && top > 0 && L.nsmall[top] == 0) top--;
   }
-  {
-    // roots that are leaves (n <= maxmemb) still have to report NaNs
-    BIT_CUDA(cudaMemcpyAsync(hp + 1, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    BIT_CUDA(cudaStreamSynchronize(s));
-    if (*reinterpret_cast<int*>(hp + 1) & 1)
-      fail(BIT_ERR_INVALID_ARGUMENT, "particle coordinates contain NaN");
-  }
+  const int b = h->lv[cur % kLevels].a;
   t->numtree = b;
-  t->depth = depth;
+  t->depth = cur;
   t->cap = cap;
   t->nodec.ensure(c, b);
   t->nodeh.ensure(c, b);
   t->kids.ensure(c, b);
-  count_launch(), k_node_centres<<<grid_for(b, 128), 128, 0, s>>>(b, t->fields.p, t->children.p, t->nummemb.p,
-                                                                 t->nodec.p, t->nodeh.p, t->kids.p);
+  t->leaf_of.ensure(c, n);
+  t->iperm.ensure(c, n);
+  t->pstart.ensure(c, b);
+  count_launch(), k_finish_nodes<<<grid_for(b, 8), 256, 0, s>>>(b, t->fields.p, t->children.p, t->nummemb.p,
+                                                               t->start.p, t->nodec.p, t->nodeh.p, t->kids.p,
+                                                               t->leaf_of.p);
+  count_launch(), k_iperm<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, t->iperm.p);
+  BIT_CHECK_LAUNCH();
   tree_sync_host(t);
-  // leaves in member order
-  std::vector<int> leaves;
+  // leaves in member order: leaf l's FP32 sources begin at record (start + l) / 2, which
+  // leaves every leaf whole records of two
+  std::vector<int> leaves, ps(b, 0);
   for (int i = 0; i < b; i++)
     if (t->h_children[8LL * i] == -1) leaves.push_back(i);
   std::sort(leaves.begin(), leaves.end(), [&](int p, int q) { return t->h_start[p] < t->h_start[q]; });
   t->nleaves = (int)leaves.size();
-  t->pstart.ensure(c, b);
-  t->leaves.ensure(c, leaves.size());
-  BIT_CUDA(cudaMemcpyAsync(t->leaves.p, leaves.data(), leaves.size() * sizeof(int),
-                           cudaMemcpyHostToDevice, s));
-  t->leaf_of.ensure(c, n);
-  count_launch(), k_leaf_of<<<t->nleaves, 256, 0, s>>>(t->nleaves, t->leaves.p, t->start.p, t->nummemb.p,
-                                                       t->leaf_of.p, t->pstart.p);
-  t->iperm.ensure(c, n);
-  count_launch(), k_iperm<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, t->iperm.p);
-  BIT_CHECK_LAUNCH();
+  for (int l = 0; l < t->nleaves; l++) ps[leaves[l]] = (int)(((unsigned)t->h_start[leaves[l]] + (unsigned)l) >> 1);
+  BIT_CUDA(cudaMemcpyAsync(t->pstart.p, ps.data(), b * sizeof(int), cudaMemcpyHostToDevice, s));
   BIT_CUDA(cudaStreamSynchronize(s));
   t->gen++;
   t->has_moments = false;
@@ -871,19 +1248,18 @@ template struct DBuf<signed char>;
 template struct DBuf<SplitState>;
 template struct DBuf<SplitAcc>;
 template struct DBuf<int2>;
+template struct DBuf<NodeOut>;
+template struct DBuf<Ctl>;
 
 void tree_sync_host(Tree* t) {
-  cudaStream_t s = t->ctx->stream;
   const int b = t->numtree;
   t->h_nummemb.resize(b); t->h_start.resize(b); t->h_children.resize(8LL * b);
-  t->h_level.resize(b); t->h_fields.resize(13LL * b); t->h_node_sys.resize(b);
-  BIT_CUDA(cudaMemcpyAsync(t->h_nummemb.data(), t->nummemb.p, b * sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaMemcpyAsync(t->h_start.data(), t->start.p, b * sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaMemcpyAsync(t->h_children.data(), t->children.p, 8LL * b * sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaMemcpyAsync(t->h_level.data(), t->level.p, b * sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaMemcpyAsync(t->h_fields.data(), t->fields.p, 13LL * b * sizeof(double), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaMemcpyAsync(t->h_node_sys.data(), t->node_sys.p, b * sizeof(int), cudaMemcpyDeviceToHost, s));
-  BIT_CUDA(cudaStreamSynchronize(s));
+  t->h_fields.resize(13LL * b); t->h_node_sys.resize(b);
+  copy_d2h_batch(t->ctx, {{t->h_nummemb.data(), t->nummemb.p, b * sizeof(int)},
+                          {t->h_start.data(), t->start.p, b * sizeof(int)},
+                          {t->h_children.data(), t->children.p, 8LL * b * sizeof(int)},
+                          {t->h_fields.data(), t->fields.p, 13LL * b * sizeof(double)},
+                          {t->h_node_sys.data(), t->node_sys.p, b * sizeof(int)}});
   t->h_sys_leaf_sqr.assign(t->nsys, 0.0);
   for (int i = 0; i < b; i++)
     if (t->h_children[8LL * i] == -1) {
