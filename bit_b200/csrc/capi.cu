@@ -312,7 +312,6 @@ bit_status bit_ctx_set_near_config(bit_ctx* h, int tile, int threads_per_target)
   const int s = threads_per_target;
   if (s != 0 && (s < 1 || s > 32 || (s & (s - 1)))) return BIT_ERR_INVALID_ARGUMENT;
   h->c.near_tile = tile;
-  h->c.near_split = s;
   return BIT_OK;
 }
 

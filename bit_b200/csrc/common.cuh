@@ -131,9 +131,8 @@ struct EvalPlan {
   bool f32 = false;
   int force = 0;
   std::vector<LaunchClass> far_classes, near_classes;
-  DBuf<int> far_order, near_order;   // used when there is more than one class
-  const int* far_ord = nullptr;      // group order of the far / near launches
-  const int* near_ord = nullptr;
+  DBuf<int> far_order;               // used when there is more than one class
+  const int* far_ord = nullptr;      // group order of the far launches
   DBuf<int2> near_items;             // used when there is more than one near class
   const int2* near_it = nullptr;
   long long lists_version = -1;      // lists the classes were planned for
@@ -195,7 +194,8 @@ struct Lists {
   DBuf<unsigned long long> g_near;          // near pairs of each group
   DBuf<long long> part_off;
   DBuf<int> part_done;
-  DBuf<double> near_part;
+  DBuf<double> near_part, field_part;       // (fields: three sums a target)
+  long long part_total = 0;                 // sums of a potential in scratch
   long long version = 0;                    // bumped by every build
   ListSizing last;                          // the last build's sizes
   bool fallback = false;                    // the last build used count, scan and fill
@@ -221,9 +221,7 @@ struct Ctx {
   // kernel over a device work queue of all groups, 0 as one launch per class.
   int work_queue = 1;
   DBuf<int> queue_heads;  // the work queues' counters (far, near)
-  // near-field tuning knobs (bit_ctx_set_near_config): source records per tile and the cap
-  // on threads per target (0: the defaults)
-  int near_tile = 0, near_split = 0;
+  int near_tile = 0;      // bit_ctx_set_near_config: source records per CTA (0: the default)
   ListKey mac_hint;       // MAC of the last particle-target evaluation (acc < 0: none)
   ListSizing list_hint;   // sizes of the last list build of any tree
   // small device scratch for flags / counters
@@ -263,8 +261,7 @@ struct Tree {
   DBuf<int> perm, iperm;
   DBuf<double> sx, sy, sz, sq, sw;
   DBuf<double4> src64;   // (x, y, z, q)
-  DBuf<float4> src32;    // leaf-centred (x-c, y-c, z-c, q)
-  // the same for the mixed potentials, two sources to a record (x0 x1 y0 y1, z0 z1 q0 q1),
+  // leaf-centred FP32 (x-c, y-c, z-c, q), two sources to a record (x0 x1 y0 y1, z0 z1 q0 q1),
   // each leaf from record pstart[leaf]; an odd leaf's last record ends with its last source
   // once more, without charge
   DBuf<float4> src2;

@@ -42,13 +42,12 @@ __global__ void k_scatter(int n, const int* perm, const double* src, double* dst
 // charges q = w * s in tree order, written into every source representation
 __global__ void k_charges(int n, const double* w, const double* s, const int* leaf_of,
                           const int* start, const int* pstart, double* sq, double4* src64,
-                          float4* src32, float4* src2) {
+                          float4* src2) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   double q = w[e] * s[e];
   sq[e] = q;
   src64[e].w = q;
-  src32[e].w = (float)q;
   const int leaf = leaf_of[e], j = e - start[leaf];
   reinterpret_cast<float*>(src2)[8 * ((size_t)pstart[leaf] + (j >> 1)) + 6 + (j & 1)] = (float)q;
 }
@@ -275,7 +274,7 @@ struct BieOp {
     cudaStream_t s = c->stream;
     const int n = t->n;
     count_launch(), k_charges<<<grid_for(n, 256), 256, 0, s>>>(
-        n, w_s.p, x, t->leaf_of.p, t->start.p, t->pstart.p, t->sq.p, t->src64.p, t->src32.p, t->src2.p);
+        n, w_s.p, x, t->leaf_of.p, t->start.p, t->pstart.p, t->sq.p, t->src64.p, t->src2.p);
     tree_moments(t, nterms);
     bit_eval_params p = prm;
     p.precision = prec;

@@ -449,6 +449,7 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
     std::fill(K.begin(), K.end(), 1);
     tot = 0;
   }
+  L->part_total = tot;
   std::vector<std::pair<unsigned long long, int2>> it;
   for (int g = 0; g < ng; g++)
     for (int k = 0; k < K[g]; k++) it.push_back({pairs[g] / K[g], make_int2(g, k | K[g] << 16)});

@@ -152,17 +152,16 @@ __global__ void k_gather_charges(int n, const int* perm, const double* q, const 
   src64[e] = make_double4(sx[e], sy[e], sz[e], qq);
 }
 
-// FP32 sources in the coordinates of their own leaf's centre: one by one, and in records of two.
+// FP32 sources in the coordinates of their own leaf's centre, in records of two.
 __global__ void k_leaf_local(int n, const int* leaf_of, const int* start, const int* nummemb,
                              const int* pstart, const double4* nodec, const double4* src64,
-                             float4* src32, float4* src2) {
+                             float4* src2) {
   int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   double4 s = src64[e];
   const int leaf = leaf_of[e];
   double4 c = nodec[leaf];
   const float4 v = make_float4((float)(s.x - c.x), (float)(s.y - c.y), (float)(s.z - c.z), (float)s.w);
-  src32[e] = v;
   const int j = e - start[leaf];
   float* r = reinterpret_cast<float*>(src2) + 8 * ((size_t)pstart[leaf] + (j >> 1));
   auto put = [&](int h, float q) { r[h] = v.x; r[2 + h] = v.y; r[4 + h] = v.z; r[6 + h] = q; };
@@ -185,13 +184,12 @@ void tree_set_charges(Tree* t, const double* q, const double* w) {
   t->sq.ensure(c, n);
   if (w) t->sw.ensure(c, n);
   t->src64.ensure(c, n);
-  t->src32.ensure(c, n);
   t->src2.ensure(c, (size_t)n + t->nleaves + 2);  // two float4 per record
   count_launch(), k_gather_charges<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, q, w, t->sx.p, t->sy.p,
                                                     t->sz.p, t->sq.p, w ? t->sw.p : nullptr,
                                                     t->src64.p);
   count_launch(), k_leaf_local<<<grid_for(n, 256), 256, 0, s>>>(
-      n, t->leaf_of.p, t->start.p, t->nummemb.p, t->pstart.p, t->nodec.p, t->src64.p, t->src32.p, t->src2.p);
+      n, t->leaf_of.p, t->start.p, t->nummemb.p, t->pstart.p, t->nodec.p, t->src64.p, t->src2.p);
   BIT_CHECK_LAUNCH();
   t->has_charges = true;
   t->has_weights = w != nullptr;

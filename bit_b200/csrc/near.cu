@@ -38,104 +38,6 @@ namespace {
 
 constexpr int NW = 8;  // warps per CTA
 
-// Pack the set bits of a group mask (W words, lane l holds word l) into tl in ascending order.
-__device__ __forceinline__ void pack_list(unsigned wd, int W, unsigned short* tl) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  int base = 0;
-  for (int j = 0; j < W; j++) {
-    const unsigned b = __shfl_sync(0xffffffffu, wd, j);
-    if ((b >> lane) & 1u) tl[base + __popc(b & lt)] = (unsigned short)(32 * j + lane);
-    base += __popc(b);
-  }
-  __syncwarp();
-}
-
-// -------------------------------------------------------------------------------- FP64 pair
-// One pair's q / sqrt(r^2 + del) or q e^(-kappa R) / R (src/tree3d.cpp:4765-4769, 3609-3618)
-// added to acc.  1/R: the hardware seed and one third-order Newton step (rsqrt_nr); the
-// exponential: exp_scaled.  12 (Coulomb) / 25 (screened) FP64 operations.  EPS: a pair with
-// r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`).  UF: the
-// exponential may underflow.
-template <int KER, bool EPS, bool SELF, bool UF, int COPIES = kExpTabCopies>
-__device__ __forceinline__ void pair64(double x, double y, double z, double4 s, double del,
-                                       ExpScale k, const double2* tab, bool own, double& acc) {
-  const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
-  double rr = fma(dx, dx, fma(dy, dy, fma(dz, dz, del)));
-  double q = s.w;
-  if (EPS || SELF) {
-    const bool skip = (SELF && own) || (EPS && !(rr > kEpsNear));
-    q = skip ? 0.0 : q;
-    rr = skip ? 1.0 : rr;
-  }
-  double y0;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(rr));
-  const double t = rr * y0;
-  const double e = fma(-t, y0, 1.0);
-  const double f = fma(e, 0.375, 0.5);
-  if (KER == BIT_KERNEL_COULOMB) {
-    acc = fma(q * y0, fma(e, f, 1.0), acc);
-  } else {
-    const double ec = e * f;
-    const double ri = fma(y0, ec, y0);
-    acc = fma(q * exp_scaled<UF, COPIES>(fma(t, ec, t), k, tab), ri, acc);
-  }
-}
-
-struct Range64 {
-  const double4* src;  // the tile
-  int n;               // its sources
-  double del;
-  ExpScale k;
-  const double2* tab;
-};
-
-// Two targets against every source of the tile, two sources (four pairs) at a time; o0, o1:
-// the targets' own tile index (SELF).  (Four sources: 3% faster at 2M, 20% slower on leaves
-// of 55.)
-template <int KER, bool EPS, bool SELF, bool UF>
-__device__ __forceinline__ void two64(const Range64& r, double x0, double y0, double z0, double x1,
-                                      double y1, double z1, int o0, int o1, double& p0, double& p1) {
-  constexpr int UN = 2;
-  double a0[UN], a1[UN];
-#pragma unroll
-  for (int u = 0; u < UN; u++) a0[u] = a1[u] = 0.0;
-  auto add = [&](int j, int u) {
-    const double4 s = r.src[j];
-    pair64<KER, EPS, SELF, UF>(x0, y0, z0, s, r.del, r.k, r.tab, j == o0, a0[u]);
-    pair64<KER, EPS, SELF, UF>(x1, y1, z1, s, r.del, r.k, r.tab, j == o1, a1[u]);
-  };
-  int j = 0;
-#pragma unroll 1
-  for (; j + UN - 1 < r.n; j += UN) {
-#pragma unroll
-    for (int u = 0; u < UN; u++) add(j + u, u);
-  }
-#pragma unroll 1
-  for (; j < r.n; j++) add(j, 0);
-  p0 = a0[0] + a0[1];
-  p1 = a1[0] + a1[1];
-}
-
-// One target against sources j, j + step, ... of the tile.
-template <int KER, bool EPS, bool SELF, bool UF>
-__device__ __forceinline__ double one64(const Range64& r, double x, double y, double z, int o, int j,
-                                        int step) {
-  constexpr int UN = 4;
-  double a[UN] = {0.0, 0.0, 0.0, 0.0};
-  auto add = [&](int k, int u) {
-    pair64<KER, EPS, SELF, UF>(x, y, z, r.src[k], r.del, r.k, r.tab, k == o, a[u]);
-  };
-#pragma unroll 1
-  for (; j + (UN - 1) * step < r.n; j += UN * step) {
-#pragma unroll
-    for (int u = 0; u < UN; u++) add(j + u * step, u);
-  }
-#pragma unroll 1
-  for (; j < r.n; j += step) add(j, 0);
-  return (a[0] + a[2]) + (a[1] + a[3]);
-}
-
 // Every listed target against one tile; sums into the warp's row.
 template <int KER, bool EPS, bool SELF, bool UF>
 __device__ __forceinline__ void tile64(const Range64& r, const double* cx, const double* cy,
@@ -175,28 +77,6 @@ __device__ __forceinline__ void tile64(const Range64& r, const double* cx, const
 // (x0 x1 y0 y1 z0 z1 q0 q1), the target's offset from that centre formed in FP64 and rounded
 // once.  Differences, squares and sums run on packed pairs of sources (f32x2: one issue slot
 // for two), 1/r and 2^x on the MUFU.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 v;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-  return v;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 v;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-  return v;
-}
-
 struct Range32 {
   const ulonglong2* rec;  // the tile: two vectors per record of two sources
   int n;                  // its sources (the last record may be half empty: charge 0)
@@ -341,7 +221,6 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
 // Shared memory of a CTA: the exponential's table (FP64 screened), per warp two source tiles,
 // an accumulator row (a double, or a float and its error, per target) and a target list.
 // Tiles are counted in 32-byte records: one FP64 source, two FP32 ones.
-constexpr int kRec = 32;
 struct Layout {
   int recs, rows, tab;  // tab: bytes of the table
   __host__ __device__ size_t warp_bytes() const {
@@ -349,15 +228,6 @@ struct Layout {
   }
   __host__ __device__ size_t total() const { return tab + NW * warp_bytes(); }
 };
-
-// First source (a multiple of 8, or all ns) of an entry of weight wt whose work begins at P
-// that lies at or past T.
-__device__ __forceinline__ int cut(long long T, long long P, int wt, int ns) {
-  if (T <= P) return 0;
-  if (T >= P + (long long)wt * ns) return ns;
-  const long long j = (T - P + 8LL * wt - 1) / (8LL * wt) * 8;
-  return j < ns ? (int)j : ns;
-}
 
 // Returns false (in every thread) if a warp's bounded wait for a tile gave up: the error flag
 // is set, the warp has waited, bounded again, for its copies in flight, and the group's
@@ -389,14 +259,8 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
   // it begins in: the last whose prefix is at most T0
   const long long tot = a.tot[g];
   const int nv = NW * parts, v = part * NW + w;
-  const long long T0 = tot / nv * v + tot % nv * v / nv;
-  const long long T1 = tot / nv * (v + 1) + tot % nv * (v + 1) / nv;
-  long long e = e0 < e1 ? e0 - 1 : e1;  // (a group may have no near entries)
-  for (long long b = e0; b < e1; b += 32) {
-    const int c = __popc(__ballot_sync(0xffffffffu, b + lane < e1 && a.pre[b + lane] <= T0));
-    e += c;
-    if (c < 32) break;
-  }
+  const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
+  long long e = run_entry(a.pre, e0, e1, T0);
   __syncthreads();  // the rows are zero
   const double del = se->near_del;
   const ExpScale ks = exp_scale(se->kappa);
@@ -658,8 +522,6 @@ __global__ void __launch_bounds__(256) k_close(NearArgs a) {
   }
 }
 
-constexpr int kSmemMax = 227 * 1024;
-
 template <bool F32>
 void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
   Ctx* c = t->ctx;
@@ -718,7 +580,6 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
     launch_near<false>(t, L, P, a);
     return;
   }
-  a.src = t->src2.p;
   // Mixed: close pairs need r^2 < thr = max(sqradius / 1024, 2e-14) of some leaf, and the
   // FP32 r^2 is at least the system's del (a rounded sum of non-negative terms and del);
   // where del reaches the largest leaf threshold no pair can be close, and the records

@@ -34,7 +34,7 @@ __host__ __device__ __forceinline__ int near_weight(int cnt) {
 }
 
 struct NearArgs {
-  const int *order, *g_tstart, *g_tcount;
+  const int *g_tstart, *g_tcount;
   const double *tx, *ty, *tz;
   const long long *off, *moff;
   const int* cnt;
@@ -42,7 +42,7 @@ struct NearArgs {
   const unsigned* mask;
   const int *start, *nummemb;
   const double4* nodec;
-  const void* src;  // double4 in tree order; mixed: float4 (fields), records of two sources (potentials)
+  const void* src;  // double4 in tree order; mixed: records of two sources
   const double4* src64;
   const float4* nodeh;  // per node: half extents of the box, rounded up
   const double* sw;
@@ -55,9 +55,7 @@ struct NearArgs {
   int2* crec;   // up to kCloseRec (near entry, first source of the tile) per target
   int2* clist;  // (target, group) of every target with a record
   int* cn;      // entries of clist
-  int tile;     // sources per tile
-  int split;    // fields: threads per target, 0 the rule, else at most this many
-  // potentials
+  int tile;              // mixed potentials: sources per tile (k_close)
   const int* pstart;     // first record of each leaf's FP32 sources
   const int* tgt;        // targets of each near entry
   const long long* pre;  // work (near_weight x sources) of the group's entries before it
@@ -129,6 +127,156 @@ __device__ __forceinline__ void record_close(const NearArgs& a, int t, int g, lo
   const int c = atomicAdd(&a.ccnt[t], 1);
   if (c < kCloseRec) a.crec[(long long)t * kCloseRec + c] = make_int2((int)e, toff);
   if (c == 0) a.clist[atomicAdd(a.cn, 1)] = make_int2(t, g);
+}
+
+constexpr int kRec = 32;               // bytes of a source record: one FP64 source, two FP32 ones
+constexpr int kSmemMax = 227 * 1024;  // shared memory of a CTA
+
+// Pack the set bits of a group mask (W words, lane l holds word l) into tl in ascending order.
+__device__ __forceinline__ void pack_list(unsigned wd, int W, unsigned short* tl) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  int base = 0;
+  for (int j = 0; j < W; j++) {
+    const unsigned b = __shfl_sync(0xffffffffu, wd, j);
+    if ((b >> lane) & 1u) tl[base + __popc(b & lt)] = (unsigned short)(32 * j + lane);
+    base += __popc(b);
+  }
+  __syncwarp();
+}
+
+// -------------------------------------------------------------------------------- FP64 pair
+// One pair's q / sqrt(r^2 + del) or q e^(-kappa R) / R (src/tree3d.cpp:4765-4769, 3609-3618)
+// added to acc.  1/R: the hardware seed and one third-order Newton step (rsqrt_nr); the
+// exponential: exp_scaled.  12 (Coulomb) / 25 (screened) FP64 operations.  EPS: a pair with
+// r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`).  UF: the
+// exponential may underflow.
+template <int KER, bool EPS, bool SELF, bool UF, int COPIES = kExpTabCopies>
+__device__ __forceinline__ void pair64(double x, double y, double z, double4 s, double del,
+                                       ExpScale k, const double2* tab, bool own, double& acc) {
+  const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
+  double rr = fma(dx, dx, fma(dy, dy, fma(dz, dz, del)));
+  double q = s.w;
+  if (EPS || SELF) {
+    const bool skip = (SELF && own) || (EPS && !(rr > kEpsNear));
+    q = skip ? 0.0 : q;
+    rr = skip ? 1.0 : rr;
+  }
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(rr));
+  const double t = rr * y0;
+  const double e = fma(-t, y0, 1.0);
+  const double f = fma(e, 0.375, 0.5);
+  if (KER == BIT_KERNEL_COULOMB) {
+    acc = fma(q * y0, fma(e, f, 1.0), acc);
+  } else {
+    const double ec = e * f;
+    const double ri = fma(y0, ec, y0);
+    acc = fma(q * exp_scaled<UF, COPIES>(fma(t, ec, t), k, tab), ri, acc);
+  }
+}
+
+struct Range64 {
+  const double4* src;  // the tile
+  int n;               // its sources
+  double del;
+  ExpScale k;
+  const double2* tab;
+};
+
+// Two targets against every source of the tile, two sources (four pairs) at a time; o0, o1:
+// the targets' own tile index (SELF).  (Four sources: 3% faster at 2M, 20% slower on leaves
+// of 55.)
+template <int KER, bool EPS, bool SELF, bool UF>
+__device__ __forceinline__ void two64(const Range64& r, double x0, double y0, double z0, double x1,
+                                      double y1, double z1, int o0, int o1, double& p0, double& p1) {
+  constexpr int UN = 2;
+  double a0[UN], a1[UN];
+#pragma unroll
+  for (int u = 0; u < UN; u++) a0[u] = a1[u] = 0.0;
+  auto add = [&](int j, int u) {
+    const double4 s = r.src[j];
+    pair64<KER, EPS, SELF, UF>(x0, y0, z0, s, r.del, r.k, r.tab, j == o0, a0[u]);
+    pair64<KER, EPS, SELF, UF>(x1, y1, z1, s, r.del, r.k, r.tab, j == o1, a1[u]);
+  };
+  int j = 0;
+#pragma unroll 1
+  for (; j + UN - 1 < r.n; j += UN) {
+#pragma unroll
+    for (int u = 0; u < UN; u++) add(j + u, u);
+  }
+#pragma unroll 1
+  for (; j < r.n; j++) add(j, 0);
+  p0 = a0[0] + a0[1];
+  p1 = a1[0] + a1[1];
+}
+
+// One target against sources j, j + step, ... of the tile.
+template <int KER, bool EPS, bool SELF, bool UF>
+__device__ __forceinline__ double one64(const Range64& r, double x, double y, double z, int o, int j,
+                                        int step) {
+  constexpr int UN = 4;
+  double a[UN] = {0.0, 0.0, 0.0, 0.0};
+  auto add = [&](int k, int u) {
+    pair64<KER, EPS, SELF, UF>(x, y, z, r.src[k], r.del, r.k, r.tab, k == o, a[u]);
+  };
+#pragma unroll 1
+  for (; j + (UN - 1) * step < r.n; j += UN * step) {
+#pragma unroll
+    for (int u = 0; u < UN; u++) add(j + u * step, u);
+  }
+#pragma unroll 1
+  for (; j < r.n; j += step) add(j, 0);
+  return (a[0] + a[2]) + (a[1] + a[3]);
+}
+
+// Two FP32 numbers in one 64-bit register (packed arithmetic: one issue slot for two).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+
+// First source (a multiple of 8, or all ns) of an entry of weight wt whose work begins at P
+// that lies at or past T.
+__device__ __forceinline__ int cut(long long T, long long P, int wt, int ns) {
+  if (T <= P) return 0;
+  if (T >= P + (long long)wt * ns) return ns;
+  const long long j = (T - P + 8LL * wt - 1) / (8LL * wt) * 8;
+  return j < ns ? (int)j : ns;
+}
+
+// Where warp v of nv begins its run of a group's work.
+__device__ __forceinline__ long long run_begin(long long tot, int nv, int v) {
+  return tot / nv * v + tot % nv * v / nv;
+}
+// The entry of [e0, e1) that work T0 lies in: the last whose prefix is at most T0 (e1 if there is
+// no entry: a group may have none).
+__device__ __forceinline__ long long run_entry(const long long* pre, long long e0, long long e1, long long T0) {
+  const int lane = threadIdx.x & 31;
+  long long e = e0 < e1 ? e0 - 1 : e1;
+  for (long long b = e0; b < e1; b += 32) {
+    const int c = __popc(__ballot_sync(0xffffffffu, b + lane < e1 && pre[b + lane] <= T0));
+    e += c;
+    if (c < 32) break;
+  }
+  return e;
 }
 
 // The arguments common to every near-field launch of this plan (near_field.cu).

@@ -1,20 +1,18 @@
 // Near field of the fields: the leaf direct sums of treeforce / shielded_treeforce
-// (src/tree3d.cpp:923-967, 3378-3398), one CTA per target group.
+// (src/tree3d.cpp:923-967, 3378-3398), with the work shared out as the potentials' (near.cu):
+// one CTA per item, every warp a contiguous run of the group's sources, two targets a lane,
+// its own tiles and accumulator rows (three, in FP64).
 //
-// For each near entry (source leaf, bitmask over the group's targets) the CTA packs the
-// targets that need the leaf into a dense list and splits the leaf's sources across 1..32
-// threads per target, whichever keeps the most threads busy (partial sums combined by
-// warp shuffles).  Source tiles are staged in shared memory by TMA bulk
-// copies (cp.async.bulk with an mbarrier), double buffered so the next tile streams in
-// while the current one is consumed; every thread then reads each source from shared
-// memory, broadcast across the targets.  Accumulation per target is in shared memory in a
-// fixed order, so results are deterministic.
-//
-// FP64 path: the reference's arithmetic.  Mixed path: sources in FP32 relative to their
-// leaf centre, the target's offset from that centre formed in FP64 and rounded once; pairs
-// too close for FP32 coordinates are summed in FP64.
+// FP64: the reference's sums, with 1/r^3 from one reciprocal square root: 16 FP64 operations a
+// Coulomb pair, where a square root and a division took about 40.  Mixed: sources in FP32
+// relative to their leaf centre, the target's offset from that centre formed in FP64 and
+// rounded once, a tile's sums in FP32; pairs too close for FP32 coordinates are summed in FP64.
+// Bound by the FP64 pipe, mixed by issue.  Before (a square root and a division, one target a
+// thread, a barrier per tile) / now, FP64 Coulomb field, ms: 2M clustered in leaves of 1000,
+// theta = 0.7, 24.2 / 14.2 (rows of 1,000 targets leave eight warps an SM); 100k in leaves of
+// 500, theta = 0.15, 12.9 / 2.0; 300k uniform in leaves of 100 1.28 / 0.33; 20k 0.32 / 0.11.
 #include <algorithm>
-#include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 #include "fp64math.cuh"
@@ -25,342 +23,360 @@ namespace bit {
 
 namespace {
 
-constexpr int NT = 256;  // threads per CTA
+// Warps per CTA: four, so that the three rows of groups of 1,000 targets leave room for two
+// CTAs an SM.
+constexpr int NW = 4;
+// The regularised Coulomb field, the same with the reference's KERNEL_ORDER family, the
+// screened 2-D field.
+enum { F_COULOMB = 0, F_ORDER = 1, F_CURL = 2 };
 
-template <bool F32>
-struct Prec;
-// Source tile (records per TMA copy): the default, and the range a context may choose
-// (bit_ctx_set_near_config); shared memory holds two tiles.
-template <>
-struct Prec<true> {
-  using S = float4;
-  using T = float;
-  static constexpr int TILE = 1024, TILE_MIN = 256, TILE_MAX = 2048;
-};
-template <>
-struct Prec<false> {
-  using S = double4;
-  using T = double;
-  static constexpr int TILE = 512, TILE_MIN = 128, TILE_MAX = 1024;
+struct Field {
+  double del, kappa;
+  ExpScale k;
+  const double2* tab;
+  int korder;
 };
 
-// Field of eval_grad_kernel_reg (src/tree3d.cpp:73-97), KERNEL_ORDER = 0:
-// q * (-(x_j - x) / (r * r^2)).
-__device__ __forceinline__ void fpair(double x, double y, double z, double4 s, double del,
-                                      double& ax, double& ay, double& az) {
-  const double dx = s.x - x, dy = s.y - y, dz = s.z - z;
-  const double rs = dx * dx + dy * dy + dz * dz + del;
-  const double r = sqrt(rs);
-  const double t = s.w / (r * rs);
-  ax -= dx * t; ay -= dy * t; az -= dz * t;
-}
-// The same with the reference's KERNEL_ORDER family (eval_grad_kernel_reg,
-// src/tree3d.cpp:80-91): 1/(r rs) plus korder terms, each the previous one times
-// (l + 1/2)/l * del/rs.
-__device__ __forceinline__ void fpair_order(double x, double y, double z, double4 s, double del,
-                                            int korder, double& ax, double& ay, double& az) {
-  const double dx = s.x - x, dy = s.y - y, dz = s.z - z;
-  const double rs = dx * dx + dy * dy + dz * dz + del;
-  const double r = sqrt(rs);
-  double temp = 1.0 / (r * rs), f = temp;
-  for (int l = 1; l <= korder; l++) {
-    f = f * (l + 0.5) / l * del / rs;
-    temp += f;
-  }
-  const double t = s.w * temp;
-  ax -= dx * t; ay -= dy * t; az -= dz * t;
-}
-// Screened 2-D field of one pair (shielded_treeforce's leaf loop, src/tree3d.cpp:3384-3398):
-// t = q e^{-kappa r} / r^2 (kappa + 1/r), fx -= dy t, fy += dx t, no del.
-__device__ __forceinline__ void cpair(double x, double y, double z, double4 s, double kappa,
-                                      double& ax, double& ay) {
+// One pair's field in FP64, added to (ax, ay, az):
+// F_COULOMB  q (x - x_j) / (r^2 + del)^(3/2) (eval_grad_kernel_reg, src/tree3d.cpp:73-97)
+// F_ORDER    the same plus korder terms, each the previous one times (l + 1/2)/l del/rs
+//            (src/tree3d.cpp:80-91)
+// F_CURL     t (-dy, dx), t = q e^(-kappa r) / r^2 (kappa + 1/r) (src/tree3d.cpp:3384-3398)
+// 1/r^3: with y the hardware seed of 1/r and e = 1 - rs y^2 (of the rounded y^2),
+// y^3 (1 + 3/2 e + 15/8 e^2), an error of e^3 ~ 1e-17.
+template <int FK, bool SELF, bool UF>
+__device__ __forceinline__ void field64(double x, double y, double z, double4 s, const Field& f, bool own,
+                                        double& ax, double& ay, double& az) {
   const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
-  const double rs = dx * dx + dy * dy + dz * dz;
-  const double r = sqrt(rs);
-  const double t = s.w * exp(-kappa * r) / rs * (kappa + 1 / r);
-  ax -= dy * t; ay += dx * t;
-}
-
-template <class T>
-__device__ __forceinline__ T shfl_sum(T v, int tpt) {
-  for (int o = tpt >> 1; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Field of one pair, q (x - x_j) / r^3 (eval_grad_kernel_reg, src/tree3d.cpp:73-97,
-// KERNEL_ORDER = 0); CHK as acc_pot.
-template <bool CHK>
-__device__ __forceinline__ void acc_force(float xt, float yt, float zt, float4 s, float del,
-                                          float thr, float& ax, float& ay, float& az,
-                                          bool& close) {
-  const float dx = xt - s.x, dy = yt - s.y, dz = zt - s.z;
-  float rs = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, del)));
-  float q = s.w;
-  if (CHK) {
-    const bool cl = rs < thr;
-    close |= cl;
-    q = cl ? 0.f : q;
-    rs = cl ? 1.f : rs;
+  double rs = fma(dx, dx, fma(dy, dy, fma(dz, dz, f.del))), q = s.w;
+  if (SELF && own) {
+    q = 0.0;
+    rs = 1.0;
   }
-  const float ri = rsqrt_approx(rs);
-  const float tq = q * ri * ri * ri;
-  ax = fmaf(dx, tq, ax); ay = fmaf(dy, tq, ay); az = fmaf(dz, tq, az);
-}
-
-__device__ __forceinline__ void close_force(float xt, float yt, float zt, double x, double y,
-                                         double z, const float4* fs, const double4* s64,
-                                         int slice, int tpt, int ns, int selfj, float del,
-                                         float thr, double del64, double& cx, double& cy,
-                                         double& cz) {
-  for (int j = slice; j < ns; j += tpt)
-    if (j != selfj && r2_32(xt, yt, zt, fs[j], del) < thr) fpair(x, y, z, s64[j], del64, cx, cy, cz);
-}
-
-// Threads per target for an entry with cnt targets: the power of two (1..32, or up to a tuned
-// cap) that keeps the most of the CTA's threads busy over the rounds of NT units (a larger
-// split must win by 4% to be taken, since it adds a shuffle reduction and shortens each
-// thread's run).
-__device__ __forceinline__ int split_for(int cnt, int cap) {
-  const int maxtp = cap > 0 ? cap : 32;
-  int best = 1;
-  float bu = 0.f;
-  for (int tp = 1; tp <= maxtp; tp <<= 1) {
-    const int units = cnt * tp;
-    const int rounds = (units + NT - 1) / NT;
-    const float util = (float)units / (float)(rounds * NT);
-    if (util > bu + 0.04f) {
-      bu = util;
-      best = tp;
+  if constexpr (FK == F_ORDER) {
+    double temp = 1.0 / (sqrt(rs) * rs), g = temp;
+    for (int l = 1; l <= f.korder; l++) {
+      g = g * (l + 0.5) / l * f.del / rs;
+      temp += g;
+    }
+    const double t = q * temp;
+    ax = fma(dx, t, ax); ay = fma(dy, t, ay); az = fma(dz, t, az);
+  } else {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(rs));
+    if constexpr (FK == F_COULOMB) {
+      const double y2 = y0 * y0;
+      const double e = fma(-rs, y2, 1.0);
+      const double t = (q * y0) * y2 * fma(e, fma(e, 1.875, 1.5), 1.0);
+      ax = fma(dx, t, ax); ay = fma(dy, t, ay); az = fma(dz, t, az);
+    } else {
+      const double u = rs * y0;
+      const double e = fma(-u, y0, 1.0);
+      const double ec = e * fma(e, 0.375, 0.5);
+      const double ri = fma(y0, ec, y0);
+      const double ex = exp_scaled<UF, kExpTabCopies>(fma(u, ec, u), f.k, f.tab);
+      const double t = q * ex * (ri * ri) * (f.kappa + ri);
+      ax = fma(-dy, t, ax); ay = fma(dx, t, ay);
     }
   }
-  return best;
 }
 
-// Shared-memory layout of one CTA: two source tiles of `tile` records, then the
-// accumulators, the packed target list and the mbarriers (target
-// coordinates are read through L1).
-template <bool F32>
-struct Smem {
-  using S = typename Prec<F32>::S;
-  static constexpr size_t acc = 3 * kGroupMax * sizeof(double);
-  static constexpr size_t list = kGroupMax * sizeof(int);
-  static constexpr size_t bars = 64;
-  __host__ __device__ static size_t tiles(int tile) { return 2 * (size_t)tile * sizeof(S); }
-  __host__ __device__ static size_t total(int tile) { return tiles(tile) + acc + list + bars; }
+struct Vec {
+  double x, y, z;
 };
 
-// The whole near field of group g, by the whole CTA.  If a bounded wait gave up, the error
-// flag is set, and the CTA has waited, bounded again, for its copies in flight.
-template <int KER, bool F32>
-__device__ __forceinline__ void near_group(const NearArgs& a, int g) {
-  using P = Prec<F32>;
-  using S = typename P::S;
-  using T = typename P::T;
-  using L = Smem<F32>;
-  const int TILE = a.tile;
+template <int FK, bool SELF, bool UF>
+__device__ __forceinline__ void two64(const double4* src, int n, const Field& f, Vec s, Vec t, int o0, int o1,
+                                      Vec& p, Vec& r) {
+  p = r = Vec{0.0, 0.0, 0.0};
+  Vec p1 = p, r1 = p;
+  int j = 0;
+#pragma unroll 1
+  for (; j + 1 < n; j += 2) {
+    const double4 a = src[j], b = src[j + 1];
+    field64<FK, SELF, UF>(s.x, s.y, s.z, a, f, j == o0, p.x, p.y, p.z);
+    field64<FK, SELF, UF>(t.x, t.y, t.z, a, f, j == o1, r.x, r.y, r.z);
+    field64<FK, SELF, UF>(s.x, s.y, s.z, b, f, j + 1 == o0, p1.x, p1.y, p1.z);
+    field64<FK, SELF, UF>(t.x, t.y, t.z, b, f, j + 1 == o1, r1.x, r1.y, r1.z);
+  }
+  if (j < n) {
+    field64<FK, SELF, UF>(s.x, s.y, s.z, src[j], f, j == o0, p.x, p.y, p.z);
+    field64<FK, SELF, UF>(t.x, t.y, t.z, src[j], f, j == o1, r.x, r.y, r.z);
+  }
+  p.x += p1.x; p.y += p1.y; p.z += p1.z;
+  r.x += r1.x; r.y += r1.y; r.z += r1.z;
+}
+
+template <int FK, bool SELF, bool UF>
+__device__ __forceinline__ Vec one64(const double4* src, int n, const Field& f, Vec s, int o, int j, int step) {
+  Vec p{0.0, 0.0, 0.0}, q = p;
+#pragma unroll 1
+  for (; j + step < n; j += 2 * step) {
+    field64<FK, SELF, UF>(s.x, s.y, s.z, src[j], f, j == o, p.x, p.y, p.z);
+    field64<FK, SELF, UF>(s.x, s.y, s.z, src[j + step], f, j + step == o, q.x, q.y, q.z);
+  }
+  if (j < n) field64<FK, SELF, UF>(s.x, s.y, s.z, src[j], f, j == o, p.x, p.y, p.z);
+  return Vec{p.x + q.x, p.y + q.y, p.z + q.z};
+}
+
+// Mixed: one target (offset from the leaf centre, negated and doubled) against records k,
+// k + step, ...; careful: its own source, the empty half and close pairs add nothing.
+struct Tile32 {
+  const ulonglong2* rec;
+  const double4* s64;  // the tile's sources in FP64
+  int n;
+  float del, thr;
+};
+template <bool CAREFUL>
+__device__ __forceinline__ void field32(const Tile32& r, int k, f32x2 nx, f32x2 ny, f32x2 nz, int o, float& ax,
+                                        float& ay, float& az, bool& close) {
+  const ulonglong2 u = r.rec[2 * k], v = r.rec[2 * k + 1];
+  const f32x2 dx = add2(u.x, nx), dy = add2(u.y, ny), dz = add2(v.x, nz);
+  float2 f = unpack2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, pack2(r.del, r.del)))));
+  float2 q = unpack2(v.y);
+  if (CAREFUL) {
+    const bool in0 = 2 * k != o, in1 = 2 * k + 1 != o && 2 * k + 1 < r.n;
+    const bool c0 = f.x < r.thr, c1 = f.y < r.thr;
+    close |= (in0 && c0) || (in1 && c1);
+    if (!in0 || c0) { q.x = 0.f; f.x = 1.f; }
+    if (!in1 || c1) { q.y = 0.f; f.y = 1.f; }
+  }
+  const float i0 = rsqrt_approx(f.x), i1 = rsqrt_approx(f.y);
+  const float t0 = q.x * i0 * i0 * i0, t1 = q.y * i1 * i1 * i1;
+  const float2 x = unpack2(dx), y = unpack2(dy), z = unpack2(dz);
+  ax = fmaf(-x.x, t0, ax); ay = fmaf(-y.x, t0, ay); az = fmaf(-z.x, t0, az);
+  ax = fmaf(-x.y, t1, ax); ay = fmaf(-y.y, t1, ay); az = fmaf(-z.y, t1, az);
+}
+template <bool CAREFUL>
+__device__ __forceinline__ Vec sum32(const Tile32& r, double px, double py, double pz, float x, float y, float z,
+                                     double del, int o, int k0, int step) {
+  const f32x2 nx = pack2(-x, -x), ny = pack2(-y, -y), nz = pack2(-z, -z);
+  const int nr = (r.n + 1) >> 1;
+  float ax = 0.f, ay = 0.f, az = 0.f, bx = 0.f, by = 0.f, bz = 0.f;
+  bool close = false;
+  int k = k0;
+#pragma unroll 1
+  for (; k + step < nr; k += 2 * step) {
+    field32<CAREFUL>(r, k, nx, ny, nz, o, ax, ay, az, close);
+    field32<CAREFUL>(r, k + step, nx, ny, nz, o, bx, by, bz, close);
+  }
+  if (k < nr) field32<CAREFUL>(r, k, nx, ny, nz, o, ax, ay, az, close);
+  Vec p{(double)(ax + bx), (double)(ay + by), (double)(az + bz)};
+  if (CAREFUL && close) {  // this lane's close pairs, in FP64
+    const float* f = reinterpret_cast<const float*>(r.rec);
+    Field c{};
+    c.del = del;
+    for (k = k0; k < nr; k += step)
+      for (int j = 2 * k; j < min(2 * k + 2, r.n); j++) {
+        const float* s = f + 8 * (j >> 1) + (j & 1);
+        if (j != o && r2_32(x, y, z, make_float4(s[0], s[2], s[4], 0.f), r.del) < r.thr)
+          field64<F_COULOMB, false, false>(px, py, pz, r.s64[j], c, false, p.x, p.y, p.z);
+      }
+  }
+  return p;
+}
+
+struct Layout {
+  int recs, rows, tab;  // records of a tile, targets of a row, bytes of the exponential's table
+  int single;           // no scratch: part 0 takes the whole group
+  __host__ __device__ size_t warp_bytes() const {
+    return 2 * (size_t)recs * kRec + (size_t)rows * (3 * sizeof(double) + sizeof(unsigned short));
+  }
+  __host__ __device__ size_t total() const { return tab + NW * warp_bytes(); }
+};
+
+// near_item of near.cu with three sums.  FIELD kinds per launch: FK.
+template <int FK, bool F32>
+__global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L) {
+  constexpr int PER = F32 ? 2 : 1;  // sources of a record
+  __shared__ uint64_t bar[2 * NW];
+  __shared__ int s_last;
   extern __shared__ __align__(128) unsigned char sm[];
-  S* tiles = reinterpret_cast<S*>(sm);
-  const double* cx = a.tx + 0;  // group targets, indexed t0 + i below
-  const double* cy = a.ty + 0;
-  const double* cz = a.tz + 0;
-  unsigned char* rest = sm + L::tiles(TILE);
-  double* accd = reinterpret_cast<double*>(rest);
-  int* tl = reinterpret_cast<int*>(rest + L::acc);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(rest + L::acc + L::list);
-  __shared__ int s_cnt;
+  const int TILE = L.recs * PER;
+  const int2 item = a.items[blockIdx.x];
+  const int g = item.x, part = L.single ? 0 : item.y & 0xffff, parts = L.single ? 1 : item.y >> 16;
+  if (L.single && (item.y & 0xffff)) return;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (L.tab) exp_tab_fill(reinterpret_cast<double2*>(sm), tid, 32 * NW);
+  if (tid == 0) {
+    for (int k = 0; k < 2 * NW; k++) mbar_init(&bar[k], 1);
+    fence_mbar_init();
+  }
+  unsigned phase = 0;
+  unsigned char* tiles0 = sm + L.tab;
+  unsigned char* tiles = tiles0 + (size_t)w * 2 * L.recs * kRec;
+  double* rows = reinterpret_cast<double*>(tiles0 + NW * 2 * (size_t)L.recs * kRec);
+  double* row = rows + (size_t)w * 3 * L.rows;
+  unsigned short* tl = reinterpret_cast<unsigned short*>(rows + (size_t)NW * 3 * L.rows) + (size_t)w * L.rows;
 
   const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
   const SysEval* se = a.sys + a.g_sys[g];
-  const double sdel = se->near_del, skappa = se->kappa;
   const int W = (tc + 31) >> 5;
-  const long long e0 = a.off[g], e1 = e0 + a.cnt[g];
-  const long long m0 = a.moff[g];
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int k = tid; k < 3 * kGroupMax; k += NT) accd[k] = 0.0;
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  if (e0 < e1) {
-    const S* src = reinterpret_cast<const S*>(a.src);
-    const float del = (float)sdel;
-    // job iterator: (entry e, first source of the tile in the entry's leaf)
-    long long e = e0;
-    int node = a.node[e];
-    int j0 = a.start[node], jn = a.nummemb[node];
-    int toff = 0;
-    if (tid == 0) {
-      const int cnt0 = min(TILE, jn);
-      fence_proxy_async();
-      mbar_expect_tx(&bar[0], cnt0 * (unsigned)sizeof(S));
-      tma_load_1d(tiles, src + j0, cnt0 * (unsigned)sizeof(S), &bar[0]);
-    }
-    int k = 0, tpt = 1, cnt = 0;
-    while (true) {
-      const int buf = k & 1;
-      const int ns = min(TILE, jn - toff);
-      if (toff == 0 && tid < 32) {
-        // pack the targets of this entry (warp 0)
-        unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-        const int c = __popc(wd);
-        int pre = c;
-        for (int o = 1; o < 32; o <<= 1) {
-          int t = __shfl_up_sync(0xffffffffu, pre, o);
-          if (lane >= o) pre += t;
-        }
-        int base = pre - c;
-        while (wd) {
-          const int b = __ffs(wd) - 1;
-          wd &= wd - 1;
-          tl[base++] = 32 * lane + b;
-        }
-        if (lane == 31) s_cnt = pre;
-      }
-      // the next job streams into the other buffer while this one is consumed
-      long long ne = e;
-      int noff = toff + TILE;
-      if (noff >= jn) { ne = e + 1; noff = 0; }
-      if (tid == 0 && ne < e1) {
-        const int nd = a.node[ne];
-        const int cntn = min(TILE, a.nummemb[nd] - noff);
+  const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
+  const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
+  for (int i = tid; i < NW * 3 * L.rows; i += 32 * NW) rows[i] = 0.0;
+  const long long tot = a.tot[g];
+  const int nv = NW * parts, v = part * NW + w;
+  const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
+  long long e = run_entry(a.pre, e0, e1, T0);
+  __syncthreads();  // the rows are zero, the table and the barriers are there
+  Field f;
+  f.del = se->near_del;
+  f.kappa = se->kappa;
+  f.k = exp_scale(se->kappa);
+  f.tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
+  f.korder = se->kernel_order;
+  bool failed = false;
+  for (; e < e1; e++) {
+    const long long P = a.pre[e];
+    if (P >= T1) break;
+    const int node = a.node[e], ns = a.nummemb[node], cnt = a.tgt[e];
+    const int wt = near_weight(cnt);
+    const int ja = cut(T0, P, wt, ns), jb = cut(T1, P, wt, ns);
+    if (ja >= jb) continue;
+    const int s0 = a.start[node];
+    const unsigned char* src =
+        reinterpret_cast<const unsigned char*>(a.src) + (size_t)(F32 ? a.pstart[node] : s0) * kRec;
+    auto fetch = [&](int j, unsigned n) {
+      if (lane == 0) {
+        const int c = min(jb, (j / TILE + 1) * TILE) - j;
+        const unsigned bytes = (unsigned)((c + PER - 1) / PER) * kRec;
         fence_proxy_async();
-        mbar_expect_tx(&bar[buf ^ 1], cntn * (unsigned)sizeof(S));
-        tma_load_1d(tiles + (buf ^ 1) * TILE, src + a.start[nd] + noff,
-                    cntn * (unsigned)sizeof(S), &bar[buf ^ 1]);
+        mbar_expect_tx(&bar[2 * w + (n & 1)], bytes);
+        tma_load_1d(tiles + (n & 1) * L.recs * kRec, src + (size_t)(j / PER) * kRec, bytes, &bar[2 * w + (n & 1)]);
       }
-      // Every thread waits (bounded) for this job's tile; the barrier then combines the
-      // outcomes, so the whole CTA takes the same branch.  On a timeout the CTA waits,
-      // bounded again, for both copies it may still have in flight into its shared memory
-      // before it returns, and the host reports the error flag.
-      const bool landed = mbar_wait(&bar[buf], (k >> 1) & 1);
-      if (__syncthreads_or(!landed)) {
-        if (tid == 0) {
-          atomicOr(a.err, 2);
-          mbar_wait(&bar[buf], (k >> 1) & 1);
-          if (ne < e1) mbar_wait(&bar[buf ^ 1], ((k + 1) >> 1) & 1);
-        }
-        __syncthreads();
-        return;
-      }
-      if (toff == 0) {
-        cnt = s_cnt;
-        tpt = split_for(cnt, a.split);
-      }
-      const S* ts = tiles + buf * TILE;
-      const double4 c = a.nodec[node];
-      // Particle targets: target i's own source sits at its sorted position t0 + i, i.e.
-      // at tile index i + selfbase, which is inside this tile only if the target is one
-      // of the tile's sources.
-      const int selfbase = se->particles ? (t0 - (j0 + toff)) : INT_MIN;
-      const int units = cnt * tpt;
-      const int lt = __ffs(tpt) - 1;
-      // close-pair checks are needed only where a target comes within r_t of this leaf's box
-      float thr = fmaxf((float)c.w * kCloseFrac, kThrMin);  // r_t^2 = sqradius / 1024
-      // the FP32 r^2 is at least del (fmaf of non-negative squares onto del), so where del
-      // reaches thr no pair of this tile can be close: thr = 0 keeps every warp on the
-      // plain loop (no box distance is below 0), which is then exact
-      if (!(del < thr)) thr = 0.f;
-      const float4 hb = a.nodeh[node];
-      const double4* s64 = a.src64 + j0 + toff;
-      for (int u0 = 0; u0 < units; u0 += NT) {
-        const int u = u0 + tid;
-        const bool valid = u < units;
-        const int slot = u >> lt, slice = u & (tpt - 1);
-        const int i = valid ? tl[slot] : 0;
-        const int selfj = selfbase == INT_MIN ? -1 : i + selfbase;
-        const bool self_in = selfj >= 0 && selfj < ns && ((selfj - slice) & (tpt - 1)) == 0;
-        // the target's own source in this lane's slice: sum around it
-        const int je = self_in ? selfj : ns;
-        {
-          T fx = 0, fy = 0, fz = 0;
-          if constexpr (F32) {
-            const float4* fs = reinterpret_cast<const float4*>(ts);
-            const float xt = (float)(cx[t0 + i] - c.x), yt = (float)(cy[t0 + i] - c.y),
-                        zt = (float)(cz[t0 + i] - c.z);
-            const bool chk = __any_sync(0xffffffffu, valid && box_d2(xt, yt, zt, hb) < thr);
-            if (valid) {
-              bool close = false;
-              if (!chk) {
-                for (int j = slice; j < je; j += tpt)
-                  acc_force<false>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-                if (self_in)
-                  for (int j = selfj + tpt; j < ns; j += tpt)
-                    acc_force<false>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-              } else {
-                for (int j = slice; j < je; j += tpt)
-                  acc_force<true>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-                if (self_in)
-                  for (int j = selfj + tpt; j < ns; j += tpt)
-                    acc_force<true>(xt, yt, zt, fs[j], del, thr, fx, fy, fz, close);
-              }
-              if (close) {
-                double qx = 0.0, qy = 0.0, qz = 0.0;
-                close_force(xt, yt, zt, cx[t0 + i], cy[t0 + i], cz[t0 + i], fs, s64, slice, tpt,
-                            ns, selfj, del, thr, sdel, qx, qy, qz);
-                fx += (float)qx; fy += (float)qy; fz += (float)qz;
-              }
-            }
-          } else {
-            if (valid) {
-              const double4* ds = reinterpret_cast<const double4*>(ts);
-              const double x = cx[t0 + i], y = cy[t0 + i], z = cz[t0 + i];
-              const int korder = se->kernel_order;
-              if (KER == BIT_KERNEL_SCREENED) {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) cpair(x, y, z, ds[j], skappa, fx, fy);
-              } else if (korder > 0) {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) fpair_order(x, y, z, ds[j], sdel, korder, fx, fy, fz);
-              } else {
-                for (int j = slice; j < ns; j += tpt)
-                  if (j != selfj) fpair(x, y, z, ds[j], sdel, fx, fy, fz);
-              }
-            }
-          }
-          fx = shfl_sum(fx, tpt);
-          fy = shfl_sum(fy, tpt);
-          fz = shfl_sum(fz, tpt);
-          if (valid && slice == 0) {
-            accd[i] += (double)fx;
-            accd[kGroupMax + i] += (double)fy;
-            accd[2 * kGroupMax + i] += (double)fz;
-          }
-        }
-      }
-      __syncthreads();
-      k++;
-      if (ne >= e1) break;
-      if (ne != e) {
-        e = ne;
-        node = a.node[e];
-        j0 = a.start[node];
-        jn = a.nummemb[node];
-      }
-      toff = noff;
+    };
+    fetch(ja, phase);
+    const bool all = cnt == tc;
+    if (!all) {
+      const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
+      pack_list(wd, W, tl);
     }
+    const bool self = s0 < t0 + tc && t0 < s0 + ns;
+    const double4 c = a.nodec[node];
+    const float4 hb = a.nodeh[node];
+    const NearSteps st = near_steps(cnt);
+    for (int j = ja; j < jb;) {
+      const int jn = min(jb, (j / TILE + 1) * TILE);
+      if (jn < jb) fetch(jn, phase + 1);  // (its buffer's reads ended at the last __syncwarp)
+      if (!__all_sync(0xffffffffu, mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1))) {
+        if (lane == 0) {
+          atomicOr(a.err, 2);
+          mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1);
+          if (jn < jb) mbar_wait(&bar[2 * w + ((phase + 1) & 1)], ((phase + 1) >> 1) & 1);
+        }
+        __syncwarp();
+        failed = true;
+        break;
+      }
+      const unsigned char* tile = tiles + (phase & 1) * L.recs * kRec;
+      phase++;
+      const int n = jn - j, own0 = t0 - s0 - j;
+      auto add = [&](int i, const Vec& p) {
+        row[i] += p.x;
+        row[L.rows + i] += p.y;
+        if (FK != F_CURL) row[2 * L.rows + i] += p.z;
+      };
+      if constexpr (F32) {
+        Tile32 r{reinterpret_cast<const ulonglong2*>(tile), a.src64 + s0 + j, n, (float)f.del, near_close_thr(c.w)};
+        if (!(r.del < r.thr)) r.thr = 0.f;
+        auto sum = [&](int i, int k, int step) {
+          const float x = (float)(cx[i] - c.x), y = (float)(cy[i] - c.y), z = (float)(cz[i] - c.z);
+          return self || __any_sync(0xffffffffu, box_d2(x, y, z, hb) < r.thr)
+                     ? sum32<true>(r, cx[i], cy[i], cz[i], x, y, z, f.del, self ? i + own0 : -1, k, step)
+                     : sum32<false>(r, cx[i], cy[i], cz[i], x, y, z, f.del, -1, k, step);
+        };
+        for (int b = 0; b < cnt - 31; b += 32) {
+          const int i = all ? b + lane : tl[b + lane];
+          add(i, sum(i, 0, 1));
+        }
+        if (cnt & 31) {
+          const int r0 = cnt & 31, sh = near_tail_shift(r0), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+          const bool in = slot < r0;
+          const int q = (cnt & ~31) + (in ? slot : 0), i = all ? q : tl[q];
+          Vec p = sum(i, slice, 1 << sh);
+          for (int o = 1 << sh >> 1; o; o >>= 1) {
+            p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
+            p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
+            p.z += __shfl_xor_sync(0xffffffffu, p.z, o);
+          }
+          if (in && slice == 0) add(i, p);
+        }
+      } else {
+        const double4* ds = reinterpret_cast<const double4*>(tile);
+        auto run = [&](auto S, auto U) {
+          constexpr bool SELF = decltype(S)::value, UF = decltype(U)::value;
+          for (int b = 0; b < st.full; b++) {
+            const int r0 = 64 * b + lane, r1 = r0 + 32;
+            const bool v1 = r1 < cnt;  // (a partial last block holds more than 48: r0 is a target)
+            const int i0 = all ? r0 : tl[r0], i1 = v1 ? (all ? r1 : tl[r1]) : i0;
+            Vec p, q;
+            two64<FK, SELF, UF>(ds, n, f, Vec{cx[i0], cy[i0], cz[i0]}, Vec{cx[i1], cy[i1], cz[i1]}, i0 + own0,
+                                i1 + own0, p, q);
+            add(i0, p);
+            if (v1) add(i1, q);
+          }
+          int base = 64 * st.full;
+          if (st.one) {
+            const int i = all ? base + lane : tl[base + lane];
+            add(i, one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, 0, 1));
+            base += 32;
+          }
+          if (st.tail) {
+            const int sh = near_tail_shift(st.tail), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+            const bool in = slot < st.tail;
+            const int r0 = base + (in ? slot : 0), i = all ? r0 : tl[r0];
+            Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, slice, 1 << sh);
+            for (int o = 1 << sh >> 1; o; o >>= 1) {
+              p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
+              p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
+              p.z += __shfl_xor_sync(0xffffffffu, p.z, o);
+            }
+            if (in && slice == 0) add(i, p);
+          }
+        };
+        // (the careful forms only where they can matter)
+        if (FK == F_CURL && se->underflow) run(std::true_type{}, std::true_type{});
+        else if (self) run(std::true_type{}, std::false_type{});
+        else run(std::false_type{}, std::false_type{});
+      }
+      __syncwarp();
+      j = jn;
+    }
+    if (failed) break;
   }
   __syncthreads();
-  for (int i = tid; i < tc; i += NT) {
-    a.out[t0 + i] += accd[i];
-    a.out_y[t0 + i] += accd[kGroupMax + i];
-    a.out_z[t0 + i] += accd[2 * kGroupMax + i];
+  // as near_item: straight into the result, or the group's scratch and then in part order
+  auto warps_sum = [&](int d, int i) {
+    double s = 0.0;
+    for (int q = 0; q < NW; q++) s += rows[((size_t)q * 3 + d) * L.rows + i];
+    return s;
+  };
+  double* sum = a.part + 3 * a.part_off[g];
+  if (parts > 1) {
+    for (int i = tid; i < 3 * tc; i += 32 * NW) sum[(long long)part * 3 * tc + i] = warps_sum(i / tc, i % tc);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      s_last = atomicAdd(&a.part_done[g], 1) == parts - 1;
+      if (s_last) {
+        a.part_done[g] = 0;
+        __threadfence();
+      }
+    }
+    __syncthreads();
+    if (!s_last) return;
   }
-}
-
-// One launch class: CTA b takes group order[b].
-template <int KER, bool F32>
-__global__ void __launch_bounds__(NT) k_near_field(NearArgs a) {
-  near_group<KER, F32>(a, a.order[blockIdx.x]);
-}
-
-template <int KER, bool F32>
-void launch(const NearArgs& a, int ngroups, cudaStream_t s) {
-  const size_t bytes = Smem<F32>::total(a.tile);
-  ensure_smem_attr(reinterpret_cast<const void*>(k_near_field<KER, F32>),
-                   (int)Smem<F32>::total(Prec<F32>::TILE_MAX));
-  count_launch(), k_near_field<KER, F32><<<ngroups, NT, bytes, s>>>(a);
+  for (int i = tid; i < 3 * tc; i += 32 * NW) {
+    const int d = i / tc, k = i % tc;
+    double s = 0.0;
+    if (parts > 1) {
+      for (int q = 0; q < parts; q++) s += __ldcg(sum + (long long)q * 3 * tc + i);
+    } else {
+      s = warps_sum(d, k);
+    }
+    (d == 0 ? a.out : d == 1 ? a.out_y : a.out_z)[t0 + k] += s;
+  }
 }
 
 }  // namespace
@@ -379,19 +395,13 @@ NearArgs near_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const
   a.start = t->start.p;
   a.nummemb = t->nummemb.p;
   a.nodec = t->nodec.p;
-  a.src = P.f32 ? (const void*)t->src32.p : (const void*)t->src64.p;
+  a.src = P.f32 ? (const void*)t->src2.p : (const void*)t->src64.p;
   a.src64 = t->src64.p;
   a.nodeh = t->nodeh.p;
   a.sw = t->has_weights ? t->sw.p : nullptr;
   a.sys = P.sys.p;
   a.g_sys = L->g_sys.p;
   a.err = t->ctx->dev_err();
-  // the context's tile, clamped to the precision's range (0: the default)
-  const int want = t->ctx->near_tile;
-  const int lo = P.f32 ? Prec<true>::TILE_MIN : Prec<false>::TILE_MIN;
-  const int hi = P.f32 ? Prec<true>::TILE_MAX : Prec<false>::TILE_MAX;
-  a.tile = want == 0 ? (P.f32 ? Prec<true>::TILE : Prec<false>::TILE) : std::min(hi, std::max(lo, want));
-  a.split = t->ctx->near_split;
   a.tgt = L->near_tgt.p;
   a.pre = L->near_pre.p;
   a.pstart = t->pstart.p;
@@ -404,22 +414,38 @@ NearArgs near_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const
 }
 
 void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* fy, double* fz) {
-  cudaStream_t s = t->ctx->stream;
+  Ctx* c = t->ctx;
+  cudaStream_t s = c->stream;
   NearArgs a = near_args(t, L, P, t->sx.p, t->sy.p, t->sz.p);
   a.out = fx; a.out_y = fy; a.out_z = fz;
   // P.force: 1 the regularised Coulomb field (kernel order per system; FP64 beyond order
   // 0), 2 the screened 2-D field of shielded_treeforce (FP64)
+  if (P.force == 2 && P.f32) fail(BIT_ERR_INVALID_ARGUMENT, "the screened field is FP64 only");
+  bool korder = false;
+  for (const SysEval& se : P.h_sys) korder |= se.kernel_order > 0;
+  // the parts' scratch, three sums a target; without room in the memory budget a group's first
+  // part takes it whole
+  Layout lay;
+  const size_t need = 3 * (size_t)L->part_total;
+  lay.single = L->field_part.n < need && c->budget && c->in_use + need * sizeof(double) > c->budget;
+  if (!lay.single) L->field_part.ensure(c, need);
+  a.part = L->field_part.p;
+  lay.rows = L->max_targets;
+  lay.tab = P.force == 2 ? kExpTabBytes : 0;
+  lay.recs = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 64;
+  // four CTAs an SM if tiles of 32 do it
+  while (lay.recs > 32 && lay.total() > kSmemMax / 4 - 1024) lay.recs -= 16;
   for (const LaunchClass& k : P.near_classes) {
-    a.order = P.near_ord + k.begin;
-    if (P.force == 2) {
-      if (P.f32) fail(BIT_ERR_INVALID_ARGUMENT, "the screened field is FP64 only");
-      launch<BIT_KERNEL_SCREENED, false>(a, k.count, s);
-    } else if (P.f32) {
-      launch<BIT_KERNEL_COULOMB, true>(a, k.count, s);
-    } else {
-      launch<BIT_KERNEL_COULOMB, false>(a, k.count, s);
-    }
-    BIT_CHECK_LAUNCH();
+    a.items = P.near_it + k.ibegin;
+    auto go = [&](auto kernel) {
+      ensure_smem_attr(reinterpret_cast<const void*>(kernel), kSmemMax - 1024);
+      count_launch(), kernel<<<k.icount, 32 * NW, lay.total(), s>>>(a, lay);
+      BIT_CHECK_LAUNCH();
+    };
+    if (P.force == 2) go(k_near_field<F_CURL, false>);
+    else if (P.f32) go(k_near_field<F_COULOMB, true>);
+    else if (korder) go(k_near_field<F_ORDER, false>);
+    else go(k_near_field<F_COULOMB, false>);
   }
 }
 

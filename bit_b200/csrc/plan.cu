@@ -199,13 +199,9 @@ void plan_classes(Tree* t, Lists* L, EvalPlan* P) {
   }
   if (one_near) {
     P->near_classes.assign(1, LaunchClass{0, s0.kernel, s0.eps_check, s0.far_kind, 0, ng, 0, (int)L->h_items.size()});
-    P->near_ord = L->order.p;
     P->near_it = L->items.p;
   } else {
     order_by_class(L, gn, *P, ord, P->near_classes, false);
-    P->near_order.ensure(c, ng);
-    BIT_CUDA(cudaMemcpyAsync(P->near_order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, st));
-    P->near_ord = P->near_order.p;
     std::vector<int2> it;
     for (LaunchClass& k : P->near_classes) {
       k.ibegin = (int)it.size();

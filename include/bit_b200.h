@@ -113,12 +113,11 @@ bit_status bit_ctx_set_group_size(bit_ctx* ctx, int targets);
  * take (system, target group) items from a device work queue in decreasing-work order;
  * 0 launches once per class.  Results are identical either way. */
 bit_status bit_ctx_set_work_queue(bit_ctx* ctx, int on);
-/* Near-field tuning knobs (bit_b200.autotune): `tile` source records per TMA tile (a power
- * of two, 128..2048; 0: the default).  Fields: clamped to 256..2048 for the mixed path and
- * 128..1024 for FP64, default 1024 / 512.  Potentials: shared by a CTA's eight warps, an
- * eighth each (32..128, default 64, less where shared memory is short).  And, for fields, the
- * cap on threads that share one target's sources (a power of two, 1..32; 0: the default
- * rule).  Results change only in FP rounding order. */
+/* Near-field tuning knobs (bit_b200.autotune): `tile` source records per CTA (a power of two,
+ * 128..2048; 0: the default, 512), shared by its eight warps, an eighth each (32..128 records,
+ * less where shared memory is short); `threads_per_target` (a power of two, 1..32; 0) is
+ * accepted and has no effect: targets share a source's lanes as their number asks.  Results
+ * change only in FP rounding order. */
 bit_status bit_ctx_set_near_config(bit_ctx* ctx, int tile, int threads_per_target);
 bit_status bit_ctx_stream(const bit_ctx* ctx, void** stream);
 /* Bytes currently allocated by the context and its trees. */
