@@ -162,8 +162,7 @@ struct ListSizing {
   double acc = -1;                          // the build's MAC parameter
   int points = 0;
   unsigned long long totals[4] = {0, 0, 0, 0};  // far entries, far words, near entries, near words
-  long long stage[2] = {0, 0};              // largest group: far, near staging words
-                                            // (entries x (mask words + 1))
+  long long visits = 0;                     // most nodes that a group visited
 };
 
 struct Lists {
@@ -198,9 +197,9 @@ struct Lists {
   long long part_total = 0;                 // sums of a potential in scratch
   long long version = 0;                    // bumped by every build
   ListSizing last;                          // the last build's sizes
-  bool fallback = false;                    // the last build used count, scan and fill
-  DBuf<unsigned> gstage;                    // per resident CTA: staging of one group's entries
-  DBuf<int> head;                           // the single-pass build's work counter
+  bool fallback = false;                    // the last build was run again, with more room
+  DBuf<unsigned> gstage;                    // per resident CTA: the visits of one group
+  DBuf<int> head;                           // the build's work counter
   // The lists also serve alt_key when alt_valid: the build checked that MAC at every
   // (target, node) it visited and no decision differed, so that MAC's own traversal
   // would have visited the same nodes and emitted the same entries.
@@ -272,7 +271,7 @@ struct Tree {
   DBuf<double> fields;   // 13 per node
   DBuf<double4> nodec;   // (xmid, ymid, zmid, sqradius)
   DBuf<float4> nodeh;    // half extents of the box about the midpoint (rounded up)
-  DBuf<int2> kids;       // children: (first index or -1, count | slot order 3 bits each)
+  DBuf<int2> kids;       // children: (first index, count), or a leaf (-1, members)
   // host mirror of the node structure
   std::vector<int> h_nummemb, h_start, h_children, h_perm;
   std::vector<double> h_fields;

@@ -2,26 +2,38 @@
 // (src/tree3d.cpp:4679-4778, 3448-3627, 851-971) for a whole group of targets at once.
 //
 // A group is up to 1024 consecutive targets (a run of consecutive small leaves, a leaf, or
-// a chunk of one; for external points, 256 consecutive points in Morton order).  One CTA walks the tree for the group,
-// one thread per target, one 32-bit mask word per warp.  At a node every active target
+// a chunk of one; for external points, 256 consecutive points in Morton order).  One CTA walks
+// the tree for the group, with a 32-bit mask word per 32 targets.  At a node every active target
 // evaluates the reference's acceptance test in FP64 without contraction
 // (sqradius < acc * ((dx*dx + dy*dy + dz*dz + add) - sub)); the node becomes a far entry
-// for the accepting targets, and the others descend into the children in the reference's
-// children[] order, or get a near entry at a leaf.  Entries carry the group's bitmask.
-// Restricted to one target, the entries are exactly its reference traversal, in order.
-// In a forest the walk starts at the root of the group's system, with that system's MAC.
+// for the accepting targets, and the others descend into the children, or get a near entry at
+// a leaf.  Entries carry the group's bitmask.  Restricted to one target, the entries are
+// exactly those of its reference traversal.  In a forest the walk starts at the root of the
+// group's system, with that system's MAC.
 //
-// Single pass: a persistent kernel whose CTAs take groups from a device counter; each CTA
-// stages a group's entries in its own region of global memory, then reserves room in the
-// global lists with one atomic per list and copies them out (a group's entries stay
-// contiguous and in order; groups land in completion order, addressed by begin/count).
-// The lists are written in place, into arrays sized from an estimate, and the staging
-// regions are sized from the largest group of the previous build (of this tree, else the
-// context's last build under the same MAC; a first build uses an allowance; no region is
-// larger than the tree's worst case, every node a far entry and every leaf a near one).
-// A group that overflows its staging region, or a reservation that runs past the arrays,
-// makes the whole build fall back to a count pass, a prefix sum and a fill pass; so does
-// a context whose memory budget has no room for the staging.
+// k_lists is a persistent kernel whose CTAs take groups from a device counter and visit each
+// group's nodes breadth first, which is by increasing index, up to 256 waiting nodes at a time:
+// one thread per node tests the box of the group's targets, the warps test the nodes that this
+// leaves open against the targets they hold (one mask word or up to four a warp), then
+// one thread per node places its far or near entry and its children by prefix sums.  What the
+// group has visited (its reject masks above all) stays in the CTA's own region of global
+// memory; the CTA then reserves room in the global lists with one atomic per list and writes
+// the entries out (a group's entries are contiguous and in the order of the visits; groups land
+// in completion order, addressed by begin/count).
+//
+// The lists are written in place, into arrays sized from an estimate, and the regions from the
+// group with the most visits of the previous build (of this tree, else the context's last build
+// under the same MAC; a first build uses an allowance).  Where a group overflows its region, or
+// a reservation runs past the arrays, the build is run again, with four times the room a group
+// (up to every node of the tree), or with room for the totals that this run counted: the same
+// lists, later.  A memory budget limits the regions to as many as fit.
+//
+// Bound by issue and latency (tensor and FP64 pipes idle, everything in L1 and L2).  Walking
+// depth first, one node at a time and a thread per target, against this; a whole build with its
+// host part, us: 2M particles, leaves of 1000: 3200 -> 1250; 300k, leaves of 100: 3500 -> 750;
+// 200k, 500: 517 -> 258; 50k, 300: 235 -> 140; 10k, 200: 117 -> 82.  Of that the box test took
+// the kernel from 1310 to 545 (2M) and from 200 to 116 (200k): half of the issue slots went to
+// tests whose outcome the group shares.
 //
 // Optionally the walk also evaluates a second MAC (another kernel's parameters, e.g. the
 // Coulomb test's (r^2 + del) - del next to the screened r^2 - mac_del) at every (target,
@@ -29,6 +41,7 @@
 // and emit the same entries, so the lists serve both MACs bit for bit; one differing
 // decision anywhere and they serve only their own.
 #include <algorithm>
+#include <climits>
 #include <numeric>
 #include <vector>
 
@@ -39,18 +52,16 @@ namespace bit {
 
 namespace {
 
-constexpr int LT = 1024;          // threads of the list builder (one per target of a group)
-constexpr int LSTK = 256;         // traversal stack entries per group
-constexpr size_t STACK_BYTES = 32 * LSTK * sizeof(int);  // per-warp node stacks
-constexpr long long STAGE_FIRST[2] = {768 * 33, 192 * 33};  // first build: far, near words
-
-enum { MODE_COUNT = 0, MODE_FILL = 1, MODE_STAGE = 2 };
+constexpr long long kVisitsFirst = 768;  // first build: visits of a group
+constexpr int kVisitWords = 7;           // of a visit's record, next to its mask words
+constexpr int QT = 256;                  // threads of the builder
+constexpr size_t kRegionBytes = 1u << 30;  // of all regions, one at least
 
 struct ListArgs {
   const int *g_tstart, *g_tcount;
   const double *tx, *ty, *tz;
   const double4* nodec;
-  const int2* kids;  // per node: (first child, count | slot order), a leaf (-1, members)
+  const int2* kids;  // per node: (first child, count), a leaf (-1, members)
   const SysEval* sys;  // per system: MAC parameters
   const int* g_sys;    // per group: system (its root is node g_sys[g])
   // per group
@@ -66,16 +77,16 @@ struct ListArgs {
   unsigned *far_mask, *near_mask;
   unsigned long long* totals;  // far entries, far words, near entries, near words
   unsigned long long* pairs;   // far pairs, near pairs
-  int* err;                    // 1: stack overflow, 2: staging or arena overflow,
+  int* err;                    // 1: a region overflowed, 2: the arrays did,
                                // 4: the alternative MAC disagreed somewhere
-  unsigned long long cap[4];   // MODE_STAGE: room in the four output arrays
+  unsigned long long cap[4];   // room in the four output arrays
   int has_alt;                 // also evaluate a second MAC and compare its decisions
   double alt_acc, alt_add, alt_sub;
-  // MODE_STAGE (k_lists_queue): each resident CTA's own staging region in global memory,
-  // stage_far + stage_near words (far nodes | far masks, near nodes | near masks), and the
-  // work counter over the ngroups groups
+  // each resident CTA's own region in global memory, `stage` words, the most
+  // visits of any group (maximum), and the work counter over the ngroups groups
   unsigned* gstage;
-  long long stage_far, stage_near;
+  long long stage;
+  unsigned long long* visits;
   int* head;
   int ngroups;
 };
@@ -85,29 +96,13 @@ __device__ __forceinline__ bool alt_ok(const ListArgs& a, double s, double w) {
   return w < dmul(a.alt_acc, dsub(dadd(s, a.alt_add), a.alt_sub));
 }
 
-// Barrier `id` (1..15) among the first `nthreads` threads of the CTA (a multiple of 32);
-// barrier 0 is __syncthreads.
-__device__ __forceinline__ void bar_sync_n(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// The per-entry targets and work prefixes of group g, whose lists begin at far / near entry
-// fo / no and mask word fmo / nmo (written by this CTA): the potentials' kernels share a
-// group's work out by them, without a pass over the masks of their own.
-__device__ void finish_group(const ListArgs& a, int g, long long nf, long long fo, long long fmo,
-                             long long nn, long long no, long long nmo) {
-  const int W = (a.g_tcount[g] + 31) >> 5;
+// The work prefixes of group g's entries, whose targets are in place: warp 0 the far list (from
+// entry fo), warp 1 the near list (from no).  The potentials' kernels share a group's work out
+// by them.
+__device__ __forceinline__ void group_prefixes(const ListArgs& a, int g, long long nf, long long fo, long long nn,
+                                               long long no) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
-  for (long long k = threadIdx.x; k < nf + nn; k += LT) {
-    const unsigned* m = k < nf ? a.far_mask + fmo + k * W : a.near_mask + nmo + (k - nf) * W;
-    int c = 0;
-    for (int q = 0; q < W; q++) c += __popc(m[q]);
-    if (k < nf) a.far_tgt[fo + k] = c;
-    else a.near_tgt[no + k - nf] = c;
-  }
-  __syncthreads();
-  if (w > 1) return;  // warp 0 the far list, warp 1 the near list
+  if (w > 1) return;
   const long long n = w ? nn : nf;
   long long run = 0;
   for (long long b = 0; b < n; b += 32) {
@@ -131,245 +126,268 @@ __device__ void finish_group(const ListArgs& a, int g, long long nf, long long f
   }
 }
 
-// The walk of group g by the whole CTA.  MODE_COUNT counts the group's entries, MODE_FILL
-// writes them at the offsets a scan gave, MODE_STAGE writes them into the CTA's staging
-// region and then copies them into room reserved with one atomic per list.
-template <int MODE>
-__device__ __forceinline__ void walk_group(const ListArgs& a, int g) {
-  __shared__ unsigned s_mask[LSTK][32];  // each warp's mask word of every stack entry
-  __shared__ unsigned s_am[2][32], s_rm[2][32];  // accept / reject words, by parity
-  __shared__ unsigned long long s_base[4];
-  __shared__ int s_flags;  // the walk's overflow (1) / full staging (2), for every warp
-  __shared__ long long s_n[2];  // the walk's far and near entry counts, for every warp
-  __shared__ unsigned long long s_np;  // the group's near pairs
-  extern __shared__ unsigned dyn[];
-  // dynamic shared memory: each warp's own copy of the node stack
-  int (*s_node)[LSTK] = reinterpret_cast<int (*)[LSTK]>(dyn);
-  unsigned* stage = MODE == MODE_STAGE
-                        ? a.gstage + (size_t)blockIdx.x * (size_t)(a.stage_far + a.stage_near)
-                        : nullptr;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
-  const int W = (tc + 31) >> 5;
-  const int i = threadIdx.x;
-  const int root = a.g_sys[g];
-  const double macc = a.sys[root].acc, madd = a.sys[root].mac_add, msub = a.sys[root].mac_sub;
-  // staging layout: far nodes | far masks, near nodes | near masks
-  const long long fcap = MODE == MODE_STAGE ? a.stage_far / (W + 1) : 0;
-  const long long ncap = MODE == MODE_STAGE ? a.stage_near / (W + 1) : 0;
-  int* sf_node = reinterpret_cast<int*>(stage);
-  unsigned* sf_mask = stage + fcap;
-  int* sn_node = reinterpret_cast<int*>(stage + a.stage_far);
-  unsigned* sn_mask = stage + a.stage_far + ncap;
-  double x = 0, y = 0, z = 0;
-  if (i < tc) { x = a.tx[t0 + i]; y = a.ty[t0 + i]; z = a.tz[t0 + i]; }
-  if (lane == 0) {
-    s_node[w][0] = root;
-    int live = tc - 32 * w;
-    s_mask[0][w] = live >= 32 ? 0xffffffffu : (live > 0 ? (1u << live) - 1u : 0u);
-  }
-  // warps without targets do not walk: their accept / reject words stay 0
-  if (threadIdx.x < 64) {
-    s_am[threadIdx.x >> 5][lane] = 0u;
-    s_rm[threadIdx.x >> 5][lane] = 0u;
-  }
-  if (threadIdx.x == 0) { s_flags = 0; s_np = 0; }
-  int sp = 1;
-  long long nf = 0, nn = 0, fpairs = 0, npairs = 0;
-  const long long fo = MODE == MODE_FILL ? a.far_off[g] : 0, no = MODE == MODE_FILL ? a.near_off[g] : 0;
-  const long long fmo = MODE == MODE_FILL ? a.far_moff[g] : 0, nmo = MODE == MODE_FILL ? a.near_moff[g] : 0;
-  bool overflow = false, full = false, differ = false;
-  __syncthreads();
-  // One barrier per visited node, after every warp has published its accept / reject
-  // words.  Every warp pushes the same children onto its own stack (all threads see the
-  // same children and the same CTA-wide decision), so no warp waits for another's push;
-  // the words alternate between two buffers, so a fast warp never overwrites words a
-  // slow one is still reading (it cannot get two barriers ahead of it).  Only the W warps
-  // that hold targets walk, on barrier 1 among their 32 W threads: they pop the same
-  // entries and take the same number of steps, while the others wait at the barrier after
-  // the walk (a group of 650 targets leaves 11 of the 32 warps idle).
-  int par = 0;
-  while (w < W && sp > 0) {
-    sp--;
-    const int node = s_node[w][sp];
-    const unsigned word = s_mask[sp][w];
-    const int2 kd = a.kids[node];  // loads alongside the centre, needed only to descend
-    bool ok = false;
-    if ((word >> lane) & 1u) {
-      const double4 c = a.nodec[node];
-      double dx = dsub(x, c.x), dy = dsub(y, c.y), dz = dsub(z, c.z);
-      double s = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-      ok = c.w < dmul(macc, dsub(dadd(s, madd), msub));
-      if (a.has_alt) differ |= ok != alt_ok(a, s, c.w);
-    }
-    const unsigned am = __ballot_sync(0xffffffffu, ok) & word;
-    const unsigned rm = word & ~am;
-    if (lane == 0) { s_am[par][w] = am; s_rm[par][w] = rm; }
-    bar_sync_n(1, 32 * W);
-    const bool anyA = __ballot_sync(0xffffffffu, s_am[par][lane] != 0u) != 0u;
-    const bool anyR = __ballot_sync(0xffffffffu, s_rm[par][lane] != 0u) != 0u;
-    par ^= 1;
-    if (anyA) {
-      if (MODE == MODE_FILL) {
-        if (threadIdx.x == 0) a.far_node[fo + nf] = node;
-        if (lane == 0 && w < W) a.far_mask[fmo + nf * W + w] = am;
-      } else if (MODE == MODE_STAGE) {
-        if (nf >= fcap) { full = true; break; }
-        if (threadIdx.x == 0) sf_node[nf] = node;
-        if (lane == 0 && w < W) sf_mask[nf * W + w] = am;
-      }
-      nf++;
-      if (lane == 0) fpairs += __popc(am);
-    }
-    if (anyR) {
-      if (kd.x < 0) {
-        if (MODE == MODE_FILL) {
-          if (threadIdx.x == 0) a.near_node[no + nn] = node;
-          if (lane == 0 && w < W) a.near_mask[nmo + nn * W + w] = rm;
-        } else if (MODE == MODE_STAGE) {
-          if (nn >= ncap) { full = true; break; }
-          if (threadIdx.x == 0) sn_node[nn] = node;
-          if (lane == 0 && w < W) sn_mask[nn * W + w] = rm;
-        }
-        nn++;
-        if (lane == 0) npairs += (long long)__popc(rm) * kd.y;
-      } else {
-        const int cnt = kd.y & 15;
-        if (sp + cnt > LSTK) { overflow = true; break; }
-        // children[k] = kd.x + order[k]; the last slot goes deepest, so children[0] pops first
-        if (lane == 0)
-          for (int k = cnt - 1, q = sp; k >= 0; k--, q++) {
-            s_node[w][q] = kd.x + ((kd.y >> (4 + 3 * k)) & 7);
-            s_mask[q][w] = rm;
-          }
-        sp += cnt;
-      }
-    }
-    __syncwarp();  // this warp's pushes, before its next pop
-  }
-  // the walk's outcome and entry counts for every warp (thread 0's warp walked)
-  if (threadIdx.x == 0) {
-    if (overflow || full) s_flags = overflow ? 1 : 2;
-    s_n[0] = nf;
-    s_n[1] = nn;
-  }
-  __syncthreads();
-  overflow = s_flags == 1;
-  full = s_flags == 2;
-  nf = s_n[0];
-  nn = s_n[1];
-  if (threadIdx.x == 0 && (overflow || full)) atomicOr(a.err, overflow ? 1 : 2);
-  if (a.has_alt && __any_sync(0xffffffffu, differ) && lane == 0) atomicOr(a.err, 4);
-  if (MODE != MODE_FILL && lane == 0 && (fpairs || npairs)) {
-    atomicAdd(&a.pairs[0], (unsigned long long)fpairs);
-    atomicAdd(&a.pairs[1], (unsigned long long)npairs);
-    if (npairs) atomicAdd(&s_np, (unsigned long long)npairs);
-  }
-  if (MODE == MODE_FILL) {
-    finish_group(a, g, nf, fo, fmo, nn, no, nmo);
-    return;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    a.g_near[g] = s_np;
-    if (MODE == MODE_COUNT) {
-      a.far_cnt[g] = (int)nf;
-      a.near_cnt[g] = (int)nn;
-    }
-  }
-  if (MODE != MODE_STAGE || overflow || full) return;
-  if (threadIdx.x == 0) {
-    s_base[0] = atomicAdd(&a.totals[0], (unsigned long long)nf);
-    s_base[1] = atomicAdd(&a.totals[1], (unsigned long long)(nf * W));
-    s_base[2] = atomicAdd(&a.totals[2], (unsigned long long)nn);
-    s_base[3] = atomicAdd(&a.totals[3], (unsigned long long)(nn * W));
-    // the arrays were sized from an estimate: past their end, the build falls back
-    if (s_base[0] + nf > a.cap[0] || s_base[1] + nf * W > a.cap[1] ||
-        s_base[2] + nn > a.cap[2] || s_base[3] + nn * W > a.cap[3]) {
-      atomicOr(a.err, 2);
-      s_base[0] = ~0ull;
-    }
-    a.far_off[g] = (long long)s_base[0];
-    a.far_moff[g] = (long long)s_base[1];
-    a.near_off[g] = (long long)s_base[2];
-    a.near_moff[g] = (long long)s_base[3];
-    a.far_cnt[g] = (int)nf;
-    a.near_cnt[g] = (int)nn;
-  }
-  __syncthreads();
-  if (s_base[0] == ~0ull) return;
-  for (int k = threadIdx.x; k < nf; k += LT) a.far_node[s_base[0] + k] = sf_node[k];
-  for (int k = threadIdx.x; k < nf * W; k += LT) a.far_mask[s_base[1] + k] = sf_mask[k];
-  for (int k = threadIdx.x; k < nn; k += LT) a.near_node[s_base[2] + k] = sn_node[k];
-  for (int k = threadIdx.x; k < nn * W; k += LT) a.near_mask[s_base[3] + k] = sn_mask[k];
-  finish_group(a, g, nf, (long long)s_base[0], (long long)s_base[1], nn, (long long)s_base[2],
-               (long long)s_base[3]);
-}
-
-// Count / fill passes: CTA b walks group b.
-template <int MODE>
-__global__ void __launch_bounds__(LT) k_lists(ListArgs a) {
-  walk_group<MODE>(a, blockIdx.x);
-}
-
-// The single-pass build: a persistent kernel whose CTAs take groups from a device counter
-// and stage each group's entries in their own global-memory region, so that a group is
-// walked once.  No CTA waits for another; the counter is the only shared state.
-__global__ void __launch_bounds__(LT) k_lists_queue(ListArgs a) {
-  __shared__ int s_item;
+// No CTA waits for another; the work counter is the only shared state.
+__global__ void __launch_bounds__(QT, 4) k_lists(ListArgs a) {
+  constexpr int QW = QT / 32;
+  constexpr int MAXJ = 32 / QW;  // mask words of a warp, at most
+  __shared__ int s_item, s_ac[QT], s_rc[QT], s_open[QT], s_nopen, s_nan;
+  __shared__ long long s_ws[QW];
+  __shared__ double s_part[QW][6], s_box[6];
+  __shared__ unsigned long long s_pairs[2], s_base[4];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  unsigned* region = a.gstage + (size_t)blockIdx.x * (size_t)a.stage;
+  bool differ = false;
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(a.head, 1);
+    __syncthreads();  // the last group's reads of shared memory and of the region
+    if (tid == 0) s_item = atomicAdd(a.head, 1);
+    if (tid < 2) s_pairs[tid] = 0;
+    if (tid == 0) s_nopen = s_nan = 0;
     __syncthreads();
     const int g = s_item;
-    __syncthreads();  // every thread has read s_item before it is overwritten
-    if (g >= a.ngroups) return;
-    walk_group<MODE_STAGE>(a, g);
-    __syncthreads();  // the group's copy-out reads precede the next group's staging writes
-  }
-}
-
-// Exclusive scan of int counts times a per-group factor (one block); the total goes to
-// *total.  tcount == nullptr: factor 1, else (tcount+31)/32 mask words per entry.
-__global__ void k_scan_cnt(const int* in, const int* tcount, long long* out, int n,
-                           unsigned long long* total) {
-  __shared__ long long ws[32];
-  __shared__ long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int base = 0; base < n; base += blockDim.x) {
-    int i = base + threadIdx.x;
-    long long v = i < n ? (long long)in[i] * (tcount ? (long long)((tcount[i] + 31) >> 5) : 1LL) : 0;
-    long long s = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      long long t = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += t;
+    if (g >= a.ngroups) break;
+    const int t0 = a.g_tstart[g], tc = a.g_tcount[g], W = (tc + 31) >> 5, root = a.g_sys[g];
+    const double macc = a.sys[root].acc, madd = a.sys[root].mac_add, msub = a.sys[root].mac_sub;
+    // visit v: its node; the visit whose reject row holds the targets that came here (-1: all),
+    // and the one whose row holds those that it rejected (itself, unless all were); the numbers
+    // it accepted and rejected; the visits that made far and near entries, in order; reject rows
+    const int vcap = (int)min(a.stage / (W + kVisitWords), (long long)INT_MAX);
+    int* vnode = reinterpret_cast<int*>(region);
+    int *vrow = vnode + vcap, *vrej = vrow + vcap, *vac = vrej + vcap, *vrc = vac + vcap, *fref = vrc + vcap, *nref = fref + vcap;
+    unsigned* R = reinterpret_cast<unsigned*>(nref + vcap);
+    auto live = [&](int j) { return tc - 32 * j >= 32 ? 0xffffffffu : (1u << (tc - 32 * j)) - 1u; };
+    // Up to four words: the warps share the nodes out (nsl of them to a word); more: each warp
+    // takes every node for words w, w + 8, ...
+    const int wp = W > 4 ? QW : (W > 2 ? 4 : W), nsl = QW / wp, j0 = w % wp, sl = w / wp;
+    double x[MAXJ], y[MAXJ], z[MAXJ];
+#pragma unroll
+    for (int i = 0; i < MAXJ; i++) {
+      const int k = 32 * (j0 + QW * i) + lane;
+      const bool in = k < tc && (i == 0 || wp == QW);
+      x[i] = in ? a.tx[t0 + k] : 0.0;
+      y[i] = in ? a.ty[t0 + k] : 0.0;
+      z[i] = in ? a.tz[t0 + k] : 0.0;
     }
-    if (lane == 31) ws[w] = s;
-    __syncthreads();
-    if (w == 0) {
-      long long t = lane < nw ? ws[lane] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        long long u = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += u;
+    // the box of the group's targets
+    {
+      double b[6] = {HUGE_VAL, HUGE_VAL, HUGE_VAL, -HUGE_VAL, -HUGE_VAL, -HUGE_VAL};
+      bool nan = false;
+#pragma unroll
+      for (int i = 0; i < MAXJ; i++) {
+        if (!(32 * (j0 + QW * i) + lane < tc && (i == 0 || wp == QW))) continue;
+        const double t[3] = {x[i], y[i], z[i]};
+        for (int q = 0; q < 3; q++) {
+          nan |= isnan(t[q]);
+          b[q] = fmin(b[q], t[q]);
+          b[3 + q] = fmax(b[3 + q], t[q]);
+        }
       }
-      if (lane < nw) ws[lane] = t;
+      for (int q = 0; q < 6; q++) {
+        for (int o = 16; o; o >>= 1) {
+          const double t = __shfl_xor_sync(0xffffffffu, b[q], o);
+          b[q] = q < 3 ? fmin(b[q], t) : fmax(b[q], t);
+        }
+        if (lane == 0) s_part[w][q] = b[q];
+      }
+      if (nan) s_nan = 1;
+      __syncthreads();
+      if (tid < 6) {
+        double t = s_part[0][tid];
+        for (int q = 1; q < QW; q++) t = tid < 3 ? fmin(t, s_part[q][tid]) : fmax(t, s_part[q][tid]);
+        s_box[tid] = t;
+      }
+    }
+    if (tid == 0) {
+      vnode[0] = root;
+      vrow[0] = -1;
     }
     __syncthreads();
-    long long pre = carry + (w ? ws[w - 1] : 0) + s - v;
-    if (i < n) out[i] = pre;
+    int head = 0, tail = 1, nf = 0, nn = 0;
+    unsigned long long fp = 0, np = 0;
+    bool full = vcap < 1;
+    while (head < tail && !full) {
+      const int c = min(QT, tail - head);
+      s_ac[tid] = s_rc[tid] = 0;
+      // One thread per node tries the whole box first.  Every operation of the test rounds
+      // monotonically, so the box's nearest point to the node bounds all targets' values from
+      // below and its farthest corner from above: the decision is theirs, bit for bit.
+      int verdict = 0;  // 1: all accept, -1: all reject, 0: open
+      if (tid < c) {
+        const double4 nd = a.nodec[vnode[head + tid]];
+        const double n3[3] = {nd.x, nd.y, nd.z};
+        double lo[3], hi[3];
+        for (int q = 0; q < 3; q++) {
+          const double d0 = dsub(s_box[q], n3[q]), d1 = dsub(s_box[3 + q], n3[q]);
+          lo[q] = n3[q] >= s_box[q] ? (n3[q] <= s_box[3 + q] ? 0.0 : d1) : d0;
+          hi[q] = fmax(fabs(d0), fabs(d1));
+        }
+        const double s0 = dadd(dadd(dmul(lo[0], lo[0]), dmul(lo[1], lo[1])), dmul(lo[2], lo[2]));
+        const double s1 = dadd(dadd(dmul(hi[0], hi[0]), dmul(hi[1], hi[1])), dmul(hi[2], hi[2]));
+        const bool all = nd.w < dmul(macc, dsub(dadd(s0, madd), msub));
+        const bool any = nd.w < dmul(macc, dsub(dadd(s1, madd), msub));
+        verdict = !s_nan && macc >= 0.0 && (all || !any) ? (all ? 1 : -1) : 0;
+        if (a.has_alt && !(a.alt_acc >= 0.0 && alt_ok(a, s0, nd.w) == all && alt_ok(a, s1, nd.w) == any)) verdict = 0;
+      }
+      const unsigned open = __ballot_sync(0xffffffffu, tid < c && !verdict);
+      int ob = 0;
+      if (lane == 0 && open) ob = atomicAdd(&s_nopen, __popc(open));
+      ob = __shfl_sync(0xffffffffu, ob, 0);
+      if ((open >> lane) & 1u) s_open[ob + __popc(open & ((1u << lane) - 1u))] = tid;
+      __syncthreads();
+      for (int kk = sl; kk < s_nopen; kk += nsl) {
+        const int k = s_open[kk], v = head + k, row = vrow[v];
+        const double4 nd = a.nodec[vnode[v]];
+        int na = 0, nr = 0;
+#pragma unroll
+        for (int i = 0; i < MAXJ; i++) {
+          const int j = j0 + QW * i;
+          if (j >= W || (i > 0 && wp != QW)) break;
+          const unsigned m = row < 0 ? live(j) : R[(size_t)row * W + j];
+          unsigned am = 0;
+          if (m) {
+            bool ok = false;
+            if ((m >> lane) & 1u) {
+              const double dx = dsub(x[i], nd.x), dy = dsub(y[i], nd.y), dz = dsub(z[i], nd.z);
+              const double s = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+              ok = nd.w < dmul(macc, dsub(dadd(s, madd), msub));
+              if (a.has_alt) differ |= ok != alt_ok(a, s, nd.w);
+            }
+            am = __ballot_sync(0xffffffffu, ok);
+          }
+          if (lane == 0) R[(size_t)v * W + j] = m & ~am;
+          na += __popc(am);
+          nr += __popc(m & ~am);
+        }
+        if (lane == 0) {
+          if (na) atomicAdd(&s_ac[k], na);
+          if (nr) atomicAdd(&s_rc[k], nr);
+        }
+      }
+      __syncthreads();
+      // one thread per node: its entry and its children, by prefix sums (far | near | children)
+      const int v = head + tid;
+      int nacc = 0, nrej = 0, nch = 0;
+      bool leaf = false;
+      int2 kd{};
+      if (tid == 0) s_nopen = 0;
+      int rej = v;
+      if (tid < c) {
+        nacc = s_ac[tid];
+        nrej = s_rc[tid];
+        if (verdict) {
+          const int row = vrow[v], cnt = row < 0 ? tc : vrc[row];
+          nacc = verdict > 0 ? cnt : 0;
+          nrej = cnt - nacc;
+          rej = row;
+        }
+        vrej[v] = rej;
+        if (nrej) {
+          kd = a.kids[vnode[v]];
+          leaf = kd.x < 0;
+          nch = leaf ? 0 : kd.y;
+        }
+        vac[v] = nacc;
+        vrc[v] = nrej;
+      }
+      const long long mine = (nacc > 0) | (long long)leaf << 21 | (long long)nch << 42;
+      long long inc = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+      }
+      if (lane == 31) s_ws[w] = inc;
+      __syncthreads();
+      long long before = 0, all = 0;
+      for (int q = 0; q < QW; q++) {
+        if (q < w) before += s_ws[q];
+        all += s_ws[q];
+      }
+      before += inc - mine;
+      constexpr long long F = (1 << 21) - 1;
+      full = tail + (int)(all >> 42) > vcap;
+      if (!full) {
+        if (nacc) {
+          fref[nf + (int)(before & F)] = v;
+          fp += nacc;
+        }
+        if (leaf) {
+          nref[nn + (int)((before >> 21) & F)] = v;
+          np += (unsigned long long)nrej * kd.y;
+        }
+        const int cb = tail + (int)(before >> 42);
+        for (int q = 0; q < nch; q++) {
+          vnode[cb + q] = kd.x + q;
+          vrow[cb + q] = rej;
+        }
+        head += c;
+        tail += (int)(all >> 42);
+        nf += (int)(all & F);
+        nn += (int)((all >> 21) & F);
+      }
+      __syncthreads();  // the region's new records; the counts are read
+    }
+    if (tid == 0) atomicMax(a.visits, (unsigned long long)tail);
+    if (full) {
+      if (tid == 0) atomicOr(a.err, 1);
+      continue;
+    }
+    for (int o = 16; o; o >>= 1) {
+      fp += __shfl_xor_sync(0xffffffffu, fp, o);
+      np += __shfl_xor_sync(0xffffffffu, np, o);
+    }
+    if (lane == 0) {
+      if (fp) atomicAdd(&s_pairs[0], fp);
+      if (np) atomicAdd(&s_pairs[1], np);
+    }
     __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = pre + v;
+    if (tid == 0) {
+      atomicAdd(&a.pairs[0], s_pairs[0]);
+      atomicAdd(&a.pairs[1], s_pairs[1]);
+      a.g_near[g] = s_pairs[1];
+      s_base[0] = atomicAdd(&a.totals[0], (unsigned long long)nf);
+      s_base[1] = atomicAdd(&a.totals[1], (unsigned long long)nf * W);
+      s_base[2] = atomicAdd(&a.totals[2], (unsigned long long)nn);
+      s_base[3] = atomicAdd(&a.totals[3], (unsigned long long)nn * W);
+      // the arrays were sized from an estimate: past their end, the build is run again
+      if (s_base[0] + nf > a.cap[0] || s_base[1] + (unsigned long long)nf * W > a.cap[1] ||
+          s_base[2] + nn > a.cap[2] || s_base[3] + (unsigned long long)nn * W > a.cap[3]) {
+        atomicOr(a.err, 2);
+        s_base[0] = ~0ull;
+      }
+      a.far_off[g] = (long long)s_base[0];
+      a.far_moff[g] = (long long)s_base[1];
+      a.near_off[g] = (long long)s_base[2];
+      a.near_moff[g] = (long long)s_base[3];
+      a.far_cnt[g] = nf;
+      a.near_cnt[g] = nn;
+    }
     __syncthreads();
+    if (s_base[0] == ~0ull) continue;
+    const long long fo = (long long)s_base[0], fmo = (long long)s_base[1], no = (long long)s_base[2],
+                    nmo = (long long)s_base[3];
+    for (int k = tid; k < nf; k += QT) {
+      const int v = fref[k];
+      a.far_node[fo + k] = vnode[v];
+      a.far_tgt[fo + k] = vac[v];
+    }
+    for (int k = tid; k < nn; k += QT) {
+      const int v = nref[k];
+      a.near_node[no + k] = vnode[v];
+      a.near_tgt[no + k] = vrc[v];
+    }
+    // a warp per entry, a lane per word
+    for (int k = w; k < nf + nn; k += QW) {
+      const int v = k < nf ? fref[k] : nref[k - nf];
+      if (lane < W) {
+        auto row = [&](int q) { return q < 0 ? live(lane) : R[(size_t)q * W + lane]; };
+        const unsigned r = vrc[v] ? row(vrej[v]) : 0u;
+        if (k < nf) a.far_mask[fmo + (long long)k * W + lane] = row(vrow[v]) & ~r;
+        else a.near_mask[nmo + (long long)(k - nf) * W + lane] = r;
+      }
+    }
+    __syncthreads();  // the entries' nodes and targets
+    group_prefixes(a, g, nf, fo, nn, no);
   }
-  if (threadIdx.x == 0) *total = (unsigned long long)carry;
-}
-
-void set_stage_attr() {
-  // static + dynamic shared memory is above the 48 KB default
-  ensure_smem_attr(reinterpret_cast<const void*>(k_lists_queue), (int)STACK_BYTES);
-  ensure_smem_attr(reinterpret_cast<const void*>(k_lists<MODE_COUNT>), (int)STACK_BYTES);
-  ensure_smem_attr(reinterpret_cast<const void*>(k_lists<MODE_FILL>), (int)STACK_BYTES);
+  if (a.has_alt && __any_sync(0xffffffffu, differ) && lane == 0) atomicOr(a.err, 4);
 }
 
 }  // namespace
@@ -502,9 +520,8 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->far_cnt.ensure(c, ng);
   L->near_cnt.ensure(c, ng);
   L->g_near.ensure(c, ng);
-  DBuf<unsigned long long> cnt;  // totals[4], pairs[2], err (as the 7th word)
+  DBuf<unsigned long long> cnt;  // totals[4], pairs[2], err (as the 7th word), most visits
   cnt.ensure(c, 8);
-  BIT_CUDA(cudaMemsetAsync(cnt.p, 0, 8 * sizeof(unsigned long long), s));
   ListArgs a{};
   a.g_tstart = L->g_tstart.p;
   a.g_tcount = L->g_tcount.p;
@@ -526,9 +543,6 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     a.alt_add = alt->add_del;
     a.alt_sub = alt->sub_del;
   }
-  // Single pass straight into the lists, sized from an estimate: the last build's totals
-  // scaled by the group count, else a per-group allowance.  A group that does not fit
-  // its staging area or the arrays makes the build fall back to count, scan and fill.
   long long words = 0;
   for (int g = 0; g < ng; g++) words += (tc[g] + 31) / 32;
   // sizes of this tree's last build, else of the context's last build under the same MAC
@@ -546,100 +560,74 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     cap[2] = 48ull * ng + 1024;
     cap[3] = 48ull * words + 1024;
   }
-  L->far_node.ensure(c, cap[0]);
-  L->far_mask.ensure(c, cap[1]);
-  L->near_node.ensure(c, cap[2]);
-  L->near_mask.ensure(c, cap[3]);
-  for (int k = 0; k < 4; k++) a.cap[k] = cap[k];
-  auto point_at_lists = [&] {
-    L->far_tgt.ensure(c, L->far_node.n);
-    L->near_tgt.ensure(c, L->near_node.n);
-    L->far_pre.ensure(c, L->far_node.n);
-    L->near_pre.ensure(c, L->near_node.n);
-    a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
-    a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
-    a.far_tgt = L->far_tgt.p; a.near_tgt = L->near_tgt.p;
-    a.far_pre = L->far_pre.p; a.near_pre = L->near_pre.p;
-  };
-  point_at_lists();
-  L->far_tot.ensure(c, ng);
-  L->near_tot.ensure(c, ng);
-  a.far_tot = L->far_tot.p; a.near_tot = L->near_tot.p;
-  set_stage_attr();
-  // staging: one region per resident CTA.  A group's entries number at most the tree's
-  // nodes (far) and leaves (near), each with at most 32 mask words.
+  // one region per resident CTA; a group visits a node once at most
   int maxw = 1;
   for (int g = 0; g < ng; g++) maxw = std::max(maxw, (tc[g] + 31) / 32);
   L->max_targets = 32 * maxw;
   int per_sm = 0;
-  BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists_queue, LT, STACK_BYTES));
-  const int slots = std::max(1, std::min(ng, c->num_sms * std::max(per_sm, 1)));
-  const long long worst[2] = {(maxw + 1LL) * std::max(t->numtree, 1),
-                              (maxw + 1LL) * std::max(t->nleaves, 1)};
-  long long want[2];
-  for (int k = 0; k < 2; k++)
-    want[k] = std::min(worst[k], hint && hint->stage[k] > 0
-                                     ? hint->stage[k] + hint->stage[k] / 4 + 64
-                                     : STAGE_FIRST[k]);
-  a.stage_far = want[0];
-  a.stage_near = want[1];
-  const size_t stage_words = (size_t)slots * (size_t)(want[0] + want[1]);
-  const bool staged = L->gstage.n >= stage_words ||
-                      !c->budget || c->in_use + stage_words * sizeof(unsigned) <= c->budget;
+  BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists, QT, 0));
+  const long long nodes = std::max(t->numtree, 1);
+  long long visits0 = 1;  // at least this many
+  long long visits = std::min(nodes, hint && hint->visits > 0 ? hint->visits + hint->visits / 4 + 64 : kVisitsFirst);
+  L->far_tot.ensure(c, ng);
+  L->near_tot.ensure(c, ng);
+  L->head.ensure(c, 1);
+  a.far_tot = L->far_tot.p; a.near_tot = L->near_tot.p;
+  a.visits = cnt.p + 7;
+  a.head = L->head.p;
+  a.ngroups = ng;
   unsigned long long h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   std::vector<int> hf(ng), hn(ng);
   std::vector<unsigned long long> hp(ng);
-  auto read_back = [&] {
+  int err = 0;
+  L->fallback = false;
+  for (;;) {
+    L->far_node.ensure(c, cap[0]);
+    L->far_mask.ensure(c, cap[1]);
+    L->near_node.ensure(c, cap[2]);
+    L->near_mask.ensure(c, cap[3]);
+    L->far_tgt.ensure(c, L->far_node.n);
+    L->near_tgt.ensure(c, L->near_node.n);
+    L->far_pre.ensure(c, L->far_node.n);
+    L->near_pre.ensure(c, L->near_node.n);
+    for (int k = 0; k < 4; k++) a.cap[k] = cap[k];
+    a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
+    a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
+    a.far_tgt = L->far_tgt.p; a.near_tgt = L->near_tgt.p;
+    a.far_pre = L->far_pre.p; a.near_pre = L->near_pre.p;
+    const long long per = (long long)(maxw + kVisitWords) * sizeof(unsigned);  // bytes a visit
+    size_t room = kRegionBytes;
+    if (c->budget) {
+      const size_t held = c->in_use - L->gstage.n * sizeof(unsigned);
+      room = std::min(room, std::max(L->gstage.n * sizeof(unsigned), c->budget > held ? c->budget - held : 0));
+      visits = std::min(visits, std::max<long long>(room / per, visits0));
+    }
+    a.stage = visits * (maxw + kVisitWords);
+    long long slots = std::min<long long>(ng, (long long)c->num_sms * std::max(per_sm, 1));
+    slots = std::min<long long>(slots, room / (visits * per));
+    slots = std::max(slots, 1LL);
+    L->gstage.ensure(c, (size_t)slots * (size_t)a.stage);
+    a.gstage = L->gstage.p;
+    BIT_CUDA(cudaMemsetAsync(cnt.p, 0, 8 * sizeof(unsigned long long), s));
+    BIT_CUDA(cudaMemsetAsync(L->head.p, 0, sizeof(int), s));
+    count_launch(), k_lists<<<(unsigned)slots, QT, 0, s>>>(a);
+    BIT_CHECK_LAUNCH();
     copy_d2h_batch(c, {{h, cnt.p, 8 * sizeof(unsigned long long)},
                        {hf.data(), L->far_cnt.p, ng * sizeof(int)},
                        {hn.data(), L->near_cnt.p, ng * sizeof(int)},
                        {hp.data(), L->g_near.p, ng * sizeof(unsigned long long)}});
-  };
-  int err = 2;  // no single pass: straight to count, scan and fill
-  if (staged) {
-    L->gstage.ensure(c, stage_words);
-    L->head.ensure(c, 1);
-    BIT_CUDA(cudaMemsetAsync(L->head.p, 0, sizeof(int), s));
-    a.gstage = L->gstage.p;
-    a.head = L->head.p;
-    a.ngroups = ng;
-    count_launch(), k_lists_queue<<<slots, LT, STACK_BYTES, s>>>(a);
-    BIT_CHECK_LAUNCH();
-    read_back();
     err = (int)(h[6] & 0xffffffffu);
-    if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded (tree deeper than supported)");
-  }
-  L->fallback = (err & 2) != 0;
-  if (err & 2) {
-    // some group's lists exceed the staging area or the arrays: count, scan, fill
-    BIT_CUDA(cudaMemsetAsync(cnt.p, 0, 8 * sizeof(unsigned long long), s));
-    count_launch(), k_lists<MODE_COUNT><<<ng, LT, STACK_BYTES, s>>>(a);
-    count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->far_cnt.p, nullptr, L->far_off.p, ng, cnt.p + 0);
-    count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->far_cnt.p, L->g_tcount.p, L->far_moff.p, ng, cnt.p + 1);
-    count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->near_cnt.p, nullptr, L->near_off.p, ng, cnt.p + 2);
-    count_launch(), k_scan_cnt<<<1, 1024, 0, s>>>(L->near_cnt.p, L->g_tcount.p, L->near_moff.p, ng, cnt.p + 3);
-    read_back();
-    err = (int)(h[6] & 0xffffffffu);  // this pass walked every group to the end
-    if (err & 1) fail(BIT_ERR_CAPACITY, "traversal stack capacity exceeded");
-    L->far_node.ensure(c, h[0]);
-    L->far_mask.ensure(c, h[1]);
-    L->near_node.ensure(c, h[2]);
-    L->near_mask.ensure(c, h[3]);
-    point_at_lists();
-    count_launch(), k_lists<MODE_FILL><<<ng, LT, STACK_BYTES, s>>>(a);
-    BIT_CHECK_LAUNCH();
+    if (!(err & 3)) break;
+    L->fallback = true;
+    if (err & 1) visits0 = visits + 1, visits = std::min(nodes, 4 * visits);  // (the totals are not complete)
+    else for (int k = 0; k < 4; k++) cap[k] = h[k];
   }
   ListSizing& z = L->last;
   z.ngroups = ng;
   z.acc = key.acc;
   z.points = key.points;
   for (int k = 0; k < 4; k++) z.totals[k] = h[k];
-  z.stage[0] = z.stage[1] = 0;
-  for (int g = 0; g < ng; g++) {
-    const long long w1 = (tc[g] + 31) / 32 + 1;
-    z.stage[0] = std::max(z.stage[0], w1 * hf[g]);
-    z.stage[1] = std::max(z.stage[1], w1 * hn[g]);
-  }
+  z.visits = (long long)h[7];
   c->list_hint = z;
   L->nfar = (long long)h[0];
   L->nnear = (long long)h[2];

@@ -995,9 +995,8 @@ __global__ void __launch_bounds__(256) k_finish_nodes(int numtree, const double*
                                                       float4* nodeh, int2* kids, int* leaf_of) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
   if (i >= numtree) return;
-  // children[] holds base + order[c] in its first nchild slots (consecutive node
-  // indices, in another order), so one int2 gives the traversal all of them:
-  // (base, nchild | order[c] << (4 + 3c)); a leaf is (-1, nummemb)
+  // a node's children are consecutive indices (children[] holds them in the reference's own
+  // order), so one int2 gives the traversal all of them: (first, count); a leaf is (-1, nummemb)
   const int* ch = children + 8LL * i;
   if (ch[0] == -1)
     for (int e = start[i] + lane; e < start[i] + nummemb[i]; e += 32) leaf_of[e] = i;
@@ -1007,9 +1006,7 @@ __global__ void __launch_bounds__(256) k_finish_nodes(int numtree, const double*
     base = min(base, ch[c]);
     cnt++;
   }
-  int code = cnt;
-  for (int c = 0; c < cnt; c++) code |= (ch[c] - base) << (4 + 3 * c);
-  kids[i] = cnt ? make_int2(base, code) : make_int2(-1, nummemb[i]);
+  kids[i] = cnt ? make_int2(base, cnt) : make_int2(-1, nummemb[i]);
   const double* f = fields + 13LL * i;
   nodec[i] = make_double4(f[6], f[7], f[8], f[12]);
   // half extents about the midpoint, rounded up to FP32 (a box the members are inside of)

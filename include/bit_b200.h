@@ -87,7 +87,7 @@ typedef struct {
   long long far_entries, near_entries, batches;
   int numtree, nleaves, depth, nterms;
   int far_launches, near_launches;
-  int list_fallback; /* the last list build used the count / scan / fill passes */
+  int list_fallback; /* the last list build outran its estimate and was run again with room */
   int lists_shared;  /* the last evaluation reused lists built for another MAC (the
                         context's previous one): every acceptance decision of that
                         traversal was also checked under this MAC and agreed, so the
