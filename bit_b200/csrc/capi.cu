@@ -198,16 +198,6 @@ void eval_particles_sorted(Tree* t, const std::vector<bit_eval_params>& prm) {
   t->stats.lists_shared = t->plists.shared ? 1 : 0;
 }
 
-uint64_t spread3(uint64_t v) {
-  v &= 0x1fffff;
-  v = (v | v << 32) & 0x1f00000000ffffULL;
-  v = (v | v << 16) & 0x1f0000ff0000ffULL;
-  v = (v | v << 8) & 0x100f00f00f00f00fULL;
-  v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
-  v = (v | v << 2) & 0x1249249249249249ULL;
-  return v;
-}
-
 }  // namespace
 }  // namespace bit
 
@@ -624,42 +614,14 @@ bit_status bit_eval_points(bit_tree* th, const bit_eval_params* prm, int m, cons
     check_params(prm);
     if (!t->has_moments) fail(BIT_ERR_STATE, "moments not computed");
     BIT_CUDA(cudaSetDevice(c->device));
-    // spatial (Morton) order of the points so that a batch is compact
-    double lo[3] = {x[0], y[0], z[0]}, hi[3] = {x[0], y[0], z[0]};
-    for (int i = 0; i < m; i++) {
-      double v[3] = {x[i], y[i], z[i]};
-      for (int a = 0; a < 3; a++) {
-        if (std::isnan(v[a])) fail(BIT_ERR_INVALID_ARGUMENT, "point coordinates contain NaN");
-        lo[a] = std::min(lo[a], v[a]);
-        hi[a] = std::max(hi[a], v[a]);
-      }
-    }
-    std::vector<std::pair<uint64_t, int>> key(m);
-    for (int i = 0; i < m; i++) {
-      double v[3] = {x[i], y[i], z[i]};
-      uint64_t code = 0;
-      for (int a = 0; a < 3; a++) {
-        double s = hi[a] > lo[a] ? (v[a] - lo[a]) / (hi[a] - lo[a]) : 0.0;
-        uint64_t q = (uint64_t)std::min(2097151.0, std::max(0.0, s * 2097151.0));
-        code |= spread3(q) << a;
-      }
-      key[i] = {code, i};
-    }
-    std::sort(key.begin(), key.end());
-    std::vector<double> sx(m), sy(m), sz(m);
-    std::vector<int> ord(m);
-    for (int i = 0; i < m; i++) {
-      ord[i] = key[i].second;
-      sx[i] = x[ord[i]]; sy[i] = y[ord[i]]; sz[i] = z[ord[i]];
-    }
-    DBuf<double> dx, dy, dz, out;
-    DBuf<int> dord;
-    dx.ensure(c, m); dy.ensure(c, m); dz.ensure(c, m); out.ensure(c, m); dord.ensure(c, m);
     cudaStream_t s = c->stream;
-    copy_h2d(c, dx.p, sx.data(), m * sizeof(double));
-    copy_h2d(c, dy.p, sy.data(), m * sizeof(double));
-    copy_h2d(c, dz.p, sz.data(), m * sizeof(double));
-    copy_h2d(c, dord.p, ord.data(), m * sizeof(int));
+    const double* host[3] = {x, y, z};
+    double lo[3], hi[3];
+    DBuf<double> pt[3], out;
+    DBuf<int> dord;
+    order_points(c, m, host, pt, dord, lo, hi);
+    const double *dx = pt[0].p, *dy = pt[1].p, *dz = pt[2].p;
+    out.ensure(c, m);
     Lists L;
     EvalPlan P;
     double reach = 0.0;  // of the points' box, from the tree's box centre
@@ -668,10 +630,10 @@ bit_status bit_eval_points(bit_tree* th, const bit_eval_params* prm, int m, cons
       reach += d * d;
     }
     plan_sys(t, &P, {*prm}, 1, 0, 0, std::sqrt(reach));
-    build_lists(t, &L, plan_key(t, P, 1), m, dx.p, dy.p, dz.p, P.sys.p);
+    build_lists(t, &L, plan_key(t, P, 1), m, dx, dy, dz, P.sys.p);
     plan_classes(t, &L, &P);
-    eval_far(t, &L, P, dx.p, dy.p, dz.p, out.p);
-    eval_near(t, &L, P, dx.p, dy.p, dz.p, out.p);
+    eval_far(t, &L, P, dx, dy, dz, out.p);
+    eval_near(t, &L, P, dx, dy, dz, out.p);
     DBuf<double> res;
     res.ensure(c, m);
     count_launch(), k_scatter_out<<<grid_for(m, 256), 256, 0, s>>>(m, dord.p, out.p, res.p);

@@ -17,7 +17,7 @@ namespace bit {
 constexpr int kWarp = 32;
 constexpr int kNtermsMax = BIT_NTERMS_MAX;
 constexpr int kGroupMax = 1024;   // targets per group (one CTA; 32 mask words)
-constexpr int kPointGroup = 256;  // external points per group
+constexpr int kPointGroup = 256;  // external points per group, at most
 constexpr int kNearParts = 8;         // near-field items of a group, at most
 constexpr long long kNearChunk = 512 << 10;  // and the pairs of one, at least
 constexpr double kEpsNear = 1e-14;  // src/constants.h:35
@@ -312,6 +312,8 @@ void tree_sync_host(Tree* t);
 void tree_set_charges(Tree* t, const double* dq, const double* dw);
 void tree_moments(Tree* t, int nterms);
 void tree_moments_sys(Tree* t, const std::vector<int>& nterms_per_system);
+void order_points(Ctx* c, int m, const double* const host[3], DBuf<double> sorted[3], DBuf<int>& ord, double lo[3],
+                  double hi[3]);
 // alt (single-system keys only, or nullptr): a second MAC checked during the traversal.
 void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const double* tx,
                  const double* ty, const double* tz, const SysEval* d_sys,
