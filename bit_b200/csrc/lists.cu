@@ -2,7 +2,7 @@
 // (src/tree3d.cpp:4679-4778, 3448-3627, 851-971) for a whole group of targets at once.
 //
 // A group is up to 1024 consecutive targets (a run of consecutive small leaves, a leaf, or
-// a chunk of one; for external points, 256 consecutive points in Morton order).  One CTA walks
+// a chunk of one; for external points, 32 to 256 consecutive points in Morton order).  One CTA walks
 // the tree for the group, with a 32-bit mask word per 32 targets.  At a node every active target
 // evaluates the reference's acceptance test in FP64 without contraction
 // (sqradius < acc * ((dx*dx + dy*dy + dz*dz + add) - sub)); the node becomes a far entry
@@ -447,6 +447,19 @@ static void particle_groups(Tree* t, int G, std::vector<int>& ts, std::vector<in
   flush();
 }
 
+// Points per group: as few as make six groups a multiprocessor, in powers of two from a mask
+// word to kPointGroup.  A small group shares less (traversal, coefficients, sources), but few
+// groups leave the chip idle.  A whole call on 200k particles (nterms 9, screened, FP64), groups
+// of 32 / 64 / 128 / 256, us: 300 points 516 / 711 / 1093 / 1739; 10k 635 / 721 / 844 / 1112;
+// 27k 786 / 801 / 1006 / 1121; 40k 1008 / 922 / 1110 / 1271; 60k 1366 / 1155 / 1160 / 1416; 140k
+// 3737 / 3232 / 3072 / 3002; 1M 22256 / 18659 / 17114 / 15959; other trees and kernels cross at
+// 20k to 27k, 50k to 60k and 100k to 130k.
+static int point_group(int m, int sms) {
+  int size = 32;
+  while (size < kPointGroup && m > 6LL * sms * size) size *= 2;
+  return size;
+}
+
 // The potentials' near-field items, heaviest first: a group's near work in one item, or in up
 // to kNearParts equal parts of at least kNearChunk pairs each, whose sums meet in scratch
 // (near_part).  The count follows from the group's own lists alone, so that its result does
@@ -495,9 +508,10 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   std::vector<int> ts, tc, gsys;
   if (key.points) {
     if (t->nsys != 1) fail(BIT_ERR_INVALID_ARGUMENT, "external points need a single-system tree");
-    for (int e = 0; e < ntargets; e += kPointGroup) {
+    const int size = point_group(ntargets, c->num_sms);
+    for (int e = 0; e < ntargets; e += size) {
       ts.push_back(e);
-      tc.push_back(std::min(kPointGroup, ntargets - e));
+      tc.push_back(std::min(size, ntargets - e));
       gsys.push_back(0);
     }
   } else {

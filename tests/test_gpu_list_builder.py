@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("m", [1, 32, 33, 65, 97, 128, 129, 160, 225, 256, 289, 513])
-def test_points_of_every_mask_width(ctx, orc, m):
+def test_points_of_every_remainder(ctx, orc, m):
     import bit_b200 as B
     from bit_b200 import workloads
     x, y, z, q = workloads.clustered_blobs(4000, seed=m)
@@ -22,6 +22,29 @@ def test_points_of_every_mask_width(ctx, orc, m):
     for acc in (0.02, 0.3, 0.9):
         want = T.evaluate(orc.params(orc.COULOMB, orc.MODE_CONSISTENT, acc=acc, del_=1e-3), points=pts)
         got = t.evaluate(B.params(B.COULOMB, B.CONSISTENT, B.FP64, acc=acc, del_=1e-3), points=pts)
+        assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+    t.treeempty()
+
+
+@pytest.mark.parametrize("size", [32, 33, 64, 65, 96, 128, 129, 160, 256, 288, 992, 1024])
+def test_packed_leaves_of_every_mask_width(orc, size):
+    """Runs of small leaves packed to groups of up to `size` targets: 1 to 32 mask words."""
+    import bit_b200 as B
+    from bit_b200 import workloads
+    ctx = B.Context()
+    ctx.set_group_size(size)
+    n = 4000
+    x, y, z, q = workloads.clustered_blobs(n, seed=size)
+    t = ctx.treemake(x, y, z, 9)
+    t.treemoments(q, 2)
+    T = orc.Tree(x, y, z, 9)
+    T.compute_moments(q, 2)
+    for acc in (0.02, 0.3, 0.9):
+        nf, nn, _ = T.count(orc.params(orc.COULOMB, acc=acc, del_=1e-3))
+        want = T.evaluate(orc.params(orc.COULOMB, orc.MODE_CONSISTENT, acc=acc, del_=1e-3))
+        got = t.evaluate(B.params(B.COULOMB, B.CONSISTENT, B.FP64, acc=acc, del_=1e-3))
+        st = t.stats()
+        assert st["far_pairs"] == nf and st["near_pairs"] - n == nn
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
     t.treeempty()
 
