@@ -112,7 +112,7 @@ struct SysEval {
   int kernel, nterms;
   int near_sign, eps_check, self_term, particles;
   int kernel_order;  // regularised Coulomb field: the reference's KERNEL_ORDER (src/problem.h:13)
-  int far_kind;      // potentials: bit 0 screened, bit 1 regularised (far_add > 0)
+  int far_kind;      // bit 0 screened, bit 1 regularised (far_add not 0)
   int underflow;     // some pair's exp(-kappa R) may fall below the smallest normal number
   int pad_;
 };

@@ -14,7 +14,8 @@
 // target-centre offset is formed in FP64; the mixed path rounds it once to FP32 and runs
 // the evaluation in FP32, accumulating with two-sum.
 //
-// Forces: the reference's recurrences (gen_farfield.py) on the moments themselves.
+// Fields: the gradients of the same polynomials (k_far_field); with a kernel order, the
+// reference's recurrences (gen_farfield.py) on the moments themselves.
 #include <algorithm>
 
 #include "common.cuh"
@@ -385,13 +386,125 @@ __global__ void __launch_bounds__(32 * NW, 2) k_far_queue(FarArgs a, int count, 
   }
 }
 
-// Field kinds of k_far_force: the regularised Coulomb field of treetaylorforce with
-// KERNEL_ORDER = 0 (FK_COULOMB) or with the system's kernel order (FK_COULOMB_KORDER, FP64),
-// and the screened 2-D field of shielded_treetaylorforce (FK_SCREENED_CURL, FP64).
-constexpr int FK_COULOMB = 0, FK_COULOMB_KORDER = 1, FK_SCREENED_CURL = 2;
+// ---- fields -------------------------------------------------------------------------------
 
-template <int NT, int FK, class T>
-__global__ void __launch_bounds__(32 * NWF) k_far_force(FarArgs a) {
+// Far field of the vector fields: the regularised Coulomb field of treetaylorforce (KIND 0 or
+// FAR_REG) and the screened 2-D field of shielded_treetaylorforce (KIND FAR_SCREENED), as the
+// gradients of the potentials' polynomials (gen_harmonics.py).  A CTA takes up to kFieldChunk
+// targets of a group, so that the three rows of FP64 sums a warp keeps stay small: the
+// recurrence kernel that this replaces had rows for a whole group of 1024, 130 KB, and so four
+// warps a multiprocessor.  Entries are shared out to the warps as in far_group (by the work of
+// the whole group), and rows are summed in warp order.  Bound by the FP64 / FP32 pipe: 1,252
+// flops a pair (nterms 9, delta > 0) against the recurrence's 3,455.  Before / now, FP64 with delta,
+// without, mixed, screened, ms: 2M clustered, nterms 9: 32.3 / 11.3, 32.2 / 7.3, 27.3 / 7.1, 41.8 /
+// 10.3; 150k, 9: 1.14 / 0.44, 1.14 / 0.29, 0.99 / 0.29, 1.47 / 0.39; 20k, 6: 0.145 / 0.077, 0.144 /
+// 0.070, 0.119 / 0.064, 0.152 / 0.082.  Mixed against FP64, 2M: 3.4e-7 / 1.9e-7.
+constexpr int kFieldChunk = 256;
+// CTAs of eight warps per SM: two (128 registers) hold every order without spills; three (80)
+// do up to nterms 4, 230 -> 198 us on 100k in leaves of 100, but cost 50k, nterms 7, 165 -> 183.
+// (One CTA, 166 registers: 2M 13.3 ms.)
+constexpr int field_blocks(int nt) { return nt <= 4 ? 3 : 2; }
+
+template <int NT, int KIND, class T>
+__global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArgs a) {
+  constexpr int NW = NWP;
+  constexpr int CNT = far_count(NT, KIND);
+  constexpr int TP = far_block(NT, KIND);
+  constexpr int WC = kFieldChunk / 32;
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ uint64_t bar[NW];
+  const int g = a.order[blockIdx.x], c0 = blockIdx.y * kFieldChunk;
+  const int t0 = a.g_tstart[g] + c0, gc = a.g_tcount[g], tc = min(gc - c0, kFieldChunk);
+  if (tc <= 0) return;  // (the whole CTA)
+  far_bars_init<NW>(bar);
+  const int rows = a.rows;
+  double* accb = reinterpret_cast<double*>(sm);  // [NW][3][rows]
+  T* msb = reinterpret_cast<T*>(accb + NW * 3 * rows);
+  unsigned short* tlb = reinterpret_cast<unsigned short*>(msb + NW * a.stride);
+  const int W = (gc + 31) >> 5, w0 = blockIdx.y * WC, wn = (tc + 31) >> 5;
+  const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
+  for (int i = tid; i < NW * 3 * rows; i += 32 * NW) accb[i] = 0.0;
+  double* row = accb + w * 3 * rows;
+  T* M = msb + w * a.stride;
+  unsigned short* tl = tlb + w * rows;
+  const T* coef = reinterpret_cast<const T*>(a.coef);
+  const SysEval* se = a.sys + a.g_sys[g];
+  const T tadd = (T)se->far_add, tk = (T)se->kappa;
+  const long long tot = a.tot[g];
+  long long eb = 0, ee = 0;
+  for (long long b = e0; b < e1; b += 32) {
+    const bool in = b + lane < e1;
+    const long long P = in ? a.pre[b + lane] * NW : 0;
+    eb += __popc(__ballot_sync(0xffffffffu, in && P < w * tot));
+    ee += __popc(__ballot_sync(0xffffffffu, in && P < (w + 1) * tot));
+  }
+  __syncthreads();  // the rows are zero, the barriers ready
+  bool failed = false;
+  unsigned phase = 0;
+  for (long long e = e0 + eb; e < e0 + ee; e++) {
+    const int node = a.node[e];
+    if (lane == 0) {
+      fence_proxy_async();
+      mbar_expect_tx(&bar[w], TP * (unsigned)sizeof(T));
+      tma_load_1d(M, coef + (long long)node * a.stride, TP * (unsigned)sizeof(T), &bar[w]);
+    }
+    const unsigned wd = lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
+    const bool all = a.tgt[e] == gc;
+    const int cnt = all ? tc : __reduce_add_sync(0xffffffffu, __popc(wd));
+    const double4 c = a.nodec[node];
+    if (!all && cnt) warp_pack(wd, wn, tl);
+    const bool landed = __all_sync(0xffffffffu, mbar_wait(&bar[w], phase & 1));
+    phase++;
+    if (!landed) {
+      if (lane == 0) {
+        atomicOr(a.err, 8);
+        mbar_wait(&bar[w], (phase - 1) & 1);
+      }
+      __syncwarp();
+      failed = true;
+      break;
+    }
+    const T H = M[CNT];
+    for (int r = lane; r < cnt; r += 32) {
+      const int i = all ? r : tl[r];
+      const T dx = (T)(cx[i] - c.x), dy = (T)(cy[i] - c.y), dz = (T)(cz[i] - c.z);
+      const T r2 = dx * dx + dy * dy + dz * dz;
+      T fx, fy, fz;
+      if constexpr (KIND == 0) Harmonics<NT>::template ghc<T>(dx, dy, dz, r2, tadd, tk, H, M, fx, fy, fz);
+      else if constexpr (KIND == FAR_REG) Harmonics<NT>::template grc<T>(dx, dy, dz, r2, tadd, tk, H, M, fx, fy, fz);
+      else Harmonics<NT>::template ghs<T>(dx, dy, dz, r2, tadd, tk, H, M, fx, fy, fz);
+      if constexpr (KIND == FAR_SCREENED) {  // the curl: (d phi / dy, -d phi / dx)
+        row[i] -= (double)fy;
+        row[rows + i] += (double)fx;
+      } else {
+        row[i] += (double)fx;
+        row[rows + i] += (double)fy;
+        row[2 * rows + i] += (double)fz;
+      }
+    }
+    __syncwarp();
+  }
+  if (__syncthreads_or(failed)) return;
+  for (int i = tid; i < tc; i += 32 * NW) {
+    double sx = 0, sy = 0, sz = 0;
+    for (int q = 0; q < NW; q++) {
+      sx += accb[(q * 3 + 0) * rows + i];
+      sy += accb[(q * 3 + 1) * rows + i];
+      sz += accb[(q * 3 + 2) * rows + i];
+    }
+    a.out[t0 + i] = sx;
+    a.out_y[t0 + i] = sy;
+    a.out_z[t0 + i] = sz;
+  }
+}
+
+// The regularised Coulomb field with the systems' kernel orders (FP64): the reference's
+// recurrences (gen_farfield.py) on the moments themselves.
+template <int NT>
+__global__ void __launch_bounds__(32 * NWF) k_far_force_korder(FarArgs a) {
+  using T = double;
   constexpr int TT = num_terms(NT);
   constexpr int TP = FarField<NT>::kPadded;
   constexpr int NW = NWF;
@@ -416,7 +529,7 @@ __global__ void __launch_bounds__(32 * NWF) k_far_force(FarArgs a) {
   unsigned short* tl = tlb + w * kGroupMax;
   double* row = accb + w * 3 * kGroupMax;
   const SysEval* se = a.sys + a.g_sys[g];
-  const T tadd = (T)se->far_add, tk = (T)se->kappa, tdel = (T)se->near_del;
+  const T tadd = (T)se->far_add, tdel = (T)se->near_del;
   const int korder = se->kernel_order;
   for (long long e = e0 + w; e < e1; e += NW) {
     const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
@@ -433,10 +546,7 @@ __global__ void __launch_bounds__(32 * NWF) k_far_force(FarArgs a) {
       const T dx = (T)(cx[i] - c.x), dy = (T)(cy[i] - c.y), dz = (T)(cz[i] - c.z);
       const T rs = dx * dx + dy * dy + dz * dz + tadd;
       T fx = 0, fy = 0, fz = 0;
-      if constexpr (FK == FK_COULOMB) FarField<NT>::template force<T>(dx, dy, dz, rs, M, fx, fy, fz);
-      else if constexpr (FK == FK_COULOMB_KORDER)
-        FarField<NT>::template force_korder<T>(dx, dy, dz, rs, tdel, korder, M, fx, fy, fz);
-      else FarField<NT>::template screened_curl<T>(dx, dy, dz, rs, tk, M, fx, fy);
+      FarField<NT>::template force_korder<T>(dx, dy, dz, rs, tdel, korder, M, fx, fy, fz);
       row[i] += (double)fx;
       row[kGroupMax + i] += (double)fy;
       row[2 * kGroupMax + i] += (double)fz;
@@ -475,11 +585,22 @@ void launch_far(const FarArgs& a, int ng, cudaStream_t s) {
   count_launch(), k_far<NT, KIND, T, NW><<<ng, 32 * NW, far_smem<T, NW>(a), s>>>(a);
 }
 
-template <int NT, int FK, class T>
-void launch_force(const FarArgs& a, int ng, cudaStream_t s) {
-  const size_t bytes = force_smem(FarField<NT>::kPadded * sizeof(T));
-  set_smem(k_far_force<NT, FK, T>, bytes);
-  count_launch(), k_far_force<NT, FK, T><<<ng, 32 * NWF, bytes, s>>>(a);
+template <int NT>
+void launch_korder(const FarArgs& a, int ng, cudaStream_t s) {
+  const size_t bytes = force_smem(FarField<NT>::kPadded * sizeof(double));
+  set_smem(k_far_force_korder<NT>, bytes);
+  count_launch(), k_far_force_korder<NT><<<ng, 32 * NWF, bytes, s>>>(a);
+}
+
+template <class T>
+constexpr size_t field_smem(int stride, int rows) {
+  return NWP * (3 * (size_t)rows * sizeof(double) + (size_t)stride * sizeof(T) + (size_t)rows * sizeof(unsigned short));
+}
+
+template <int NT, int KIND, class T>
+void launch_field(const FarArgs& a, int ng, int chunks, cudaStream_t s) {
+  set_smem(k_far_field<NT, KIND, T>, field_smem<double>(far_block(kNtermsMax, FAR_REG), kFieldChunk));
+  count_launch(), k_far_field<NT, KIND, T><<<dim3(ng, chunks), 32 * NWP, field_smem<T>(a.stride, a.rows), s>>>(a);
 }
 
 FarArgs far_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
@@ -596,16 +717,24 @@ void eval_far_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* fy
   bool korder = false;
   for (const SysEval& se : P.h_sys) korder |= se.kernel_order > 0;
   if (f32 && (curl || korder)) fail(BIT_ERR_INVALID_ARGUMENT, "this field is FP64 only");
+  if (!korder) {
+    if (f32) far_coefs<float>(t, P, a, s);
+    else far_coefs<double>(t, P, a, s);
+  }
+  a.rows = std::min(L->max_targets, kFieldChunk);
+  const int chunks = (L->max_targets + kFieldChunk - 1) / kFieldChunk;
   for (const LaunchClass& k : P.far_classes) {
     a.order = P.far_ord + k.begin;
     const int ng = k.count;
     switch (k.nterms) {
-#define CASE(N)                                                            \
-  case N:                                                                  \
-    if (f32) launch_force<N, FK_COULOMB, float>(a, ng, s);                 \
-    else if (curl) launch_force<N, FK_SCREENED_CURL, double>(a, ng, s);    \
-    else if (korder) launch_force<N, FK_COULOMB_KORDER, double>(a, ng, s); \
-    else launch_force<N, FK_COULOMB, double>(a, ng, s);                    \
+#define CASE(N)                                                                            \
+  case N:                                                                                  \
+    if (korder) launch_korder<N>(a, ng, s);                                                \
+    else if (curl) launch_field<N, FAR_SCREENED, double>(a, ng, chunks, s);                \
+    else if (f32 && k.kind) launch_field<N, FAR_REG, float>(a, ng, chunks, s);             \
+    else if (f32) launch_field<N, 0, float>(a, ng, chunks, s);                             \
+    else if (k.kind) launch_field<N, FAR_REG, double>(a, ng, chunks, s);                   \
+    else launch_field<N, 0, double>(a, ng, chunks, s);                                     \
     break;
       CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)
 #undef CASE

@@ -726,18 +726,10 @@ def main(out):
         parts.append(f"  static constexpr int kPadded = {len(table)};")
         parts.append("  // canonical (i outer, j, k inner) index of the k-th moment in shell order")
         parts.append(f"  static __device__ __forceinline__ int canon(int k) {{ return kShellCanon{nt}[k]; }}")
-        parts.append("  template <class T> static __device__ __forceinline__ void force("
-                     "T dx, T dy, T dz, T rs, const T* __restrict__ M, T& fx, T& fy, T& fz) {")
-        parts += gen_force(nt)
-        parts.append("  }")
         parts.append("  template <class T> static __device__ __forceinline__ void force_korder("
                      "T dx, T dy, T dz, T rs, T del, int korder, const T* __restrict__ M, "
                      "T& fx, T& fy, T& fz) {")
         parts += gen_force_korder(nt)
-        parts.append("  }")
-        parts.append("  template <class T> static __device__ __forceinline__ void screened_curl("
-                     "T dx, T dy, T dz, T dist2, T kappa, const T* __restrict__ M, T& fx, T& fy) {")
-        parts += gen_screened_curl(nt)
         parts.append("  }")
         parts.append("};")
     parts.append("}  // namespace bit")

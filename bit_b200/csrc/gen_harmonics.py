@@ -28,9 +28,19 @@ beta_(s+1) = beta_s + x^2 beta_(s-1) / ((2s + 1)(2s - 1)), x = kappa rho: every 
 B_lm = Q_lm(z) Re / Im (x + i y)^m, Q_mm = 1, Q_(l+1)m = z Q_lm - c_lm |.|^2 Q_(l-1)m,
 c_lm = (l^2 - m^2)/(4 l^2 - 1): the associated Legendre function, scaled to a leading 1.
 
-Written per nterms: four evaluation functions (delta = 0 or not, kappa = 0 or not), the
-order in which they read a cluster's coefficients, and, once for all orders, the table of
-the harmonic moments A in terms of the shell-order Cartesian moments.
+The gradient of the same polynomial (treetaylorforce, :456-810; shielded_treetaylorforce,
+:2745-2973) reads the same coefficients.  With U_lm the coefficient times its radial factor,
+S = sum U_lm B_lm(v) and the derivative of the radial factors by Euler's theorem,
+
+  grad phi = c (S_v - d' (S + 2 v.S_v + sum U'_lm B_lm(v))),   S_v = grad_v S at fixed U,
+
+where U' is 2 s per term of E_(l+s) (delta > 0), and kappa^2 H r g_(l-1) / (2l - 1) in the place
+of g_l (screened, delta = 0).  S_v needs no further harmonics: d/dz B_lm = k_lm B_(l-1)m, and
+as a function of z and |v|^2, d/d|v|^2 Q_lm = n_lm Q_(l-1)(m+1).
+
+Written per nterms: four evaluation functions (delta = 0 or not, kappa = 0 or not), three of
+the gradient, the order in which they read a cluster's coefficients, and, once for all orders,
+the table of the harmonic moments A in terms of the shell-order Cartesian moments.
 
 Usage: python gen_harmonics.py <out.cuh>
 """
@@ -315,11 +325,219 @@ def gen_eval(nt, reg, scr):
     return L
 
 
+def grad_constants(lmax):
+    """{(l, m): (k_lm, n_lm)} of the header, from Q_lm as polynomials in z and n2 = |.|^2."""
+    Q = {}
+    for m in range(lmax + 2):
+        for l in range(m, lmax + 1):
+            if l == m:
+                Q[l, m] = {(0, 0): Fraction(1)}
+                continue
+            q = {(i + 1, j): c for (i, j), c in Q[l - 1, m].items()}
+            if l - 2 >= m:
+                for (i, j), c in Q[l - 2, m].items():
+                    q[i, j + 1] = q.get((i, j + 1), 0) - rec_c(l - 1, m) * c
+            Q[l, m] = {w: c for w, c in q.items() if c}
+
+    def ratio(a, b):
+        if not a:
+            return Fraction(0)
+        w = next(iter(b))
+        f = a[w] / b[w]
+        assert a == {v: f * c for v, c in b.items()}
+        return f
+    out = {}
+    for (l, m), q in Q.items():
+        dz, dn = {}, {}
+        for (i, j), c in q.items():  # d/dz with n2 following z, d/dn2 alone
+            if i:
+                dz[i - 1, j] = dz.get((i - 1, j), 0) + i * c
+            if j:
+                dz[i + 1, j - 1] = dz.get((i + 1, j - 1), 0) + 2 * j * c
+                dn[i, j - 1] = dn.get((i, j - 1), 0) + j * c
+        dz = {w: c for w, c in dz.items() if c}
+        out[l, m] = (ratio(dz, Q.get((l - 1, m), {(0, 0): 1})), ratio(dn, Q.get((l - 1, m + 1), {(0, 0): 1})))
+    return out
+
+
+GRADIENTS = [("ghc", False, False), ("ghs", False, True), ("grc", True, False)]
+
+
+def gen_grad(nt, reg, scr):
+    """Minus the gradient of one cluster's potential: arguments as gen_eval's, into fx, fy, fz."""
+    L = []
+    top = nt - 1
+    K = grad_constants(top)
+    if not reg:
+        L += ["  const T ri = rsqrt_t(r2);",
+              "  const T vx = dx * ri, vy = dy * ri, vz = dz * ri;"]
+        if top >= 1:
+            L.append("  const T eta = H * ri;")
+        if scr:
+            L += ["  const T r = r2 * ri;",
+                  "  const T x = kappa * r;",
+                  "  const T g0 = exp_t(-x) * ri;",
+                  "  const T h0 = x * g0;"]
+            if top >= 1:
+                L += ["  const T g1 = eta * fma_t(x, g0, g0);",
+                      "  const T kh = kappa * H;", "  const T kr = kh * x;"]
+            if top >= 2:
+                L.append("  const T kh2 = kh * kh;")
+            for l in range(2, nt):
+                c = Fraction(1, (2 * l - 1) * (2 * l - 3))
+                L.append(f"  const T g{l} = fma_t({lit(c)}, kh2 * g{l - 2}, eta * g{l - 1});")
+            for l in range(1, nt):
+                L.append(f"  const T h{l} = " + (f"{lit(Fraction(1, 2 * l - 1))} * (kr * g{l - 1});" if l > 1
+                                                 else f"kr * g{l - 1};"))
+        else:
+            L.append("  const T g0 = ri;")
+            for l in range(1, nt):
+                L.append(f"  const T g{l} = g{l - 1} * eta;")
+        n2 = None
+    else:
+        L += ["  const T rho2 = r2 + add;",
+              "  const T ri = rsqrt_t(rho2);"]
+        if top >= 1:
+            L += ["  const T eta = H * ri;",
+                  "  const T f = eta * ri;",
+                  "  const T vx = dx * f, vy = dy * f, vz = dz * f;"]
+        if top >= 2:
+            L += ["  const T n2 = fma_t(vx, vx, fma_t(vy, vy, vz * vz));",
+                  "  const T t1 = eta * eta;",
+                  "  const T t2 = t1 * t1;"]
+            for s in range(3, 2 * (top // 2) + 1):
+                L.append(f"  const T t{s} = t{s - 1} * t1;")
+            for s in range(2, 2 * (top // 2) + 1):
+                L.append(f"  const T y{s} = {lit(2 * s)} * t{s};")
+        n2 = "n2"
+    ld = Loads(L)
+
+    def column(m):
+        """q{m}_l for l > m, once (Q_mm = 1)."""
+        for l in range(m + 1, nt):
+            if l == m + 1:
+                L.append(f"  const T q{m}_{l} = vz;")
+                continue
+            c = lit(-rec_c(l - 1, m))
+            prev = f"q{m}_{l - 2}" if l - 2 > m else None
+            if n2:
+                tail = f"{c} * n2" if prev is None else f"{c} * (n2 * {prev})"
+            else:
+                tail = c if prev is None else f"{c} * {prev}"
+            L.append(f"  const T q{m}_{l} = fma_t(vz, q{m}_{l - 1}, {tail});")
+
+    Q = lambda l, m: None if l == m else f"q{m}_{l}"
+    have = set()
+
+    def add(P, a, b):
+        """P += a * b; a or b None stands for 1."""
+        e = a if b is None else b if a is None else None
+        if P in have:
+            L.append(f"  {P} = {e} + {P};" if e else f"  {P} = fma_t({a}, {b}, {P});")
+        else:
+            L.append(f"  T {P} = {e};" if e else f"  T {P} = {a} * {b};")
+            have.add(P)
+
+    mono = ld.get()
+    column(0)
+    for m in range(nt):
+        if m == 1:
+            L.append("  const T c1 = vx, s1 = vy;")
+        elif m > 1:
+            L += [f"  const T c{m} = fma_t(vx, c{m - 1}, -(vy * s{m - 1}));",
+                  f"  const T s{m} = fma_t(vx, s{m - 1}, vy * c{m - 1});"]
+        if m < top:
+            column(m + 1)
+        for l in range(m, nt):
+            if (l, m) != (0, 0):
+                k, n = K[l, m]
+                if l - 1 >= m:
+                    w = Q(l - 1, m)
+                    L.append(f"  const T z{m}_{l} = " + (f"{lit(k)} * {w};" if w else f"{lit(k)};"))
+                if l - 1 >= m + 1:
+                    w = Q(l - 1, m + 1)
+                    L.append(f"  const T n{m}_{l} = " + (f"{lit(2 * n)} * {w};" if w else f"{lit(2 * n)};"))
+            for part in range(2 if m else 1):
+                pq = f"{'pq'[part]}{m}"
+                nm = f"u{m}_{l}_{part}"
+                if reg:
+                    u = g = None
+                    for s in radial_set(nt, l, True):
+                        if (l, m, s) == (0, 0, 0):
+                            continue
+                        mv = ld.get()
+                        u = (mv if s == 0 else f"{mv} * t{s}") if u is None else f"fma_t({mv}, t{s}, {u})"
+                        if s:
+                            g = f"{mv} * y{s}" if g is None else f"fma_t({mv}, y{s}, {g})"
+                else:
+                    mv = mono if (l, m) == (0, 0) else ld.get()
+                    u = f"{mv} * g{l}"
+                    g = f"{mv} * h{l}" if scr else None
+                if u is not None:
+                    L.append(f"  const T {nm} = {u};")
+                    if reg or (l, m) != (0, 0):  # (delta = 0: the monopole is added at the end)
+                        add(pq, nm, Q(l, m))
+                    if l - 1 >= m:
+                        add("z" + pq, nm, f"z{m}_{l}")
+                    if l - 1 >= m + 1:
+                        add("n" + pq, nm, f"n{m}_{l}")
+                if g is not None:
+                    L.append(f"  const T v{nm} = {g};")
+                    add("g" + pq, "v" + nm, Q(l, m))
+        # the sums of this m: S, its derivatives, and the radial part
+        for sp, tot in (("", "S"), ("z", "Sz"), ("n", "N"), ("g", "G")):
+            if sp + f"p{m}" in have:
+                add(tot, sp + f"p{m}", f"c{m}" if m else None)
+            if m and sp + f"q{m}" in have:
+                add(tot, sp + f"q{m}", f"s{m}")
+        if m and f"p{m}" in have:
+            mm = lit(m)
+            if m == 1:
+                add("Sx", "p1", None)
+                add("Sy", "q1", None)
+            else:
+                L.append(f"  const T a{m} = {mm} * p{m}, e{m} = {mm} * q{m};")
+                add("Sx", f"a{m}", f"c{m - 1}")
+                add("Sx", f"e{m}", f"s{m - 1}")
+                add("Sy", f"e{m}", f"c{m - 1}")
+                add("Sy", f"-a{m}", f"s{m - 1}")
+    if "N" in have:
+        add("Sx", "vx", "N")
+        add("Sy", "vy", "N")
+    e = "S" if "S" in have else None
+    if "Sz" in have:
+        L.append(f"  const T dot = fma_t(vx, Sx, fma_t(vy, Sy, vz * Sz));")
+        e = f"fma_t(T(2), dot, {e})"
+    if "G" in have:
+        e = f"{e} + G" if e else "G"
+    if reg:
+        L.append(f"  const T R = {f'{mono} + ({e})' if e else mono};")
+        L.append("  const T i2 = ri * ri;")
+        for a in "xyz":  # (ri^3 would leave the range of FP32 earlier than the field does)
+            w = f"(d{a} * ri)"
+            L.append(f"  f{a} = i2 * " + (f"fma_t({w}, R, -(eta * S{a}));" if "Sz" in have else f"({w} * R);"))
+    else:
+        L.append(f"  const T R = " + (f"fma_t({mono}, g0, {e});" if e else f"{mono} * g0;"))
+        for a in "xyz":
+            L.append(f"  f{a} = ri * " + (f"fma_t(v{a}, R, -S{a});" if "Sz" in have else f"(v{a} * R);"))
+    return L
+
+
+def field_flops_per_pair(nt):
+    """Flops per pair of the fields: "force" (delta > 0), "force0" (delta = 0), "curl"."""
+    f = lambda reg, scr: (lambda c: 2 * c[0] + c[1])(count_ops(gen_grad(nt, reg, scr)))
+    return {"force": f(True, False), "force0": f(False, False), "curl": f(False, True)}
+
+
 def ops_per_pair(nt, reg, scr):
     """(fma, other) floating-point instructions of one evaluation."""
+    return count_ops(gen_eval(nt, reg, scr))
+
+
+def count_ops(lines):
     import re
     fma = other = 0
-    for ln in gen_eval(nt, reg, scr):
+    for ln in lines:
         if "ld4(" in ln:
             continue
         e = re.sub(r"T\([^()]*\)", "C", ln.split("=", 1)[-1])
@@ -398,6 +616,12 @@ def main(out):
             parts.append(f"  template <class T> static __device__ __forceinline__ T {nm}("
                          "T dx, T dy, T dz, T r2, T add, T kappa, T H, const T* __restrict__ M) {")
             parts += ["  " + ln for ln in gen_eval(nt, reg, scr)]
+            parts.append("  }")
+        for nm, reg, scr in GRADIENTS:
+            parts.append(f"  template <class T> static __device__ __forceinline__ void {nm}("
+                         "T dx, T dy, T dz, T r2, T add, T kappa, T H, const T* __restrict__ M, T& fx, T& fy, "
+                         "T& fz) {")
+            parts += ["  " + ln for ln in gen_grad(nt, reg, scr)]
             parts.append("  }")
         parts.append("};")
     parts.append("}  // namespace bit")

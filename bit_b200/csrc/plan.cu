@@ -44,6 +44,7 @@ SysEval make_sys_eval(const bit_eval_params& p, int nterms, int points, int forc
     s.near_sign = 1;
     s.eps_check = 0;
     s.particles = 1;
+    s.far_kind = 1;
     return s;
   }
   if (force) {
@@ -55,6 +56,7 @@ SysEval make_sys_eval(const bit_eval_params& p, int nterms, int points, int forc
     s.near_sign = 1;
     s.eps_check = 0;
     s.particles = 1;
+    s.far_kind = p.del != 0.0 ? 2 : 0;  // (a field's del may be negative)
     return s;
   }
   switch (p.kernel) {

@@ -6,6 +6,7 @@ Tolerance: both sides sum a few hundred products of size at most eta^n (eta = 0.
 largest cluster-radius ratio here) times sum |q| e^(-kappa R) / R, so each side's rounding
 is below about 500 * 1.1e-16 * sum_n eta^n = 4e-13 of that scale."""
 import math
+import re
 
 import numpy as np
 import pytest
@@ -92,3 +93,46 @@ def test_harmonic_moments_keep_every_cartesian_moment():
             assert deg * (deg + 1) * (deg + 2) // 6 <= p < (deg + 1) * (deg + 2) * (deg + 3) // 6
             A[i, p] = f
     assert np.linalg.matrix_rank(A / np.abs(A).max(axis=1, keepdims=True)) == n
+
+
+@pytest.mark.parametrize("nt", range(1, 11))
+def test_gradients_equal_the_taylor_recurrences(nt):
+    """The generated gradients against the literal field sums: Coulomb with and without delta,
+    and the screened curl (d phi/dy, -d phi/dx).  A field term is at most (n + 1) / R times its
+    potential's, so the scale is that of the potential times nterms / R."""
+    g, t = gen(), gen_taylor()
+    args = ["dx", "dy", "dz", "rs", "M", "fx", "fy", "fz"]
+
+    def fields(lines, names):
+        out = lines + ["  return fx, fy, fz;"]
+        return compile_lines([re.sub(r"f([xyz]) \+= (\w+)", r"f\1 = \2", ln) for ln in out], names)
+
+    coulomb = fields(t.gen_force(nt), args)
+    curl = fields(t.gen_screened_curl(nt), ["dx", "dy", "dz", "dist2", "kappa", "M", "fx", "fy", "fz"])
+    shells = list(t.shells(nt - 1))
+    rng = np.random.default_rng(nt)
+    for name, reg, scr in g.GRADIENTS:
+        f = fields(g.gen_grad(nt, reg, scr), ARGS)
+        for trial in range(12):
+            radius = 10.0 ** rng.uniform(-5, 1)
+            y = rng.uniform(-1, 1, (30, 3)) * radius / math.sqrt(3.0)
+            q = rng.uniform(-1, 1, 30)
+            M = np.array([np.sum(q * y[:, 0] ** v[0] * y[:, 1] ** v[1] * y[:, 2] ** v[2])
+                          for v in shells])
+            d = rng.standard_normal(3)
+            d *= radius / math.sqrt(rng.uniform(0.05, 0.75)) / np.linalg.norm(d)
+            delta = radius ** 2 * 10.0 ** rng.uniform(-6, 3) if reg else 0.0
+            kappa = rng.uniform(0.0, 4.0) / radius if scr else 0.0
+            r2 = float(d @ d)
+            R2 = r2 + delta
+            H = 2.0 ** (math.floor(math.log2(max(radius, math.sqrt(delta)))) + 1)
+            pad = np.concatenate([M, np.zeros(-len(M) % 4)])
+            got = f(*d, r2, delta, kappa, H, coefficients(g, nt, reg, M, kappa, delta, H))
+            if scr:
+                want = curl(*d, R2, kappa, pad, 0.0, 0.0, 0.0)
+                got = (-got[1], got[0], 0.0)
+            else:
+                want = coulomb(*d, R2, pad, 0.0, 0.0, 0.0)
+            scale = np.abs(q).sum() * math.exp(-kappa * math.sqrt(R2)) / R2 * (nt + kappa * math.sqrt(R2))
+            scale *= 1.0 + (kappa * radius) ** (nt - 1) / math.factorial(nt - 1)
+            assert np.max(np.abs(np.subtract(got, want))) <= TOL * scale, (name, trial, got, want)
