@@ -17,6 +17,7 @@ namespace bit {
 constexpr int kWarp = 32;
 constexpr int kNtermsMax = BIT_NTERMS_MAX;
 constexpr int kGroupMax = 1024;   // targets per group (one CTA; 32 mask words)
+constexpr int kFieldChunk = 256;       // targets of a CTA of the fields' kernels, at most
 constexpr int kPointGroup = 256;  // external points per group, at most
 constexpr int kNearParts = 8;         // near-field items of a group, at most
 constexpr long long kNearChunk = 512 << 10;  // and the pairs of one, at least
@@ -170,6 +171,7 @@ struct Lists {
   bool valid = false;
   int ngroups = 0;
   int ntargets = 0;                         // targets the groups cover
+  int field_chunk = kFieldChunk;            // targets of a CTA of the fields' kernels
   int max_targets = 0;                      // of the largest group, rounded up to 32
   long long nfar = 0, nnear = 0;            // entries
   long long far_pairs = 0, near_pairs = 0;  // interactions

@@ -68,7 +68,8 @@ struct FarArgs {
   const long long* mom_off;  // first moment of each node
   const void* coef;          // float or double: every node's coefficients (potential kernels)
   int stride;                // elements from one node's coefficients to the next's
-  int rows;                  // targets of the largest group, rounded up to 32 (potentials)
+  int rows;                  // targets of the largest group (fields: chunk), rounded up to 32
+  int chunk;                 // fields: targets of a CTA, at most
   int* err;                  // device error flags (a bounded wait that gave up: 8)
   const int* tgt;            // targets of each far entry (potentials)
   const long long* pre;      // targets of the group's entries before it
@@ -390,8 +391,8 @@ __global__ void __launch_bounds__(32 * NW, 2) k_far_queue(FarArgs a, int count, 
 
 // Far field of the vector fields: the regularised Coulomb field of treetaylorforce (KIND 0 or
 // FAR_REG) and the screened 2-D field of shielded_treetaylorforce (KIND FAR_SCREENED), as the
-// gradients of the potentials' polynomials (gen_harmonics.py).  A CTA takes up to kFieldChunk
-// targets of a group, so that the three rows of FP64 sums a warp keeps stay small: the
+// gradients of the potentials' polynomials (gen_harmonics.py).  A CTA takes a chunk of a
+// group's targets (32 to 256, Lists::field_chunk), so that the three rows of FP64 sums a warp keeps stay small: the
 // recurrence kernel that this replaces had rows for a whole group of 1024, 130 KB, and so four
 // warps a multiprocessor.  Entries are shared out to the warps as in far_group (by the work of
 // the whole group), and rows are summed in warp order.  Bound by the FP64 / FP32 pipe: 1,252
@@ -399,7 +400,6 @@ __global__ void __launch_bounds__(32 * NW, 2) k_far_queue(FarArgs a, int count, 
 // without, mixed, screened, ms: 2M clustered, nterms 9: 32.3 / 11.3, 32.2 / 7.3, 27.3 / 7.1, 41.8 /
 // 10.3; 150k, 9: 1.14 / 0.44, 1.14 / 0.29, 0.99 / 0.29, 1.47 / 0.39; 20k, 6: 0.145 / 0.077, 0.144 /
 // 0.070, 0.119 / 0.064, 0.152 / 0.082.  Mixed against FP64, 2M: 3.4e-7 / 1.9e-7.
-constexpr int kFieldChunk = 256;
 // CTAs of eight warps per SM: two (128 registers) hold every order without spills; three (80)
 // do up to nterms 4, 230 -> 198 us on 100k in leaves of 100, but cost 50k, nterms 7, 165 -> 183.
 // (One CTA, 166 registers: 2M 13.3 ms.)
@@ -410,18 +410,17 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   constexpr int NW = NWP;
   constexpr int CNT = far_count(NT, KIND);
   constexpr int TP = far_block(NT, KIND);
-  constexpr int WC = kFieldChunk / 32;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ uint64_t bar[NW];
-  const int g = a.order[blockIdx.x], c0 = blockIdx.y * kFieldChunk;
-  const int t0 = a.g_tstart[g] + c0, gc = a.g_tcount[g], tc = min(gc - c0, kFieldChunk);
+  const int g = a.order[blockIdx.x], c0 = blockIdx.y * a.chunk;
+  const int t0 = a.g_tstart[g] + c0, gc = a.g_tcount[g], tc = min(gc - c0, a.chunk);
   if (tc <= 0) return;  // (the whole CTA)
   far_bars_init<NW>(bar);
   const int rows = a.rows;
   double* accb = reinterpret_cast<double*>(sm);  // [NW][3][rows]
   T* msb = reinterpret_cast<T*>(accb + NW * 3 * rows);
   unsigned short* tlb = reinterpret_cast<unsigned short*>(msb + NW * a.stride);
-  const int W = (gc + 31) >> 5, w0 = blockIdx.y * WC, wn = (tc + 31) >> 5;
+  const int W = (gc + 31) >> 5, w0 = c0 >> 5, wn = (tc + 31) >> 5;
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
@@ -721,8 +720,9 @@ void eval_far_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* fy
     if (f32) far_coefs<float>(t, P, a, s);
     else far_coefs<double>(t, P, a, s);
   }
-  a.rows = std::min(L->max_targets, kFieldChunk);
-  const int chunks = (L->max_targets + kFieldChunk - 1) / kFieldChunk;
+  a.chunk = L->field_chunk;
+  a.rows = std::min(L->max_targets, a.chunk);
+  const int chunks = (L->max_targets + a.chunk - 1) / a.chunk;
   for (const LaunchClass& k : P.far_classes) {
     a.order = P.far_ord + k.begin;
     const int ng = k.count;

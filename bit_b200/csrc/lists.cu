@@ -460,6 +460,21 @@ static int point_group(int m, int sms) {
   return size;
 }
 
+// Targets of a CTA of the fields' kernels, which keep three sums a target and warp: at most
+// kFieldChunk, and fewer where the groups would leave the chip idle.  Far + near, FP64 Coulomb
+// field, chunks of 32 / 64 / 128 / 256, us: 2k in leaves of 500 61 / 78 / 96 / 132; 8k, 300: 100 /
+// 108 / 136 / 197; 20k, 200: 168 / 153 / 180 / 186; 50k, 300: 460 / 388 / 392 / 485; 100k, 300: 854 /
+// 667 / 587 / 600; 150k, 600: 1817 / 1361 / 1138 / 1045; 2M, 1000, ms: 42.8 / 31.0 / 25.2 / 22.3 (whole
+// groups of 1000: 25.2).
+static int field_chunk(const std::vector<int>& tc, int sms) {
+  for (int size = kFieldChunk; size > 32; size /= 2) {
+    long long chunks = 0;
+    for (int k : tc) chunks += (k + size - 1) / size;
+    if (2 * chunks >= 5LL * sms) return size;
+  }
+  return 32;
+}
+
 // The potentials' near-field items, heaviest first: a group's near work in one item, or in up
 // to kNearParts equal parts of at least kNearChunk pairs each, whose sums meet in scratch
 // (near_part).  The count follows from the group's own lists alone, so that its result does
@@ -578,6 +593,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   int maxw = 1;
   for (int g = 0; g < ng; g++) maxw = std::max(maxw, (tc[g] + 31) / 32);
   L->max_targets = 32 * maxw;
+  L->field_chunk = field_chunk(tc, c->num_sms);
   int per_sm = 0;
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists, QT, 0));
   const long long nodes = std::max(t->numtree, 1);

@@ -1,6 +1,6 @@
 // Near field of the fields: the leaf direct sums of treeforce / shielded_treeforce
 // (src/tree3d.cpp:923-967, 3378-3398), with the work shared out as the potentials' (near.cu):
-// one CTA per item, every warp a contiguous run of the group's sources, two targets a lane,
+// one CTA per item and chunk of the group's targets, every warp a contiguous run of the group's sources, two targets a lane,
 // its own tiles and accumulator rows (three, in FP64).
 //
 // FP64: the reference's sums, with 1/r^3 from one reciprocal square root: 16 FP64 operations a
@@ -8,9 +8,10 @@
 // relative to their leaf centre, the target's offset from that centre formed in FP64 and
 // rounded once, a tile's sums in FP32; pairs too close for FP32 coordinates are summed in FP64.
 // Bound by the FP64 pipe, mixed by issue.  Before (a square root and a division, one target a
-// thread, a barrier per tile) / now, FP64 Coulomb field, ms: 2M clustered in leaves of 1000,
-// theta = 0.7, 24.2 / 14.2 (rows of 1,000 targets leave eight warps an SM); 100k in leaves of
-// 500, theta = 0.15, 12.9 / 2.0; 300k uniform in leaves of 100 1.28 / 0.33; 20k 0.32 / 0.11.
+// thread, a barrier per tile) / now, ms: 2M clustered in leaves of 1000, theta = 0.7, FP64 Coulomb
+// 24.2 / 11.0, mixed 7.6 / 6.1, screened 40.3 / 21.1; 100k uniform in leaves of 100 0.57 / 0.16, 0.47 /
+// 0.11, 0.70 / 0.24; 50k in leaves of 300 1.03 / 0.24, 0.47 / 0.13, 1.50 / 0.47; 20k 0.33 / 0.09,
+// 0.21 / 0.06, 0.42 / 0.13.
 #include <algorithm>
 #include <type_traits>
 
@@ -23,8 +24,7 @@ namespace bit {
 
 namespace {
 
-// Warps per CTA: four, so that the three rows of groups of 1,000 targets leave room for two
-// CTAs an SM.
+// Warps per CTA: with chunks of 256 targets, their three rows leave room for four CTAs an SM.
 constexpr int NW = 4;
 // The regularised Coulomb field, the same with the reference's KERNEL_ORDER family, the
 // screened 2-D field.
@@ -178,6 +178,7 @@ __device__ __forceinline__ Vec sum32(const Tile32& r, double px, double py, doub
 
 struct Layout {
   int recs, rows, tab;  // records of a tile, targets of a row, bytes of the exponential's table
+  int chunk;            // targets of a CTA, at most
   int single;           // no scratch: part 0 takes the whole group
   __host__ __device__ size_t warp_bytes() const {
     return 2 * (size_t)recs * kRec + (size_t)rows * (3 * sizeof(double) + sizeof(unsigned short));
@@ -209,9 +210,11 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   double* row = rows + (size_t)w * 3 * L.rows;
   unsigned short* tl = reinterpret_cast<unsigned short*>(rows + (size_t)NW * 3 * L.rows) + (size_t)w * L.rows;
 
-  const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
+  const int gc = a.g_tcount[g], c0 = blockIdx.y * L.chunk, tc = min(gc - c0, L.chunk);
+  if (tc <= 0) return;  // (the whole CTA)
+  const int t0 = a.g_tstart[g] + c0, chunks = (gc + L.chunk - 1) / L.chunk;
   const SysEval* se = a.sys + a.g_sys[g];
-  const int W = (tc + 31) >> 5;
+  const int W = (gc + 31) >> 5, w0 = c0 >> 5, wn = (tc + 31) >> 5;  // words of the group, the chunk
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
   for (int i = tid; i < NW * 3 * L.rows; i += 32 * NW) rows[i] = 0.0;
@@ -230,10 +233,14 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   for (; e < e1; e++) {
     const long long P = a.pre[e];
     if (P >= T1) break;
-    const int node = a.node[e], ns = a.nummemb[node], cnt = a.tgt[e];
-    const int wt = near_weight(cnt);
+    const int node = a.node[e], ns = a.nummemb[node], ec = a.tgt[e];
+    const int wt = near_weight(ec);  // (the work is shared out by the whole group's)
     const int ja = cut(T0, P, wt, ns), jb = cut(T1, P, wt, ns);
     if (ja >= jb) continue;
+    const bool all = ec == gc;
+    const unsigned wd = !all && lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
+    const int cnt = all ? tc : __reduce_add_sync(0xffffffffu, __popc(wd));
+    if (!cnt) continue;
     const int s0 = a.start[node];
     const unsigned char* src =
         reinterpret_cast<const unsigned char*>(a.src) + (size_t)(F32 ? a.pstart[node] : s0) * kRec;
@@ -247,11 +254,7 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
       }
     };
     fetch(ja, phase);
-    const bool all = cnt == tc;
-    if (!all) {
-      const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-      pack_list(wd, W, tl);
-    }
+    if (!all) pack_list(wd, wn, tl);
     const bool self = s0 < t0 + tc && t0 < s0 + ns;
     const double4 c = a.nodec[node];
     const float4 hb = a.nodeh[node];
@@ -353,29 +356,28 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
     return s;
   };
   double* sum = a.part + 3 * a.part_off[g];
-  if (parts > 1) {
-    for (int i = tid; i < 3 * tc; i += 32 * NW) sum[(long long)part * 3 * tc + i] = warps_sum(i / tc, i % tc);
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-      s_last = atomicAdd(&a.part_done[g], 1) == parts - 1;
-      if (s_last) {
-        a.part_done[g] = 0;
-        __threadfence();
-      }
-    }
-    __syncthreads();
-    if (!s_last) return;
+  double* out[3] = {a.out, a.out_y, a.out_z};
+  if (parts == 1) {
+    for (int i = tid; i < 3 * tc; i += 32 * NW) out[i / tc][t0 + i % tc] += warps_sum(i / tc, i % tc);
+    return;
   }
-  for (int i = tid; i < 3 * tc; i += 32 * NW) {
-    const int d = i / tc, k = i % tc;
-    double s = 0.0;
-    if (parts > 1) {
-      for (int q = 0; q < parts; q++) s += __ldcg(sum + (long long)q * 3 * tc + i);
-    } else {
-      s = warps_sum(d, k);
+  for (int i = tid; i < 3 * tc; i += 32 * NW)
+    sum[((long long)part * 3 + i / tc) * gc + c0 + i % tc] = warps_sum(i / tc, i % tc);
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    s_last = atomicAdd(&a.part_done[g], 1) == parts * chunks - 1;
+    if (s_last) {
+      a.part_done[g] = 0;
+      __threadfence();
     }
-    (d == 0 ? a.out : d == 1 ? a.out_y : a.out_z)[t0 + k] += s;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  for (int i = tid; i < 3 * gc; i += 32 * NW) {
+    double s = 0.0;
+    for (int q = 0; q < parts; q++) s += __ldcg(sum + (long long)q * 3 * gc + i);
+    out[i / gc][t0 - c0 + i % gc] += s;
   }
 }
 
@@ -430,7 +432,9 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
   lay.single = L->field_part.n < need && c->budget && c->in_use + need * sizeof(double) > c->budget;
   if (!lay.single) L->field_part.ensure(c, need);
   a.part = L->field_part.p;
-  lay.rows = L->max_targets;
+  lay.chunk = L->field_chunk;
+  lay.rows = std::min(L->max_targets, lay.chunk);
+  const int chunks = (L->max_targets + lay.chunk - 1) / lay.chunk;
   lay.tab = P.force == 2 ? kExpTabBytes : 0;
   lay.recs = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 64;
   // four CTAs an SM if tiles of 32 do it
@@ -439,7 +443,7 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
     a.items = P.near_it + k.ibegin;
     auto go = [&](auto kernel) {
       ensure_smem_attr(reinterpret_cast<const void*>(kernel), kSmemMax - 1024);
-      count_launch(), kernel<<<k.icount, 32 * NW, lay.total(), s>>>(a, lay);
+      count_launch(), kernel<<<dim3(k.icount, chunks), 32 * NW, lay.total(), s>>>(a, lay);
       BIT_CHECK_LAUNCH();
     };
     if (P.force == 2) go(k_near_field<F_CURL, false>);

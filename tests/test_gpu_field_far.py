@@ -35,6 +35,23 @@ def test_groups_around_the_chunks(ctx, orc, maxmemb):
     compare(ctx, orc, x, y, z, q, maxmemb, 5, 0.8, 1e-3)
 
 
+@pytest.mark.parametrize("n,maxmemb", [(20000, 200), (50000, 300), (100000, 300), (150000, 1000)])
+def test_larger_systems_take_larger_chunks(ctx, orc, n, maxmemb):
+    import bit_b200 as B
+    from bit_b200 import workloads
+    x, y, z, q = workloads.clustered_blobs(n, seed=n)
+    t = ctx.treemake(x, y, z, maxmemb)
+    t.treemoments(q, 4)
+    T = orc.Tree(x, y, z, maxmemb)
+    T.compute_moments(q, 4)
+    tg = workloads.sample_targets(n, 400, seed=1)
+    want = np.stack(T.evaluate_force(1e-3, 0.7, targets=tg))
+    for prec, tol in ((B.FP64, 1e-12), (B.MIXED, 2e-6)):
+        got = np.stack(t.treeforce(0.7, 1e-3, prec))[:, tg]
+        assert np.max(np.abs(got - want)) <= tol * np.max(np.abs(want))
+    t.treeempty()
+
+
 @pytest.mark.parametrize("nterms", range(1, 11))
 @pytest.mark.parametrize("delta", [1e-2, 0.0, -1e-9])
 def test_every_order_and_sign_of_delta(ctx, orc, nterms, delta):
