@@ -221,12 +221,31 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
 // Shared memory of a CTA: the exponential's table (FP64 screened), per warp two source tiles,
 // an accumulator row (a double, or a float and its error, per target) and a target list.
 // Tiles are counted in 32-byte records: one FP64 source, two FP32 ones.
+// A group's tiles are as large as its own rows leave room for beside a second CTA, so that its
+// sums do not depend on the other groups of the launch.  At most 128 records: 64 / 96 / 128, FP64
+// screened, FP64 Coulomb, mixed screened, mixed Coulomb, us: 2M in leaves of 1000 17223 / 17073 /
+// 17032, 7530 / 7407 / 7370, 5921 / 5794 / 5757, 3765 / 3618 / 3569; 20k, 500: 367 / 363 / 361, 150 / 144
+// / 140, 127 / 121 / 121, 88 / 82 / 82; 300k, 100: 516 / 477 / 478, 320 / 281 / 279, 295 / 295 / 295, 248 /
+// 246 / 248.
 struct Layout {
-  int recs, rows, tab;  // tab: bytes of the table
-  __host__ __device__ size_t warp_bytes() const {
+  int cap, tab;  // records of a tile at most; bytes of the table
+  static __host__ __device__ int rows(int tc) { return (tc + 31) / 32 * 32; }
+  template <bool F32>
+  static __host__ __device__ int recs(int cap, int rows) {
+    constexpr int room = (kSmemMax / 2 - 1024 - (F32 ? 0 : kExpTabBytes)) / NW;
+    const int n = (room - rows * (int)(sizeof(double) + sizeof(unsigned short))) / (2 * kRec) / 16 * 16;
+    return n < 16 ? 16 : (n < cap ? n : cap);
+  }
+  static __host__ __device__ size_t warp_bytes(int recs, int rows) {
     return 2 * (size_t)recs * kRec + (size_t)rows * (sizeof(double) + sizeof(unsigned short));
   }
-  __host__ __device__ size_t total() const { return tab + NW * warp_bytes(); }
+  // for every group of up to `most` targets
+  template <bool F32>
+  size_t total(int most) const {
+    size_t b = 0;
+    for (int r = 32; r <= most; r += 32) b = std::max(b, warp_bytes(recs<F32>(cap, r), r));
+    return tab + NW * b;
+  }
 };
 
 // Returns false (in every thread) if a warp's bounded wait for a tile gave up: the error flag
@@ -237,24 +256,25 @@ template <int KER, bool EPS, bool F32>
 __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, int2 item, uint64_t* bar,
                                           unsigned& phase) {
   constexpr int PER = F32 ? 2 : 1;  // sources of a record
-  const int TILE = L.recs * PER;
-  const int g = item.x, part = item.y & 0xffff, parts = item.y >> 16;
+  const int g = item.x, ROWS = Layout::rows(a.g_tcount[g]), RECS = Layout::recs<F32>(L.cap, ROWS);
+  const int TILE = RECS * PER;
+  const int part = item.y & 0xffff, parts = item.y >> 16;
   __shared__ int s_last;
   extern __shared__ __align__(128) unsigned char sm[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const double2* tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
   unsigned char* tiles0 = sm + L.tab;
-  unsigned char* tiles = tiles0 + (size_t)w * 2 * L.recs * kRec;
-  double* rows = reinterpret_cast<double*>(tiles0 + NW * 2 * (size_t)L.recs * kRec);
-  double* row = rows + (size_t)w * L.rows;
-  unsigned short* tl = reinterpret_cast<unsigned short*>(rows + (size_t)NW * L.rows) + (size_t)w * L.rows;
+  unsigned char* tiles = tiles0 + (size_t)w * 2 * RECS * kRec;
+  double* rows = reinterpret_cast<double*>(tiles0 + NW * 2 * (size_t)RECS * kRec);
+  double* row = rows + (size_t)w * ROWS;
+  unsigned short* tl = reinterpret_cast<unsigned short*>(rows + (size_t)NW * ROWS) + (size_t)w * ROWS;
 
   const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
   const SysEval* se = a.sys + a.g_sys[g];
   const int W = (tc + 31) >> 5;
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
-  for (int i = tid; i < NW * L.rows; i += 32 * NW) rows[i] = 0.0;
+  for (int i = tid; i < NW * ROWS; i += 32 * NW) rows[i] = 0.0;
   // this warp's run [T0, T1) of the group's work (all parts' warps share it), and the entry
   // it begins in: the last whose prefix is at most T0
   const long long tot = a.tot[g];
@@ -282,7 +302,7 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
         const unsigned bytes = (unsigned)((cnt_j + PER - 1) / PER) * kRec;
         fence_proxy_async();
         mbar_expect_tx(&bar[2 * w + (n & 1)], bytes);
-        tma_load_1d(tiles + (n & 1) * L.recs * kRec, src + (size_t)(j / PER) * kRec, bytes,
+        tma_load_1d(tiles + (n & 1) * RECS * kRec, src + (size_t)(j / PER) * kRec, bytes,
                     &bar[2 * w + (n & 1)]);
       }
     };
@@ -320,7 +340,7 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
         failed = true;
         break;
       }
-      const unsigned char* tile = tiles + (phase & 1) * L.recs * kRec;
+      const unsigned char* tile = tiles + (phase & 1) * RECS * kRec;
       phase++;
       const int own = t0 - s0 - j;
       if constexpr (F32) {
@@ -328,8 +348,8 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
         r32.n = jn - j;
         float* row32 = reinterpret_cast<float*>(row);
         const int toff = j / TILE * TILE;
-        if (self) tile32<KER, true>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, own, row32, L.rows, t0, g, e, toff);
-        else tile32<KER, false>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, 0, row32, L.rows, t0, g, e, toff);
+        if (self) tile32<KER, true>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, own, row32, ROWS, t0, g, e, toff);
+        else tile32<KER, false>(a, r32, cx, cy, cz, c, hb, tl, all, cnt, 0, row32, ROWS, t0, g, e, toff);
       } else {
         const Range64 r{reinterpret_cast<const double4*>(tile), jn - j, del, ks, tab};
         if (KER != BIT_KERNEL_COULOMB && se->underflow) {
@@ -348,10 +368,10 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
   auto warps_sum = [&](int i) {
     double s = 0.0;
     for (int q = 0; q < NW; q++) {
-      const double* x = rows + (size_t)q * L.rows;
+      const double* x = rows + (size_t)q * ROWS;
       if (F32) {
         const float* f = reinterpret_cast<const float*>(x);
-        s += (double)f[i] + (double)f[L.rows + i];
+        s += (double)f[i] + (double)f[ROWS + i];
       } else {
         s += x[i];
       }
@@ -488,7 +508,7 @@ __device__ double close_sum(const NearArgs& a, const SysEval* se, int t, int g, 
     for (int k = 0; k < nrec; k++) {
       if (k && r[k].x == r[k - 1].x && r[k].y == r[k - 1].y) continue;
       const int node = a.node[r[k].x];
-      tile(node, r[k].y, min(r[k].y + a.tile, a.nummemb[node]));
+      tile(node, r[k].y, min(r[k].y + 2 * Layout::recs<true>(a.cap, Layout::rows(a.g_tcount[g])), a.nummemb[node]));
     }
   } else {
     const int i = t - a.g_tstart[g], W = (a.g_tcount[g] + 31) >> 5;
@@ -527,25 +547,22 @@ void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
   Ctx* c = t->ctx;
   cudaStream_t s = c->stream;
   Layout lay;
-  lay.rows = L->max_targets;
   lay.tab = 0;
   for (const LaunchClass& k : P.near_classes)
     if (!F32 && k.kernel != BIT_KERNEL_COULOMB) lay.tab = kExpTabBytes;
   // a context's tile setting counts the records of a CTA's eight warps
-  lay.recs = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 64;
-  // two CTAs an SM: rows of 1,024 targets and the table leave room for tiles of 48
-  while (lay.recs > 16 && lay.total() > kSmemMax / 2 - 1024) lay.recs -= 16;
-  a.tile = lay.recs * (F32 ? 2 : 1);
+  lay.cap = a.cap = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 128;
+  const size_t bytes = lay.total<F32>(L->max_targets);
   if (c->work_queue && P.near_classes.size() > 1) {
     const int count = (int)L->h_items.size();
     a.items = L->items.p;
     ensure_smem_attr(reinterpret_cast<const void*>(k_near_queue<F32>), kSmemMax - 1024);
     int per_sm = 0;
-    BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32>, 32 * NW, lay.total()));
+    BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32>, 32 * NW, bytes));
     const int grid = std::max(1, std::min(count, c->num_sms * std::max(per_sm, 1)));
     c->queue_heads.ensure(c, 2);
     BIT_CUDA(cudaMemsetAsync(c->queue_heads.p + 1, 0, sizeof(int), s));
-    count_launch(), k_near_queue<F32><<<grid, 32 * NW, lay.total(), s>>>(a, lay, count, c->queue_heads.p + 1);
+    count_launch(), k_near_queue<F32><<<grid, 32 * NW, bytes, s>>>(a, lay, count, c->queue_heads.p + 1);
     BIT_CHECK_LAUNCH();
     return;
   }
@@ -553,7 +570,7 @@ void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
     a.items = P.near_it + k.ibegin;
     auto go = [&](auto kernel) {
       ensure_smem_attr(reinterpret_cast<const void*>(kernel), kSmemMax - 1024);
-      count_launch(), kernel<<<k.icount, 32 * NW, lay.total(), s>>>(a, lay);
+      count_launch(), kernel<<<k.icount, 32 * NW, bytes, s>>>(a, lay);
       BIT_CHECK_LAUNCH();
     };
     const bool eps = !F32 && k.eps;

@@ -55,7 +55,7 @@ struct NearArgs {
   int2* crec;   // up to kCloseRec (near entry, first source of the tile) per target
   int2* clist;  // (target, group) of every target with a record
   int* cn;      // entries of clist
-  int tile;              // mixed potentials: sources per tile (k_close)
+  int cap;               // mixed potentials: records of a tile at most (k_close)
   const int* pstart;     // first record of each leaf's FP32 sources
   const int* tgt;        // targets of each near entry
   const long long* pre;  // work (near_weight x sources) of the group's entries before it
