@@ -171,6 +171,7 @@ struct Lists {
   bool valid = false;
   int ngroups = 0;
   int ntargets = 0;                         // targets the groups cover
+  int far_chunk = kGroupMax;                // targets of a CTA of the potentials' far kernel
   int field_chunk = kFieldChunk;            // targets of a CTA of the fields' kernels
   int max_targets = 0;                      // of the largest group, rounded up to 32
   long long nfar = 0, nnear = 0;            // entries

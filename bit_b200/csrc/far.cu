@@ -68,8 +68,8 @@ struct FarArgs {
   const long long* mom_off;  // first moment of each node
   const void* coef;          // float or double: every node's coefficients (potential kernels)
   int stride;                // elements from one node's coefficients to the next's
-  int rows;                  // targets of the largest group (fields: chunk), rounded up to 32
-  int chunk;                 // fields: targets of a CTA, at most
+  int chunk;                 // targets of a CTA, at most
+  int rows;                  // those of the largest chunk, rounded up to 32
   int* err;                  // device error flags (a bounded wait that gave up: 8)
   const int* tgt;            // targets of each far entry (potentials)
   const long long* pre;      // targets of the group's entries before it
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kCoefThreads)
 // set, the warp has waited (bounded again) for that copy, and the group's result is not
 // valid.
 template <int NT, int KIND, class T, int NW>
-__device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar, unsigned& phase) {
+__device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint64_t* bar, unsigned& phase) {
   constexpr int CNT = far_count(NT, KIND);
   constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
@@ -255,8 +255,8 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
   T* accb = msb + NW * a.stride;
   unsigned short* tlb = reinterpret_cast<unsigned short*>(accb + NW * ROW);
 
-  const int t0 = a.g_tstart[g], tc = a.g_tcount[g];
-  const int W = (tc + 31) >> 5;
+  const int gc = a.g_tcount[g], t0 = a.g_tstart[g] + c0, tc = min(gc - c0, a.chunk);
+  const int W = (gc + 31) >> 5, w0 = c0 >> 5, wn = (tc + 31) >> 5;  // words of the group, the chunk
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
@@ -294,11 +294,15 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, uint64_t* bar
       mbar_expect_tx(&bar[w], TP * (unsigned)sizeof(T));
       tma_load_1d(M, coef + (long long)node * a.stride, TP * (unsigned)sizeof(T), &bar[w]);
     }
-    const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
-    const int cnt = a.tgt[e];
+    const unsigned wd = lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
+    int cnt = a.tgt[e];
     const double4 c = a.nodec[node];
-    const bool all = cnt == tc;  // a cluster accepted by the whole group needs no list
-    if (!all) warp_pack(wd, W, tl);
+    const bool all = cnt == gc;  // a cluster accepted by the whole group needs no list
+    if (all) cnt = tc;
+    else {
+      if (tc < gc) cnt = __reduce_add_sync(0xffffffffu, __popc(wd));
+      warp_pack(wd, wn, tl);
+    }
     const bool landed = __all_sync(0xffffffffu, mbar_wait(&bar[w], phase & 1));
     phase++;
     if (!landed) {
@@ -343,13 +347,16 @@ __device__ __forceinline__ void far_bars_init(uint64_t* bar) {
   }
 }
 
-// One launch class: CTA b takes group order[b].
+// One launch class: CTA (b, k) takes chunk k of group order[b].  A target's sum is the same
+// whatever the chunks: its entries are shared out to the warps by the whole group's work.
 template <int NT, int KIND, class T, int NW>
 __global__ void __launch_bounds__(32 * NW, far_blocks(NT)) k_far(FarArgs a) {
   __shared__ uint64_t bar[NW];
+  const int g = a.order[blockIdx.x], c0 = blockIdx.y * a.chunk;
+  if (c0 >= a.g_tcount[g]) return;  // (the whole CTA)
   far_bars_init<NW>(bar);
   unsigned phase = 0;
-  far_group<NT, KIND, T, NW>(a, a.order[blockIdx.x], bar, phase);
+  far_group<NT, KIND, T, NW>(a, g, c0, bar, phase);
 }
 
 // Persistent work queue over the groups of every class: each CTA takes the next item
@@ -374,7 +381,7 @@ __global__ void __launch_bounds__(32 * NW, 2) k_far_queue(FarArgs a, int count, 
     bool ok = true;
     switch (se->nterms * 4 + se->far_kind) {
 #define FK(N, K) \
-  case 4 * N + K: ok = far_group<N, K, T, NW>(a, g, bar, phase); break;
+  case 4 * N + K: ok = far_group<N, K, T, NW>(a, g, 0, bar, phase); break;
 #define FQ(N) FK(N, 0) FK(N, 1) FK(N, 2) FK(N, 3)
       FQ(1) FQ(2) FQ(3) FQ(4) FQ(5) FQ(6) FQ(7) FQ(8) FQ(9) FQ(10)
 #undef FQ
@@ -579,9 +586,9 @@ constexpr size_t kFarSmemMax =
     NWP * ((far_block(kNtermsMax, FAR_REG) + kGroupMax) * sizeof(double) + kGroupMax * sizeof(unsigned short));
 
 template <int NT, int KIND, class T, int NW>
-void launch_far(const FarArgs& a, int ng, cudaStream_t s) {
+void launch_far(const FarArgs& a, int ng, int chunks, cudaStream_t s) {
   set_smem(k_far<NT, KIND, T, NW>, kFarSmemMax);
-  count_launch(), k_far<NT, KIND, T, NW><<<ng, 32 * NW, far_smem<T, NW>(a), s>>>(a);
+  count_launch(), k_far<NT, KIND, T, NW><<<dim3(ng, chunks), 32 * NW, far_smem<T, NW>(a), s>>>(a);
 }
 
 template <int NT>
@@ -671,6 +678,7 @@ void eval_far(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const doub
               const double* tz, double* out) {
   FarArgs a = far_args(t, L, P, tx, ty, tz);
   a.out = out;
+  a.chunk = kGroupMax;
   a.rows = L->max_targets;
   cudaStream_t s = t->ctx->stream;
   const bool f32 = P.f32;
@@ -686,14 +694,17 @@ void eval_far(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const doub
     BIT_CHECK_LAUNCH();
     return;
   }
+  a.chunk = L->far_chunk;
+  a.rows = std::min(L->max_targets, a.chunk);
+  const int chunks = (L->max_targets + a.chunk - 1) / a.chunk;
   for (const LaunchClass& k : P.far_classes) {
     a.order = P.far_ord + k.begin;
     const int ng = k.count;
     switch (k.nterms * 4 + k.kind) {
 #define FK(N, K)                                             \
   case 4 * N + K:                                            \
-    if (f32) launch_far<N, K, float, NWP>(a, ng, s);         \
-    else launch_far<N, K, double, NWP>(a, ng, s);            \
+    if (f32) launch_far<N, K, float, NWP>(a, ng, chunks, s);         \
+    else launch_far<N, K, double, NWP>(a, ng, chunks, s);            \
     break;
 #define CASE(N) FK(N, 0) FK(N, 1) FK(N, 2) FK(N, 3)
       CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10)

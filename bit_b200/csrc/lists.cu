@@ -460,20 +460,30 @@ static int point_group(int m, int sms) {
   return size;
 }
 
-// Targets of a CTA of the fields' kernels, which keep three sums a target and warp: at most
-// kFieldChunk, and fewer where the groups would leave the chip idle.  Far + near, FP64 Coulomb
-// field, chunks of 32 / 64 / 128 / 256, us: 2k in leaves of 500 61 / 78 / 96 / 132; 8k, 300: 100 /
-// 108 / 136 / 197; 20k, 200: 168 / 153 / 180 / 186; 50k, 300: 460 / 388 / 392 / 485; 100k, 300: 854 /
-// 667 / 587 / 600; 150k, 600: 1817 / 1361 / 1138 / 1045; 2M, 1000, ms: 42.8 / 31.0 / 25.2 / 22.3 (whole
-// groups of 1000: 25.2).
-static int field_chunk(const std::vector<int>& tc, int sms) {
-  for (int size = kFieldChunk; size > 32; size /= 2) {
+// Targets of a CTA: `top`, or less where the groups' chunks of that size would be fewer than
+// `enough`.
+static int chunk_size(const std::vector<int>& tc, int top, long long enough) {
+  for (int size = top; size > 32; size /= 2) {
     long long chunks = 0;
     for (int k : tc) chunks += (k + size - 1) / size;
-    if (2 * chunks >= 5LL * sms) return size;
+    if (chunks >= enough) return size;
   }
   return 32;
 }
+// The potentials' far kernel (two CTAs of eight warps a multiprocessor): whole groups from 1.25
+// chunks a multiprocessor.  A chunk reads its group's coefficients again.  Screened / with delta,
+// FP64, chunks of 32 / 64 / 128 / 256 / 512 / whole groups, us: 20k in leaves of 500 (64 groups)
+// 67, 76 / 55, 61 / 47, 60 / 54, 65 / 63, 77 / 63, 78; 50k, 1000 (64) 109, 122 / 74, 86 / 63, 77 / 63, 83 /
+// 83, 102 / 112, 143; 10k, 200 (64) 44, 49 / 37, 43 / 41, 49 / 41, 49 / 43, 49 / 43, 49; 50k, 300 (260)
+// 156, 178 / 119, 135 / 101, 120 / 95, 118 / 100, 127 / 102, 127; 200k, 500 (750) 698, 807 / 463, 552 / 337,
+// 427 / 277, 362 / 246, 334 / 248, 339.
+static int far_chunk(const std::vector<int>& tc, int sms) { return chunk_size(tc, kGroupMax, 5LL * sms / 4); }
+// The fields' kernels, which keep three sums a target and warp: at most kFieldChunk, and from
+// 2.5 chunks a multiprocessor.  Far + near, FP64 Coulomb field, chunks of 32 / 64 / 128 / 256, us:
+// 2k in leaves of 500 61 / 78 / 96 / 132; 8k, 300: 100 / 108 / 136 / 197; 20k, 200: 168 / 153 / 180 /
+// 186; 50k, 300: 460 / 388 / 392 / 485; 100k, 300: 854 / 667 / 587 / 600; 150k, 600: 1817 / 1361 / 1138 /
+// 1045; 2M, 1000, ms: 42.8 / 31.0 / 25.2 / 22.3 (whole groups: 25.2).
+static int field_chunk(const std::vector<int>& tc, int sms) { return chunk_size(tc, kFieldChunk, 5LL * sms / 2); }
 
 // The potentials' near-field items, heaviest first: a group's near work in one item, or in up
 // to kNearParts equal parts of at least kNearChunk pairs each, whose sums meet in scratch
@@ -594,6 +604,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   for (int g = 0; g < ng; g++) maxw = std::max(maxw, (tc[g] + 31) / 32);
   L->max_targets = 32 * maxw;
   L->field_chunk = field_chunk(tc, c->num_sms);
+  L->far_chunk = far_chunk(tc, c->num_sms);
   int per_sm = 0;
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists, QT, 0));
   const long long nodes = std::max(t->numtree, 1);

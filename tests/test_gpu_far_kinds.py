@@ -32,3 +32,28 @@ def test_far_kinds_match_oracle(ctx, orc, nterms, n, maxmemb):
         mixed = t.evaluate(B.params(kb, B.CONSISTENT, B.MIXED, acc=0.6, **kw))
         assert np.linalg.norm(mixed - want) < 1e-6 * np.linalg.norm(want), (kern, kw)
     t.treeempty()
+
+
+@pytest.mark.parametrize("n,maxmemb", [(2500, 1000), (12000, 900), (30000, 1000), (60000, 1000), (200000, 1000)])
+def test_every_chunk_of_a_group(ctx, orc, n, maxmemb):
+    """Few large groups are cut into chunks of 32 targets and up, many are taken whole; a target's
+    result does not depend on it: alone and beside a larger system it is the same."""
+    import bit_b200 as B
+    from bit_b200 import workloads
+    x, y, z, q = workloads.clustered_blobs(n, seed=n)
+    t = ctx.treemake(x, y, z, maxmemb)
+    t.treemoments(q, 4)
+    T = orc.Tree(x, y, z, maxmemb)
+    T.compute_moments(q, 4)
+    tg = workloads.sample_targets(n, 400, seed=2)
+    want = T.evaluate(orc.params(orc.SCREENED, orc.MODE_CONSISTENT, acc=0.8, kappa=1.0), targets=tg)
+    p = B.params(B.SCREENED, B.CONSISTENT, B.FP64, acc=0.8, kappa=1.0)
+    got = t.evaluate(p)
+    assert np.linalg.norm(got[tg] - want) < 1e-12 * np.linalg.norm(want)
+    t.treeempty()
+    X, Y, Z, Q = workloads.uniform_cube(250000, seed=1)
+    f = ctx.forest(np.concatenate([x, X]), np.concatenate([y, Y]), np.concatenate([z, Z]), [n, 250000], maxmemb)
+    f.set_charges(np.concatenate([q, Q]))
+    f.moments([4, 4])
+    assert np.array_equal(f.evaluate([p, p])[:n], got)
+    f.treeempty()
