@@ -282,7 +282,10 @@ bit_status bit_ctx_destroy(bit_ctx* h) {
     if (c.stage_ev[i]) cudaEventSynchronize(c.stage_ev[i]);
     if (c.stage[i]) cudaFreeHost(c.stage[i]);
     if (c.stage_ev[i]) cudaEventDestroy(c.stage_ev[i]);
+    if (c.side_ev[i]) cudaEventDestroy(c.side_ev[i]);
+    if (c.side[i]) cudaStreamDestroy(c.side[i]);
   }
+  if (c.fork_ev) cudaEventDestroy(c.fork_ev);
   if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);
   delete h;
   return BIT_OK;

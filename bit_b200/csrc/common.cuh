@@ -240,6 +240,9 @@ struct Ctx {
   DBuf<int2> close_rec, close_list;
   void* stage[2] = {nullptr, nullptr};            // pinned staging chunks for host copies
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+  // the tree build's larger nodes run beside the smaller ones (made at their first use)
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t side_ev[2] = {nullptr, nullptr}, fork_ev = nullptr;
   int* dev_err() {
     if (!err_flag) {
       err_flag = static_cast<int*>(dev_alloc(this, 64));

@@ -79,6 +79,24 @@ __device__ void box_fields(double* f, double x0, double x1, double y0, double y1
   f[12] = dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
 }
 
+// box_fields by a warp, lanes 0..2 an axis and a quotient each; bb: smallest and (negated) largest
+// coordinate of each axis.
+__device__ void warp_box_fields(double* f, const double* bb) {
+  const int lane = threadIdx.x & 31, a = lane < 3 ? lane : 0;
+  const double lo = bb[2 * a], hi = -bb[2 * a + 1];
+  const double mid = dmul(0.5, dadd(hi, lo)), ext = dsub(hi, lo), half = dsub(hi, mid), sq = dmul(half, half);
+  const double ey = __shfl_sync(0xffffffffu, ext, 1), ez = __shfl_sync(0xffffffffu, ext, 2);
+  const double ex = __shfl_sync(0xffffffffu, ext, 0);
+  const double s1 = __shfl_sync(0xffffffffu, sq, 1), s2 = __shfl_sync(0xffffffffu, sq, 2);
+  if (lane < 3) {
+    f[2 * lane] = lo;
+    f[2 * lane + 1] = hi;
+    f[6 + lane] = mid;
+    f[9 + lane] = fabs(__ddiv_rn(lane == 2 ? ey : ex, lane == 0 ? ey : ez));
+    if (lane == 0) f[12] = dadd(dadd(sq, s1), s2);
+  }
+}
+
 // What a split leaves for k_make_children: the child slots and the order of children[].
 struct NodeOut {
   int nchild;
@@ -92,7 +110,7 @@ struct Level {
   int a, b;            // its nodes
   int nact;            // nodes to split, numbered in no particular order
   int nsmall[kClasses], nbig;  // of those, by class
-  int arrive;          // CTAs of the level's last k_node_split that are done
+  int arrive;          // CTAs of the level's k_node_split launches that are done
 };
 struct Ctl {
   Level lv[kLevels];
@@ -325,17 +343,41 @@ constexpr int SW = ST / 32;  // warps of a CTA
 struct NodeShared {
   Program g;
   double pf[13], f[8][13];      // the node's box, the slots'
-  double red[SW][14];           // per warp: min / max of x, y, z and the count, of both halves
+  double red[SW][14];           // per warp: combine's values of both halves
   double part[2][14], all[14];  // the CTA's (by parity of the bisection), the node's
   int wcnt[SW][8], tot[8];      // members of each slot, per warp and in the CTA
   int made;
 };
 
-// Value v = 7 h + q of a bisection: q = 2 d the smallest, 2 d + 1 the largest coordinate of
-// axis d in half h, 6 the count.
+// Value v = 7 h + q of a bisection: q = 2 d the smallest coordinate of axis d in half h, 2 d + 1
+// the largest's negative, 6 the count.
 __device__ __forceinline__ double combine(int v, double a, double b) {
-  const int q = v % 7;
-  return q == 6 ? a + b : ((q & 1) ? (b > a ? b : a) : (b < a ? b : a));
+  return v % 7 == 6 ? a + b : (b < a ? b : a);
+}
+template <class T>
+__device__ __forceinline__ void least(T& a, T b) { a = b < a ? b : a; }
+// The warp's least of each of v[0..11], by halves: lane l is left with that of value
+// 6 (l >> 4) + 3 (l >> 3 & 1) + (l >> 1 & 3) in v[0] (l >> 1 & 3 < 3).  13 exchanges, where twelve
+// butterflies make 60, and the exchanges bounded a bisection.
+template <class T>
+__device__ __forceinline__ void warp_least12(T (&v)[12]) {
+  const int lane = threadIdx.x & 31;
+  auto halve = [&](int o, int n) {  // v[0..2n): the lanes of bit o keep the second n
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < 6; q++)
+      if (q < n) {
+        const T a = v[q], b = v[q + n], r = __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+        v[q] = up ? b : a;
+        least(v[q], r);
+      }
+  };
+  halve(16, 6);
+  halve(8, 3);
+  v[3] = v[2];
+  halve(4, 2);
+  halve(2, 1);
+  least(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
 }
 
 // Split every node of class C at level lev: a cluster of CTAs holds a node's members in shared
@@ -343,10 +385,10 @@ __device__ __forceinline__ double combine(int v, double a, double b) {
 // register.  A bisection is a pass over the thread's members, a reduction over the warp, the
 // CTA and (through distributed shared memory) the cluster, and one thread's step of the
 // program, which every CTA takes for itself.  The members then go to the children's ranges in
-// order, in place: all of them were read before any is written.  The level's last CTA (of the
-// launch with `last`) scans the child counts.
+// order, in place: all of them were read before any is written.  The level's last CTA, of the
+// `total` of its launches, scans the child counts.
 template <int C>
-__global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) {
+__global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int total) {
   constexpr int CS = kClassCtas[C], ROWS = kClassRows[C];
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ NodeShared N;
@@ -393,9 +435,9 @@ __global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) 
       const int dir = N.g.dir, src = N.g.src;
       const double mid = (src < 0 ? N.pf : N.f[src])[6 + dir];
       const unsigned want = src < 0 ? 15u : (unsigned)src;
-      double v[14];
+      double v[12];
 #pragma unroll
-      for (int q = 0; q < 14; q++) v[q] = q % 7 == 6 ? 0.0 : ((q % 7) & 1 ? -inf : inf);
+      for (int q = 0; q < 12; q++) v[q] = inf;
       int n0 = 0, n1 = 0;
       unsigned up = 0;
       const double* cs = dir == 0 ? xs : (dir == 1 ? ys : zs);
@@ -405,34 +447,19 @@ __global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) 
         const double x = xs[o] + 0.0, y = ys[o] + 0.0, z = zs[o] + 0.0;
         if (cs[o] <= mid) {
           n0++;
-          v[0] = x < v[0] ? x : v[0]; v[1] = x > v[1] ? x : v[1];
-          v[2] = y < v[2] ? y : v[2]; v[3] = y > v[3] ? y : v[3];
-          v[4] = z < v[4] ? z : v[4]; v[5] = z > v[5] ? z : v[5];
+          least(v[0], x); least(v[1], -x); least(v[2], y); least(v[3], -y); least(v[4], z); least(v[5], -z);
         } else {
           up |= 1u << i;
           n1++;
-          v[7] = x < v[7] ? x : v[7]; v[8] = x > v[8] ? x : v[8];
-          v[9] = y < v[9] ? y : v[9]; v[10] = y > v[10] ? y : v[10];
-          v[11] = z < v[11] ? z : v[11]; v[12] = z > v[12] ? z : v[12];
+          least(v[6], x); least(v[7], -x); least(v[8], y); least(v[9], -y); least(v[10], z); least(v[11], -z);
         }
       }
       n0 = __reduce_add_sync(0xffffffffu, n0);
       n1 = __reduce_add_sync(0xffffffffu, n1);
-      if (n0)  // (the whole warp)
-#pragma unroll
-        for (int q = 0; q < 6; q++)
-#pragma unroll
-          for (int o = 16; o; o >>= 1) v[q] = combine(q, v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
-      if (n1)
-#pragma unroll
-        for (int q = 7; q < 13; q++)
-#pragma unroll
-          for (int o = 16; o; o >>= 1) v[q] = combine(q, v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
-      v[6] = n0;
-      v[13] = n1;
-      if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < 14; q++) N.red[w][q] = v[q];
+      warp_least12(v);
+      if (!(lane & 1) && (lane & 6) != 6) N.red[w][7 * (lane >> 4) + 3 * ((lane >> 3) & 1) + (lane & 6) / 2] = v[0];
+      if (lane == 0) N.red[w][6] = n0;
+      if (lane == 16) N.red[w][13] = n1;
       __syncthreads();
       if (w < 14) {  // warp q: value q over the CTA's warps
         double x = N.red[lane & (SW - 1)][w];
@@ -454,10 +481,10 @@ __global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) 
       const bool any0 = N.all[6] > 0.0, any1 = N.all[13] > 0.0;
       const int d0 = N.g.c1, d1 = any0 ? N.g.c2 : N.g.c1;
       __syncthreads();  // every thread has read the bisection in hand
-      if (lane == 0 && w < 2 && (w ? any1 : any0)) {  // a half's fields, one warp each
-        const double* bb = &N.all[7 * w];
-        box_fields(N.f[w ? d1 : d0], bb[0], bb[1], bb[2], bb[3], bb[4], bb[5]);
-        N.g.n[w ? d1 : d0] = (int)bb[6];
+      if (w < 2 && (w ? any1 : any0)) {  // a half's fields, one warp each, a lane an axis
+        const int slot = w ? d1 : d0;
+        warp_box_fields(N.f[slot], &N.all[7 * w]);
+        if (lane == 0) N.g.n[slot] = (int)N.all[7 * w + 6];
       }
       for (int i = 0; i < rows; i++)
         if (((unsigned)(lab >> (4 * i)) & 15u) == want)
@@ -530,11 +557,10 @@ __global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) 
     if (CS > 1) cluster.sync();  // the cluster's reads of each other's counts are done
     else __syncthreads();
   }
-  if (!last) return;
   // the level's last CTA: where each node's children begin
   __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(&lv->arrive, 1) == (int)gridDim.x - 1;
+  if (tid == 0) s_last = atomicAdd(&lv->arrive, 1) == total - 1;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -573,14 +599,18 @@ __global__ void __launch_bounds__(ST) k_node_split(Arrays A, int lev, int last) 
 template <int C>
 constexpr size_t split_smem() { return (size_t)kClassRows[C] * ST * (3 * sizeof(double) + sizeof(int)); }
 
-// `nodes`: at most that many nodes of the class.
+// CTAs for at most `nodes` nodes of class C.
 template <int C>
-void launch_split(const Ctx* c, const Arrays& A, int lev, int last, long long nodes, cudaStream_t s) {
-  ensure_smem_attr(reinterpret_cast<const void*>(k_node_split<C>), (int)split_smem<C>());
+int split_ctas(const Ctx* c, long long nodes) {
   const int per_sm = C == 2 ? 1 : 2;
   const long long fit = std::max(1, c->num_sms * per_sm / kClassCtas[C]);
+  return (int)(std::max(1LL, std::min(nodes, fit)) * kClassCtas[C]);
+}
+template <int C>
+void launch_split(const Arrays& A, int lev, int ctas, int total, cudaStream_t s) {
+  ensure_smem_attr(reinterpret_cast<const void*>(k_node_split<C>), (int)split_smem<C>());
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(std::max(1LL, std::min(nodes, fit)) * kClassCtas[C]));
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(ST);
   cfg.dynamicSmemBytes = split_smem<C>();
   cfg.stream = s;
@@ -591,7 +621,41 @@ void launch_split(const Ctx* c, const Arrays& A, int lev, int last, long long no
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   count_launch();
-  BIT_CUDA(cudaLaunchKernelEx(&cfg, k_node_split<C>, A, lev, last));
+  BIT_CUDA(cudaLaunchKernelEx(&cfg, k_node_split<C>, A, lev, total));
+}
+
+// One level's classes, the larger ones on the context's side streams: their nodes are disjoint,
+// none fills the chip, and one after the other they took 144 us a level of 100k particles
+// where together they take the longest's 53.  The side streams' work ends with this object.
+struct SplitFork {
+  Ctx* c;
+  cudaStream_t s;
+  int n;  // side streams in use
+  SplitFork(Ctx* c_, cudaStream_t s_, int n_) : c(c_), s(s_), n(n_) {
+    if (n == 0) return;
+    for (int k = 0; k < 2; k++)
+      if (!c->side[k]) {
+        BIT_CUDA(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
+        BIT_CUDA(cudaEventCreateWithFlags(&c->side_ev[k], cudaEventDisableTiming));
+      }
+    if (!c->fork_ev) BIT_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
+    BIT_CUDA(cudaEventRecord(c->fork_ev, s));
+    for (int k = 0; k < n; k++) BIT_CUDA(cudaStreamWaitEvent(c->side[k], c->fork_ev, 0));
+  }
+  ~SplitFork() {
+    for (int k = 0; k < n; k++) {
+      cudaEventRecord(c->side_ev[k], c->side[k]);
+      cudaStreamWaitEvent(s, c->side_ev[k], 0);
+    }
+  }
+};
+void split_level(Ctx* c, const Arrays& A, int lev, int top, long long n, long long actl, cudaStream_t s) {
+  const int g0 = split_ctas<0>(c, actl), g1 = top >= 1 ? split_ctas<1>(c, n / class_members(0) + 1) : 0,
+            g2 = top >= 2 ? split_ctas<2>(c, n / class_members(1) + 1) : 0;
+  const SplitFork f(c, s, top);
+  if (top >= 2) launch_split<2>(A, lev, g2, g0 + g1 + g2, c->side[1]);
+  if (top >= 1) launch_split<1>(A, lev, g1, g0 + g1 + g2, c->side[0]);
+  launch_split<0>(A, lev, g0, g0 + g1 + g2, s);
 }
 
 // The children of level lev's nodes, one warp per node: their records, and the lists of the
@@ -1180,10 +1244,7 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
     // empty launches).
     const int batch = nbig > 0 ? 1 : 4;
     for (int k = 0; k < batch; k++) {
-      // (a class's nodes are disjoint and larger than the class below)
-      if (top >= 2) launch_split<2>(c, A, cur + k, 0, n / class_members(1) + 1, s);
-      if (top >= 1) launch_split<1>(c, A, cur + k, 0, n / class_members(0) + 1, s);
-      launch_split<0>(c, A, cur + k, 1, actl, s);
+      split_level(c, A, cur + k, top, n, actl, s);
       make_children(cur + k);
     }
     BIT_CHECK_LAUNCH();
