@@ -282,6 +282,8 @@ bit_status bit_ctx_destroy(bit_ctx* h) {
     if (c.stage_ev[i]) cudaEventSynchronize(c.stage_ev[i]);
     if (c.stage[i]) cudaFreeHost(c.stage[i]);
     if (c.stage_ev[i]) cudaEventDestroy(c.stage_ev[i]);
+  }
+  for (int i = 0; i < 3; i++) {
     if (c.side_ev[i]) cudaEventDestroy(c.side_ev[i]);
     if (c.side[i]) cudaStreamDestroy(c.side[i]);
   }

@@ -241,8 +241,9 @@ struct Ctx {
   void* stage[2] = {nullptr, nullptr};            // pinned staging chunks for host copies
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   // the tree build's larger nodes run beside the smaller ones (made at their first use)
-  cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t side_ev[2] = {nullptr, nullptr}, fork_ev = nullptr;
+  cudaStream_t side[3] = {nullptr, nullptr, nullptr};
+  cudaEvent_t side_ev[3] = {nullptr, nullptr, nullptr}, fork_ev = nullptr;
+  int clusters16 = -1;  // whether the device takes clusters of 16 of its largest CTAs (-1: not asked)
   int* dev_err() {
     if (!err_flag) {
       err_flag = static_cast<int*>(dev_alloc(this, 64));

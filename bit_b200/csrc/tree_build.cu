@@ -7,8 +7,8 @@
 // src/tree3d.cpp:1163-1304), each needing the member count and bounding box of both
 // halves of the slot it splits (min/max are order independent, so the result is exact).
 //
-// A node of at most kSmallNode members is one cluster's work (k_node_split: one, four or eight
-// CTAs by its size): the members stay in shared memory through the whole program, and go to
+// A node of up to 57,344 (114,688) members is one cluster's work (k_node_split: one to sixteen CTAs
+// by its size): the members stay in shared memory through the whole program, and go to
 // the children's ranges in one stable scatter, members in ascending original index (the
 // reference's member order).  The level's last CTA scans the child counts, k_make_children
 // appends the children and sorts out which of them are to be split, all from device-side
@@ -22,10 +22,13 @@
 // Field arithmetic (midpoints, aspect ratios, sqradius) is the reference's, with no FMA
 // contraction.
 //
-// Bound by launches and latency.  With the passes for every node (18 launches and a round trip
-// a level), before / now: 10k uniform in leaves of 200 700 / 220 us, 100k clustered in leaves
-// of 500 1,757 / 780, 2M in leaves of 1000 4,200 / 2,900; with one CTA up to 16,384 members
-// that read them from L2 at every bisection: 320, 1,190, 4,030.
+// Bound by latency: launches, and in a node's CTA its scans and reductions, one bisection after
+// the other.  With the passes for every node (18 launches and a round trip a level), before /
+// now: 2k uniform in leaves of 50 744 / 172 us, 10k, 200: 693 / 183, 50k clustered, 300: 1,663 / 412,
+// 100k, 500: 1,845 / 500, 200k, 500: 2,105 / 700, 2M, 1000: 4,149 / 2,490, 48 systems 1,279 / 535.  With
+// one CTA up to 16,384 members that read them from L2 at every bisection: 10k 320, 100k 1,190.
+// Doing the bisection in hand and a foreseen one in one pass (four passes for seven) gave
+// nothing: a pass's own scan and reduction take the time, not its barriers.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -43,16 +46,18 @@ namespace cg = cooperative_groups;
 constexpr int CH = 2048;  // members per chunk (one block)
 constexpr int TB = 256;   // threads per block
 // Nodes that a cluster of CTAs splits with its members in shared memory, by size: one CTA of
-// up to 3,584 members (two such CTAs an SM), four of those, eight of 7,168.  Larger nodes take
-// all SMs.
-constexpr int kClasses = 3;
-constexpr int kClassCtas[kClasses] = {1, 4, 8};
-constexpr int kClassRows[kClasses] = {7, 7, 14};  // members of a thread
-constexpr int ST = 512;                           // threads of a CTA
+// up to 3,584 members (two such CTAs an SM), four of those, eight or sixteen of 7,168.  Larger
+// nodes take all SMs; so do those of the last class where larger ones are there to take along:
+// it is used for trees and forests whose roots all fit it (a build of 100k clustered particles in
+// leaves of 500 580 -> 500 us, of 48 systems of up to 100k 705 -> 535; with a larger root the
+// passes are made in any case).
+constexpr int kClasses = 4;
+constexpr int kClassCtas[kClasses] = {1, 4, 8, 16};
+constexpr int kClassRows[kClasses] = {7, 7, 14, 14};  // members of a thread
+constexpr int ST = 512;                               // threads of a CTA
 __host__ __device__ constexpr int class_members(int c) {
-  return (c == 0 ? 1 : c == 1 ? 4 : 8) * (c == 2 ? 14 : 7) * ST;
+  return (c == 0 ? 1 : c == 1 ? 4 : c == 2 ? 8 : 16) * (c >= 2 ? 14 : 7) * ST;
 }
-constexpr int kSmallNode = class_members(kClasses - 1);
 static_assert(CH % TB == 0, "a chunk is a whole number of block strides");
 
 __device__ __forceinline__ unsigned long long okey(double v) {
@@ -288,26 +293,26 @@ struct Lists2 {
 };
 
 // Node `node` of level lev (its record L) joins the list it belongs to; act: its number among
-// the nodes to split, or -1.
+// the nodes to split, or -1; small: the largest node that a cluster takes.
 __device__ __forceinline__ void enlist(int node, int cnt, int maxmemb, Level* L, int lev,
-                                       const Lists2& ls, int* act, int* nch) {
+                                       const Lists2& ls, int* act, int* nch, int small) {
   nch[node] = 0;
   if (cnt <= maxmemb) {
     act[node] = -1;
     return;
   }
   act[node] = atomicAdd(&L->nact, 1);
-  if (cnt > kSmallNode) {
+  if (cnt > small) {
     ls.big[lev & 1][atomicAdd(&L->nbig, 1)] = node;
     return;
   }
-  const int c = cnt <= class_members(0) ? 0 : cnt <= class_members(1) ? 1 : 2;
+  const int c = cnt <= class_members(0) ? 0 : cnt <= class_members(1) ? 1 : cnt <= class_members(2) ? 2 : 3;
   ls.small[c][lev & 1][atomicAdd(&L->nsmall[c], 1)] = node;
 }
 
 __global__ void k_root_init(int nsys, const int* sys_start, const int* sys_n, const int* sys_maxmemb,
                             const SplitAcc* acc, int* nummemb, int* start, int* children,
-                            double* fields, int* node_sys, Ctl* ctl, Lists2 ls, int* act, int* nch) {
+                            double* fields, int* node_sys, Ctl* ctl, Lists2 ls, int* act, int* nch, int small) {
   const int sy = blockIdx.x * blockDim.x + threadIdx.x;
   if (sy >= nsys) return;
   double f[13];
@@ -319,7 +324,7 @@ __global__ void k_root_init(int nsys, const int* sys_start, const int* sys_n, co
   node_sys[sy] = sy;
   for (int c = 0; c < 8; c++) children[8LL * sy + c] = -1;
   if (sy == 0) ctl->lv[0].b = nsys;
-  enlist(sy, sys_n[sy], sys_maxmemb[sy], &ctl->lv[0], 0, ls, act, nch);
+  enlist(sy, sys_n[sy], sys_maxmemb[sy], &ctl->lv[0], 0, ls, act, nch, small);
 }
 
 struct Arrays {
@@ -334,10 +339,10 @@ struct Arrays {
   Ctl* ctl;
   Lists2 ls;
   double lim;
-  int cap;
+  int cap, small;
 };
 
-// ---- nodes of up to kSmallNode members ------------------------------------------------------
+// ---- nodes of one cluster -------------------------------------------------------------------
 constexpr int SW = ST / 32;  // warps of a CTA
 
 struct NodeShared {
@@ -602,7 +607,7 @@ constexpr size_t split_smem() { return (size_t)kClassRows[C] * ST * (3 * sizeof(
 // CTAs for at most `nodes` nodes of class C.
 template <int C>
 int split_ctas(const Ctx* c, long long nodes) {
-  const int per_sm = C == 2 ? 1 : 2;
+  const int per_sm = C >= 2 ? 1 : 2;
   const long long fit = std::max(1, c->num_sms * per_sm / kClassCtas[C]);
   return (int)(std::max(1LL, std::min(nodes, fit)) * kClassCtas[C]);
 }
@@ -624,6 +629,30 @@ void launch_split(const Arrays& A, int lev, int ctas, int total, cudaStream_t s)
   BIT_CUDA(cudaLaunchKernelEx(&cfg, k_node_split<C>, A, lev, total));
 }
 
+// The sixteen-CTA class needs room for such a cluster (a size past the portable eight).
+bool clusters_of_16(Ctx* c) {
+  if (c->clusters16 < 0) {
+    auto* f = reinterpret_cast<const void*>(k_node_split<3>);
+    ensure_smem_attr(f, (int)split_smem<3>());
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(ST);
+    cfg.dynamicSmemBytes = split_smem<3>();
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 16;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess;
+    if (!ok) cudaGetLastError();  // (the eight-CTA class and the passes do without it)
+    c->clusters16 = ok && n > 0;
+  }
+  return c->clusters16 > 0;
+}
+
 // One level's classes, the larger ones on the context's side streams: their nodes are disjoint,
 // none fills the chip, and one after the other they took 144 us a level of 100k particles
 // where together they take the longest's 53.  The side streams' work ends with this object.
@@ -633,7 +662,7 @@ struct SplitFork {
   int n;  // side streams in use
   SplitFork(Ctx* c_, cudaStream_t s_, int n_) : c(c_), s(s_), n(n_) {
     if (n == 0) return;
-    for (int k = 0; k < 2; k++)
+    for (int k = 0; k < n; k++)
       if (!c->side[k]) {
         BIT_CUDA(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
         BIT_CUDA(cudaEventCreateWithFlags(&c->side_ev[k], cudaEventDisableTiming));
@@ -651,11 +680,13 @@ struct SplitFork {
 };
 void split_level(Ctx* c, const Arrays& A, int lev, int top, long long n, long long actl, cudaStream_t s) {
   const int g0 = split_ctas<0>(c, actl), g1 = top >= 1 ? split_ctas<1>(c, n / class_members(0) + 1) : 0,
-            g2 = top >= 2 ? split_ctas<2>(c, n / class_members(1) + 1) : 0;
+            g2 = top >= 2 ? split_ctas<2>(c, n / class_members(1) + 1) : 0,
+            g3 = top >= 3 ? split_ctas<3>(c, n / class_members(2) + 1) : 0, all = g0 + g1 + g2 + g3;
   const SplitFork f(c, s, top);
-  if (top >= 2) launch_split<2>(A, lev, g2, g0 + g1 + g2, c->side[1]);
-  if (top >= 1) launch_split<1>(A, lev, g1, g0 + g1 + g2, c->side[0]);
-  launch_split<0>(A, lev, g0, g0 + g1 + g2, s);
+  if (top >= 3) launch_split<3>(A, lev, g3, all, c->side[2]);
+  if (top >= 2) launch_split<2>(A, lev, g2, all, c->side[1]);
+  if (top >= 1) launch_split<1>(A, lev, g1, all, c->side[0]);
+  launch_split<0>(A, lev, g0, all, s);
 }
 
 // The children of level lev's nodes, one warp per node: their records, and the lists of the
@@ -692,7 +723,7 @@ __global__ void __launch_bounds__(256) k_make_children(Arrays A, int lev) {
       A.nummemb[node] = n;
       A.start[node] = A.start[p] + off;
       A.node_sys[node] = sys;
-      enlist(node, n, A.sys_maxmemb[sys], nx, lev + 1, A.ls, A.act, A.nch);
+      enlist(node, n, A.sys_maxmemb[sys], nx, lev + 1, A.ls, A.act, A.nch, A.small);
     }
   }
   if (first) ctl->cur = lev + 1;
@@ -1124,13 +1155,15 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   // nodes: an estimate, grown when it is short; nodes to split at one level: more than maxmemb
   // members each
   long long capl = 64, actl = 1;
-  bool big = false;
+  int most = 0;  // members of the largest node to split
   for (int k = 0; k < nsys; k++) {
     const int m = t->h_sys_maxmemb[k];
     capl += 16LL * (t->h_sys_n[k] / std::max(m, 1) + 1) + 8;
     actl += t->h_sys_n[k] / (m + 1LL);
-    big |= t->h_sys_n[k] > std::max(m, kSmallNode);
+    if (t->h_sys_n[k] > m) most = std::max(most, t->h_sys_n[k]);
   }
+  const int small_node = most <= class_members(3) && clusters_of_16(c) ? class_members(3) : class_members(2);
+  const bool big = most > small_node;
   int cap = (int)std::min<long long>(capl, 1LL << 30);
   DBuf<int> act, nch, cscan, small, big0, big1;
   DBuf<NodeOut> out;
@@ -1139,7 +1172,7 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   t->fields.ensure(c, 13LL * cap); t->node_sys.ensure(c, cap);
   act.ensure(c, cap); nch.ensure(c, cap); cscan.ensure(c, cap);
   small.ensure(c, 2 * kClasses * actl);
-  big0.ensure(c, n / kSmallNode + 1); big1.ensure(c, n / kSmallNode + 1);
+  big0.ensure(c, n / class_members(2) + 1); big1.ensure(c, n / class_members(2) + 1);
   out.ensure(c, actl);
   ctl.ensure(c, 1);
   BIT_CUDA(cudaMemsetAsync(ctl.p, 0, sizeof(Ctl), s));
@@ -1157,6 +1190,7 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   A.ls.big[0] = big0.p;
   A.ls.big[1] = big1.p;
   A.lim = 1.0 / std::sqrt(2.0);  // src/tree3d.cpp:1371
+  A.small = small_node;
   auto point_at_nodes = [&] {
     A.nummemb = t->nummemb.p; A.start = t->start.p; A.children = t->children.p;
     A.node_sys = t->node_sys.p; A.fields = t->fields.p;
@@ -1175,16 +1209,13 @@ void tree_build(Tree* t, const double* x, const double* y, const double* z) {
   }
   count_launch(), k_root_init<<<grid_for(nsys, 128), 128, 0, s>>>(
       nsys, t->sys_start.p, t->sys_n.p, t->sys_maxmemb.p, acc.p, t->nummemb.p, t->start.p, t->children.p,
-      t->fields.p, t->node_sys.p, ctl.p, A.ls, act.p, nch.p);
+      t->fields.p, t->node_sys.p, ctl.p, A.ls, act.p, nch.p, small_node);
   BIT_CHECK_LAUNCH();
 
   const unsigned gsplit = (unsigned)std::max(1LL, std::min(actl, 2LL * c->num_sms));
   // the largest class a system's root may be in: the first levels launch no more
   int top = 0;
-  for (int k = 0; k < nsys; k++)
-    if (t->h_sys_n[k] > t->h_sys_maxmemb[k])
-      for (int q = top + 1; q < kClasses; q++)
-        if (t->h_sys_n[k] > class_members(q - 1)) top = q;
+  while (top + 1 < kClasses && most > class_members(top) && class_members(top + 1) <= small_node) top++;
   auto sync_ctl = [&] {
     BIT_CUDA(cudaMemcpyAsync(h, ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     BIT_CUDA(cudaStreamSynchronize(s));

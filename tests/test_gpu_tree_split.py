@@ -1,5 +1,5 @@
 """The tree build where nodes change from one CTA's work to a cluster's (3,584 and 14,336
-members) and to all SMs' (57,344), on shapes that exercise every branch of the split program:
+members; 57,344 and 114,688 to all SMs'), on shapes that exercise every branch of the split program:
 bit for bit the oracle's tree."""
 import numpy as np
 import pytest
@@ -34,7 +34,8 @@ def shape(kind, n, seed):
 
 
 @pytest.mark.parametrize("n,maxmemb", [(1, 1), (2, 1), (700, 1), (3584, 60), (3585, 60), (14336, 500),
-                                       (14337, 64), (57344, 800), (57345, 800), (90001, 30000)])
+                                       (14337, 64), (57344, 800), (57345, 800), (90001, 30000), (114688, 900),
+                                       (114689, 900), (150001, 60000)])
 @pytest.mark.parametrize("kind", ["cube", "blobs", "slab", "rod", "plane", "line", "graded", "lattice"])
 def test_tree_matches_oracle_around_the_limits(ctx, orc, kind, n, maxmemb):
     import bit_b200
