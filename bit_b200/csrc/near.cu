@@ -83,18 +83,21 @@ struct Range32 {
   float del, kl2, thr;    // kl2 = -kappa log2(e); pairs below thr are close (near.cuh)
 };
 
-// A target against one record; careful: the target's own source (index o), the empty half and
+// A target against one record.  M_WATCH: also the least r^2, from which the caller sees that a
+// close pair was among them; M_CAREFUL: the target's own source (index o), the empty half and
 // close pairs add nothing, and `close` tells that there was a close one.  Only the differences
 // and r^2 are packed: what follows the MUFU stays scalar, since gathering its results into
 // pairs costs a move each.
-template <int KER, bool CAREFUL>
+enum { M_PLAIN = 0, M_WATCH = 1, M_CAREFUL = 2 };
+template <int KER, int MODE>
 __device__ __forceinline__ void pair32(const Range32& r, int k, f32x2 nx, f32x2 ny, f32x2 nz, int o,
-                                       float2& acc, bool& close) {
+                                       float2& acc, float& least, bool& close) {
   const ulonglong2 u = r.rec[2 * k], v = r.rec[2 * k + 1];
   const f32x2 dx = add2(u.x, nx), dy = add2(u.y, ny), dz = add2(v.x, nz);
   float2 f = unpack2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, pack2(r.del, r.del)))));
   float2 q = unpack2(v.y);
-  if (CAREFUL) {
+  if (MODE == M_WATCH) least = fminf(least, fminf(f.x, f.y));
+  if (MODE == M_CAREFUL) {
     const bool in0 = 2 * k != o, in1 = 2 * k + 1 != o && 2 * k + 1 < r.n;
     const bool c0 = f.x < r.thr, c1 = f.y < r.thr;
     close |= (in0 && c0) || (in1 && c1);
@@ -118,45 +121,57 @@ struct Target32 {
       : nx(pack2(-x, -x)), ny(pack2(-y, -y)), nz(pack2(-z, -z)), own(o) {}
 };
 
-template <int KER, bool CAREFUL>
+template <int KER, int MODE>
 __device__ __forceinline__ void two32(const Range32& r, const Target32& a, const Target32& b, float& p0,
                                       float& p1, bool& c0, bool& c1) {
   float2 s0{0.f, 0.f}, s1{0.f, 0.f}, t0{0.f, 0.f}, t1{0.f, 0.f};
+  float m0 = HUGE_VALF, m1 = HUGE_VALF;
   const int nr = (r.n + 1) >> 1;
   int k = 0;
 #pragma unroll 1
   for (; k + 1 < nr; k += 2) {
-    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c0);
-    pair32<KER, CAREFUL>(r, k, b.nx, b.ny, b.nz, b.own, t0, c1);
-    pair32<KER, CAREFUL>(r, k + 1, a.nx, a.ny, a.nz, a.own, s1, c0);
-    pair32<KER, CAREFUL>(r, k + 1, b.nx, b.ny, b.nz, b.own, t1, c1);
+    pair32<KER, MODE>(r, k, a.nx, a.ny, a.nz, a.own, s0, m0, c0);
+    pair32<KER, MODE>(r, k, b.nx, b.ny, b.nz, b.own, t0, m1, c1);
+    pair32<KER, MODE>(r, k + 1, a.nx, a.ny, a.nz, a.own, s1, m0, c0);
+    pair32<KER, MODE>(r, k + 1, b.nx, b.ny, b.nz, b.own, t1, m1, c1);
   }
   if (k < nr) {
-    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c0);
-    pair32<KER, CAREFUL>(r, k, b.nx, b.ny, b.nz, b.own, t0, c1);
+    pair32<KER, MODE>(r, k, a.nx, a.ny, a.nz, a.own, s0, m0, c0);
+    pair32<KER, MODE>(r, k, b.nx, b.ny, b.nz, b.own, t0, m1, c1);
   }
   p0 = (s0.x + s0.y) + (s1.x + s1.y);
   p1 = (t0.x + t0.y) + (t1.x + t1.y);
+  if (MODE == M_WATCH) {
+    c0 = m0 < r.thr;
+    c1 = m1 < r.thr;
+  }
 }
 
 // One target against records k, k + step, ...
-template <int KER, bool CAREFUL>
+template <int KER, int MODE>
 __device__ __forceinline__ float one32(const Range32& r, const Target32& a, int k, int step, bool& c) {
   float2 s0{0.f, 0.f}, s1{0.f, 0.f};
+  float m = HUGE_VALF;
   const int nr = (r.n + 1) >> 1;
 #pragma unroll 1
   for (; k + step < nr; k += 2 * step) {
-    pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c);
-    pair32<KER, CAREFUL>(r, k + step, a.nx, a.ny, a.nz, a.own, s1, c);
+    pair32<KER, MODE>(r, k, a.nx, a.ny, a.nz, a.own, s0, m, c);
+    pair32<KER, MODE>(r, k + step, a.nx, a.ny, a.nz, a.own, s1, m, c);
   }
-  if (k < nr) pair32<KER, CAREFUL>(r, k, a.nx, a.ny, a.nz, a.own, s0, c);
+  if (k < nr) pair32<KER, MODE>(r, k, a.nx, a.ny, a.nz, a.own, s0, m, c);
+  if (MODE == M_WATCH) c = m < r.thr;
   return (s0.x + s0.y) + (s1.x + s1.y);
 }
 
 // Every listed target against one tile of leaf `entry` (centre c, half extents hb); compensated
 // sums into the warp's row (rows values, then rows errors).  own0: the tile index of target
-// 0's own source if the leaf holds targets of the group (SELF).  A warp takes the careful
-// loops where one of its targets comes within the close distance of the leaf's box.
+// 0's own source if the leaf holds targets of the group (SELF).  A warp takes the careful loop
+// in its own leaf (without close pairs: where the tile holds the own source of one of its
+// targets), and where the watching loop, taken within the close distance of the leaf's box, has
+// met a close pair (rare; the pairs that both loops add are the same, bit for bit).  2M clustered
+// in leaves of 1000, us: the careful loop in all these places, screened 5761, regularised 5018,
+// Coulomb with a delta past the close distance 3571; as it is 5401, 4875, 3375; watching in the
+// own leaf too 5640, 4873, 3375 (a close pair in 40% of its tiles).
 template <int KER, bool SELF>
 __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, const double* cx,
                                        const double* cy, const double* cz, double4 c, float4 hb,
@@ -170,6 +185,18 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
   auto near_box = [&](const Target32& t) {
     return box_d2(unpack2(t.nx).x, unpack2(t.ny).x, unpack2(t.nz).x, hb) < r.thr;
   };
+  auto own_in = [&](const Target32& t) { return (unsigned)t.own < (unsigned)r.n; };
+  auto one = [&](const Target32& t, int k, int step, bool& cl) {
+    float p = 0.f;
+    bool careful = SELF && (r.thr > 0.f || __any_sync(0xffffffffu, own_in(t)));
+    if (!careful) {
+      if (SELF || !__any_sync(0xffffffffu, near_box(t))) return one32<KER, M_PLAIN>(r, t, k, step, cl);
+      p = one32<KER, M_WATCH>(r, t, k, step, cl);
+      careful = __any_sync(0xffffffffu, cl);
+      cl = false;
+    }
+    return careful ? one32<KER, M_CAREFUL>(r, t, k, step, cl) : p;
+  };
   auto add = [&](int i, float p, bool close) {
     two_sum(row[i], row[rows + i], p);
     if (close) record_close(a, t0 + i, g, e, toff);
@@ -181,10 +208,18 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
     const Target32 x = target(i0), y = target(i1);
     float p0, p1;
     bool c0 = false, c1 = false;
-    if (SELF || __any_sync(0xffffffffu, near_box(x) || near_box(y)))
-      two32<KER, true>(r, x, y, p0, p1, c0, c1);
-    else
-      two32<KER, false>(r, x, y, p0, p1, c0, c1);
+    bool careful = SELF && (r.thr > 0.f || __any_sync(0xffffffffu, own_in(x) || own_in(y)));
+    if (!careful) {
+      // (in the own leaf no pair can be close here)
+      if (!SELF && __any_sync(0xffffffffu, near_box(x) || near_box(y))) {
+        two32<KER, M_WATCH>(r, x, y, p0, p1, c0, c1);
+        careful = __any_sync(0xffffffffu, c0 || c1);
+        c0 = c1 = false;
+      } else {
+        two32<KER, M_PLAIN>(r, x, y, p0, p1, c0, c1);
+      }
+    }
+    if (careful) two32<KER, M_CAREFUL>(r, x, y, p0, p1, c0, c1);
     add(i0, p0, c0);
     if (v1) add(i1, p1, c1);
   }
@@ -193,8 +228,7 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
     const int i = all ? base + lane : tl[base + lane];
     const Target32 x = target(i);
     bool cl = false;
-    const float p = SELF || __any_sync(0xffffffffu, near_box(x)) ? one32<KER, true>(r, x, 0, 1, cl)
-                                                                : one32<KER, false>(r, x, 0, 1, cl);
+    const float p = one(x, 0, 1, cl);
     add(i, p, cl);
     base += 32;
   }
@@ -205,8 +239,7 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
     const int i = all ? r0 : tl[r0];
     const Target32 x = target(i);
     bool cl = false;
-    float p = SELF || __any_sync(0xffffffffu, near_box(x)) ? one32<KER, true>(r, x, slice, 1 << sh, cl)
-                                                          : one32<KER, false>(r, x, slice, 1 << sh, cl);
+    float p = one(x, slice, 1 << sh, cl);
     int c = cl;
     for (int o = 1 << sh >> 1; o; o >>= 1) {
       p += __shfl_xor_sync(0xffffffffu, p, o);

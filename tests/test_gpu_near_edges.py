@@ -103,3 +103,27 @@ def test_points_with_no_near_entries(ctx, orc, m):
         for prec, tol in ((B.FP64, 1e-12), (B.MIXED, 1e-6)):
             check(t.evaluate(B.params(kb, B.CONSISTENT, prec, acc=0.4, **kw), points=pts), want, tol)
     t.treeempty()
+
+
+@pytest.mark.parametrize("n,maxmemb", [(3000, 100), (9000, 700)])
+def test_close_pairs_across_leaves(ctx, orc, n, maxmemb):
+    """Partners on either side of the tree's first cuts, 1e-7 to 1e-3 apart: the loop that watches
+    for close pairs meets them in other leaves than the target's own, and is done again."""
+    import bit_b200 as B
+    rng = np.random.default_rng(n)
+    p = rng.uniform(-1, 1, (3, n))
+    for a in range(3):
+        i = rng.choice(n, 60, replace=False)
+        gap = 10.0 ** rng.uniform(-7, -3, 30)
+        p[:, i[30:]] = p[:, i[:30]]
+        p[a, i[:30]], p[a, i[30:]] = gap / 2, -gap / 2
+    p[:, 0], p[:, 1] = 1.0, -1.0  # the box is symmetric: cuts through 0
+    q = rng.uniform(-1, 1, n)
+    t = ctx.treemake(*p, maxmemb)
+    t.treemoments(q, 2)
+    tg = np.arange(n, dtype=np.int32)
+    for kb, ko, kw in kernels(B, orc):
+        want = orc.direct(*p, q, orc.params(ko, orc.MODE_CONSISTENT, acc=0.0, **kw), tg)
+        for prec, tol in ((B.FP64, 1e-12), (B.MIXED, 1e-6)):
+            check(t.evaluate(B.params(kb, B.CONSISTENT, prec, acc=0.0, **kw)), want, tol)
+    t.treeempty()
