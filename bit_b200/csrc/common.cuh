@@ -20,7 +20,7 @@ constexpr int kGroupMax = 1024;   // targets per group (one CTA; 32 mask words)
 constexpr int kFieldChunk = 256;       // targets of a CTA of the fields' kernels, at most
 constexpr int kPointGroup = 256;  // external points per group, at most
 constexpr int kNearParts = 8;         // near-field items of a group, at most
-constexpr long long kNearChunk = 512 << 10;  // and the pairs of one, at least
+constexpr long long kNearChunk = 512 << 10, kNearChunkMin = 32 << 10;  // and the pairs of one
 constexpr double kEpsNear = 1e-14;  // src/constants.h:35
 
 __host__ __device__ constexpr int num_terms(int n) { return n * (n + 1) * (n + 2) / 6; }

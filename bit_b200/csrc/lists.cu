@@ -485,19 +485,32 @@ static int far_chunk(const std::vector<int>& tc, int sms) { return chunk_size(tc
 // 1045; 2M, 1000, ms: 42.8 / 31.0 / 25.2 / 22.3 (whole groups: 25.2).
 static int field_chunk(const std::vector<int>& tc, int sms) { return chunk_size(tc, kFieldChunk, 5LL * sms / 2); }
 
-// The potentials' near-field items, heaviest first: a group's near work in one item, or in up
-// to kNearParts equal parts of at least kNearChunk pairs each, whose sums meet in scratch
-// (near_part).  The count follows from the group's own lists alone, so that its result does
+// The near-field items, heaviest first: a group's near work in one item, or in up to kNearParts
+// equal parts of at least `chunk` pairs each, whose sums meet in scratch (near_part).  A part
+// packs its targets for fewer sources, so parts are only as many as give a system four items a
+// multiprocessor: chunk is a share of the system's pairs, between kNearChunkMin and kNearChunk
+// (groups of packed leaves, set for throughput: kNearChunk).  Screened FP64 / mixed, us, chunks
+// of 512k against this: 20k in leaves of 500 359 / 121 -> 117 / 68; 50k, 300: 426 / 160 -> 248 / 144; 10k,
+// 200: 89 / 51 -> 46 / 41; 200k, 500: 1332 / 470 either way; 64k for all: 1369 / 559 at 200k, 17.3 for 17.0
+// ms at 2M, 48 packed systems 3.2 for 2.8 ms.  (Cutting a group's targets instead gave nothing: most
+// lists are short.)  The count follows from the system's own lists alone, so that its result does
 // not depend on what else is evaluated; without room in the memory budget for the scratch,
 // every group is one item.
 static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& pairs,
-                       const std::vector<int>& tc) {
+                       const std::vector<int>& tc, const std::vector<int>& sys, bool packed) {
   const int ng = (int)pairs.size();
   std::vector<int> K(ng);
+  std::vector<unsigned long long> of_sys(ng ? 1 + *std::max_element(sys.begin(), sys.end()) : 0, 0);
+  for (int g = 0; g < ng; g++) of_sys[sys[g]] += pairs[g];
+  auto chunk = [&](int s) {
+    const unsigned long long share = of_sys[s] / (unsigned long long)(4 * c->num_sms);
+    return packed ? (unsigned long long)kNearChunk
+                  : std::min<unsigned long long>(kNearChunk, std::max<unsigned long long>(kNearChunkMin, share));
+  };
   std::vector<long long> off(ng, 0);
   long long tot = 0;
   for (int g = 0; g < ng; g++) {
-    K[g] = (int)std::max(1ull, std::min<unsigned long long>(kNearParts, pairs[g] / kNearChunk));
+    K[g] = (int)std::max(1ull, std::min<unsigned long long>(kNearParts, pairs[g] / chunk(sys[g])));
     off[g] = tot;
     if (K[g] > 1) tot += (long long)K[g] * tc[g];
   }
@@ -683,7 +696,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->h_work = wk;
   L->order.ensure(c, ng);
   BIT_CUDA(cudaMemcpyAsync(L->order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s));
-  near_items(L, c, hp, tc);  // (synchronises)
+  near_items(L, c, hp, tc, gsys, key.group > 0 && !key.points);  // (synchronises)
   L->key = key;
   L->valid = true;
   L->version++;

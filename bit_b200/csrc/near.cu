@@ -18,12 +18,12 @@
 // FP64: bound by the FP64 pipe (12 operations a Coulomb pair, 25 a screened one; the kernel
 // this replaces, one target a thread and a barrier per tile, was held up by shared-memory
 // wavefronts).  Mixed: by the MUFU (one or two a pair) and issue.  Before / now, ms, default
-// settings: 2M clustered (leaves of 1000, theta = 0.7, 9.25 G pairs) FP64 screened 20.7 / 17.1,
-// Coulomb 13.4 / 7.5, mixed 6.0 / 5.9 and 3.6 / 3.8; 100k, theta = 0.15 (1.61 G pairs): 10.8 /
-// 3.1, 6.5 / 1.34, mixed 2.26 / 1.16, 1.72 / 0.60; 300k uniform in leaves of 100: 1.17 / 0.50,
-// 0.75 / 0.32, mixed 0.68 / 0.29, 0.50 / 0.24.  Eight warps a CTA: four are 5% faster in the
-// mixed 2M case and up to 50% slower on 20k; parts of at least 512k pairs: 64k cost 10% at
-// 200k for 10% at 20k.
+// settings: 2M clustered (leaves of 1000, theta = 0.7, 8.6 G pairs) FP64 screened 20.7 / 17.0,
+// Coulomb 13.4 / 7.4, mixed 6.0 / 5.4 and 3.6 / 3.4; 100k, theta = 0.15 (1.6 G pairs): 10.8 / 3.1,
+// 6.5 / 1.3, mixed 2.26 / 1.12, 1.72 / 0.57; 300k uniform in leaves of 100: 1.17 / 0.48, 0.75 / 0.28,
+// mixed 0.68 / 0.30, 0.50 / 0.25; 20k in leaves of 500 0.71 / 0.12, 0.41 / 0.06, 0.20 / 0.07, 0.16 /
+// 0.04.  Eight warps a CTA: four are 5% faster in the
+// mixed 2M case and up to 50% slower on 20k.
 #include <algorithm>
 #include <climits>
 

@@ -10,8 +10,8 @@
 // Bound by the FP64 pipe, mixed by issue.  Before (a square root and a division, one target a
 // thread, a barrier per tile) / now, ms: 2M clustered in leaves of 1000, theta = 0.7, FP64 Coulomb
 // 24.2 / 11.0, mixed 7.6 / 6.1, screened 40.3 / 21.1; 100k uniform in leaves of 100 0.57 / 0.16, 0.47 /
-// 0.11, 0.70 / 0.24; 50k in leaves of 300 1.03 / 0.24, 0.47 / 0.13, 1.50 / 0.47; 20k 0.33 / 0.09,
-// 0.21 / 0.06, 0.42 / 0.13.
+// 0.11, 0.70 / 0.24; 50k in leaves of 300 1.03 / 0.20, 0.47 / 0.13, 1.50 / 0.33; 20k 0.33 / 0.08,
+// 0.21 / 0.06, 0.42 / 0.10.
 #include <algorithm>
 #include <type_traits>
 
