@@ -46,7 +46,7 @@ FLOPS_NEAR = {"screened": 14, "coulomb": 11}     # per near pair (rsqrt, exp cou
 # FP64 pipe operations the FP64 near kernel issues per pair (its own rsqrt and exp spelled
 # out: 3 differences, 3 for r^2 + del, 4 for the Newton step, 11 for exp, the products):
 # the instruction-level ceiling of that kernel is peak / 2 / ops pairs per second
-FP64_OPS_NEAR = {"screened": 26, "coulomb": 13}
+FP64_OPS_NEAR = {"screened": 25, "coulomb": 12}
 # Accuracy-matched parameters: (p, theta, N0) at which the plain FP64 treecode reaches 1e-6
 # relative L2 against the FP64 direct sum on these workloads (measured; the run reports
 # the errors it reaches)

@@ -14,10 +14,10 @@ group of targets.  It pays off for many small leaves (batched uneven systems: 35
 and costs where near entries then cover too few targets (the icosphere solves: 70% slower),
 so tune_group times it on the caller's own workload.
 
-The near field's source tile (records per TMA copy into shared memory) and the cap on the
-threads that split one target's sources (bit_ctx_set_near_config) are tuned per
-(nterms, kernel, N0, precision) by tune_near on the same seeded systems; tune() chains
-N0 and the near-field knobs for one workload class.
+The limit on the near field's source tile (bit_ctx_set_near_config; its second knob, the
+threads that split one target's sources, has no effect) is tuned per (nterms, kernel, N0,
+precision) by tune_near on the same seeded systems; tune() chains N0 and the near-field
+knobs for one workload class.
 """
 import math
 

@@ -114,7 +114,7 @@ bit_status bit_ctx_set_group_size(bit_ctx* ctx, int targets);
  * 0 launches once per class.  Results are identical either way. */
 bit_status bit_ctx_set_work_queue(bit_ctx* ctx, int on);
 /* Near-field tuning knobs (bit_b200.autotune): `tile` source records per CTA (a power of two,
- * 128..2048; 0: the default, 512), shared by its eight warps, an eighth each (32..128 records,
+ * 128..2048; 0: the default, 1024), shared by its eight warps, an eighth each (32..128 records,
  * less where shared memory is short); `threads_per_target` (a power of two, 1..32; 0) is
  * accepted and has no effect: targets share a source's lanes as their number asks.  Results
  * change only in FP rounding order. */
