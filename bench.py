@@ -60,10 +60,10 @@ MATCHED_BATCH_ACC = {5: 0.015, 7: 0.05, 9: 0.1}   # theta by nterms (p = 4, 6, 8
 # i.e. 135 and 78 MB scaled by N; the full-size launches read more (sources re-read by
 # groups of several waves once the 126 MB L2 no longer holds them).
 TRAFFIC = {
-    "k_near<SCREENED, F64>": 266.19e6, "k_near<COULOMB, F64>": 225.88e6,
-    "k_far<9, SCREENED, double>": 102.06e6, "k_far<9, COULOMB, double>": 102.54e6,
-    "k_near<SCREENED, F32>": 131.96e6, "k_near<COULOMB, F32>": 114.60e6,
-    "k_far<9, SCREENED, float>": 98.32e6, "k_far<9, COULOMB, float>": 98.96e6,
+    "k_near<SCREENED, F64>": 387.8e6, "k_near<COULOMB, F64>": 390.1e6,
+    "k_far<9, SCREENED, double>": 105.1e6, "k_far<9, COULOMB, double>": 111.1e6,
+    "k_near<SCREENED, F32>": 220.1e6, "k_near<COULOMB, F32>": 195.4e6,
+    "k_far<9, SCREENED, float>": 103.4e6, "k_far<9, COULOMB, float>": 106.2e6,
 }
 TRAFFIC_SOURCE = ("ncu launch list of the full-size step (gpu__time_duration.sum, "
                   "dram__bytes_read.sum, dram__bytes_write.sum; one pass per launch), "
@@ -357,8 +357,9 @@ def run_bit(args):
             line["accuracy_matched"]["serving"] = run_serving(ctx, args, matched=True)
     if args.cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(x, y, z, q, n, args)
-        # the same lists, so the same interactions per eval
-        line["cpu_baseline"]["interactions_per_s"] = line["cpu_baseline"]["value"] * inter / evals
+        # the same lists, so the same interactions per eval (no value: no reference build here)
+        if line["cpu_baseline"]["value"]:
+            line["cpu_baseline"]["interactions_per_s"] = line["cpu_baseline"]["value"] * inter / evals
     line["gpu_launches"] = launches[B.FP64] * args.steps
     line["gpu_launches_per_step"] = launches[B.FP64]
     print(json.dumps(line), flush=True)

@@ -25,7 +25,7 @@
 // Bound by latency: launches, and in a node's CTA its scans and reductions, one bisection after
 // the other.  With the passes for every node (18 launches and a round trip a level), before /
 // now: 2k uniform in leaves of 50 744 / 172 us, 10k, 200: 693 / 183, 50k clustered, 300: 1,663 / 412,
-// 100k, 500: 1,845 / 500, 200k, 500: 2,105 / 700, 2M, 1000: 4,149 / 2,490, 48 systems 1,279 / 535.  With
+// 100k, 500: 1,845 / 500, 200k, 500: 2,105 / 689, 2M, 1000: 4,149 / 2,130, 48 systems 1,279 / 535.  With
 // one CTA up to 16,384 members that read them from L2 at every bisection: 10k 320, 100k 1,190.
 // Doing the bisection in hand and a foreseen one in one pass (four passes for seven) gave
 // nothing: a pass's own scan and reduction take the time, not its barriers.
@@ -836,9 +836,9 @@ __global__ void __launch_bounds__(TB, 6)
   const int node = list[ck.x];
   const int e1 = min(ck.y + CH, A.start[node] + A.nummemb[node]);
   int cnt[2] = {0, 0};
-  unsigned long long mn[2][3], mx[2][3];
-  for (int h = 0; h < 2; h++)
-    for (int d = 0; d < 3; d++) { mn[h][d] = ~0ULL; mx[h][d] = 0ULL; }
+  unsigned long long v[12];  // per half and axis: the smallest key, the largest's complement
+#pragma unroll
+  for (int q = 0; q < 12; q++) v[q] = ~0ULL;
   // this thread's members e = ck.y + tid + k TB: every label first, then the unrolled
   // loop, so the members' loads overlap instead of waiting one after the other
   constexpr int PER = CH / TB;
@@ -858,50 +858,48 @@ __global__ void __launch_bounds__(TB, 6)
       lab[e] = (signed char)l;
     }
     if (hc && l == cu.src) {
-      int h = (coord(cu.dir, sx, sy, sz, e) <= cu.mid) ? 0 : 1;
-      double v[3] = {sx[e], sy[e], sz[e]};
+      const bool h = !(coord(cu.dir, sx, sy, sz, e) <= cu.mid);
+      const double x[3] = {sx[e], sy[e], sz[e]};
       cnt[h]++;
+#pragma unroll
       for (int d = 0; d < 3; d++) {
-        unsigned long long k = okey(v[d]);
-        mn[h][d] = k < mn[h][d] ? k : mn[h][d];
-        mx[h][d] = k > mx[h][d] ? k : mx[h][d];
+        const unsigned long long k = okey(x[d]);
+        if (h) {
+          least(v[6 + 2 * d], k);
+          least(v[7 + 2 * d], ~k);
+        } else {
+          least(v[2 * d], k);
+          least(v[2 * d + 1], ~k);
+        }
       }
     }
   }
-  // warp, then CTA reductions; one set of global atomics per CTA (min / max / sum are
+  // warp (by halves: a build of 2M 2,465 -> 2,130 us, of 800k 935 -> 842), then CTA reductions;
+  // one set of global atomics per CTA (min / max / sum are
   // order-independent, so the result is exact whatever the order)
   constexpr int NW = TB / 32;
   __shared__ int s_c[NW][2];
-  __shared__ unsigned long long s_m[NW][2][3], s_M[NW][2][3];
+  __shared__ unsigned long long s_v[NW][12];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int h = 0; h < 2; h++) {
-    const int c = warp_sum(cnt[h]);
-    unsigned long long m[3], M[3];
-    for (int d = 0; d < 3; d++) { m[d] = warp_min(mn[h][d]); M[d] = warp_max(mx[h][d]); }
-    if (lane == 0) {
-      s_c[w][h] = c;
-      for (int d = 0; d < 3; d++) { s_m[w][h][d] = m[d]; s_M[w][h][d] = M[d]; }
-    }
+    const int c = __reduce_add_sync(0xffffffffu, cnt[h]);
+    if (lane == 0) s_c[w][h] = c;
   }
+  warp_least12(v);
+  if (!(lane & 1) && (lane & 6) != 6) s_v[w][6 * (lane >> 4) + 3 * ((lane >> 3) & 1) + (lane & 6) / 2] = v[0];
   __syncthreads();
-  if (hc && threadIdx.x < 2 * 7) {  // thread (h, v): v = 0..5 min/max of one axis, v = 6 count
-    const int h = threadIdx.x / 7, v = threadIdx.x % 7;
+  if (hc && threadIdx.x < 2 * 7) {  // thread (h, q): q = 0..5 smallest / largest of an axis, 6 count
+    const int h = threadIdx.x / 7, q = threadIdx.x % 7;
     int c = 0;
-    for (int q = 0; q < NW; q++) c += s_c[q][h];
+    for (int k = 0; k < NW; k++) c += s_c[k][h];
     if (c > 0) {
-      if (v == 6) {
+      if (q == 6) {
         atomicAdd(&acc[ck.x].cnt[h], c);
       } else {
-        const int d = v >> 1;
-        if (v & 1) {
-          unsigned long long M = 0;
-          for (int q = 0; q < NW; q++) M = s_M[q][h][d] > M ? s_M[q][h][d] : M;
-          atomicMax(&acc[ck.x].mx[h][d], M);
-        } else {
-          unsigned long long m = ~0ULL;
-          for (int q = 0; q < NW; q++) m = s_m[q][h][d] < m ? s_m[q][h][d] : m;
-          atomicMin(&acc[ck.x].mn[h][d], m);
-        }
+        unsigned long long m = ~0ULL;
+        for (int k = 0; k < NW; k++) least(m, s_v[k][6 * h + q]);
+        if (q & 1) atomicMax(&acc[ck.x].mx[h][q >> 1], ~m);
+        else atomicMin(&acc[ck.x].mn[h][q >> 1], m);
       }
     }
   }
