@@ -149,8 +149,9 @@ __device__ __forceinline__ void pack_list(unsigned wd, int W, unsigned short* tl
 // One pair's q / sqrt(r^2 + del) or q e^(-kappa R) / R (src/tree3d.cpp:4765-4769, 3609-3618)
 // added to acc.  1/R: the hardware seed and one third-order Newton step (rsqrt_nr); the
 // exponential: exp_scaled.  12 (Coulomb) / 25 (screened) FP64 operations.  EPS: a pair with
-// r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`).  UF: the
-// exponential may underflow.
+// r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`); both are evaluated
+// with charge 0 at R = 1.  UF: the exponential may underflow; without, kappa R of every pair and
+// kappa itself are below kExpNoUnderflow (SysEval::underflow).
 template <int KER, bool EPS, bool SELF, bool UF, int COPIES = kExpTabCopies>
 __device__ __forceinline__ void pair64(double x, double y, double z, double4 s, double del,
                                        ExpScale k, const double2* tab, bool own, double& acc) {
