@@ -18,88 +18,129 @@ namespace bit {
 // Device memory: a per-context cache of freed blocks.  All work of a context runs on its
 // one stream, so a block freed after a launch can be handed to a later launch on the same
 // stream without a device synchronisation (stream order protects it).  The HBM budget
-// bounds live + cached bytes; cached blocks are released first when it would be exceeded.
+// bounds live + cached bytes.  At the budget a cached block is cut: the request takes its
+// front, the rest stays cached, and neighbours join again when they are freed; a request
+// served whole by whatever larger block there was held that block's bytes for as long as it
+// lived, and a few small ones could use the budget up.
 static size_t round_block(size_t b) {
   const size_t g = b < (1u << 20) ? 512 : (size_t)2 << 20;
   return (b + g - 1) / g * g;
 }
 
-static void release_cache(Ctx* c) {
-  for (auto& kv : c->cache) cudaFree(kv.second);
-  c->cache.clear();
-  c->cached = 0;
+// Give the largest block that is free as a whole back to the device; false: there is none.
+static bool drop_largest(Ctx* c) {
+  for (auto it = c->cache.rbegin(); it != c->cache.rend(); ++it) {
+    const auto blk = c->blocks.find(it->second);
+    if (blk->second.size != blk->second.whole) continue;
+    cudaFree(it->second);
+    c->cached -= it->first;
+    c->cache.erase(std::next(it).base());
+    c->blocks.erase(blk);
+    return true;
+  }
+  return false;
+}
+
+size_t ctx_releasable(const Ctx* c) {
+  size_t n = 0;
+  for (const auto& f : c->cache)
+    if (c->blocks.at(f.second).whole == f.first) n += f.first;
+  return n;
+}
+
+size_t ctx_room(const Ctx* c) {
+  if (!c->budget) return SIZE_MAX;
+  const size_t held = c->in_use + c->cached - ctx_releasable(c);
+  const size_t room = std::max(c->budget > held ? c->budget - held : 0, c->cache.empty() ? 0 : c->cache.rbegin()->first);
+  return room < (1u << 20) ? room / 512 * 512 : std::max<size_t>((1u << 20) - 512, room >> 21 << 21);
 }
 
 void ctx_trim(Ctx* c, size_t keep) {
   if (c->in_use + c->cached <= keep) return;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  // largest blocks first
-  while (!c->cache.empty() && c->in_use + c->cached > keep) {
-    auto it = std::prev(c->cache.end());
-    cudaFree(it->second);
-    c->cached -= it->first;
-    c->cache.erase(it);
-  }
+  while (c->in_use + c->cached > keep && drop_largest(c)) {}
 }
 
-// Over the budget, a request is served from any larger cached block (it costs no memory),
-// and otherwise only as many cached blocks are freed, largest first, as the new block needs:
-// every cudaFree waits for the device, and freeing the whole cache for one small block
-// stalled served requests by hundreds of milliseconds.
-static void release_for(Ctx* c, size_t bytes) {
-  while (!c->cache.empty() && c->in_use + c->cached + bytes > c->budget) {
-    auto it = std::prev(c->cache.end());
-    cudaFree(it->second);
-    c->cached -= it->first;
-    c->cache.erase(it);
+// Scratch between two list builds, which a request that does not fit may have: the regions of
+// every tree's builder.  False: there was none.
+static bool reclaim(Ctx* c) {
+  bool any = false;
+  for (Tree* t : c->trees) {
+    any |= t->plists.gstage.p != nullptr;
+    t->plists.gstage.release();
   }
+  return any;
 }
 
 void* dev_alloc(Ctx* c, size_t bytes) {
   bytes = round_block(bytes);
-  auto it = c->cache.lower_bound(bytes);
+  auto it = c->cache.lower_bound({bytes, nullptr});
   const bool tight = c->budget && c->in_use + c->cached + bytes > c->budget;
   if (it != c->cache.end() && (it->first <= 2 * bytes || tight)) {
-    void* p = it->second;
-    size_t sz = it->first;
+    char* p = it->second;
     c->cache.erase(it);
-    c->cached -= sz;
-    c->in_use += sz;
+    Ctx::Block& b = c->blocks[p];
+    if (tight && b.size > bytes) {
+      c->blocks[p + bytes] = Ctx::Block{b.size - bytes, b.whole, b.base, false};
+      c->cache.insert({b.size - bytes, p + bytes});
+      b.size = bytes;
+    }
+    b.live = true;
+    c->cached -= b.size;
+    c->in_use += b.size;
     c->peak = std::max(c->peak, c->in_use);
-    c->allocs.push_back({p, sz});
     return p;
   }
-  if (tight) release_for(c, bytes);
-  if (c->budget && c->in_use + bytes > c->budget)
+  if (c->budget && c->in_use + c->cached - ctx_releasable(c) + bytes > c->budget) {
+    if (reclaim(c)) return dev_alloc(c, bytes);
     fail(BIT_ERR_BUDGET, "allocation of " + std::to_string(bytes) + " bytes exceeds the HBM budget");
+  }
+  // Only as many cached blocks are freed, largest first, as the new block needs: every cudaFree
+  // waits for the device, and freeing the whole cache for one small block stalled served requests
+  // by hundreds of milliseconds.
+  while (c->budget && c->in_use + c->cached + bytes > c->budget && drop_largest(c)) {}
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    release_cache(c);
+    while (drop_largest(c)) {}
     e = cudaMalloc(&p, bytes);
   }
   BIT_CUDA(e);
   c->in_use += bytes;
   c->peak = std::max(c->peak, c->in_use);
-  c->allocs.push_back({p, bytes});
+  char* q = static_cast<char*>(p);
+  c->blocks[q] = Ctx::Block{bytes, bytes, q, true};
   return p;
 }
 
-void dev_free(Ctx* c, void* p) {
-  if (!p) return;
-  for (size_t i = 0; i < c->allocs.size(); i++)
-    if (c->allocs[i].first == p) {
-      size_t sz = c->allocs[i].second;
-      c->in_use -= sz;
-      c->allocs[i] = c->allocs.back();
-      c->allocs.pop_back();
-      c->cache.insert({sz, p});
-      c->cached += sz;
-      return;
-    }
-  cudaFree(p);
+void dev_free(Ctx* c, void* ptr) {
+  if (!ptr) return;
+  auto it = c->blocks.find(static_cast<char*>(ptr));
+  if (it == c->blocks.end()) {
+    cudaFree(ptr);
+    return;
+  }
+  c->in_use -= it->second.size;
+  c->cached += it->second.size;
+  it->second.live = false;
+  // join a free neighbour of the same cudaMalloc
+  auto joins = [&](auto a, auto b) { return !a->second.live && !b->second.live && a->second.base == b->second.base; };
+  auto next = std::next(it);
+  if (next != c->blocks.end() && joins(it, next)) {
+    c->cache.erase({next->second.size, next->first});
+    it->second.size += next->second.size;
+    c->blocks.erase(next);
+  }
+  if (it != c->blocks.begin() && joins(std::prev(it), it)) {
+    auto prev = std::prev(it);
+    c->cache.erase({prev->second.size, prev->first});
+    prev->second.size += it->second.size;
+    c->blocks.erase(it);
+    it = prev;
+  }
+  c->cache.insert({it->second.size, it->first});
 }
 
 // Blocking device-to-host copy ordered on the context's stream (the legacy default stream
@@ -248,6 +289,9 @@ bit_status bit_ctx_create(bit_ctx** out, const bit_ctx_opts* opts) {
     }
     BIT_CUDA(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
     BIT_CUDA(cudaMallocHost(&c.h_pinned, 64 * sizeof(long long)));
+    // what lives as long as the context has blocks of its own, not cut from a larger one
+    c.dev_err();
+    c.queue_heads.ensure(&c, 2);
   });
   if (st != BIT_OK) {
     delete h;
@@ -276,7 +320,9 @@ bit_status bit_ctx_destroy(bit_ctx* h) {
   c.close_n.release();
   c.close_rec.release();
   c.close_list.release();
-  release_cache(&c);
+  c.queue_heads.release();
+  dev_free(&c, c.err_flag);
+  while (drop_largest(&c)) {}
   if (c.h_pinned) cudaFreeHost(c.h_pinned);
   for (int i = 0; i < 2; i++) {
     if (c.stage_ev[i]) cudaEventSynchronize(c.stage_ev[i]);

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <initializer_list>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -72,6 +73,9 @@ struct D2H {
 void copy_d2h_batch(Ctx* c, std::initializer_list<D2H> list);
 // Free cached (unused) blocks until live + cached bytes are at most `keep`.
 void ctx_trim(Ctx* c, size_t keep);
+// The cached bytes that this could free, and the largest block to be had within the budget.
+size_t ctx_releasable(const Ctx* c);
+size_t ctx_room(const Ctx* c);
 
 template <class T>
 struct DBuf {
@@ -185,8 +189,8 @@ struct Lists {
   DBuf<int> far_node, near_node;            // entry -> node
   DBuf<unsigned> far_mask, near_mask;       // (tcount+31)/32 words per entry
   DBuf<int> order;                          // groups by decreasing work
-  DBuf<int> far_tgt, near_tgt;              // targets of each entry
-  DBuf<long long> far_pre, near_pre;        // work of the group's entries before it
+  DBuf<unsigned short> far_tgt, near_tgt;   // targets of each entry (at most kGroupMax)
+  DBuf<long long> far_pre, near_pre;        // of every 32nd entry: work of its group's before it
   DBuf<long long> far_tot, near_tot;        // per group: work of all its entries
   std::vector<long long> h_work;            // estimated work of each group
   // the potentials' near-field items (group, part | parts << 16), heaviest first; groups of
@@ -229,8 +233,13 @@ struct Ctx {
   // small device scratch for flags / counters
   DBuf<long long> scratch_ll;
   long long* h_pinned = nullptr;  // pinned host staging for small read-backs (64 entries)
-  std::vector<std::pair<void*, size_t>> allocs;  // live device allocations and their sizes
-  std::multimap<size_t, void*> cache;             // freed blocks kept for reuse, by size
+  struct Block {
+    size_t size, whole;  // bytes; those of the cudaMalloc that it is (a part of), at base
+    char* base;
+    bool live;
+  };
+  std::map<char*, Block> blocks;                  // all of the context's device memory
+  std::set<std::pair<size_t, char*>> cache;       // freed blocks kept for reuse, by size
   size_t cached = 0;                              // bytes held in `cache`
   std::vector<Tree*> trees;                       // trees built by this context
   long long launches = 0;                         // kernels launched by this context

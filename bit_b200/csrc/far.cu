@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "near.cuh"
 #include "tma.cuh"
 
 namespace bit {
@@ -71,8 +72,8 @@ struct FarArgs {
   int chunk;                 // targets of a CTA, at most
   int rows;                  // those of the largest chunk, rounded up to 32
   int* err;                  // device error flags (a bounded wait that gave up: 8)
-  const int* tgt;            // targets of each far entry (potentials)
-  const long long* pre;      // targets of the group's entries before it
+  const unsigned short* tgt;  // targets of each far entry
+  const long long* pre;      // of every 32nd: targets of its group's entries before it
   const long long* tot;      // per group: targets of all its entries
   const SysEval* sys;        // per system: far_add, kappa, far_sign
   const int* g_sys;          // per group: system
@@ -232,6 +233,15 @@ __global__ void __launch_bounds__(kCoefThreads)
   }
 }
 
+// The group's first far entry, of [e0, e1), whose work begins at or past share / nw (e1: none does).
+__device__ __forceinline__ long long far_begin(const FarArgs& a, long long e0, long long e1, long long share, int nw) {
+  const long long T = (share + nw - 1) / nw;
+  if (T <= 0) return e0;
+  long long P;
+  const long long e = run_entry(a.pre, e0, e1, T - 1, [&](long long k) { return (long long)a.tgt[k]; }, P);
+  return min(e + 1, e1);
+}
+
 // The far field of one target group g (the CTA's whole work for that group).  Bound by the
 // FP64 / FP32 pipe and issue: 244 instructions a pair (nterms 9, screened) where the
 // reference's recurrence took 1,333 (FP64) and 1,118 (FP32); 324 against 738 and 683 with
@@ -275,15 +285,10 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
   // round-robin deal this replaces left warps idle at the group's closing barrier.  The
   // split depends on the lists only, so results stay deterministic.
   const long long tot = a.tot[g];
-  long long eb = 0, ee = 0;
-  for (long long b = e0; b < e1; b += 32) {
-    const bool in = b + lane < e1;
-    const long long P = in ? a.pre[b + lane] * NW : 0;
-    eb += __popc(__ballot_sync(0xffffffffu, in && P < w * tot));
-    ee += __popc(__ballot_sync(0xffffffffu, in && P < (w + 1) * tot));
-  }
+  const long long ee = far_begin(a, e0, e1, (w + 1) * tot, NW);
+  long long e = far_begin(a, e0, e1, w * tot, NW);
   __syncthreads();  // the rows are zero
-  for (long long e = e0 + eb; e < e0 + ee; e++) {
+  for (; e < ee; e++) {
     const int node = a.node[e];
     // The cluster's coefficients, its whole block (TP values, 16-byte aligned in global and
     // shared memory), by one TMA bulk copy into the warp's slot while the warp packs the
@@ -439,17 +444,12 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   const SysEval* se = a.sys + a.g_sys[g];
   const T tadd = (T)se->far_add, tk = (T)se->kappa;
   const long long tot = a.tot[g];
-  long long eb = 0, ee = 0;
-  for (long long b = e0; b < e1; b += 32) {
-    const bool in = b + lane < e1;
-    const long long P = in ? a.pre[b + lane] * NW : 0;
-    eb += __popc(__ballot_sync(0xffffffffu, in && P < w * tot));
-    ee += __popc(__ballot_sync(0xffffffffu, in && P < (w + 1) * tot));
-  }
+  const long long ee = far_begin(a, e0, e1, (w + 1) * tot, NW);
+  long long e = far_begin(a, e0, e1, w * tot, NW);
   __syncthreads();  // the rows are zero, the barriers ready
   bool failed = false;
   unsigned phase = 0;
-  for (long long e = e0 + eb; e < e0 + ee; e++) {
+  for (; e < ee; e++) {
     const int node = a.node[e];
     if (lane == 0) {
       fence_proxy_async();

@@ -26,7 +26,8 @@
 // under the same MAC; a first build uses an allowance).  Where a group overflows its region, or
 // a reservation runs past the arrays, the build is run again, with four times the room a group
 // (up to every node of the tree), or with room for the totals that this run counted: the same
-// lists, later.  A memory budget limits the regions to as many as fit.
+// lists, later.  A memory budget limits the regions to as many as fit beside the lists, down to one,
+// and what is allocated after them may have their room (dev_alloc).
 //
 // Bound by issue and latency (tensor and FP64 pipes idle, everything in L1 and L2).  Walking
 // depth first, one node at a time and a thread per target, against this; a whole build with its
@@ -68,9 +69,10 @@ struct ListArgs {
   long long *far_off, *near_off, *far_moff, *near_moff;
   int *far_cnt, *near_cnt;
   unsigned long long* g_near;  // near pairs of each group
-  // per entry: its targets, and the work of the group's entries before it (far: targets,
-  // near: near_weight x sources); per group: that of all
-  int *far_tgt, *near_tgt;
+  // per entry: its targets; for the entries whose index is a multiple of 32, the work of their
+  // group's entries before them (far: targets, near: near_weight x sources; run_entry finds the
+  // others' from it); per group: that of all
+  unsigned short *far_tgt, *near_tgt;
   long long *far_pre, *near_pre, *far_tot, *near_tot;
   // lists
   int *far_node, *near_node;
@@ -114,9 +116,9 @@ __device__ __forceinline__ void group_prefixes(const ListArgs& a, int g, long lo
       const long long t = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += t;
     }
-    if (k < n) {
-      if (w) a.near_pre[no + k] = run + inc - v;
-      else a.far_pre[fo + k] = run + inc - v;
+    if (k < n && !((w ? no + k : fo + k) & 31)) {
+      if (w) a.near_pre[(no + k) >> 5] = run + inc - v;
+      else a.far_pre[(fo + k) >> 5] = run + inc - v;
     }
     run += __shfl_sync(0xffffffffu, inc, 31);
   }
@@ -367,12 +369,12 @@ __global__ void __launch_bounds__(QT, 4) k_lists(ListArgs a) {
     for (int k = tid; k < nf; k += QT) {
       const int v = fref[k];
       a.far_node[fo + k] = vnode[v];
-      a.far_tgt[fo + k] = vac[v];
+      a.far_tgt[fo + k] = (unsigned short)vac[v];
     }
     for (int k = tid; k < nn; k += QT) {
       const int v = nref[k];
       a.near_node[no + k] = vnode[v];
-      a.near_tgt[no + k] = vrc[v];
+      a.near_tgt[no + k] = (unsigned short)vrc[v];
     }
     // a warp per entry, a lane per word
     for (int k = w; k < nf + nn; k += QW) {
@@ -497,7 +499,7 @@ static int field_chunk(const std::vector<int>& tc, int sms) { return chunk_size(
 // not depend on what else is evaluated; without room in the memory budget for the scratch,
 // every group is one item.
 static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& pairs,
-                       const std::vector<int>& tc, const std::vector<int>& sys, bool packed) {
+                       const std::vector<int>& tc, const std::vector<int>& sys, bool packed, size_t later) {
   const int ng = (int)pairs.size();
   std::vector<int> K(ng);
   std::vector<unsigned long long> of_sys(ng ? 1 + *std::max_element(sys.begin(), sys.end()) : 0, 0);
@@ -514,7 +516,9 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
     off[g] = tot;
     if (K[g] > 1) tot += (long long)K[g] * tc[g];
   }
-  if (L->near_part.n < (size_t)tot && c->budget && c->in_use + tot * sizeof(double) > c->budget) {
+  auto fits = [&] { return L->near_part.n >= (size_t)tot || tot * sizeof(double) + later <= ctx_room(c); };
+  if (!fits()) L->gstage.release();
+  if (!fits()) {
     std::fill(K.begin(), K.end(), 1);
     tot = 0;
   }
@@ -621,7 +625,6 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   int per_sm = 0;
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists, QT, 0));
   const long long nodes = std::max(t->numtree, 1);
-  long long visits0 = 1;  // at least this many
   long long visits = std::min(nodes, hint && hint->visits > 0 ? hint->visits + hint->visits / 4 + 64 : kVisitsFirst);
   L->far_tot.ensure(c, ng);
   L->near_tot.ensure(c, ng);
@@ -642,20 +645,15 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     L->near_mask.ensure(c, cap[3]);
     L->far_tgt.ensure(c, L->far_node.n);
     L->near_tgt.ensure(c, L->near_node.n);
-    L->far_pre.ensure(c, L->far_node.n);
-    L->near_pre.ensure(c, L->near_node.n);
+    L->far_pre.ensure(c, L->far_node.n / 32 + 1);
+    L->near_pre.ensure(c, L->near_node.n / 32 + 1);
     for (int k = 0; k < 4; k++) a.cap[k] = cap[k];
     a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
     a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
     a.far_tgt = L->far_tgt.p; a.near_tgt = L->near_tgt.p;
     a.far_pre = L->far_pre.p; a.near_pre = L->near_pre.p;
     const long long per = (long long)(maxw + kVisitWords) * sizeof(unsigned);  // bytes a visit
-    size_t room = kRegionBytes;
-    if (c->budget) {
-      const size_t held = c->in_use - L->gstage.n * sizeof(unsigned);
-      room = std::min(room, std::max(L->gstage.n * sizeof(unsigned), c->budget > held ? c->budget - held : 0));
-      visits = std::min(visits, std::max<long long>(room / per, visits0));
-    }
+    const size_t room = std::min(kRegionBytes, std::max(L->gstage.n * sizeof(unsigned), ctx_room(c)));
     a.stage = visits * (maxw + kVisitWords);
     long long slots = std::min<long long>(ng, (long long)c->num_sms * std::max(per_sm, 1));
     slots = std::min<long long>(slots, room / (visits * per));
@@ -673,9 +671,10 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     err = (int)(h[6] & 0xffffffffu);
     if (!(err & 3)) break;
     L->fallback = true;
-    if (err & 1) visits0 = visits + 1, visits = std::min(nodes, 4 * visits);  // (the totals are not complete)
+    if (err & 1) visits = std::min(nodes, 4 * visits);  // (the totals are not complete)
     else for (int k = 0; k < 4; k++) cap[k] = h[k];
   }
+  if (key.points) L->gstage.release();
   ListSizing& z = L->last;
   z.ngroups = ng;
   z.acc = key.acc;
@@ -696,7 +695,10 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->h_work = wk;
   L->order.ensure(c, ng);
   BIT_CUDA(cudaMemcpyAsync(L->order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s));
-  near_items(L, c, hp, tc, gsys, key.group > 0 && !key.points);  // (synchronises)
+  // what an evaluation takes beside the lists and its parts' scratch: sums, close pairs, coefficients
+  const size_t later = (size_t)ntargets * (2 * sizeof(double) + 28) +
+                       (size_t)nodes * (3 * num_terms(std::max(t->nterms, 1)) / 2 + 4) * sizeof(double);
+  near_items(L, c, hp, tc, gsys, key.group > 0 && !key.points, later);  // (synchronises)
   L->key = key;
   L->valid = true;
   L->version++;

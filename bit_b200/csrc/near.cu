@@ -313,18 +313,20 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
   const long long tot = a.tot[g];
   const int nv = NW * parts, v = part * NW + w;
   const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
-  long long e = run_entry(a.pre, e0, e1, T0);
+  long long P;
+  long long e = run_entry(a.pre, e0, e1, T0, [&](long long k) { return near_work(a, k); }, P);
+  long long d0 = T0 - P, d1 = T1 - P;  // the run, from where the entry's work begins
   __syncthreads();  // the rows are zero
   const double del = se->near_del;
   const ExpScale ks = exp_scale(se->kappa);
   const float kl2 = (float)(-se->kappa * 1.4426950408889634);  // -kappa log2(e)
   bool failed = false;
-  for (; e < e1; e++) {
-    const long long P = a.pre[e];
-    if (P >= T1) break;
+  for (; e < e1 && d1 > 0; e++) {
     const int node = a.node[e], ns = a.nummemb[node], cnt = a.tgt[e];
     const int wt = near_weight(cnt);
-    const int ja = cut(T0, P, wt, ns), jb = cut(T1, P, wt, ns);
+    const int ja = cut(d0, wt, ns), jb = cut(d1, wt, ns);
+    d0 -= (long long)wt * ns;
+    d1 -= (long long)wt * ns;
     if (ja >= jb) continue;
     const int s0 = a.start[node];
     const unsigned char* src = reinterpret_cast<const unsigned char*>(a.src) +

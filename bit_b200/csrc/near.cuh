@@ -57,8 +57,8 @@ struct NearArgs {
   int* cn;      // entries of clist
   int cap;               // mixed potentials: records of a tile at most (k_close)
   const int* pstart;     // first record of each leaf's FP32 sources
-  const int* tgt;        // targets of each near entry
-  const long long* pre;  // work (near_weight x sources) of the group's entries before it
+  const unsigned short* tgt;  // targets of each near entry
+  const long long* pre;  // of every 32nd: work (near_weight x sources) of its group's before it
   const long long* tot;  // per group: work of all its entries
   const int* leaf_of;  // leaf of each sorted position
   const int2* items;   // (group, part | parts << 16)
@@ -254,12 +254,12 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   return v;
 }
 
-// First source (a multiple of 8, or all ns) of an entry of weight wt whose work begins at P
-// that lies at or past T.
-__device__ __forceinline__ int cut(long long T, long long P, int wt, int ns) {
-  if (T <= P) return 0;
-  if (T >= P + (long long)wt * ns) return ns;
-  const long long j = (T - P + 8LL * wt - 1) / (8LL * wt) * 8;
+// First source (a multiple of 8, or all ns) of an entry of weight wt that lies d or more into its
+// work.
+__device__ __forceinline__ int cut(long long d, int wt, int ns) {
+  if (d <= 0) return 0;
+  if (d >= (long long)wt * ns) return ns;
+  const long long j = (d + 8LL * wt - 1) / (8LL * wt) * 8;
   return j < ns ? (int)j : ns;
 }
 
@@ -267,17 +267,38 @@ __device__ __forceinline__ int cut(long long T, long long P, int wt, int ns) {
 __device__ __forceinline__ long long run_begin(long long tot, int nv, int v) {
   return tot / nv * v + tot % nv * v / nv;
 }
-// The entry of [e0, e1) that work T0 lies in: the last whose prefix is at most T0 (e1 if there is
-// no entry: a group may have none).
-__device__ __forceinline__ long long run_entry(const long long* pre, long long e0, long long e1, long long T0) {
+// The entry of a group's [e0, e1) that work T lies in: the last that begins at T or before (e1 if
+// there is no entry: a group may have none); P: where it begins.  pre: where the work of every
+// 32nd entry of the list begins (kept for those alone, and counts in 16 bits: a list of small
+// leaves at a small theta is most of a request's memory); work: an entry's.  By a whole warp.
+template <class Work>
+__device__ __forceinline__ long long run_entry(const long long* pre, long long e0, long long e1, long long T,
+                                               Work work, long long& P) {
   const int lane = threadIdx.x & 31;
-  long long e = e0 < e1 ? e0 - 1 : e1;
-  for (long long b = e0; b < e1; b += 32) {
-    const int c = __popc(__ballot_sync(0xffffffffu, b + lane < e1 && pre[b + lane] <= T0));
-    e += c;
+  P = 0;
+  if (e0 >= e1) return e1;
+  long long k = e0 >> 5;  // the block of 32 entries
+  for (long long b = k + 1, last = (e1 - 1) >> 5; b <= last; b += 32) {
+    const int c = __popc(__ballot_sync(0xffffffffu, b + lane <= last && pre[b + lane] <= T));
+    k += c;
     if (c < 32) break;
   }
-  return e;
+  const bool first = (k << 5) <= e0;
+  const long long s = first ? e0 : k << 5, begin = first ? 0 : pre[k];
+  const bool in = s + lane < min(e1, (k + 1) << 5);
+  const long long v = in ? work(s + lane) : 0;
+  long long inc = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  const int n = __popc(__ballot_sync(0xffffffffu, in && begin + inc - v <= T));
+  P = begin + __shfl_sync(0xffffffffu, inc - v, n - 1);
+  return s + n - 1;
+}
+// A group's near entry: its work.
+__device__ __forceinline__ long long near_work(const NearArgs& a, long long e) {
+  return (long long)near_weight(a.tgt[e]) * a.nummemb[a.node[e]];
 }
 
 // The arguments common to every near-field launch of this plan (near_field.cu).

@@ -221,7 +221,9 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   const long long tot = a.tot[g];
   const int nv = NW * parts, v = part * NW + w;
   const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
-  long long e = run_entry(a.pre, e0, e1, T0);
+  long long P;
+  long long e = run_entry(a.pre, e0, e1, T0, [&](long long k) { return near_work(a, k); }, P);
+  long long d0 = T0 - P, d1 = T1 - P;  // the run, from where the entry's work begins
   __syncthreads();  // the rows are zero, the table and the barriers are there
   Field f;
   f.del = se->near_del;
@@ -230,12 +232,12 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   f.tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
   f.korder = se->kernel_order;
   bool failed = false;
-  for (; e < e1; e++) {
-    const long long P = a.pre[e];
-    if (P >= T1) break;
+  for (; e < e1 && d1 > 0; e++) {
     const int node = a.node[e], ns = a.nummemb[node], ec = a.tgt[e];
     const int wt = near_weight(ec);  // (the work is shared out by the whole group's)
-    const int ja = cut(T0, P, wt, ns), jb = cut(T1, P, wt, ns);
+    const int ja = cut(d0, wt, ns), jb = cut(d1, wt, ns);
+    d0 -= (long long)wt * ns;
+    d1 -= (long long)wt * ns;
     if (ja >= jb) continue;
     const bool all = ec == gc;
     const unsigned wd = !all && lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
@@ -429,7 +431,7 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
   // part takes it whole
   Layout lay;
   const size_t need = 3 * (size_t)L->part_total;
-  lay.single = L->field_part.n < need && c->budget && c->in_use + need * sizeof(double) > c->budget;
+  lay.single = L->field_part.n < need && (need + 6 * (size_t)t->n) * sizeof(double) > ctx_room(c);
   if (!lay.single) L->field_part.ensure(c, need);
   a.part = L->field_part.p;
   lay.chunk = L->field_chunk;
