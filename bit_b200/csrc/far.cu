@@ -196,7 +196,10 @@ __global__ void __launch_bounds__(kCoefThreads)
     s_m[p] = ldexp(M[t], -he * d);
   }
   if (threadIdx.x == 0) {
-    const double kh = kind & FAR_SCREENED ? ldexp(se->kappa, he) : 0.0;
+    // (kappa H is held where its powers stay in range: past 2^13 every accepted pair's exponential
+    // is 0 in FP32, past 2^100 in FP64, and a coefficient of infinity would make the 0 a NaN)
+    const double cap = sizeof(T) == 4 ? 0x1p13 : 0x1p100;
+    const double kh = kind & FAR_SCREENED ? fmin(fabs(ldexp(se->kappa, he)), cap) : 0.0;
     const double k2 = kh * kh, dd = ldexp(delta, -2 * he);
     for (int k = 0; k < KMAX; k++)
       for (int s = 0; s < 2 * KMAX; s++) s_e[k][s] = 0.0;

@@ -171,6 +171,11 @@ def lit(v):
     return f"T({float(v)!r})"
 
 
+# Past X_MAX = kappa rho the exponential is 0 in either precision, and so is the result: kappa rho
+# is held there, and kappa H at KH_MAX, so that no factor beside that 0 is infinite.
+X_MAX, KH_MAX = 2.0 ** 20, 2.0 ** 50
+
+
 class Loads:
     """A cluster's coefficients, four at a time, where they are first needed."""
 
@@ -206,7 +211,7 @@ def gen_eval(nt, reg, scr):
             if top >= 1:
                 L.append("  const T g1 = eta * fma_t(x, g0, g0);")
             if top >= 2:
-                L += ["  const T kh = kappa * H;", "  const T kh2 = kh * kh;"]
+                L += [f"  const T kh = min(kappa * H, {lit(KH_MAX)});", "  const T kh2 = kh * kh;"]
             for l in range(2, nt):
                 c = Fraction(1, (2 * l - 1) * (2 * l - 3))
                 L.append(f"  const T g{l} = fma_t({lit(c)}, kh2 * g{l - 2}, eta * g{l - 1});")
@@ -229,7 +234,7 @@ def gen_eval(nt, reg, scr):
             for s in range(3, 2 * (top // 2) + 1):
                 L.append(f"  const T t{s} = t{s - 1} * t1;")
         if scr:
-            L += ["  const T x = kappa * (rho2 * ri);",
+            L += [f"  const T x = min(kappa * (rho2 * ri), {lit(X_MAX)});",
                   "  const T b0 = exp_t(-x);"]
             if top >= 1:
                 L.append("  const T b1 = fma_t(x, b0, b0);")
@@ -375,12 +380,12 @@ def gen_grad(nt, reg, scr):
             L.append("  const T eta = H * ri;")
         if scr:
             L += ["  const T r = r2 * ri;",
-                  "  const T x = kappa * r;",
+                  f"  const T x = min(kappa * r, {lit(X_MAX)});",
                   "  const T g0 = exp_t(-x) * ri;",
                   "  const T h0 = x * g0;"]
             if top >= 1:
                 L += ["  const T g1 = eta * fma_t(x, g0, g0);",
-                      "  const T kh = kappa * H;", "  const T kr = kh * x;"]
+                      f"  const T kh = min(kappa * H, {lit(KH_MAX)});", "  const T kr = kh * x;"]
             if top >= 2:
                 L.append("  const T kh2 = kh * kh;")
             for l in range(2, nt):

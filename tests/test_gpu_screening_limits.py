@@ -64,3 +64,26 @@ def test_field_at_the_limit_of_the_unchecked_exponential(ctx, kappa, extent):
     check(fy, d[0] * w)
     assert not np.any(fz)
     t.treeempty()
+
+
+@pytest.mark.parametrize("nterms", [3, 9, 10])
+@pytest.mark.parametrize("kappa", [3e3, 1e5, 1e7, 1e12, 1e25])
+def test_far_field_of_clusters_many_screening_lengths_wide(ctx, nterms, kappa):
+    """Accepted clusters lie so many screening lengths away that their potential is 0; powers of
+    kappa times their size, up to the eighth, and of kappa times the distance leave FP32's range."""
+    import bit_b200 as B
+    from bit_b200 import workloads
+    x, y, z, q = workloads.clustered_blobs(4000, seed=3)
+    far = np.random.default_rng(4).uniform(-1, 1, (100, 3)) * 10.0 ** np.arange(1, 11).repeat(10)[:, None] + 50.0
+    t = ctx.treemake(x, y, z, 60)
+    t.treemoments(q, nterms)
+    for kernel, delta in ((B.SCREENED, 0.0), (B.SCREENED_REG, 1e-4)):
+        got = {}
+        for prec in (B.FP64, B.MIXED):
+            p = B.params(kernel, B.CONSISTENT, prec, kappa=kappa, del_=delta, acc=0.5)
+            got[prec] = t.evaluate(p)
+            assert not np.any(t.evaluate(p, points=far))
+        assert np.all(np.isfinite(got[B.FP64]))
+        # (FP32 holds nothing below 1e-45; kappa R rounds to 6e-8 of at most 100)
+        assert np.max(np.abs(got[B.MIXED] - got[B.FP64])) <= 1e-5 * np.max(np.abs(got[B.FP64])) + 1e-40
+    t.treeempty()
