@@ -262,6 +262,7 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
   constexpr int CNT = far_count(NT, KIND);
   constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ long long s_begin[NW];
   const int rows = a.rows;
   const int ROW = WarpAcc<T>::words * rows;
   T* msb = reinterpret_cast<T*>(sm);  // per warp a slot of a.stride elements
@@ -288,9 +289,10 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
   // round-robin deal this replaces left warps idle at the group's closing barrier.  The
   // split depends on the lists only, so results stay deterministic.
   const long long tot = a.tot[g];
-  const long long ee = far_begin(a, e0, e1, (w + 1) * tot, NW);
   long long e = far_begin(a, e0, e1, w * tot, NW);
-  __syncthreads();  // the rows are zero
+  if (lane == 0) s_begin[w] = e;
+  __syncthreads();  // the rows are zero, the runs' beginnings there
+  const long long ee = w + 1 < NW ? s_begin[w + 1] : e1;
   for (; e < ee; e++) {
     const int node = a.node[e];
     // The cluster's coefficients, its whole block (TP values, 16-byte aligned in global and
@@ -427,6 +429,7 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ uint64_t bar[NW];
+  __shared__ long long s_begin[NW];
   const int g = a.order[blockIdx.x], c0 = blockIdx.y * a.chunk;
   const int t0 = a.g_tstart[g] + c0, gc = a.g_tcount[g], tc = min(gc - c0, a.chunk);
   if (tc <= 0) return;  // (the whole CTA)
@@ -447,9 +450,10 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   const SysEval* se = a.sys + a.g_sys[g];
   const T tadd = (T)se->far_add, tk = (T)se->kappa;
   const long long tot = a.tot[g];
-  const long long ee = far_begin(a, e0, e1, (w + 1) * tot, NW);
   long long e = far_begin(a, e0, e1, w * tot, NW);
-  __syncthreads();  // the rows are zero, the barriers ready
+  if (lane == 0) s_begin[w] = e;
+  __syncthreads();  // the rows are zero, the runs' beginnings there, the barriers ready
+  const long long ee = w + 1 < NW ? s_begin[w + 1] : e1;
   bool failed = false;
   unsigned phase = 0;
   for (; e < ee; e++) {
