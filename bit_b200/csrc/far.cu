@@ -148,11 +148,11 @@ __host__ __device__ constexpr int far_block(int nt, int kind) {
 }
 
 // Exponent of H = 2^e, the smallest power of two above the cluster's radius and (regularised)
-// sqrt(delta): the scaled evaluation then works with ratios H / distance of at most about
-// one, and scaling by H is exact.  A cluster of coincident particles has moments of degree 0
-// only, and takes the lowest exponent.
+// sqrt(|delta|; a field's may be negative): the scaled evaluation then works with ratios H /
+// distance of at most about one, powers of delta / H^2 stay in range, and scaling by H is exact.
+// A cluster of coincident particles has moments of degree 0 only, and takes the lowest exponent.
 __device__ __forceinline__ int far_scale_exp(double sqradius, double delta) {
-  const double s = fmax(sqradius, delta);
+  const double s = fmax(sqradius, fabs(delta));
   if (!(s > 0.0)) return -100;
   if (!(s < 1e300)) return 100;
   const int e = ilogb(sqrt(s)) + 1;
