@@ -85,6 +85,28 @@ struct Vec {
   double x, y, z;
 };
 
+// The field of a tile's sources j, j + step, ... by the plain formulas: where field64 leaves NaN
+// (an r^2 past FP64's range counts as 0, one of 0 as infinite).
+template <int FK>
+__device__ __noinline__ Vec plain64(const double4* src, int n, double x, double y, double z, double del,
+                                    double kappa, int o, int j, int step) {
+  Vec p{0.0, 0.0, 0.0};
+  for (; j < n; j += step) {
+    if (j == o) continue;
+    const double4 s = src[j];
+    const double dx = x - s.x, dy = y - s.y, dz = z - s.z;
+    const double rs = dx * dx + dy * dy + dz * dz + del, r = sqrt(rs);
+    if (FK == F_CURL) {
+      const double t = s.w * exp(-kappa * r) / rs * (kappa + 1 / r);
+      p.x -= dy * t; p.y += dx * t;
+    } else {
+      const double t = s.w / (r * rs);
+      p.x += dx * t; p.y += dy * t; p.z += dz * t;
+    }
+  }
+  return p;
+}
+
 template <int FK, bool SELF, bool UF>
 __device__ __forceinline__ void two64(const double4* src, int n, const Field& f, Vec s, Vec t, int o0, int o1,
                                       Vec& p, Vec& r) {
@@ -309,6 +331,10 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
         }
       } else {
         const double4* ds = reinterpret_cast<const double4*>(tile);
+        auto plain = [&](Vec& p, int i, int k, int step) {
+          if (FK != F_ORDER && isnan(p.x))  // (a pair's factor is NaN in all components)
+            p = plain64<FK>(ds, n, cx[i], cy[i], cz[i], f.del, f.kappa, i + own0, k, step);
+        };
         auto run = [&](auto S, auto U) {
           constexpr bool SELF = decltype(S)::value, UF = decltype(U)::value;
           for (int b = 0; b < st.full; b++) {
@@ -318,13 +344,17 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
             Vec p, q;
             two64<FK, SELF, UF>(ds, n, f, Vec{cx[i0], cy[i0], cz[i0]}, Vec{cx[i1], cy[i1], cz[i1]}, i0 + own0,
                                 i1 + own0, p, q);
+            plain(p, i0, 0, 1);
+            plain(q, i1, 0, 1);
             add(i0, p);
             if (v1) add(i1, q);
           }
           int base = 64 * st.full;
           if (st.one) {
             const int i = all ? base + lane : tl[base + lane];
-            add(i, one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, 0, 1));
+            Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, 0, 1);
+            plain(p, i, 0, 1);
+            add(i, p);
             base += 32;
           }
           if (st.tail) {
@@ -332,6 +362,7 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
             const bool in = slot < st.tail;
             const int r0 = base + (in ? slot : 0), i = all ? r0 : tl[r0];
             Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, slice, 1 << sh);
+            plain(p, i, slice, 1 << sh);
             for (int o = 1 << sh >> 1; o; o >>= 1) {
               p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
               p.y += __shfl_xor_sync(0xffffffffu, p.y, o);

@@ -1,8 +1,9 @@
 """Fields at the ends of their arguments' ranges: a negative delta (the entry points take any finite
-one) beside clusters of no extent."""
+one) beside clusters of no extent, and distances whose squares leave FP64's range."""
 import numpy as np
 import pytest
 
+from test_gpu_field_direct_edges import check, coulomb_field, curl_field
 from test_gpu_field_far import compare
 
 pytestmark = pytest.mark.gpu
@@ -18,3 +19,24 @@ def test_negative_delta_beside_clusters_of_one_particle(ctx, orc, nterms, scale)
     g = np.stack(np.meshgrid(*[np.arange(9.0)] * 3, indexing="ij")).reshape(3, -1)
     x, y, z = (g + rng.uniform(-0.1, 0.1, g.shape)) * scale
     compare(ctx, orc, x, y, z, rng.uniform(-1, 1, g.shape[1]), 1, nterms, 0.5, -0.3 * scale ** 2, 1e-5)
+
+
+@pytest.mark.parametrize("n", [1, 20, 33, 49, 70, 150])
+def test_distances_whose_squares_overflow(ctx, n):
+    """n particles near the origin and n some 1e160 away, 1e150 apart: a pair of the two kinds, or of
+    two of the far ones, adds 0."""
+    import bit_b200 as B
+    rng = np.random.default_rng(n)
+    p = rng.uniform(-1, 1, (3, 2 * n))
+    p[:, n:] = 1e160 * (1.0 + 1e-10 * p[:, n:])
+    q = rng.uniform(-1, 1, 2 * n)
+    near = slice(0, n)
+    for maxmemb in (2 * n, n):
+        t = ctx.treemake(*p, maxmemb)
+        t.treemoments(q, 2)
+        for got, want in ((t.treeforce(0.0, 1e-3), coulomb_field(*p[:, near], q[near], 1e-3)),
+                          (t.field(B.FIELD_SCREENED, acc=0.0, kappa=1.5), curl_field(*p[:, near], q[near], 1.5))):
+            got = np.stack(got)
+            assert not np.any(got[:, n:])
+            check(got[:, near], want, 1e-12)
+        t.treeempty()
