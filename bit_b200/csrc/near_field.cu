@@ -86,7 +86,8 @@ struct Vec {
 };
 
 // The field of a tile's sources j, j + step, ... by the plain formulas: where field64 leaves NaN
-// (an r^2 past FP64's range counts as 0, one of 0 as infinite).
+// (an r^2 past FP64's range counts as 0, one of 0 as infinite), and where a screened field grows
+// with the distance (kappa < 0, which the entry points take) past exp_scaled's domain.
 template <int FK>
 __device__ __noinline__ Vec plain64(const double4* src, int n, double x, double y, double z, double del,
                                     double kappa, int o, int j, int step) {
@@ -331,8 +332,9 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
         }
       } else {
         const double4* ds = reinterpret_cast<const double4*>(tile);
+        const bool grows = FK == F_CURL && f.kappa < 0.0 && se->underflow;
         auto plain = [&](Vec& p, int i, int k, int step) {
-          if (FK != F_ORDER && isnan(p.x))  // (a pair's factor is NaN in all components)
+          if (FK != F_ORDER && (grows || isnan(p.x)))  // (a pair's factor is NaN in all components)
             p = plain64<FK>(ds, n, cx[i], cy[i], cz[i], f.del, f.kappa, i + own0, k, step);
         };
         auto run = [&](auto S, auto U) {

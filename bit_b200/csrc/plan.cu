@@ -107,10 +107,10 @@ void plan_sys(Tree* t, EvalPlan* P, const std::vector<bit_eval_params>& prm, int
     // the largest kappa R of a pair: the sources lie within the root box's half diagonal of
     // its centre, particle targets too; a pair that is left out (the target's own source, or
     // one below the limit on r^2) is evaluated at R = 1 in place of its own distance
-    const double half = std::sqrt(t->h_fields[13LL * s + 12]);
+    // (a field's kappa may be negative)
+    const double kap = std::fabs(h[s].kappa), half = std::sqrt(t->h_fields[13LL * s + 12]);
     const double far = half + (points ? reach : half);
-    h[s].underflow = !(h[s].kappa * std::sqrt(far * far + h[s].near_del) < kExpNoUnderflow &&
-                       h[s].kappa < kExpNoUnderflow);
+    h[s].underflow = !(kap * std::sqrt(far * far + h[s].near_del) < kExpNoUnderflow && kap < kExpNoUnderflow);
   }
   P->f32 = prm[0].precision == BIT_PREC_MIXED;
   P->force = force;

@@ -1,5 +1,6 @@
 """Fields at the ends of their arguments' ranges: a negative delta (the entry points take any finite
-one) beside clusters of no extent, and distances whose squares leave FP64's range."""
+one) beside clusters of no extent, distances whose squares leave FP64's range, and screened fields
+that grow with the distance (kappa < 0, which the entry points take too)."""
 import numpy as np
 import pytest
 
@@ -40,3 +41,34 @@ def test_distances_whose_squares_overflow(ctx, n):
             assert not np.any(got[:, n:])
             check(got[:, near], want, 1e-12)
         t.treeempty()
+
+
+@pytest.mark.parametrize("extent", [10.0, 690.0, 703.0, 760.0])
+@pytest.mark.parametrize("n", [40, 300])
+def test_screened_field_that_grows(ctx, n, extent):
+    """kappa < 0 to where exp(-kappa R) nears FP64's largest number, e^709.78, and past it, where the
+    field is infinite (or infinities of either sign meet); kappa R rounds as in the tests of the
+    strong screening, so 1e-12 of the terms' sizes."""
+    import bit_b200 as B
+    rng = np.random.default_rng(n)
+    p = rng.uniform(0, 1, (3, n))
+    p[:, 0], p[:, 1] = 0.0, 1.0
+    kappa = -3.0
+    p *= extent / 3.0 / np.sqrt(3.0)
+    q = rng.uniform(-1, 1, n) * 1e-6
+    t = ctx.treemake(*p, 40)
+    t.treemoments(q, 2)
+    fx, fy, fz = t.field(B.FIELD_SCREENED, acc=0.0, kappa=kappa)
+    t.treeempty()
+    d = (p[:, :, None] - p[:, None, :]).astype(np.longdouble)
+    r = np.sqrt((d * d).sum(0))
+    np.fill_diagonal(r, 1.0)
+    w = q * np.exp(-np.longdouble(kappa) * r) / (r * r) * (kappa + 1 / r)
+    np.fill_diagonal(w, 0.0)
+    most = np.max(-kappa * r, axis=1)
+    inside, outside = most < 709.5, most > 710.0
+    assert np.any(outside) == (extent > 710)
+    for got, terms in ((fx, -d[1] * w), (fy, d[0] * w)):
+        assert np.all(np.abs(got - terms.sum(1))[inside] <= 1e-12 * np.abs(terms).sum(1)[inside])
+        assert not np.any(np.isfinite(got[outside]))
+    assert not np.any(fz)
