@@ -496,8 +496,8 @@ static int field_chunk(const std::vector<int>& tc, int sms) { return chunk_size(
 // 200: 89 / 51 -> 46 / 41; 200k, 500: 1332 / 470 either way; 64k for all: 1369 / 559 at 200k, 17.3 for 17.0
 // ms at 2M, 48 packed systems 3.2 for 2.8 ms.  (Cutting a group's targets instead gave nothing: most
 // lists are short.)  The count follows from the system's own lists alone, so that its result does
-// not depend on what else is evaluated; without room in the memory budget for the scratch,
-// every group is one item.
+// not depend on what else is evaluated.  Without room in the memory budget for the scratch every
+// group is one item that takes its parts one after the other: the same sums, later.
 static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& pairs,
                        const std::vector<int>& tc, const std::vector<int>& sys, bool packed, size_t later) {
   const int ng = (int)pairs.size();
@@ -518,14 +518,14 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
   }
   auto fits = [&] { return L->near_part.n >= (size_t)tot || tot * sizeof(double) + later <= ctx_room(c); };
   if (!fits()) L->gstage.release();
-  if (!fits()) {
-    std::fill(K.begin(), K.end(), 1);
-    tot = 0;
-  }
+  L->part_seq = !fits();
+  if (L->part_seq) tot = 0;
   L->part_total = tot;
   std::vector<std::pair<unsigned long long, int2>> it;
-  for (int g = 0; g < ng; g++)
-    for (int k = 0; k < K[g]; k++) it.push_back({pairs[g] / K[g], make_int2(g, k | K[g] << 16)});
+  for (int g = 0; g < ng; g++) {
+    const int items = L->part_seq ? 1 : K[g];
+    for (int k = 0; k < items; k++) it.push_back({pairs[g] / items, make_int2(g, k | K[g] << 16)});
+  }
   std::stable_sort(it.begin(), it.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
   L->h_items.resize(it.size());
   for (size_t i = 0; i < it.size(); i++) L->h_items[i] = it[i].second;

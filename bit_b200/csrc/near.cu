@@ -262,6 +262,7 @@ __device__ __forceinline__ void tile32(const NearArgs& a, const Range32& r, cons
 // 246 / 248.
 struct Layout {
   int cap, tab;  // records of a tile at most; bytes of the table
+  int seq;       // groups that take their parts in turn: where the sums of those done begin
   static __host__ __device__ int rows(int tc) { return (tc + 31) / 32 * 32; }
   template <bool F32>
   static __host__ __device__ int recs(int cap, int rows) {
@@ -281,18 +282,16 @@ struct Layout {
   }
 };
 
-// Returns false (in every thread) if a warp's bounded wait for a tile gave up: the error flag
-// is set, the warp has waited, bounded again, for its copies in flight, and the group's
-// result is not valid.  phase: this warp's count of completed copies, over the items of a
-// queue.
+// Part `part` of group g's work, of `parts`: the CTA's warps' sums into their rows.  Returns false
+// (in every thread) if a warp's bounded wait for a tile gave up: the error flag is set, the
+// warp has waited, bounded again, for its copies in flight, and the group's result is not
+// valid.  phase: this warp's count of completed copies, over the items of a queue.
 template <int KER, bool EPS, bool F32>
-__device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, int2 item, uint64_t* bar,
-                                          unsigned& phase) {
+__device__ __forceinline__ bool near_part(const NearArgs& a, const Layout& L, int g, int part, int parts,
+                                          uint64_t* bar, unsigned& phase) {
   constexpr int PER = F32 ? 2 : 1;  // sources of a record
-  const int g = item.x, ROWS = Layout::rows(a.g_tcount[g]), RECS = Layout::recs<F32>(L.cap, ROWS);
+  const int ROWS = Layout::rows(a.g_tcount[g]), RECS = Layout::recs<F32>(L.cap, ROWS);
   const int TILE = RECS * PER;
-  const int part = item.y & 0xffff, parts = item.y >> 16;
-  __shared__ int s_last;
   extern __shared__ __align__(128) unsigned char sm[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const double2* tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
@@ -399,7 +398,20 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
     }
     if (failed) break;
   }
-  const bool ok = !__syncthreads_or(failed);
+  return !__syncthreads_or(failed);
+}
+
+// An item.  Returns false as near_part does.  SEQ: all parts of the group, one after the other,
+// their sums kept in shared memory and added in part order as those in the scratch are.
+template <int KER, bool EPS, bool F32, bool SEQ>
+__device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, int2 item, uint64_t* bar,
+                                          unsigned& phase) {
+  __shared__ int s_last;
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int g = item.x, part = item.y & 0xffff, parts = item.y >> 16, tid = threadIdx.x;
+  const int t0 = a.g_tstart[g], tc = a.g_tcount[g], ROWS = Layout::rows(tc), W = (tc + 31) >> 5;
+  const double* rows = reinterpret_cast<const double*>(
+      sm + L.tab + NW * 2 * (size_t)Layout::recs<F32>(L.cap, ROWS) * kRec);
   auto warps_sum = [&](int i) {
     double s = 0.0;
     for (int q = 0; q < NW; q++) {
@@ -413,11 +425,21 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
     }
     return s;
   };
+  double* seq = reinterpret_cast<double*>(sm + L.seq);
+  bool ok = near_part<KER, EPS, F32>(a, L, g, part, parts, bar, phase);
+  if (SEQ && parts > 1) {
+    for (int q = 0;;) {
+      for (int i = tid; i < tc; i += 32 * NW) seq[i] = (q ? seq[i] : 0.0) + warps_sum(i);
+      __syncthreads();  // the rows are read
+      if (!ok || ++q == parts) break;
+      ok = near_part<KER, EPS, F32>(a, L, g, q, parts, bar, phase);
+    }
+  }
   // this item's sums: straight into the result, or the group's scratch, which the CTA that
   // completes the group adds up in part order (a failed item counts too: the error flag
   // stands, and the count is left at 0 for the next evaluation)
   double* sum = a.part + a.part_off[g];
-  if (parts > 1) {
+  if (!SEQ && parts > 1) {
     for (int i = tid; i < tc; i += 32 * NW) sum[(long long)part * tc + i] = warps_sum(i);
     __threadfence();
     __syncthreads();
@@ -433,16 +455,20 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
   }
   for (int i = tid; i < tc; i += 32 * NW) {
     double s = 0.0;
-    if (parts > 1) {
+    if (SEQ && parts > 1) {
+      s = seq[i];
+    } else if (parts > 1) {
       for (int q = 0; q < parts; q++) s += __ldcg(sum + (long long)q * tc + i);
     } else {
       s = warps_sum(i);
     }
     double self = 0.0;
+    const SysEval* se = a.sys + a.g_sys[g];
     if (se->self_term) {
       // the reference's self term, where the target's own leaf is one of its near entries;
       // added, not subtracted (src/tree3d.cpp:3596)
       const int leaf = a.leaf_of[t0 + i];
+      const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
       for (long long k = e0; k < e1; k++)
         if (a.node[k] == leaf) {
           if ((a.mask[m0 + (k - e0) * W + (i >> 5)] >> (i & 31)) & 1u)
@@ -467,17 +493,17 @@ __device__ __forceinline__ void near_init(const Layout& L, uint64_t* bar) {
 }
 
 // One launch class: CTA b takes item b.
-template <int KER, bool EPS, bool F32>
+template <int KER, bool EPS, bool F32, bool SEQ>
 __global__ void __launch_bounds__(32 * NW, 2) k_near(NearArgs a, Layout L) {
   __shared__ uint64_t bar[2 * NW];
   near_init(L, bar);
   unsigned phase = 0;
-  near_item<KER, EPS, F32>(a, L, a.items[blockIdx.x], bar, phase);
+  near_item<KER, EPS, F32, SEQ>(a, L, a.items[blockIdx.x], bar, phase);
 }
 
 // Persistent work queue over the items of every class (as k_far_queue): the same device code
 // per item, so the results are identical.
-template <bool F32>
+template <bool F32, bool SEQ>
 __global__ void __launch_bounds__(32 * NW, 2) k_near_queue(NearArgs a, Layout L, int count, int* head) {
   __shared__ int s_item;
   __shared__ uint64_t bar[2 * NW];
@@ -495,11 +521,11 @@ __global__ void __launch_bounds__(32 * NW, 2) k_near_queue(NearArgs a, Layout L,
     // (the mixed path applies the limit on r^2 in its FP64 pass over close pairs)
     const bool eps = !F32 && se->eps_check;
     if (se->kernel == BIT_KERNEL_COULOMB)
-      ok = eps ? near_item<BIT_KERNEL_COULOMB, !F32, F32>(a, L, item, bar, phase)
-               : near_item<BIT_KERNEL_COULOMB, false, F32>(a, L, item, bar, phase);
+      ok = eps ? near_item<BIT_KERNEL_COULOMB, !F32, F32, SEQ>(a, L, item, bar, phase)
+               : near_item<BIT_KERNEL_COULOMB, false, F32, SEQ>(a, L, item, bar, phase);
     else
-      ok = eps ? near_item<BIT_KERNEL_SCREENED, !F32, F32>(a, L, item, bar, phase)
-               : near_item<BIT_KERNEL_SCREENED, false, F32>(a, L, item, bar, phase);
+      ok = eps ? near_item<BIT_KERNEL_SCREENED, !F32, F32, SEQ>(a, L, item, bar, phase)
+               : near_item<BIT_KERNEL_SCREENED, false, F32, SEQ>(a, L, item, bar, phase);
     if (!ok) return;
     __syncthreads();  // the item's last reads of shared memory precede the next item's writes
   }
@@ -577,7 +603,7 @@ __global__ void __launch_bounds__(256) k_close(NearArgs a) {
   }
 }
 
-template <bool F32>
+template <bool F32, bool SEQ>
 void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
   Ctx* c = t->ctx;
   cudaStream_t s = c->stream;
@@ -587,17 +613,19 @@ void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
     if (!F32 && k.kernel != BIT_KERNEL_COULOMB) lay.tab = kExpTabBytes;
   // a context's tile setting counts the records of a CTA's eight warps
   lay.cap = a.cap = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 128;
-  const size_t bytes = lay.total<F32>(L->max_targets);
+  size_t bytes = lay.total<F32>(L->max_targets);
+  lay.seq = (int)((bytes + 15) / 16 * 16);
+  if (SEQ) bytes = lay.seq + L->max_targets * sizeof(double);
   if (c->work_queue && P.near_classes.size() > 1) {
     const int count = (int)L->h_items.size();
     a.items = L->items.p;
-    ensure_smem_attr(reinterpret_cast<const void*>(k_near_queue<F32>), kSmemMax - 1024);
+    ensure_smem_attr(reinterpret_cast<const void*>(k_near_queue<F32, SEQ>), kSmemMax - 1024);
     int per_sm = 0;
-    BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32>, 32 * NW, bytes));
+    BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_near_queue<F32, SEQ>, 32 * NW, bytes));
     const int grid = std::max(1, std::min(count, c->num_sms * std::max(per_sm, 1)));
     c->queue_heads.ensure(c, 2);
     BIT_CUDA(cudaMemsetAsync(c->queue_heads.p + 1, 0, sizeof(int), s));
-    count_launch(), k_near_queue<F32><<<grid, 32 * NW, bytes, s>>>(a, lay, count, c->queue_heads.p + 1);
+    count_launch(), k_near_queue<F32, SEQ><<<grid, 32 * NW, bytes, s>>>(a, lay, count, c->queue_heads.p + 1);
     BIT_CHECK_LAUNCH();
     return;
   }
@@ -610,11 +638,11 @@ void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
     };
     const bool eps = !F32 && k.eps;
     if (k.kernel == BIT_KERNEL_COULOMB) {
-      if (eps) go(k_near<BIT_KERNEL_COULOMB, !F32, F32>);
-      else go(k_near<BIT_KERNEL_COULOMB, false, F32>);
+      if (eps) go(k_near<BIT_KERNEL_COULOMB, !F32, F32, SEQ>);
+      else go(k_near<BIT_KERNEL_COULOMB, false, F32, SEQ>);
     } else {
-      if (eps) go(k_near<BIT_KERNEL_SCREENED, !F32, F32>);
-      else go(k_near<BIT_KERNEL_SCREENED, false, F32>);
+      if (eps) go(k_near<BIT_KERNEL_SCREENED, !F32, F32, SEQ>);
+      else go(k_near<BIT_KERNEL_SCREENED, false, F32, SEQ>);
     }
   }
 }
@@ -629,7 +657,8 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
   NearArgs a = near_args(t, L, P, tx, ty, tz);
   a.out = out;
   if (!P.f32) {
-    launch_near<false>(t, L, P, a);
+    if (L->part_seq) launch_near<false, true>(t, L, P, a);
+    else launch_near<false, false>(t, L, P, a);
     return;
   }
   // Mixed: close pairs need r^2 < thr = max(sqradius / 1024, 2e-14) of some leaf, and the
@@ -654,7 +683,8 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
     a.clist = c->close_list.p;
     a.cn = c->close_n.p;
   }
-  launch_near<true>(t, L, P, a);
+  if (L->part_seq) launch_near<true, true>(t, L, P, a);
+  else launch_near<true, false>(t, L, P, a);
   if (close_possible) {
     count_launch(), k_close<<<c->num_sms * 4, 256, 0, s>>>(a);
     BIT_CHECK_LAUNCH();

@@ -202,15 +202,15 @@ __device__ __forceinline__ Vec sum32(const Tile32& r, double px, double py, doub
 struct Layout {
   int recs, rows, tab;  // records of a tile, targets of a row, bytes of the exponential's table
   int chunk;            // targets of a CTA, at most
-  int single;           // no scratch: part 0 takes the whole group
+  int seq;              // no scratch: a group's first item takes the parts in turn, sums from here
   __host__ __device__ size_t warp_bytes() const {
     return 2 * (size_t)recs * kRec + (size_t)rows * (3 * sizeof(double) + sizeof(unsigned short));
   }
   __host__ __device__ size_t total() const { return tab + NW * warp_bytes(); }
 };
 
-// near_item of near.cu with three sums.  FIELD kinds per launch: FK.
-template <int FK, bool F32>
+// near_item of near.cu with three sums.  Field kinds per launch: FK.  SEQ as there.
+template <int FK, bool F32, bool SEQ>
 __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L) {
   constexpr int PER = F32 ? 2 : 1;  // sources of a record
   __shared__ uint64_t bar[2 * NW];
@@ -218,8 +218,9 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   extern __shared__ __align__(128) unsigned char sm[];
   const int TILE = L.recs * PER;
   const int2 item = a.items[blockIdx.x];
-  const int g = item.x, part = L.single ? 0 : item.y & 0xffff, parts = L.single ? 1 : item.y >> 16;
-  if (L.single && (item.y & 0xffff)) return;
+  const int g = item.x, parts = item.y >> 16;
+  int part = item.y & 0xffff;
+  if (SEQ && part) return;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   if (L.tab) exp_tab_fill(reinterpret_cast<double2*>(sm), tid, 32 * NW);
   if (tid == 0) {
@@ -240,131 +241,96 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
   const int W = (gc + 31) >> 5, w0 = c0 >> 5, wn = (tc + 31) >> 5;  // words of the group, the chunk
   const long long e0 = a.off[g], e1 = e0 + a.cnt[g], m0 = a.moff[g];
   const double *cx = a.tx + t0, *cy = a.ty + t0, *cz = a.tz + t0;
-  for (int i = tid; i < NW * 3 * L.rows; i += 32 * NW) rows[i] = 0.0;
   const long long tot = a.tot[g];
-  const int nv = NW * parts, v = part * NW + w;
-  const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
-  long long P;
-  long long e = run_entry(a.pre, e0, e1, T0, [&](long long k) { return near_work(a, k); }, P);
-  long long d0 = T0 - P, d1 = T1 - P;  // the run, from where the entry's work begins
-  __syncthreads();  // the rows are zero, the table and the barriers are there
   Field f;
   f.del = se->near_del;
   f.kappa = se->kappa;
   f.k = exp_scale(se->kappa);
   f.tab = reinterpret_cast<const double2*>(sm) + (lane & (kExpTabCopies - 1));
   f.korder = se->kernel_order;
-  bool failed = false;
-  for (; e < e1 && d1 > 0; e++) {
-    const int node = a.node[e], ns = a.nummemb[node], ec = a.tgt[e];
-    const int wt = near_weight(ec);  // (the work is shared out by the whole group's)
-    const int ja = cut(d0, wt, ns), jb = cut(d1, wt, ns);
-    d0 -= (long long)wt * ns;
-    d1 -= (long long)wt * ns;
-    if (ja >= jb) continue;
-    const bool all = ec == gc;
-    const unsigned wd = !all && lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
-    const int cnt = all ? tc : __reduce_add_sync(0xffffffffu, __popc(wd));
-    if (!cnt) continue;
-    const int s0 = a.start[node];
-    const unsigned char* src =
-        reinterpret_cast<const unsigned char*>(a.src) + (size_t)(F32 ? a.pstart[node] : s0) * kRec;
-    auto fetch = [&](int j, unsigned n) {
-      if (lane == 0) {
-        const int c = min(jb, (j / TILE + 1) * TILE) - j;
-        const unsigned bytes = (unsigned)((c + PER - 1) / PER) * kRec;
-        fence_proxy_async();
-        mbar_expect_tx(&bar[2 * w + (n & 1)], bytes);
-        tma_load_1d(tiles + (n & 1) * L.recs * kRec, src + (size_t)(j / PER) * kRec, bytes, &bar[2 * w + (n & 1)]);
-      }
-    };
-    fetch(ja, phase);
-    if (!all) pack_list(wd, wn, tl);
-    const bool self = s0 < t0 + tc && t0 < s0 + ns;
-    const double4 c = a.nodec[node];
-    const float4 hb = a.nodeh[node];
-    const NearSteps st = near_steps(cnt);
-    for (int j = ja; j < jb;) {
-      const int jn = min(jb, (j / TILE + 1) * TILE);
-      if (jn < jb) fetch(jn, phase + 1);  // (its buffer's reads ended at the last __syncwarp)
-      if (!__all_sync(0xffffffffu, mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1))) {
+  auto warps_sum = [&](int d, int i) {
+    double s = 0.0;
+    for (int q = 0; q < NW; q++) s += rows[((size_t)q * 3 + d) * L.rows + i];
+    return s;
+  };
+  double* seq = reinterpret_cast<double*>(sm + L.seq);
+  for (;;) {  // once, or (SEQ) every part
+    for (int i = tid; i < NW * 3 * L.rows; i += 32 * NW) rows[i] = 0.0;
+    const int nv = NW * parts, v = part * NW + w;
+    const long long T0 = run_begin(tot, nv, v), T1 = run_begin(tot, nv, v + 1);
+    long long P;
+    long long e = run_entry(a.pre, e0, e1, T0, [&](long long k) { return near_work(a, k); }, P);
+    long long d0 = T0 - P, d1 = T1 - P;  // the run, from where the entry's work begins
+    __syncthreads();  // the rows are zero, the table and the barriers are there
+    bool failed = false;
+    for (; e < e1 && d1 > 0; e++) {
+      const int node = a.node[e], ns = a.nummemb[node], ec = a.tgt[e];
+      const int wt = near_weight(ec);  // (the work is shared out by the whole group's)
+      const int ja = cut(d0, wt, ns), jb = cut(d1, wt, ns);
+      d0 -= (long long)wt * ns;
+      d1 -= (long long)wt * ns;
+      if (ja >= jb) continue;
+      const bool all = ec == gc;
+      const unsigned wd = !all && lane < wn ? a.mask[m0 + (e - e0) * W + w0 + lane] : 0u;
+      const int cnt = all ? tc : __reduce_add_sync(0xffffffffu, __popc(wd));
+      if (!cnt) continue;
+      const int s0 = a.start[node];
+      const unsigned char* src =
+          reinterpret_cast<const unsigned char*>(a.src) + (size_t)(F32 ? a.pstart[node] : s0) * kRec;
+      auto fetch = [&](int j, unsigned n) {
         if (lane == 0) {
-          atomicOr(a.err, 2);
-          mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1);
-          if (jn < jb) mbar_wait(&bar[2 * w + ((phase + 1) & 1)], ((phase + 1) >> 1) & 1);
+          const int c = min(jb, (j / TILE + 1) * TILE) - j;
+          const unsigned bytes = (unsigned)((c + PER - 1) / PER) * kRec;
+          fence_proxy_async();
+          mbar_expect_tx(&bar[2 * w + (n & 1)], bytes);
+          tma_load_1d(tiles + (n & 1) * L.recs * kRec, src + (size_t)(j / PER) * kRec, bytes, &bar[2 * w + (n & 1)]);
         }
-        __syncwarp();
-        failed = true;
-        break;
-      }
-      const unsigned char* tile = tiles + (phase & 1) * L.recs * kRec;
-      phase++;
-      const int n = jn - j, own0 = t0 - s0 - j;
-      auto add = [&](int i, const Vec& p) {
-        row[i] += p.x;
-        row[L.rows + i] += p.y;
-        if (FK != F_CURL) row[2 * L.rows + i] += p.z;
       };
-      if constexpr (F32) {
-        Tile32 r{reinterpret_cast<const ulonglong2*>(tile), a.src64 + s0 + j, n, (float)f.del, near_close_thr(c.w)};
-        if (!(r.del < r.thr)) r.thr = 0.f;
-        auto sum = [&](int i, int k, int step) {
-          const float x = (float)(cx[i] - c.x), y = (float)(cy[i] - c.y), z = (float)(cz[i] - c.z);
-          return self || __any_sync(0xffffffffu, box_d2(x, y, z, hb) < r.thr)
-                     ? sum32<true>(r, cx[i], cy[i], cz[i], x, y, z, f.del, self ? i + own0 : -1, k, step)
-                     : sum32<false>(r, cx[i], cy[i], cz[i], x, y, z, f.del, -1, k, step);
-        };
-        for (int b = 0; b < cnt - 31; b += 32) {
-          const int i = all ? b + lane : tl[b + lane];
-          add(i, sum(i, 0, 1));
+      fetch(ja, phase);
+      if (!all) pack_list(wd, wn, tl);
+      const bool self = s0 < t0 + tc && t0 < s0 + ns;
+      const double4 c = a.nodec[node];
+      const float4 hb = a.nodeh[node];
+      const NearSteps st = near_steps(cnt);
+      for (int j = ja; j < jb;) {
+        const int jn = min(jb, (j / TILE + 1) * TILE);
+        if (jn < jb) fetch(jn, phase + 1);  // (its buffer's reads ended at the last __syncwarp)
+        if (!__all_sync(0xffffffffu, mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1))) {
+          if (lane == 0) {
+            atomicOr(a.err, 2);
+            mbar_wait(&bar[2 * w + (phase & 1)], (phase >> 1) & 1);
+            if (jn < jb) mbar_wait(&bar[2 * w + ((phase + 1) & 1)], ((phase + 1) >> 1) & 1);
+          }
+          __syncwarp();
+          failed = true;
+          break;
         }
-        if (cnt & 31) {
-          const int r0 = cnt & 31, sh = near_tail_shift(r0), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
-          const bool in = slot < r0;
-          const int q = (cnt & ~31) + (in ? slot : 0), i = all ? q : tl[q];
-          Vec p = sum(i, slice, 1 << sh);
-          for (int o = 1 << sh >> 1; o; o >>= 1) {
-            p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
-            p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
-            p.z += __shfl_xor_sync(0xffffffffu, p.z, o);
-          }
-          if (in && slice == 0) add(i, p);
-        }
-      } else {
-        const double4* ds = reinterpret_cast<const double4*>(tile);
-        const bool grows = FK == F_CURL && f.kappa < 0.0 && se->underflow;
-        auto plain = [&](Vec& p, int i, int k, int step) {
-          if (FK != F_ORDER && (grows || isnan(p.x)))  // (a pair's factor is NaN in all components)
-            p = plain64<FK>(ds, n, cx[i], cy[i], cz[i], f.del, f.kappa, i + own0, k, step);
+        const unsigned char* tile = tiles + (phase & 1) * L.recs * kRec;
+        phase++;
+        const int n = jn - j, own0 = t0 - s0 - j;
+        auto add = [&](int i, const Vec& p) {
+          row[i] += p.x;
+          row[L.rows + i] += p.y;
+          if (FK != F_CURL) row[2 * L.rows + i] += p.z;
         };
-        auto run = [&](auto S, auto U) {
-          constexpr bool SELF = decltype(S)::value, UF = decltype(U)::value;
-          for (int b = 0; b < st.full; b++) {
-            const int r0 = 64 * b + lane, r1 = r0 + 32;
-            const bool v1 = r1 < cnt;  // (a partial last block holds more than 48: r0 is a target)
-            const int i0 = all ? r0 : tl[r0], i1 = v1 ? (all ? r1 : tl[r1]) : i0;
-            Vec p, q;
-            two64<FK, SELF, UF>(ds, n, f, Vec{cx[i0], cy[i0], cz[i0]}, Vec{cx[i1], cy[i1], cz[i1]}, i0 + own0,
-                                i1 + own0, p, q);
-            plain(p, i0, 0, 1);
-            plain(q, i1, 0, 1);
-            add(i0, p);
-            if (v1) add(i1, q);
+        if constexpr (F32) {
+          Tile32 r{reinterpret_cast<const ulonglong2*>(tile), a.src64 + s0 + j, n, (float)f.del, near_close_thr(c.w)};
+          if (!(r.del < r.thr)) r.thr = 0.f;
+          auto sum = [&](int i, int k, int step) {
+            const float x = (float)(cx[i] - c.x), y = (float)(cy[i] - c.y), z = (float)(cz[i] - c.z);
+            return self || __any_sync(0xffffffffu, box_d2(x, y, z, hb) < r.thr)
+                       ? sum32<true>(r, cx[i], cy[i], cz[i], x, y, z, f.del, self ? i + own0 : -1, k, step)
+                       : sum32<false>(r, cx[i], cy[i], cz[i], x, y, z, f.del, -1, k, step);
+          };
+          for (int b = 0; b < cnt - 31; b += 32) {
+            const int i = all ? b + lane : tl[b + lane];
+            add(i, sum(i, 0, 1));
           }
-          int base = 64 * st.full;
-          if (st.one) {
-            const int i = all ? base + lane : tl[base + lane];
-            Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, 0, 1);
-            plain(p, i, 0, 1);
-            add(i, p);
-            base += 32;
-          }
-          if (st.tail) {
-            const int sh = near_tail_shift(st.tail), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
-            const bool in = slot < st.tail;
-            const int r0 = base + (in ? slot : 0), i = all ? r0 : tl[r0];
-            Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, slice, 1 << sh);
-            plain(p, i, slice, 1 << sh);
+          if (cnt & 31) {
+            const int r0 = cnt & 31, sh = near_tail_shift(r0), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+            const bool in = slot < r0;
+            const int q = (cnt & ~31) + (in ? slot : 0), i = all ? q : tl[q];
+            Vec p = sum(i, slice, 1 << sh);
             for (int o = 1 << sh >> 1; o; o >>= 1) {
               p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
               p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
@@ -372,28 +338,71 @@ __global__ void __launch_bounds__(32 * NW, 4) k_near_field(NearArgs a, Layout L)
             }
             if (in && slice == 0) add(i, p);
           }
-        };
-        // (the careful forms only where they can matter)
-        if (FK == F_CURL && se->underflow) run(std::true_type{}, std::true_type{});
-        else if (self) run(std::true_type{}, std::false_type{});
-        else run(std::false_type{}, std::false_type{});
+        } else {
+          const double4* ds = reinterpret_cast<const double4*>(tile);
+          const bool grows = FK == F_CURL && f.kappa < 0.0 && se->underflow;
+          auto plain = [&](Vec& p, int i, int k, int step) {
+            if (FK != F_ORDER && (grows || isnan(p.x)))  // (a pair's factor is NaN in all components)
+              p = plain64<FK>(ds, n, cx[i], cy[i], cz[i], f.del, f.kappa, i + own0, k, step);
+          };
+          auto run = [&](auto S, auto U) {
+            constexpr bool SELF = decltype(S)::value, UF = decltype(U)::value;
+            for (int b = 0; b < st.full; b++) {
+              const int r0 = 64 * b + lane, r1 = r0 + 32;
+              const bool v1 = r1 < cnt;  // (a partial last block holds more than 48: r0 is a target)
+              const int i0 = all ? r0 : tl[r0], i1 = v1 ? (all ? r1 : tl[r1]) : i0;
+              Vec p, q;
+              two64<FK, SELF, UF>(ds, n, f, Vec{cx[i0], cy[i0], cz[i0]}, Vec{cx[i1], cy[i1], cz[i1]}, i0 + own0,
+                                  i1 + own0, p, q);
+              plain(p, i0, 0, 1);
+              plain(q, i1, 0, 1);
+              add(i0, p);
+              if (v1) add(i1, q);
+            }
+            int base = 64 * st.full;
+            if (st.one) {
+              const int i = all ? base + lane : tl[base + lane];
+              Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, 0, 1);
+              plain(p, i, 0, 1);
+              add(i, p);
+              base += 32;
+            }
+            if (st.tail) {
+              const int sh = near_tail_shift(st.tail), slot = lane >> sh, slice = lane & ((1 << sh) - 1);
+              const bool in = slot < st.tail;
+              const int r0 = base + (in ? slot : 0), i = all ? r0 : tl[r0];
+              Vec p = one64<FK, SELF, UF>(ds, n, f, Vec{cx[i], cy[i], cz[i]}, i + own0, slice, 1 << sh);
+              plain(p, i, slice, 1 << sh);
+              for (int o = 1 << sh >> 1; o; o >>= 1) {
+                p.x += __shfl_xor_sync(0xffffffffu, p.x, o);
+                p.y += __shfl_xor_sync(0xffffffffu, p.y, o);
+                p.z += __shfl_xor_sync(0xffffffffu, p.z, o);
+              }
+              if (in && slice == 0) add(i, p);
+            }
+          };
+          // (the careful forms only where they can matter)
+          if (FK == F_CURL && se->underflow) run(std::true_type{}, std::true_type{});
+          else if (self) run(std::true_type{}, std::false_type{});
+          else run(std::false_type{}, std::false_type{});
+        }
+        __syncwarp();
+        j = jn;
       }
-      __syncwarp();
-      j = jn;
+      if (failed) break;
     }
-    if (failed) break;
+    __syncthreads();
+    if (!SEQ || parts == 1) break;
+    for (int i = tid; i < 3 * tc; i += 32 * NW) seq[i] = (part ? seq[i] : 0.0) + warps_sum(i / tc, i % tc);
+    __syncthreads();  // the rows are read
+    if (++part == parts) break;
   }
-  __syncthreads();
   // as near_item: straight into the result, or the group's scratch and then in part order
-  auto warps_sum = [&](int d, int i) {
-    double s = 0.0;
-    for (int q = 0; q < NW; q++) s += rows[((size_t)q * 3 + d) * L.rows + i];
-    return s;
-  };
   double* sum = a.part + 3 * a.part_off[g];
   double* out[3] = {a.out, a.out_y, a.out_z};
-  if (parts == 1) {
-    for (int i = tid; i < 3 * tc; i += 32 * NW) out[i / tc][t0 + i % tc] += warps_sum(i / tc, i % tc);
+  if (SEQ || parts == 1) {
+    for (int i = tid; i < 3 * tc; i += 32 * NW)
+      out[i / tc][t0 + i % tc] += parts == 1 ? warps_sum(i / tc, i % tc) : seq[i];
     return;
   }
   for (int i = tid; i < 3 * tc; i += 32 * NW)
@@ -460,12 +469,12 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
   if (P.force == 2 && P.f32) fail(BIT_ERR_INVALID_ARGUMENT, "the screened field is FP64 only");
   bool korder = false;
   for (const SysEval& se : P.h_sys) korder |= se.kernel_order > 0;
-  // the parts' scratch, three sums a target; without room in the memory budget a group's first
-  // part takes it whole
+  // the parts' scratch, three sums a target; without room in the memory budget for that or for the
+  // potentials' the parts are taken in turn
   Layout lay;
   const size_t need = 3 * (size_t)L->part_total;
-  lay.single = L->field_part.n < need && (need + 6 * (size_t)t->n) * sizeof(double) > ctx_room(c);
-  if (!lay.single) L->field_part.ensure(c, need);
+  const bool seq = L->part_seq || (L->field_part.n < need && (need + 6 * (size_t)t->n) * sizeof(double) > ctx_room(c));
+  if (!seq) L->field_part.ensure(c, need);
   a.part = L->field_part.p;
   lay.chunk = L->field_chunk;
   lay.rows = std::min(L->max_targets, lay.chunk);
@@ -474,17 +483,24 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
   lay.recs = c->near_tile ? std::min(128, std::max(32, c->near_tile / 8)) : 64;
   // four CTAs an SM if tiles of 32 do it
   while (lay.recs > 32 && lay.total() > kSmemMax / 4 - 1024) lay.recs -= 16;
+  lay.seq = (int)((lay.total() + 15) / 16 * 16);
+  const size_t bytes = seq ? lay.seq + 3 * lay.rows * sizeof(double) : lay.total();
   for (const LaunchClass& k : P.near_classes) {
     a.items = P.near_it + k.ibegin;
     auto go = [&](auto kernel) {
       ensure_smem_attr(reinterpret_cast<const void*>(kernel), kSmemMax - 1024);
-      count_launch(), kernel<<<dim3(k.icount, chunks), 32 * NW, lay.total(), s>>>(a, lay);
+      count_launch(), kernel<<<dim3(k.icount, chunks), 32 * NW, bytes, s>>>(a, lay);
       BIT_CHECK_LAUNCH();
     };
-    if (P.force == 2) go(k_near_field<F_CURL, false>);
-    else if (P.f32) go(k_near_field<F_COULOMB, true>);
-    else if (korder) go(k_near_field<F_ORDER, false>);
-    else go(k_near_field<F_COULOMB, false>);
+    auto run = [&](auto S) {
+      constexpr bool SEQ = decltype(S)::value;
+      if (P.force == 2) go(k_near_field<F_CURL, false, SEQ>);
+      else if (P.f32) go(k_near_field<F_COULOMB, true, SEQ>);
+      else if (korder) go(k_near_field<F_ORDER, false, SEQ>);
+      else go(k_near_field<F_COULOMB, false, SEQ>);
+    };
+    if (seq) run(std::true_type{});
+    else run(std::false_type{});
   }
 }
 
