@@ -81,15 +81,20 @@ void* dev_alloc(Ctx* c, size_t bytes) {
     char* p = it->second;
     c->cache.erase(it);
     Ctx::Block& b = c->blocks[p];
-    if (tight && b.size > bytes) {
-      c->blocks[p + bytes] = Ctx::Block{b.size - bytes, b.whole, b.base, false};
-      c->cache.insert({b.size - bytes, p + bytes});
-      b.size = bytes;
-    }
     b.live = true;
-    c->cached -= b.size;
-    c->in_use += b.size;
+    const size_t size = tight ? bytes : b.size;
+    c->cached -= size;
+    c->in_use += size;
     c->peak = std::max(c->peak, c->in_use);
+    if (size < b.size) {
+      char* const rest = p + size;
+      const Ctx::Block r{b.size - size, b.whole, p, b.next, false};
+      if (b.next) c->blocks[b.next].prev = rest;
+      b.size = size;
+      b.next = rest;
+      c->cache.insert({r.size, rest});
+      c->blocks[rest] = r;
+    }
     return p;
   }
   if (c->budget && c->in_use + c->cached - ctx_releasable(c) + bytes > c->budget) {
@@ -111,13 +116,14 @@ void* dev_alloc(Ctx* c, size_t bytes) {
   c->in_use += bytes;
   c->peak = std::max(c->peak, c->in_use);
   char* q = static_cast<char*>(p);
-  c->blocks[q] = Ctx::Block{bytes, bytes, q, true};
+  c->blocks[q] = Ctx::Block{bytes, bytes, nullptr, nullptr, true};
   return p;
 }
 
 void dev_free(Ctx* c, void* ptr) {
   if (!ptr) return;
-  auto it = c->blocks.find(static_cast<char*>(ptr));
+  char* p = static_cast<char*>(ptr);
+  auto it = c->blocks.find(p);
   if (it == c->blocks.end()) {
     cudaFree(ptr);
     return;
@@ -125,22 +131,25 @@ void dev_free(Ctx* c, void* ptr) {
   c->in_use -= it->second.size;
   c->cached += it->second.size;
   it->second.live = false;
-  // join a free neighbour of the same cudaMalloc
-  auto joins = [&](auto a, auto b) { return !a->second.live && !b->second.live && a->second.base == b->second.base; };
-  auto next = std::next(it);
-  if (next != c->blocks.end() && joins(it, next)) {
-    c->cache.erase({next->second.size, next->first});
-    it->second.size += next->second.size;
-    c->blocks.erase(next);
+  // `from` (free) becomes part of `to` (free), its neighbour before it
+  auto join = [&](char* to, char* from) {
+    Ctx::Block &a = c->blocks[to], &b = c->blocks[from];
+    a.size += b.size;
+    a.next = b.next;
+    if (b.next) c->blocks[b.next].prev = to;
+    c->blocks.erase(from);
+  };
+  char *next = it->second.next, *prev = it->second.prev;
+  if (next && !c->blocks[next].live) {
+    c->cache.erase({c->blocks[next].size, next});
+    join(p, next);
   }
-  if (it != c->blocks.begin() && joins(std::prev(it), it)) {
-    auto prev = std::prev(it);
-    c->cache.erase({prev->second.size, prev->first});
-    prev->second.size += it->second.size;
-    c->blocks.erase(it);
-    it = prev;
+  if (prev && !c->blocks[prev].live) {
+    c->cache.erase({c->blocks[prev].size, prev});
+    join(prev, p);
+    p = prev;
   }
-  c->cache.insert({it->second.size, it->first});
+  c->cache.insert({c->blocks[p].size, p});
 }
 
 // Blocking device-to-host copy ordered on the context's stream (the legacy default stream

@@ -9,6 +9,7 @@
 #include <map>
 #include <set>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "bit_b200.h"
@@ -236,11 +237,11 @@ struct Ctx {
   DBuf<long long> scratch_ll;
   long long* h_pinned = nullptr;  // pinned host staging for small read-backs (64 entries)
   struct Block {
-    size_t size, whole;  // bytes; those of the cudaMalloc that it is (a part of), at base
-    char* base;
+    size_t size, whole;  // bytes; those of the cudaMalloc that it is (a part of)
+    char *prev, *next;   // its neighbours of the same cudaMalloc, or null
     bool live;
   };
-  std::map<char*, Block> blocks;                  // all of the context's device memory
+  std::unordered_map<char*, Block> blocks;        // all of the context's device memory
   std::set<std::pair<size_t, char*>> cache;       // freed blocks kept for reuse, by size
   size_t cached = 0;                              // bytes held in `cache`
   std::vector<Tree*> trees;                       // trees built by this context
