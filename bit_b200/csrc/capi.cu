@@ -215,13 +215,18 @@ double ev_sec(Tree* t, int i) {
   return ms * 1e-3;
 }
 
-// Errors raised on the device (a bounded wait that gave up) since the last check.
+// Errors raised on the device (a bounded wait that gave up) since the last check.  A work queue
+// whose CTAs gave up leaves items undone, so the counts of done parts do not come back to 0 by
+// themselves.
 void check_dev_err(Ctx* c) {
   if (!c->err_flag) return;
   int e = 0;
   d2h(c, &e, c->err_flag, sizeof(int));
   if (e) {
     BIT_CUDA(cudaMemsetAsync(c->err_flag, 0, sizeof(int), c->stream));
+    for (Tree* t : c->trees)
+      if (t->plists.part_done.p)
+        BIT_CUDA(cudaMemsetAsync(t->plists.part_done.p, 0, t->plists.part_done.n * sizeof(int), c->stream));
     fail(BIT_ERR_CUDA, "a device-side wait gave up (error flags " + std::to_string(e) + ")");
   }
 }

@@ -58,9 +58,20 @@ __global__ void k_wait_check(int limit, int* err) {
   if (__syncthreads_or(!landed) && threadIdx.x == 0) atomicOr(err, 16);
 }
 
+// What a near-field queue that gave up may leave: groups with one of their parts done.
+__global__ void k_wait_leave(int n, int* part_done) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < n) part_done[g] = 1;
+}
+
 }  // namespace
 
 void device_wait_check(Ctx* c, int limit) {
+  for (Tree* t : c->trees)
+    if (t->plists.valid) {
+      const int n = t->plists.ngroups;
+      count_launch(), k_wait_leave<<<grid_for(n, 128), 128, 0, c->stream>>>(n, t->plists.part_done.p);
+    }
   count_launch(), k_wait_check<<<1, 128, 0, c->stream>>>(limit, c->dev_err());
   BIT_CHECK_LAUNCH();
   BIT_CUDA(cudaStreamSynchronize(c->stream));

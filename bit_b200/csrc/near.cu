@@ -436,8 +436,8 @@ __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, in
     }
   }
   // this item's sums: straight into the result, or the group's scratch, which the CTA that
-  // completes the group adds up in part order (a failed item counts too: the error flag
-  // stands, and the count is left at 0 for the next evaluation)
+  // completes the group adds up in part order (a failed item counts too; the host sets the counts
+  // back when it reports the error)
   double* sum = a.part + a.part_off[g];
   if (!SEQ && parts > 1) {
     for (int i = tid; i < tc; i += 32 * NW) sum[(long long)part * tc + i] = warps_sum(i);

@@ -265,8 +265,9 @@ bit_status bit_device_fp64_math_error(bit_ctx* ctx, long long n, double* exp_ulp
  * attempts), on a barrier that nothing ever completes, combines the outcome for the CTA
  * and raises the context's device error flag.  Returns BIT_ERR_CUDA ("a device-side wait
  * gave up", flag 16) with the flag then cleared, so the context stays usable for later
- * calls.  No copy is in flight, nothing faults and nothing hangs.  A diagnostic of the
- * failure path; no reference counterpart. */
+ * calls.  The near-field parts that the context's trees count as done are left behind first, as
+ * by a work queue that gave up, and set back with the flag.  No copy is in flight, nothing faults
+ * and nothing hangs.  A diagnostic of the failure path; no reference counterpart. */
 bit_status bit_device_wait_check(bit_ctx* ctx, int limit);
 
 bit_status bit_tree_stats(const bit_tree* tree, bit_stats* st);
