@@ -655,16 +655,19 @@ bool clusters_of_16(Ctx* c) {
 
 // One level's classes, the larger ones on the context's side streams: their nodes are disjoint,
 // none fills the chip, and one after the other they took 144 us a level of 100k particles
-// where together they take the longest's 53.  The side streams' work ends with this object.
+// where together they take the longest's 53.  They have the context's stream's priority: its caller
+// chose that for all of a build.  The side streams' work ends with this object.
 struct SplitFork {
   Ctx* c;
   cudaStream_t s;
   int n;  // side streams in use
   SplitFork(Ctx* c_, cudaStream_t s_, int n_) : c(c_), s(s_), n(n_) {
     if (n == 0) return;
+    int priority = 0;
+    BIT_CUDA(cudaStreamGetPriority(s, &priority));
     for (int k = 0; k < n; k++)
       if (!c->side[k]) {
-        BIT_CUDA(cudaStreamCreateWithFlags(&c->side[k], cudaStreamNonBlocking));
+        BIT_CUDA(cudaStreamCreateWithPriority(&c->side[k], cudaStreamNonBlocking, priority));
         BIT_CUDA(cudaEventCreateWithFlags(&c->side_ev[k], cudaEventDisableTiming));
       }
     if (!c->fork_ev) BIT_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
