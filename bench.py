@@ -151,21 +151,21 @@ def run_bit(args):
     ctx = B.Context(local, stream=stream.cuda_stream)
     # measured CUDA-core FMA peaks of this device: the roofline denominators
     peaks = {"fp64": ctx.fma_peak(B.FP64) / 1e12, "fp32": ctx.fma_peak(B.MIXED) / 1e12}
-    # the autotuner's near-field (tile, threads-per-target cap) per (precision, kernel) of
+    # the autotuner's near-field (tile, 0) per (precision, kernel) of
     # this class (p = 8, N0 = 1000, clustered), measured on a seeded system of the step's
     # size (a 200k sample chose settings that were slower at 2M)
     near_cfg, tuned = {}, {}
     if args.tune:
         from bit_b200 import autotune
         for prec, pname in ((B.FP64, "fp64"), (B.MIXED, "mixed")):
-            default = (1024 if prec == B.MIXED else 512, 0)
+            default = (1024, 0)
             for kern, kname, kw in ((B.SCREENED, "screened", dict(kappa=KAPPA)),
                                     (B.COULOMB, "coulomb", dict(del_=DEL))):
                 best, times = autotune.tune_near(ctx, NTERMS, kern, n, ACC, MAXMEMB,
                                                  precision=prec, dist="clustered", **kw)
                 near_cfg[(prec, kern)] = best
                 tuned[f"{pname}_{kname}"] = {
-                    "tile": best[0], "threads_per_target": best[1],
+                    "tile": best[0],
                     "near_speedup_vs_default": times[default] / times[best] if default in times else None}
         ctx.set_near_config(0, 0)
 
@@ -911,7 +911,7 @@ def main():
     ap.add_argument("--no-matched", dest="matched", action="store_false",
                     help="skip the accuracy-matched (1e-6 vs direct sum) runs")
     ap.add_argument("--no-tune", dest="tune", action="store_false",
-                    help="default near-field tile and threads per target instead of tuned ones")
+                    help="the default near-field tile instead of tuned ones")
     args = ap.parse_args()
     if args.impl == "reference":
         run_reference(args)

@@ -1,5 +1,5 @@
 """Autotuner for the treecode's launch shape: the leaf size N0 (maxmemb), the leaf packing
-(target-batch size), and the near field's source tile and threads per target.
+(target-batch size), and the limit on the near field's source tile.
 
 N0 trades near-field work (larger leaves: more direct pairs) against far-field and list
 work (smaller leaves: more clusters, more entries).  The best value depends on the
@@ -15,9 +15,9 @@ and costs where near entries then cover too few targets (the icosphere solves: 7
 so tune_group times it on the caller's own workload.
 
 The limit on the near field's source tile (bit_ctx_set_near_config; its second knob, the
-threads that split one target's sources, has no effect) is tuned per (nterms, kernel, N0,
-precision) by tune_near on the same seeded systems; tune() chains N0 and the near-field
-knobs for one workload class.
+threads that split one target's sources, has no effect and stays 0) is tuned per (nterms,
+kernel, N0, precision) by tune_near on the same seeded systems; tune() chains N0 and the tile
+for one workload class.
 """
 import math
 
@@ -89,15 +89,15 @@ def tune_group(ctx, run, candidates=GROUP_CANDIDATES, repeats=2):
     return best, times
 
 
-NEAR_TILES = {"mixed": (512, 1024, 2048), "fp64": (256, 512, 1024)}
-NEAR_SPLITS = (0, 4, 8, 16, 32)
+# records of a CTA: 32, 64 and 128 a warp (1024 is the default, and 2048 the same)
+NEAR_TILES = (256, 512, 1024)
 
 
 def tune_near(ctx, nterms, kernel, n, acc, n0, del_=0.0, kappa=1.0, precision=None,
               dist="uniform", seed=0, repeats=2):
-    """The fastest near-field (tile, threads-per-target cap) for systems of about n
-    particles with leaf size n0, timed on the near field's device time of a seeded system.
-    Leaves the context set to it and returns ((tile, split), {(tile, split): seconds})."""
+    """The fastest near-field (tile, 0) for systems of about n particles with leaf size n0,
+    timed on the near field's device time of a seeded system.  Leaves the context set to it and
+    returns ((tile, 0), {(tile, 0): seconds})."""
     import bit_b200 as B
     prec = B.MIXED if precision is None else precision
     key = ("near", nterms, kernel, prec, _bucket(n), dist, acc, n0)
@@ -110,14 +110,13 @@ def tune_near(ctx, nterms, kernel, n, acc, n0, del_=0.0, kappa=1.0, precision=No
     t = ctx.treemake(x, y, z, n0)
     t.treemoments(q, nterms)
     times = {}
-    for tile in NEAR_TILES["mixed" if prec == B.MIXED else "fp64"]:
-        for split in NEAR_SPLITS:
-            ctx.set_near_config(tile, split)
-            best = float("inf")
-            for _ in range(repeats):
-                t.evaluate(prm)
-                best = min(best, t.stats()["t_near"])
-            times[(tile, split)] = best
+    for tile in NEAR_TILES:
+        ctx.set_near_config(tile, 0)
+        best = float("inf")
+        for _ in range(repeats):
+            t.evaluate(prm)
+            best = min(best, t.stats()["t_near"])
+        times[(tile, 0)] = best
     t.treeempty()
     best = min(times, key=times.get)
     ctx.set_near_config(*best)
@@ -126,9 +125,9 @@ def tune_near(ctx, nterms, kernel, n, acc, n0, del_=0.0, kappa=1.0, precision=No
 
 
 def tune(ctx, nterms, kernel, n, acc, del_=0.0, kappa=1.0, precision=None, dist="uniform"):
-    """N0, then the near-field tile and threads-per-target cap, for one (p, kernel) class
-    of systems of about n particles.  Returns {"n0", "tile", "threads_per_target"} and
-    leaves the context set to the near-field choice."""
+    """N0, then the near-field tile, for one (p, kernel) class of systems of about n particles.
+    Returns {"n0", "tile", "threads_per_target"} (the last 0) and leaves the context set to the
+    near-field choice."""
     n0, _ = tune_n0(ctx, nterms, kernel, n, acc, del_=del_, kappa=kappa, precision=precision,
                     dist=dist)
     (tile, split), _ = tune_near(ctx, nterms, kernel, n, acc, n0, del_=del_, kappa=kappa,
