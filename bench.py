@@ -300,7 +300,7 @@ def run_bit(args):
                   "gpu_launches_per_step": launches[B.MIXED]},
         "fma_peaks_tflops": peaks,
         "autotune": {"near_config": tuned,
-                     "note": "near-field source tile and threads-per-target cap chosen per "
+                     "note": "near-field source tile chosen per "
                              "(precision, kernel) on a seeded clustered system of the step's size, N0=1000, "
                              "p=8, theta=0.7; applied to every step"} if tuned else None,
     }

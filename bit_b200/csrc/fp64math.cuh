@@ -1,21 +1,17 @@
-// FP64 exponential and reciprocal square root for the near field's pair loops, free of
-// branches so that the independent pairs of an unrolled loop interleave.
+// FP64 exponential for the near field's and the direct sums' pair loops, free of branches so that
+// the independent pairs of an unrolled loop interleave.
 //
-// exp_tang: P. T. P. Tang's table-driven method ("Table-driven implementation of the
-// exponential function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989).  With
-// L = ln 2 / 64, t = n L + r, n = 64 m + j (0 <= j < 64), |r| <= L / 2:
-// exp(t) = 2^m * 2^(j/64) * e^r.  n comes from the round-to-integer constant 1.5 * 2^52;
-// r from two FMAs with L split into a double and its remainder; e^r - 1 from its Taylor
-// polynomial of degree 5 (truncation below 4e-17 relative for |r| <= 0.0055); 2^(j/64)
-// from a table of the 64 values as a leading double and a trailing correction (computed
-// to 80 digits), combined as lead + (trail + lead (e^r - 1)) as Tang does; 2^m is added to
-// the exponent field.  Domain: finite t <= 709.  Below t = -707 (exp(t) < 1e-307, where
-// 2^m no longer fits a normal exponent) the result is 0.  Measured on B200 over 4M
-// arguments in [-707, 0] against a long-double exp: within 1 ulp, as CUDA's exp.
-//
-// rsqrt_nr: the hardware approximation rsqrt.approx.ftz.f64 refined by one third-order
-// Newton step, y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2, which takes a seed error e0 to
-// about (5/16) e0^3.  Domain: normal positive x.
+// P. T. P. Tang's table-driven method ("Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989).  With L = ln 2 / 64,
+// t = n L + r, n = 64 m + j (0 <= j < 64), |r| <= L / 2: exp(t) = 2^m * 2^(j/64) * e^r.  n comes
+// from the round-to-integer constant 1.5 * 2^52; r from two FMAs with L split into a double
+// and its remainder; e^r - 1 from its Taylor polynomial of degree 5 (truncation below 4e-17
+// relative for |r| <= 0.0055); 2^(j/64) from a table of the 64 values as a leading double and
+// a trailing correction (computed to 80 digits), combined as lead + (trail + lead (e^r - 1)) as
+// Tang does; 2^m is added to the exponent field.  exp_tang is the method for any argument, which
+// exp_scaled, the form that the kernels run, is checked beside (mathcheck.cu); domain of exp_tang:
+// finite t <= 709, and below t = -707 (exp(t) < 1e-307, where 2^m no longer fits a normal exponent)
+// the result is 0.
 #pragma once
 
 namespace bit {
@@ -63,14 +59,7 @@ constexpr double kExpLlo = 0x1.abc9e3b39803fp-62;
 constexpr double kRoundShift = 0x1.8p52;  // adding it rounds a double below 2^51 to an integer
 
 // Tang's exp; the table is read through the read-only data cache (a warp's lanes gather
-// from 64 entries in eight 128-byte lines).  SMALL: the caller guarantees |t| < 8
-// (kSmallExpArg), so exp(t) cannot underflow and the result needs no check; the value is
-// the full form's.  At 2M clustered, p = 8, theta = 0.7 the screened FP64 near field takes
-// 2% less time (20.3 -> 19.9 ms) with the small form where every pair of a target's tile
-// has kappa r < 8.  (Dropping the second reduction step as well gained another 2% but
-// moved results by up to 3 ulps, so it is not done.)
-constexpr double kSmallExpArg = 8.0;
-template <bool SMALL = false>
+// from 64 entries in eight 128-byte lines).
 __device__ __forceinline__ double exp_tang(double t) {
   const double kd = fma(t, kExpInvL, kRoundShift);
   const int n = __double2loint(kd);  // rint(t / L), two's complement in the low word
@@ -87,18 +76,18 @@ __device__ __forceinline__ double exp_tang(double t) {
   const double v = s.x + fma(s.x, p, s.y);
   const int m = n >> 6;
   const double e = __hiloint2double(__double2hiint(v) + (m << 20), __double2loint(v));
-  if (SMALL) return e;
   return n < -65280 ? 0.0 : e;  // m < -1020: exp(t) < 1e-307
 }
 
-// The same exponential for exp(-kappa r), kappa fixed: the argument in units of L = ln 2 / 64
+// The kernels' form: exp(-kappa r), kappa fixed: the argument in units of L = ln 2 / 64
 // is r * (64 kappa / ln 2), with that factor as a leading double and a correction, so that
 // neither kappa r nor the reduction rounds it: n = rint(r nh), f = r nh - n (one fma, exact)
 // + r nl, |f| <= 1/2, and e^(f L) - 1 from the same Taylor polynomial with L^k folded into
 // its coefficients.  One operation less than -kappa r and exp_tang, and no rounded product.
 // tab: this lane's copy of the table in shared memory (exp_tab_fill): 4 copies of 16-byte
 // entries side by side, so that at most two of the 8 lanes served together meet in a bank
-// (the gather through L1 took up to eight wavefronts a load; 8 copies were no faster).  exp(-kappa r) below 1e-307 is 0.
+// (the gather through L1 took up to eight wavefronts a load; 8 copies were no faster).
+// exp(-kappa r) below 1e-307 is 0.  Within 1 ulp of CUDA's exp over 16M arguments on B200.
 struct ExpScale {
   double nh, nl;  // -64 kappa / ln 2
 };
@@ -115,7 +104,8 @@ constexpr int kExpTabBytes = 64 * kExpTabCopies * 16;
 __device__ __forceinline__ void exp_tab_fill(double2* tab, int tid, int threads) {
   for (int i = tid; i < 64 * kExpTabCopies; i += threads) tab[i] = kExp2Tab64[i / kExpTabCopies];
 }
-// COPIES: of the table at tab (1: kExp2Tab64 itself).  UF: the result is checked for underflow; without, kappa r < kExpNoUnderflow is required.
+// COPIES: of the table at tab (1: kExp2Tab64 itself).  UF: the result is checked for underflow;
+// without, |kappa r| < kExpNoUnderflow is required.
 template <bool UF, int COPIES>
 __device__ __forceinline__ double exp_scaled(double r, ExpScale k, const double2* tab) {
   const double kd = fma(r, k.nh, kRoundShift);
@@ -133,14 +123,6 @@ __device__ __forceinline__ double exp_scaled(double r, ExpScale k, const double2
   const double e = __hiloint2double(__double2hiint(v) + ((n >> 6) << 20), __double2loint(v));
   if (!UF) return e;
   return kd < kRoundShift - 65280.0 ? 0.0 : e;  // below 2^-1020, however far
-}
-
-__device__ __forceinline__ double rsqrt_nr(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  const double c = fma(e, 0.375, 0.5);
-  return fma(y, e * c, y);
 }
 
 }  // namespace bit

@@ -1,10 +1,13 @@
-// Agreement of the near field's own FP64 exp and rsqrt (fp64math.cuh) with CUDA's exp and
-// rsqrt on the device: the largest difference, in units in the last place of CUDA's
-// result, over n seeded arguments (exp: t uniform in [-707, 0] for the full form and in
-// (-8, 0] for the small-argument form, the larger of the two; rsqrt: x log-uniform in
-// [1e-12, 1e6]).  A test holds both to a bound.
+// Agreement of the FP64 arithmetic of the near field's pairs with CUDA's exp and rsqrt on the
+// device: the largest difference, in units in the last place of CUDA's result, over n seeded
+// arguments.  exp: exp_scaled, with and without the check for underflow, kappa log-uniform in [1e-3,
+// 1e3] and kappa r uniform in [0, 700) (both with 24 bits, so that their product is exact), and
+// exp_tang, t uniform in [-707, 0].  rsqrt: the reciprocal square root inside pair64, both kernels',
+// x log-uniform in [1e-12, 1e6].  B200, 16M arguments: exp 1 ulp, rsqrt 2.  A test holds both to a
+// bound.
 #include "common.cuh"
 #include "fp64math.cuh"
+#include "near.cuh"
 #include "tma.cuh"
 
 namespace bit {
@@ -28,15 +31,28 @@ __device__ __forceinline__ double ulp_diff(double a, double b) {
 }
 
 __global__ void k_math_check(long long n, unsigned long long* worst) {
+  __shared__ double2 s_tab[64 * kExpTabCopies];
+  exp_tab_fill(s_tab, threadIdx.x, blockDim.x);
+  __syncthreads();
+  const double2* tab = s_tab + (threadIdx.x & (kExpTabCopies - 1));
   double we = 0.0, wr = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const double t = -707.0 * unit(2 * i);
     const double x = exp10(-12.0 + 18.0 * unit(2 * i + 1));
-    const double ts = -kSmallExpArg * unit(2 * i + 1);
     we = fmax(we, ulp_diff(exp_tang(t), exp(t)));
-    we = fmax(we, ulp_diff(exp_tang<true>(ts), exp(ts)));
-    wr = fmax(wr, ulp_diff(rsqrt_nr(x), rsqrt(x)));
+    const float kappa = (float)exp10(-3.0 + 6.0 * unit(2 * i + 1));
+    const float r = __fdiv_rz((float)(699.9 * unit(2 * i)), kappa);
+    const ExpScale k = exp_scale(kappa);
+    const double e = exp(-(double)kappa * r);
+    we = fmax(we, ulp_diff(exp_scaled<true, kExpTabCopies>(r, k, tab), e));
+    we = fmax(we, ulp_diff(exp_scaled<false, kExpTabCopies>(r, k, tab), e));
+    // a source of charge 1 at the target, delta = x (kappa = 0: the exponential is 1)
+    const double4 one = make_double4(0.0, 0.0, 0.0, 1.0);
+    double c = 0.0, s = 0.0;
+    pair64<BIT_KERNEL_COULOMB, false, false, false>(0.0, 0.0, 0.0, one, x, k, tab, false, c);
+    pair64<BIT_KERNEL_SCREENED, false, false, false>(0.0, 0.0, 0.0, one, x, exp_scale(0.0), tab, false, s);
+    wr = fmax(wr, fmax(ulp_diff(c, rsqrt(x)), ulp_diff(s, rsqrt(x))));
   }
   // non-negative doubles order as their bit patterns
   atomicMax(worst, (unsigned long long)__double_as_longlong(we));

@@ -147,7 +147,8 @@ __device__ __forceinline__ void pack_list(unsigned wd, int W, unsigned short* tl
 
 // -------------------------------------------------------------------------------- FP64 pair
 // One pair's q / sqrt(r^2 + del) or q e^(-kappa R) / R (src/tree3d.cpp:4765-4769, 3609-3618)
-// added to acc.  1/R: the hardware seed and one third-order Newton step (rsqrt_nr); the
+// added to acc.  1/R: the hardware seed rsqrt.approx.ftz.f64 and one third-order Newton step,
+// y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2, which takes a seed error e0 to about (5/16) e0^3; the
 // exponential: exp_scaled.  12 (Coulomb) / 25 (screened) FP64 operations.  EPS: a pair with
 // r^2 <= 1e-14 adds nothing; SELF: nor does the target's own source (`own`); both are evaluated
 // with charge 0 at R = 1.  UF: the exponential may underflow; without, kappa R of every pair and
