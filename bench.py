@@ -56,9 +56,6 @@ MATCHED_BATCH_ACC = {5: 0.015, 7: 0.05, 9: 0.1}   # theta by nterms (p = 4, 6, 8
 # DRAM bytes (read + write) per launch of the full-size kernels (clustered N = 2M, p = 8,
 # theta = 0.7, N0 = 1000, the near field at its default tile), from an ncu launch list of
 # one step taking dram__bytes_read.sum and dram__bytes_write.sum in one pass per launch.
-# Captures of the 200k case give 13.5 MB (FP64 near) and 7.8 MB (FP64 far) per launch,
-# i.e. 135 and 78 MB scaled by N; the full-size launches read more (sources re-read by
-# groups of several waves once the 126 MB L2 no longer holds them).
 TRAFFIC = {
     "k_near<SCREENED, F64>": 387.8e6, "k_near<COULOMB, F64>": 390.1e6,
     "k_far<9, SCREENED, double>": 105.1e6, "k_far<9, COULOMB, double>": 111.1e6,

@@ -80,20 +80,6 @@ struct FarArgs {
   double *out, *out_y, *out_z;
 };
 
-// Pack the set bits of a group mask (W words, lane l holds word l) into tl in ascending
-// order: word by word, each lane placing its own bit.
-__device__ __forceinline__ void warp_pack(unsigned wd, int W, unsigned short* tl) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  int base = 0;
-  for (int j = 0; j < W; j++) {
-    const unsigned b = __shfl_sync(0xffffffffu, wd, j);
-    if ((b >> lane) & 1u) tl[base + __popc(b & lt)] = (unsigned short)(32 * j + lane);
-    base += __popc(b);
-  }
-  __syncwarp();
-}
-
 template <class T>
 struct WarpAcc;  // per-warp accumulator rows in shared memory
 template <>
@@ -311,7 +297,7 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
     if (all) cnt = tc;
     else {
       if (tc < gc) cnt = __reduce_add_sync(0xffffffffu, __popc(wd));
-      warp_pack(wd, wn, tl);
+      pack_list(wd, wn, tl);
     }
     const bool landed = __all_sync(0xffffffffu, mbar_wait(&bar[w], phase & 1));
     phase++;
@@ -467,7 +453,7 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
     const bool all = a.tgt[e] == gc;
     const int cnt = all ? tc : __reduce_add_sync(0xffffffffu, __popc(wd));
     const double4 c = a.nodec[node];
-    if (!all && cnt) warp_pack(wd, wn, tl);
+    if (!all && cnt) pack_list(wd, wn, tl);
     const bool landed = __all_sync(0xffffffffu, mbar_wait(&bar[w], phase & 1));
     phase++;
     if (!landed) {
@@ -547,7 +533,7 @@ __global__ void __launch_bounds__(32 * NWF) k_far_force_korder(FarArgs a) {
   for (long long e = e0 + w; e < e1; e += NW) {
     const unsigned wd = lane < W ? a.mask[m0 + (e - e0) * W + lane] : 0u;
     const int cnt = __reduce_add_sync(0xffffffffu, __popc(wd));
-    warp_pack(wd, W, tl);
+    pack_list(wd, W, tl);
     const int node = a.node[e];
     const double4 c = a.nodec[node];
     T* M = msb + w * TP;

@@ -579,8 +579,6 @@ def main(out):
     arr("unsigned short", "kHarmBegin", begin)
     arr("unsigned char", "kHarmShell", idx)
     arr("double", "kHarmFactor", val, repr)
-    parts.append("// degree l + 2k of harmonic moment h")
-    arr("unsigned char", "kHarmDegree", [h[0] + 2 * h[3] for h in hl])
     parts.append("// Coefficient p of an order: l, s, the harmonic moment of its k = 0, the number of k, and")
     parts.append("// the distance in the list from one k to the next is found from the degree (harm_index).")
     parts.append("struct HarmCoef { unsigned char l, s, m, part; };")

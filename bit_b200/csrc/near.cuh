@@ -96,8 +96,9 @@ __device__ __forceinline__ void two_sum(float& s, float& e, float b) {
 // thr >= 2e-14).  Every other pair keeps at most ~4e-6 relative error, far below 1e-6 of a
 // target's total.  Close pairs can only occur where a target lies within r_t of the source
 // leaf's box (its own leaf, or a neighbour's boundary), and only where the kernel's del is
-// below thr (FP32 r^2 >= del), so a warp runs the checked loop on those tiles and the plain
-// loop, with no test at all, everywhere else.
+// below thr (FP32 r^2 >= del).  Everywhere else a warp runs the plain loop, with no test at all;
+// near the box the potentials' warps watch the least r^2 and take the tile again, testing every
+// pair, where a close one was met (tile32), and the fields' test every pair at once.
 constexpr float kCloseFrac = 1.0f / 1024.0f;  // (1/32)^2
 constexpr float kThrMin = 2e-14f;             // above the 1e-14 skip of src/constants.h:35
 // r_t^2 of a leaf of squared radius sqradius

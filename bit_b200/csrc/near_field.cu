@@ -1,7 +1,7 @@
 // Near field of the fields: the leaf direct sums of treeforce / shielded_treeforce
 // (src/tree3d.cpp:923-967, 3378-3398), with the work shared out as the potentials' (near.cu):
-// one CTA per item and chunk of the group's targets, every warp a contiguous run of the group's sources, two targets a lane,
-// its own tiles and accumulator rows (three, in FP64).
+// one CTA per item and chunk of the group's targets, every warp a contiguous run of the group's
+// sources, two targets a lane (mixed: one), its own tiles and accumulator rows (three, in FP64).
 //
 // FP64: the reference's sums, with 1/r^3 from one reciprocal square root: 16 FP64 operations a
 // Coulomb pair, where a square root and a division took about 40.  Mixed: sources in FP32
