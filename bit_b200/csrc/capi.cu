@@ -697,10 +697,10 @@ bit_status bit_eval_points(bit_tree* th, const bit_eval_params* prm, int m, cons
     plan_sys(t, &P, {*prm}, 1, 0, 0, std::sqrt(reach));
     build_lists(t, &L, plan_key(t, P, 1), m, dx, dy, dz, P.sys.p);
     plan_classes(t, &L, &P);
-    eval_far(t, &L, P, dx, dy, dz, out.p);
-    eval_near(t, &L, P, dx, dy, dz, out.p);
     DBuf<double> res;
     res.ensure(c, m);
+    eval_far(t, &L, P, dx, dy, dz, out.p);
+    eval_near(t, &L, P, dx, dy, dz, out.p);
     count_launch(), k_scatter_out<<<grid_for(m, 256), 256, 0, s>>>(m, dord.p, out.p, res.p);
     BIT_CHECK_LAUNCH();
     copy_d2h(c, pot, res.p, m * sizeof(double));
@@ -748,14 +748,14 @@ bit_status bit_eval_field(bit_tree* th, const bit_field_params* fp, double* fx, 
     prepare_particles(t, {p}, fp->kind == BIT_FIELD_SCREENED ? 2 : 1, fp->kernel_order);
     const int n = t->n;
     t->fx_sorted.ensure(c, n); t->fy_sorted.ensure(c, n); t->fz_sorted.ensure(c, n);
+    DBuf<double> o;
+    o.ensure(c, 3LL * n);
     ev_rec(t, EV_FAR);
     eval_far_force(t, &t->plists, t->pplan, t->fx_sorted.p, t->fy_sorted.p, t->fz_sorted.p);
     ev_rec(t, EV_FAR + 1);
     ev_rec(t, EV_NEAR);
     eval_near_force(t, &t->plists, t->pplan, t->fx_sorted.p, t->fy_sorted.p, t->fz_sorted.p);
     ev_rec(t, EV_NEAR + 1);
-    DBuf<double> o;
-    o.ensure(c, 3LL * n);
     cudaStream_t s = c->stream;
     count_launch(), k_scatter_out<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, t->fx_sorted.p, o.p);
     count_launch(), k_scatter_out<<<grid_for(n, 256), 256, 0, s>>>(n, t->perm.p, t->fy_sorted.p, o.p + n);

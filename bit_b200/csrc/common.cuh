@@ -195,9 +195,7 @@ struct Lists {
   DBuf<long long> far_tot, near_tot;        // per group: work of all its entries
   std::vector<long long> h_work;            // estimated work of each group
   // the near-field items (group, part | parts << 16), heaviest first; groups of several parts add
-  // them up in near_part (from part_off[g]) when part_done[g] is complete.  part_seq: no room for
-  // that; one item per group, of part 0, whose CTA takes the parts one after the other
-  bool part_seq = false;
+  // them up in near_part (from part_off[g]) when part_done[g] is complete
   std::vector<int2> h_items;
   DBuf<int2> items;
   DBuf<unsigned long long> g_near;          // near pairs of each group

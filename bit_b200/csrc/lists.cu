@@ -496,10 +496,10 @@ static int field_chunk(const std::vector<int>& tc, int sms) { return chunk_size(
 // 200: 89 / 51 -> 46 / 41; 200k, 500: 1332 / 470 either way; 64k for all: 1369 / 559 at 200k, 17.3 for 17.0
 // ms at 2M, 48 packed systems 3.2 for 2.8 ms.  (Cutting a group's targets instead gave nothing: most
 // lists are short.)  The count follows from the system's own lists alone, so that its result does
-// not depend on what else is evaluated.  Without room in the memory budget for the scratch every
-// group is one item that takes its parts one after the other: the same sums, later.
+// not depend on what else is evaluated, nor on the memory budget: without room for the scratch a
+// group's first item takes the parts one after the other (near.cu), the same sums, later.
 static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& pairs,
-                       const std::vector<int>& tc, const std::vector<int>& sys, bool packed, size_t later) {
+                       const std::vector<int>& tc, const std::vector<int>& sys, bool packed) {
   const int ng = (int)pairs.size();
   std::vector<int> K(ng);
   std::vector<unsigned long long> of_sys(ng ? 1 + *std::max_element(sys.begin(), sys.end()) : 0, 0);
@@ -516,16 +516,10 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
     off[g] = tot;
     if (K[g] > 1) tot += (long long)K[g] * tc[g];
   }
-  auto fits = [&] { return L->near_part.n >= (size_t)tot || tot * sizeof(double) + later <= ctx_room(c); };
-  if (!fits()) L->gstage.release();
-  L->part_seq = !fits();
-  if (L->part_seq) tot = 0;
   L->part_total = tot;
   std::vector<std::pair<unsigned long long, int2>> it;
-  for (int g = 0; g < ng; g++) {
-    const int items = L->part_seq ? 1 : K[g];
-    for (int k = 0; k < items; k++) it.push_back({pairs[g] / items, make_int2(g, k | K[g] << 16)});
-  }
+  for (int g = 0; g < ng; g++)
+    for (int k = 0; k < K[g]; k++) it.push_back({pairs[g] / K[g], make_int2(g, k | K[g] << 16)});
   std::stable_sort(it.begin(), it.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
   L->h_items.resize(it.size());
   for (size_t i = 0; i < it.size(); i++) L->h_items[i] = it[i].second;
@@ -533,7 +527,6 @@ static void near_items(Lists* L, Ctx* c, const std::vector<unsigned long long>& 
   L->items.ensure(c, it.size());
   L->part_off.ensure(c, ng);
   L->part_done.ensure(c, ng);
-  L->near_part.ensure(c, tot);
   BIT_CUDA(cudaMemcpyAsync(L->items.p, L->h_items.data(), it.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
   BIT_CUDA(cudaMemcpyAsync(L->part_off.p, off.data(), ng * sizeof(long long), cudaMemcpyHostToDevice, s));
   BIT_CUDA(cudaMemsetAsync(L->part_done.p, 0, ng * sizeof(int), s));
@@ -674,7 +667,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     if (err & 1) visits = std::min(nodes, 4 * visits);  // (the totals are not complete)
     else for (int k = 0; k < 4; k++) cap[k] = h[k];
   }
-  if (key.points) L->gstage.release();
+  if (key.points) L->gstage.release();  // (dev_alloc finds the trees' own lists only)
   ListSizing& z = L->last;
   z.ngroups = ng;
   z.acc = key.acc;
@@ -695,10 +688,7 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   L->h_work = wk;
   L->order.ensure(c, ng);
   BIT_CUDA(cudaMemcpyAsync(L->order.p, ord.data(), ng * sizeof(int), cudaMemcpyHostToDevice, s));
-  // what an evaluation takes beside the lists and its parts' scratch: sums, close pairs, coefficients
-  const size_t later = (size_t)ntargets * (2 * sizeof(double) + 28) +
-                       (size_t)nodes * (3 * num_terms(std::max(t->nterms, 1)) / 2 + 4) * sizeof(double);
-  near_items(L, c, hp, tc, gsys, key.group > 0 && !key.points, later);  // (synchronises)
+  near_items(L, c, hp, tc, gsys, key.group > 0 && !key.points);  // (synchronises)
   L->key = key;
   L->valid = true;
   L->version++;

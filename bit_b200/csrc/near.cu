@@ -401,14 +401,15 @@ __device__ __forceinline__ bool near_part(const NearArgs& a, const Layout& L, in
   return !__syncthreads_or(failed);
 }
 
-// An item.  Returns false as near_part does.  SEQ: all parts of the group, one after the other,
-// their sums kept in shared memory and added in part order as those in the scratch are.
+// An item.  Returns false as near_part does.  SEQ: without scratch a group's first item takes all of
+// its parts, one after the other, and adds their sums in shared memory in the same order.
 template <int KER, bool EPS, bool F32, bool SEQ>
 __device__ __forceinline__ bool near_item(const NearArgs& a, const Layout& L, int2 item, uint64_t* bar,
                                           unsigned& phase) {
   __shared__ int s_last;
   extern __shared__ __align__(128) unsigned char sm[];
   const int g = item.x, part = item.y & 0xffff, parts = item.y >> 16, tid = threadIdx.x;
+  if (SEQ && part) return true;
   const int t0 = a.g_tstart[g], tc = a.g_tcount[g], ROWS = Layout::rows(tc), W = (tc + 31) >> 5;
   const double* rows = reinterpret_cast<const double*>(
       sm + L.tab + NW * 2 * (size_t)Layout::recs<F32>(L.cap, ROWS) * kRec);
@@ -607,6 +608,7 @@ template <bool F32, bool SEQ>
 void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
   Ctx* c = t->ctx;
   cudaStream_t s = c->stream;
+  a.part = L->near_part.p;
   Layout lay;
   lay.tab = 0;
   for (const LaunchClass& k : P.near_classes)
@@ -649,6 +651,14 @@ void launch_near(Tree* t, Lists* L, const EvalPlan& P, NearArgs& a) {
 
 }  // namespace
 
+bool parts_in_turn(Ctx* c, Lists* L, DBuf<double>& part, size_t count) {
+  if (part.n >= count) return false;
+  if (count * sizeof(double) > ctx_room(c)) L->gstage.release();
+  if (count * sizeof(double) > ctx_room(c)) return true;
+  part.ensure(c, count);
+  return false;
+}
+
 // One launch per (kernel, eps check) class over its items, or one work queue over all.
 void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
                const double* tz, double* out) {
@@ -657,7 +667,7 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
   NearArgs a = near_args(t, L, P, tx, ty, tz);
   a.out = out;
   if (!P.f32) {
-    if (L->part_seq) launch_near<false, true>(t, L, P, a);
+    if (parts_in_turn(c, L, L->near_part, L->part_total)) launch_near<false, true>(t, L, P, a);
     else launch_near<false, false>(t, L, P, a);
     return;
   }
@@ -683,7 +693,7 @@ void eval_near(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const dou
     a.clist = c->close_list.p;
     a.cn = c->close_n.p;
   }
-  if (L->part_seq) launch_near<true, true>(t, L, P, a);
+  if (parts_in_turn(c, L, L->near_part, L->part_total)) launch_near<true, true>(t, L, P, a);
   else launch_near<true, false>(t, L, P, a);
   if (close_possible) {
     count_launch(), k_close<<<c->num_sms * 4, 256, 0, s>>>(a);

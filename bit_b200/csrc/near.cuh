@@ -303,6 +303,9 @@ __device__ __forceinline__ long long near_work(const NearArgs& a, long long e) {
   return (long long)near_weight(a.tgt[e]) * a.nummemb[a.node[e]];
 }
 
+// The parts' scratch of `count` sums, or whether the parts are taken in turn for want of room: it is
+// asked for last, so that nothing an evaluation cannot do without is short of it.
+bool parts_in_turn(Ctx* c, Lists* L, DBuf<double>& part, size_t count);
 // The arguments common to every near-field launch of this plan (near_field.cu).
 NearArgs near_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const double* ty,
                    const double* tz);

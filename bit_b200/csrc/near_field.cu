@@ -453,7 +453,6 @@ NearArgs near_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const
   a.pstart = t->pstart.p;
   a.tot = L->near_tot.p;
   a.leaf_of = t->leaf_of.p;
-  a.part = L->near_part.p;
   a.part_off = L->part_off.p;
   a.part_done = L->part_done.p;
   return a;
@@ -469,12 +468,9 @@ void eval_near_force(Tree* t, Lists* L, const EvalPlan& P, double* fx, double* f
   if (P.force == 2 && P.f32) fail(BIT_ERR_INVALID_ARGUMENT, "the screened field is FP64 only");
   bool korder = false;
   for (const SysEval& se : P.h_sys) korder |= se.kernel_order > 0;
-  // the parts' scratch, three sums a target; without room in the memory budget for that or for the
-  // potentials' the parts are taken in turn
+  // the parts' scratch, three sums a target
   Layout lay;
-  const size_t need = 3 * (size_t)L->part_total;
-  const bool seq = L->part_seq || (L->field_part.n < need && (need + 6 * (size_t)t->n) * sizeof(double) > ctx_room(c));
-  if (!seq) L->field_part.ensure(c, need);
+  const bool seq = parts_in_turn(c, L, L->field_part, 3 * (size_t)L->part_total);
   a.part = L->field_part.p;
   lay.chunk = L->field_chunk;
   lay.rows = std::min(L->max_targets, lay.chunk);
