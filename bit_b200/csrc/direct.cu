@@ -45,12 +45,12 @@ __device__ __noinline__ double direct_plain(const double* x, const double* y, co
   return acc;
 }
 
-// wt: warps with targets of their own (1, 2, 4, 8); the 8 / wt warps of one target set take a
-// contiguous part of each tile each.
+// Chunks c0, c0 + 1, ... of `per` sources.  wt: warps with targets of their own (1, 2, 4, 8); the
+// 8 / wt warps of one target set take a contiguous part of each tile each.
 template <int KER, bool EPS>
 __global__ void __launch_bounds__(DT, 2) k_direct(int n, const double* x, const double* y, const double* z,
                                                   const double* q, int m, const int* tg, double del,
-                                                  double kappa, int per, int wt, double* part, int* err) {
+                                                  double kappa, int per, int c0, int wt, double* part, int* err) {
   constexpr int PK = KER == BIT_KERNEL_COULOMB ? BIT_KERNEL_COULOMB : BIT_KERNEL_SCREENED;
   __shared__ double4 S[DS];
   __shared__ double2 tab[PK == BIT_KERNEL_COULOMB ? 1 : 64 * kExpTabCopies];
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(DT, 2) k_direct(int n, const double* x, const 
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int slices = DT / 32 / wt, sl = w / wt;
   const int ti = blockIdx.x * 64 * wt + 64 * (w % wt) + lane;
-  const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
+  const int j0 = (c0 + blockIdx.y) * per, j1 = min(n, j0 + per);
   if (PK != BIT_KERNEL_COULOMB) exp_tab_fill(tab, tid, DT);
   int p[2];
   double X[2], Y[2], Z[2], acc[2] = {0.0, 0.0};
@@ -171,11 +171,12 @@ __global__ void __launch_bounds__(DT) k_direct_field(int n, const double* x, con
   }
 }
 
-// out[i] = sign * sum over chunks of part[c][i], in chunk order
-__global__ void k_direct_sum(int m, int nch, const double* part, double sign, double* out) {
+// out[i] = sign * sum over chunks of part[c][i], in chunk order; go_on: the sum of the chunks before
+// is in out already
+__global__ void k_direct_sum(int m, int nch, const double* part, bool go_on, double sign, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  double s = 0.0;
+  double s = go_on ? out[i] : 0.0;
   for (int c = 0; c < nch; c++) s += part[(long long)c * m + i];
   out[i] = sign * s;
 }
@@ -221,12 +222,20 @@ void direct_potential(Ctx* c, int n, const double* x, const double* y, const dou
   // four CTAs a resident slot (two an SM), of at least a tile each
   const int want = std::max(1, std::min(4 * 2 * c->num_sms / tiles, (n + DS - 1) / DS));
   const int per = (n + want - 1) / want, nch = (n + per - 1) / per;
+  // all chunks at once, or as many as the memory budget has room for: the sum goes on in chunk order
+  const int at_once = (int)std::max<size_t>(1, std::min<size_t>(nch, ctx_room(c) / sizeof(double) / m));
   DBuf<double> part;
-  part.ensure(c, (size_t)nch * m);
-  const dim3 grid(tiles, nch);
+  part.ensure(c, (size_t)at_once * m);
   int* err = c->dev_err();
+  const double sign = p.kernel == BIT_KERNEL_SCREENED ? -1.0 : 1.0;
   auto go = [&](auto kernel) {
-    count_launch(), kernel<<<grid, DT, 0, s>>>(n, x, y, z, q, m, tg, p.del, p.kappa, per, wt, part.p, err);
+    for (int c0 = 0; c0 < nch; c0 += at_once) {
+      const int k = std::min(at_once, nch - c0);
+      count_launch(), kernel<<<dim3(tiles, k), DT, 0, s>>>(n, x, y, z, q, m, tg, p.del, p.kappa, per, c0, wt, part.p, err);
+      BIT_CHECK_LAUNCH();
+      count_launch(), k_direct_sum<<<grid_for(m, 256), 256, 0, s>>>(m, k, part.p, c0 > 0, c0 + k < nch ? 1.0 : sign, out);
+      BIT_CHECK_LAUNCH();
+    }
   };
   // (where del alone keeps r^2 + del above the limit, no pair need check it)
   const bool eps = !(p.del > kEpsNear);
@@ -243,9 +252,6 @@ void direct_potential(Ctx* c, int n, const double* x, const double* y, const dou
       else go(k_direct<BIT_KERNEL_SCREENED_REG, false>);
       break;
   }
-  const double sign = p.kernel == BIT_KERNEL_SCREENED ? -1.0 : 1.0;
-  count_launch(), k_direct_sum<<<grid_for(m, 256), 256, 0, s>>>(m, nch, part.p, sign, out);
-  BIT_CHECK_LAUNCH();
 }
 
 }  // namespace bit

@@ -94,3 +94,24 @@ def test_forest_within_less_and_less_memory(queue):
     def run(ctx):
         np.testing.assert_array_equal(run_on(ctx), want)
     assert shrinking(peak + 2 * MB, MB // 2, run) > 3
+
+
+@pytest.mark.parametrize("m", [1, 70, 3000])
+def test_direct_sums_within_less_and_less_memory(m):
+    """The chunks of sources go a few at a time, to one, where the budget has no room for all sums."""
+    import bit_b200 as B
+    from bit_b200 import workloads
+    x, y, z, q = workloads.clustered_blobs(60000, seed=2)
+    tg = np.random.default_rng(m).choice(60000, m, replace=False).astype(np.int32)
+    prm = [B.params(B.COULOMB, B.CONSISTENT, B.FP64, del_=1e-4), B.params(B.SCREENED, B.CONSISTENT, B.FP64, kappa=1.0)]
+    free = B.Context()
+    want = [free.direct(x, y, z, q, p, tg) for p in prm]
+    peak = free.memory()[1]
+    free.close()
+    inputs = 4 * (60000 * 8 + 511) // 512 * 512 + (1 << 14)  # the least that a sum takes
+
+    def run(ctx):
+        for p, w in zip(prm, want):
+            np.testing.assert_array_equal(ctx.direct(x, y, z, q, p, tg), w)
+    done = shrinking(peak + (1 << 14), 1 << 14, run)
+    assert done >= min(60, (peak - inputs - 3 * 8 * m) // (1 << 14) - 2)
