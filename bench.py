@@ -57,10 +57,10 @@ MATCHED_BATCH_ACC = {5: 0.015, 7: 0.05, 9: 0.1}   # theta by nterms (p = 4, 6, 8
 # theta = 0.7, N0 = 1000, the near field at its default tile), from an ncu launch list of
 # one step taking dram__bytes_read.sum and dram__bytes_write.sum in one pass per launch.
 TRAFFIC = {
-    "k_near<SCREENED, F64>": 387.8e6, "k_near<COULOMB, F64>": 390.1e6,
-    "k_far<9, SCREENED, double>": 105.1e6, "k_far<9, COULOMB, double>": 111.1e6,
-    "k_near<SCREENED, F32>": 220.1e6, "k_near<COULOMB, F32>": 195.4e6,
-    "k_far<9, SCREENED, float>": 103.4e6, "k_far<9, COULOMB, float>": 106.2e6,
+    "k_near<SCREENED, F64>": 386.1e6, "k_near<COULOMB, F64>": 389.0e6,
+    "k_far<9, SCREENED, double>": 99.8e6, "k_far<9, COULOMB, double>": 105.4e6,
+    "k_near<SCREENED, F32>": 219.8e6, "k_near<COULOMB, F32>": 194.0e6,
+    "k_far<9, SCREENED, float>": 98.0e6, "k_far<9, COULOMB, float>": 100.7e6,
 }
 TRAFFIC_SOURCE = ("ncu launch list of the full-size step (gpu__time_duration.sum, "
                   "dram__bytes_read.sum, dram__bytes_write.sum; one pass per launch), "
