@@ -294,7 +294,6 @@ bit_status bit_ctx_create(bit_ctx** out, const bit_ctx_opts* opts) {
     c.device = opts ? opts->device : 0;
     if (c.device < 0 || c.device >= ndev) fail(BIT_ERR_INVALID_ARGUMENT, "bad device ordinal");
     BIT_CUDA(cudaSetDevice(c.device));
-    c.budget = opts ? opts->hbm_budget : 0;
     if (opts && opts->stream) {
       c.stream = static_cast<cudaStream_t>(opts->stream);
     } else {
@@ -303,9 +302,11 @@ bit_status bit_ctx_create(bit_ctx** out, const bit_ctx_opts* opts) {
     }
     BIT_CUDA(cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, c.device));
     BIT_CUDA(cudaMallocHost(&c.h_pinned, 64 * sizeof(long long)));
-    // what lives as long as the context has blocks of its own, not cut from a larger one
+    // what lives as long as the context has blocks of its own, not cut from a larger one (and no
+    // budget is too small for a context: the calls that allocate say so)
     c.dev_err();
     c.queue_heads.ensure(&c, 2);
+    c.budget = opts ? opts->hbm_budget : 0;
   });
   if (st != BIT_OK) {
     delete h;

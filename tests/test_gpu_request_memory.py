@@ -39,3 +39,16 @@ def test_requests_after_one_that_failed(ctx):
         assert st == 0, (n, info)
         np.testing.assert_array_equal(got, ctx.treecode_potential(x, y, z, q, 7, maxmemb, p))
     srv.close()
+
+
+def test_a_context_of_any_budget(ctx):
+    """A context is made whatever its budget; the calls that need memory fail, by themselves."""
+    import bit_b200 as B
+    x, y, z, q = np.random.default_rng(1).uniform(-1, 1, (4, 1000))
+    for budget in (1, 1000, 5000):
+        c = B.Context(hbm_budget=budget)
+        for _ in range(2):
+            with pytest.raises(B.BitError) as e:
+                c.treemake(x, y, z, 50)
+            assert e.value.status == 9
+        c.close()
