@@ -22,6 +22,7 @@ constexpr int kGroupMax = 1024;   // targets per group (one CTA; 32 mask words)
 constexpr int kFieldChunk = 256;       // targets of a CTA of the fields' kernels, at most
 constexpr int kPointGroup = 256;  // external points per group, at most
 constexpr int kNearParts = 8;         // near-field items of a group, at most
+constexpr int kFarWarps = 8;          // warps of a CTA of the far kernels: shares of a group's far work
 constexpr long long kNearChunk = 512 << 10, kNearChunkMin = 32 << 10;  // and the pairs of one
 constexpr double kEpsNear = 1e-14;  // src/constants.h:35
 
@@ -191,8 +192,9 @@ struct Lists {
   DBuf<unsigned> far_mask, near_mask;       // (tcount+31)/32 words per entry
   DBuf<int> order;                          // groups by decreasing work
   DBuf<unsigned short> far_tgt, near_tgt;   // targets of each entry (at most kGroupMax)
-  DBuf<long long> far_pre, near_pre;        // of every 32nd entry: work of its group's before it
-  DBuf<long long> far_tot, near_tot;        // per group: work of all its entries
+  DBuf<int> far_cut;                        // per group: first far entry of each of kFarWarps shares
+  DBuf<long long> near_pre;                 // of every 32nd near entry: work of its group's before it
+  DBuf<long long> near_tot;                 // per group: near work of all its entries
   std::vector<long long> h_work;            // estimated work of each group
   // the near-field items (group, part | parts << 16), heaviest first; groups of several parts add
   // them up in near_part (from part_off[g]) when part_done[g] is complete

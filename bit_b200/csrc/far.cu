@@ -73,8 +73,7 @@ struct FarArgs {
   int rows;                  // those of the largest chunk, rounded up to 32
   int* err;                  // device error flags (a bounded wait that gave up: 8)
   const unsigned short* tgt;  // targets of each far entry
-  const long long* pre;      // of every 32nd: targets of its group's entries before it
-  const long long* tot;      // per group: targets of all its entries
+  const int* cut;            // per group: first entry of each warp's share (group_shares)
   const SysEval* sys;        // per system: far_add, kappa, far_sign
   const int* g_sys;          // per group: system
   double *out, *out_y, *out_z;
@@ -112,7 +111,7 @@ constexpr int NWF = 4;  // warps per CTA, force (three accumulators)
 // / 449 (at four, nterms 6 starts to spill).  A second slot per warp (the next entry's
 // coefficients in flight during this one's evaluation) and two targets per lane were both
 // within 1% or slower.
-constexpr int NWP = 8;
+constexpr int NWP = kFarWarps;
 constexpr int far_blocks(int nt) { return nt <= 6 ? 3 : 2; }
 
 constexpr size_t force_smem(size_t moment_bytes) {
@@ -222,15 +221,6 @@ __global__ void __launch_bounds__(kCoefThreads)
   }
 }
 
-// The group's first far entry, of [e0, e1), whose work begins at or past share / nw (e1: none does).
-__device__ __forceinline__ long long far_begin(const FarArgs& a, long long e0, long long e1, long long share, int nw) {
-  const long long T = (share + nw - 1) / nw;
-  if (T <= 0) return e0;
-  long long P;
-  const long long e = run_entry(a.pre, e0, e1, T - 1, [&](long long k) { return (long long)a.tgt[k]; }, P);
-  return min(e + 1, e1);
-}
-
 // The far field of one target group g (the CTA's whole work for that group).  Bound by the
 // FP64 / FP32 pipe and issue: 244 instructions a pair (nterms 9, screened) where the
 // reference's recurrence took 1,333 (FP64) and 1,118 (FP32); 324 against 738 and 683 with
@@ -248,7 +238,6 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
   constexpr int CNT = far_count(NT, KIND);
   constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ long long s_begin[NW];
   const int rows = a.rows;
   const int ROW = WarpAcc<T>::words * rows;
   T* msb = reinterpret_cast<T*>(sm);  // per warp a slot of a.stride elements
@@ -271,14 +260,12 @@ __device__ __forceinline__ bool far_group(const FarArgs& a, int g, int c0, uint6
   bool failed = false;
   // Each warp takes a contiguous run of the group's entries holding about 1/NW of its
   // (target, cluster) pairs: the entries whose exclusive prefix P of target counts has
-  // w C <= NW P < (w + 1) C, C the group's total.  The entries' costs vary widely, so the
+  // w C <= NW P < (w + 1) C, C the group's total (cut, from the list builder).  The entries' costs vary widely, so the
   // round-robin deal this replaces left warps idle at the group's closing barrier.  The
   // split depends on the lists only, so results stay deterministic.
-  const long long tot = a.tot[g];
-  long long e = far_begin(a, e0, e1, w * tot, NW);
-  if (lane == 0) s_begin[w] = e;
-  __syncthreads();  // the rows are zero, the runs' beginnings there
-  const long long ee = w + 1 < NW ? s_begin[w + 1] : e1;
+  long long e = e0 + warp_uniform(a.cut[g * NW + w]);
+  const long long ee = e0 + warp_uniform(w + 1 < NW ? a.cut[g * NW + w + 1] : (int)(e1 - e0));
+  __syncthreads();  // the rows are zero
   for (; e < ee; e++) {
     const int node = a.node[e];
     // The cluster's coefficients, its whole block (TP values, 16-byte aligned in global and
@@ -415,7 +402,6 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   constexpr int TP = far_block(NT, KIND);
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ uint64_t bar[NW];
-  __shared__ long long s_begin[NW];
   const int g = a.order[blockIdx.x], c0 = blockIdx.y * a.chunk;
   const int t0 = a.g_tstart[g] + c0, gc = a.g_tcount[g], tc = min(gc - c0, a.chunk);
   if (tc <= 0) return;  // (the whole CTA)
@@ -435,11 +421,9 @@ __global__ void __launch_bounds__(32 * NWP, field_blocks(NT)) k_far_field(FarArg
   const T* coef = reinterpret_cast<const T*>(a.coef);
   const SysEval* se = a.sys + a.g_sys[g];
   const T tadd = (T)se->far_add, tk = (T)se->kappa;
-  const long long tot = a.tot[g];
-  long long e = far_begin(a, e0, e1, w * tot, NW);
-  if (lane == 0) s_begin[w] = e;
-  __syncthreads();  // the rows are zero, the runs' beginnings there, the barriers ready
-  const long long ee = w + 1 < NW ? s_begin[w + 1] : e1;
+  long long e = e0 + warp_uniform(a.cut[g * NW + w]);
+  const long long ee = e0 + warp_uniform(w + 1 < NW ? a.cut[g * NW + w + 1] : (int)(e1 - e0));
+  __syncthreads();  // the rows are zero, the barriers ready
   bool failed = false;
   unsigned phase = 0;
   for (; e < ee; e++) {
@@ -618,8 +602,7 @@ FarArgs far_args(Tree* t, Lists* L, const EvalPlan& P, const double* tx, const d
   a.mom_off = t->mom_off.p;
   a.err = t->ctx->dev_err();
   a.tgt = L->far_tgt.p;
-  a.pre = L->far_pre.p;
-  a.tot = L->far_tot.p;
+  a.cut = L->far_cut.p;
   a.sys = P.sys.p;
   a.g_sys = L->g_sys.p;
   return a;

@@ -69,11 +69,13 @@ struct ListArgs {
   long long *far_off, *near_off, *far_moff, *near_moff;
   int *far_cnt, *near_cnt;
   unsigned long long* g_near;  // near pairs of each group
-  // per entry: its targets; for the entries whose index is a multiple of 32, the work of their
-  // group's entries before them (far: targets, near: near_weight x sources; run_entry finds the
-  // others' from it); per group: that of all
+  // per entry: its targets.  How a group's work is shared out, far: per group the first entry of
+  // each share (work: targets); near: for the entries whose index is a multiple of 32, the work
+  // (near_weight x sources) of their group's entries before them, from which run_entry finds the
+  // others', and per group that of all
   unsigned short *far_tgt, *near_tgt;
-  long long *far_pre, *near_pre, *far_tot, *near_tot;
+  int* far_cut;
+  long long *near_pre, *near_tot;
   // lists
   int *far_node, *near_node;
   unsigned *far_mask, *near_mask;
@@ -98,15 +100,16 @@ __device__ __forceinline__ bool alt_ok(const ListArgs& a, double s, double w) {
   return w < dmul(a.alt_acc, dsub(dadd(s, a.alt_add), a.alt_sub));
 }
 
-// The work prefixes of group g's entries, whose targets are in place: warp 0 the far list (from
-// entry fo), warp 1 the near list (from no).  The potentials' kernels share a group's work out
-// by them.
-__device__ __forceinline__ void group_prefixes(const ListArgs& a, int g, long long nf, long long fo, long long nn,
-                                               long long no) {
+// How the work of group g's entries, whose targets are in place, is shared out: warp 0 the far list
+// (from entry fo; tot: its targets, all told), warp 1 the near list (from no).  A far entry belongs
+// to share w of kFarWarps where w tot <= kFarWarps P < (w + 1) tot, P the targets of those before.
+__device__ __forceinline__ void group_shares(const ListArgs& a, int g, long long nf, long long fo, long long tot,
+                                             long long nn, long long no) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (w > 1) return;
   const long long n = w ? nn : nf;
   long long run = 0;
+  int cut[kFarWarps] = {};
   for (long long b = 0; b < n; b += 32) {
     const long long k = b + lane;
     long long v = 0;
@@ -116,16 +119,20 @@ __device__ __forceinline__ void group_prefixes(const ListArgs& a, int g, long lo
       const long long t = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += t;
     }
-    if (k < n && !((w ? no + k : fo + k) & 31)) {
-      if (w) a.near_pre[(no + k) >> 5] = run + inc - v;
-      else a.far_pre[(fo + k) >> 5] = run + inc - v;
+    const long long before = run + inc - v;
+    if (w) {
+      if (k < n && !((no + k) & 31)) a.near_pre[(no + k) >> 5] = before;
+    } else {
+#pragma unroll
+      for (int q = 1; q < kFarWarps; q++)
+        cut[q] += __popc(__ballot_sync(0xffffffffu, k < n && before * kFarWarps < q * tot));
     }
     run += __shfl_sync(0xffffffffu, inc, 31);
   }
-  if (lane == 0) {
-    if (w) a.near_tot[g] = run;
-    else a.far_tot[g] = run;
-  }
+  if (lane) return;
+  if (w) a.near_tot[g] = run;
+  else
+    for (int q = 0; q < kFarWarps; q++) a.far_cut[g * kFarWarps + q] = cut[q];
 }
 
 // No CTA waits for another; the work counter is the only shared state.
@@ -387,7 +394,7 @@ __global__ void __launch_bounds__(QT, 4) k_lists(ListArgs a) {
       }
     }
     __syncthreads();  // the entries' nodes and targets
-    group_prefixes(a, g, nf, fo, nn, no);
+    group_shares(a, g, nf, fo, (long long)s_pairs[0], nn, no);
   }
   if (a.has_alt && __any_sync(0xffffffffu, differ) && lane == 0) atomicOr(a.err, 4);
 }
@@ -619,10 +626,10 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
   BIT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lists, QT, 0));
   const long long nodes = std::max(t->numtree, 1);
   long long visits = std::min(nodes, hint && hint->visits > 0 ? hint->visits + hint->visits / 4 + 64 : kVisitsFirst);
-  L->far_tot.ensure(c, ng);
+  L->far_cut.ensure(c, (size_t)ng * kFarWarps);
   L->near_tot.ensure(c, ng);
   L->head.ensure(c, 1);
-  a.far_tot = L->far_tot.p; a.near_tot = L->near_tot.p;
+  a.far_cut = L->far_cut.p; a.near_tot = L->near_tot.p;
   a.visits = cnt.p + 7;
   a.head = L->head.p;
   a.ngroups = ng;
@@ -638,13 +645,12 @@ void build_lists(Tree* t, Lists* L, const ListKey& key, int ntargets, const doub
     L->near_mask.ensure(c, cap[3]);
     L->far_tgt.ensure(c, L->far_node.n);
     L->near_tgt.ensure(c, L->near_node.n);
-    L->far_pre.ensure(c, L->far_node.n / 32 + 1);
     L->near_pre.ensure(c, L->near_node.n / 32 + 1);
     for (int k = 0; k < 4; k++) a.cap[k] = cap[k];
     a.far_node = L->far_node.p; a.far_mask = L->far_mask.p;
     a.near_node = L->near_node.p; a.near_mask = L->near_mask.p;
     a.far_tgt = L->far_tgt.p; a.near_tgt = L->near_tgt.p;
-    a.far_pre = L->far_pre.p; a.near_pre = L->near_pre.p;
+    a.near_pre = L->near_pre.p;
     const long long per = (long long)(maxw + kVisitWords) * sizeof(unsigned);  // bytes a visit
     const size_t room = std::min(kRegionBytes, std::max(L->gstage.n * sizeof(unsigned), ctx_room(c)));
     a.stage = visits * (maxw + kVisitWords);

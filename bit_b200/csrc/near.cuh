@@ -1,6 +1,8 @@
 // What the near-field kernels of the potentials (near.cu) and the fields (near_field.cu) share.
 #pragma once
 
+#include <limits.h>
+
 #include "common.cuh"
 #include "fp64math.cuh"
 
@@ -256,6 +258,15 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   return v;
 }
 
+// A value that all lanes of the warp hold, in a form whose uniformity the compiler sees: loops and
+// addresses that follow from it stay in uniform registers (k_far<9, 1, float> at 100k, theta 0.15: 230
+// us with its first entry from a plain load, 218 so).
+__device__ __forceinline__ int warp_uniform(int v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ long long warp_uniform(long long v) {
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)v), hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32));
+  return (long long)((unsigned long long)hi << 32 | lo);
+}
+
 // First source (a multiple of 8, or all ns) of an entry of weight wt that lies d or more into its
 // work.
 __device__ __forceinline__ int cut(long long d, int wt, int ns) {
@@ -279,14 +290,15 @@ __device__ __forceinline__ long long run_entry(const long long* pre, long long e
   const int lane = threadIdx.x & 31;
   P = 0;
   if (e0 >= e1) return e1;
-  long long k = e0 >> 5;  // the block of 32 entries
+  long long k = e0 >> 5, begin = 0;  // the block of 32 entries, and where it begins
   for (long long b = k + 1, last = (e1 - 1) >> 5; b <= last; b += 32) {
-    const int c = __popc(__ballot_sync(0xffffffffu, b + lane <= last && pre[b + lane] <= T));
+    const long long at = b + lane <= last ? pre[b + lane] : LLONG_MAX;
+    const int c = __popc(__ballot_sync(0xffffffffu, at <= T));
+    if (c) begin = __shfl_sync(0xffffffffu, at, c - 1);
     k += c;
     if (c < 32) break;
   }
-  const bool first = (k << 5) <= e0;
-  const long long s = first ? e0 : k << 5, begin = first ? 0 : pre[k];
+  const long long s = max(e0, k << 5);
   const bool in = s + lane < min(e1, (k + 1) << 5);
   const long long v = in ? work(s + lane) : 0;
   long long inc = v;
@@ -295,7 +307,7 @@ __device__ __forceinline__ long long run_entry(const long long* pre, long long e
     if (lane >= o) inc += t;
   }
   const int n = __popc(__ballot_sync(0xffffffffu, in && begin + inc - v <= T));
-  P = begin + __shfl_sync(0xffffffffu, inc - v, n - 1);
+  P = warp_uniform(begin + __shfl_sync(0xffffffffu, inc - v, n - 1));
   return s + n - 1;
 }
 // A group's near entry: its work.

@@ -663,10 +663,10 @@ struct SplitFork {
   int n;  // side streams in use
   SplitFork(Ctx* c_, cudaStream_t s_, int n_) : c(c_), s(s_), n(n_) {
     if (n == 0) return;
-    int priority = 0;
-    BIT_CUDA(cudaStreamGetPriority(s, &priority));
     for (int k = 0; k < n; k++)
       if (!c->side[k]) {
+        int priority = 0;
+        BIT_CUDA(cudaStreamGetPriority(s, &priority));
         BIT_CUDA(cudaStreamCreateWithPriority(&c->side[k], cudaStreamNonBlocking, priority));
         BIT_CUDA(cudaEventCreateWithFlags(&c->side_ev[k], cudaEventDisableTiming));
       }
