@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kCoefThreads)
 // reference's recurrence took 1,333 (FP64) and 1,118 (FP32); 324 against 738 and 683 with
 // delta > 0.  2M clustered, theta = 0.7, 181 M pairs, before / now: FP64 screened 17.2 / 4.1
 // ms, Coulomb (delta = 0.005) 11.0 / 5.4, screened regularised 17.2 / 7.0; mixed 9.1 / 2.6,
-// 6.1 / 3.4, 9.1 / 4.2; mixed against FP64 (relative L2, screened) 1.91e-7 / 1.78e-7.
+// 6.1 / 3.2, 9.1 / 4.2; mixed against FP64 (relative L2, screened) 1.91e-7 / 1.78e-7.
 // Shared memory: per warp an accumulator row, one cluster's coefficients and a packed target list
 // (a kernel running several orders sizes the coefficients for the largest).  bar: one
 // mbarrier per warp, phase: this warp's count of its completed copies.  Returns false (in
